@@ -51,7 +51,7 @@ extern "C" {
 #define PD_ETIMEOUT (-4)  /* pd_wait timed out, or a bounded device wait expired */
 #define PD_EDEVICE (-5)   /* a CUDA call failed (message in pd_last_error) */
 #define PD_ENOTFOUND (-6) /* unknown ticket */
-#define PD_ECANCELED (-7) /* the request was cancelled before it finished */
+#define PD_ECANCELED (-7) /* the request was cancelled before its result was taken */
 #define PD_ENODEV (-8)    /* no sm_100 device at the requested ordinal */
 
 /* ---- request flags ----
@@ -295,7 +295,9 @@ int pd_formfactor_tables(pd_ctx *ctx, const pd_formfactor *ff, uint32_t n_ff, do
  * 0 while it is pending, or a negative code. The result of a ticket is
  * independent of what else ran beside it (deterministic per-request
  * reduction). pd_wait hands the result out once: it then frees it, and a
- * second pd_wait with a non-NULL out_terms returns PD_EINVAL. */
+ * second pd_wait with a non-NULL out_terms returns PD_EINVAL. After pd_cancel
+ * a ticket whose result has not been taken never hands one out: pd_wait and
+ * pd_poll return PD_ECANCELED, whether or not the work had already finished. */
 int pd_submit(pd_ctx *ctx, const pd_request *req, uint64_t *ticket);
 int pd_wait(pd_ctx *ctx, uint64_t ticket, int timeout_ms, double *out_terms);
 int pd_poll(pd_ctx *ctx, uint64_t ticket);

@@ -68,8 +68,11 @@ struct Layout {
     uint64_t upload_bytes;
     uint64_t hres;         // host-only: pinned landing area of the [6][nq] result
     uint64_t stage_bytes;  // pinned image size (upload + result area)
-    uint64_t centroid, radius, atoms, slots, pairsum, terms, out, counter;
+    uint64_t centroid, cent_part, frames, atoms, slots, red, chunk_sums, terms, out;
     uint64_t status;  // int32 device status of the pair kernel, right after out
+    // counters and maxima that every execution starts from zero (one memset)
+    uint64_t ctl, counter, cent_done, pack_done, rad2, red_done, ctl_bytes;
+    uint64_t lat_sums;
     uint64_t lat_idx, hist, lat_err;  // lattice sets: coordinates, pair counts, error flag
     uint64_t total;
 };
@@ -104,16 +107,29 @@ Layout make_layout(const Plan &P, bool host_xyz) {
     L.upload_bytes = o;
     L.hres = o;
     L.stage_bytes = align_up(o + 6 * nq * 8 + 8, 256);  // result and status land here
-    L.centroid = take(static_cast<uint64_t>(P.n_frames) * 3 * 8);
-    L.radius = take(static_cast<uint64_t>(P.n_frames) * 8);
+    const uint64_t F = static_cast<uint64_t>(P.n_frames);
+    L.centroid = take(F * 3 * 8);
+    L.cent_part = take(F * pd::centroid_blocks(P.n_atoms) * 3 * 8);
+    L.frames = take(F * sizeof(PdFrameDev));
     L.atoms = take(static_cast<uint64_t>(P.n_pad) * P.n_frames *
                    (P.precision == PD_FP64 ? sizeof(double4) : sizeof(float4)));
     L.slots = take(static_cast<uint64_t>(P.slots_per_frame) * P.n_frames * P.nv * P.tun.K * 8);
-    L.pairsum = take(static_cast<uint64_t>(P.n_frames) * P.nv * P.n_pairs * nq * 8);
+    const PdReduceShape &sh = P.red;
+    const uint64_t red_rows = F * static_cast<uint64_t>(P.n_pairs);
+    L.red = take(red_rows * P.nv * sh.width * 8);
+    L.chunk_sums =
+        take(sh.n_chunk > 1 ? red_rows * sh.n_z * sh.n_chunk * P.nv * 128 * 8 : 0);
     L.terms = take(static_cast<uint64_t>(P.n_frames) * 6 * nq * 8);
     L.out = take(6 * nq * 8 + 8);
     L.status = L.out + 6 * nq * 8;
-    L.counter = take(sizeof(int) * 4);
+    L.ctl = o;
+    L.rad2 = take(F * 8);
+    L.counter = take(sizeof(int));
+    L.cent_done = take(F * 4);
+    L.pack_done = take(F * 4);
+    L.red_done = take(sh.n_chunk > 1 ? red_rows * sh.n_z * 4 : 0);
+    L.ctl_bytes = o - L.ctl;
+    L.lat_sums = take(P.lat.size() * nq * 8);
     L.lat_idx = take(P.lat.empty() ? 0 : static_cast<uint64_t>(P.n_pad) * sizeof(int4));
     L.hist = take(static_cast<uint64_t>(P.lat_bins) * 8);
     L.lat_err = take(sizeof(int));
@@ -427,7 +443,7 @@ void stage_structure(DevPlan &dp) {
     rd.gvalid = dp.dptr<int32_t>(L.gvalid);
     rd.qv = dp.dptr<double>(L.qv);
     rd.slots = dp.dptr<double>(L.slots);
-    rd.radius = dp.dptr<double>(L.radius);
+    rd.frames = dp.dptr<PdFrameDev>(L.frames);
     rd.status = dp.dptr<int32_t>(L.status);
     rd.flags = P.test_expire ? PD_REQF_TEST_EXPIRE : 0;
     rd.qmin = P.qmin;
@@ -517,36 +533,35 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st) {
     NvtxRange nvtx("pd reduce + combine");
     const Plan &P = dp.P;
     const Layout &L = dp.L;
+    const int add_exact = dp.rank == 0 ? 1 : 0;
     PD_CUDA(ctx, pd::launch_reduce(dp.dptr<double>(L.slots), dp.dptr<int64_t>(L.lptr),
                                    dp.dptr<int64_t>(L.lidx), dp.dptr<PdPairDev>(L.pairs),
-                                   dp.dptr<double>(L.qv), P.n_pairs, P.nq, P.tun.K, P.nv,
-                                   P.n_frames, P.slots_per_frame, dp.dptr<double>(L.radius),
-                                   P.qmin, P.dq, P.precision == PD_FP32_FP64RED ? 1 : 0,
-                                   dp.rank == 0 ? 1 : 0, dp.dptr<double>(L.pairsum), st));
+                                   dp.dptr<double>(L.qv), dp.dptr<PdFrameDev>(L.frames), P.red,
+                                   P.nv, P.n_frames, P.precision == PD_FP32_FP64RED ? 1 : 0,
+                                   add_exact, dp.dptr<double>(L.chunk_sums),
+                                   dp.dptr<unsigned int>(L.red_done), dp.dptr<double>(L.red), st));
     if (!P.lat.empty()) {
         PD_CUDA(ctx, pd::launch_lattice_sums(
                          reinterpret_cast<const unsigned long long *>(dp.dptr<char>(L.hist)),
                          dp.dptr<PdLatDev>(L.lat), static_cast<int>(P.lat.size()),
-                         dp.dptr<double>(L.qv), P.nq, dp.rank == 0 ? 1 : 0,
-                         dp.dptr<int>(L.lat_err), dp.dptr<double>(L.pairsum), st));
+                         dp.dptr<double>(L.qv), P.nq, add_exact, dp.dptr<int>(L.lat_err),
+                         dp.dptr<double>(L.lat_sums), st));
         ctx->launches += 1;
     }
-    PD_CUDA(ctx, pd::launch_combine(dp.dptr<double>(L.pairsum), dp.dptr<PdClassDev>(L.cls),
-                                    dp.dptr<PdPairDev>(L.pairs), P.n_cls, P.n_pairs, P.nq, P.nv,
-                                    P.n_frames, dp.dptr<double>(L.ffA),
-                                    P.has_exc ? dp.dptr<double>(L.ffC) : nullptr,
-                                    P.has_hyd ? dp.dptr<double>(L.ffW) : nullptr,
-                                    dp.rank == 0 ? 1 : 0, dp.dptr<double>(L.terms), st));
-    ctx->launches += 2;
     double *dst = out_dev ? out_dev : dp.dptr<double>(L.out);
+    double *terms = P.n_frames > 1 ? dp.dptr<double>(L.terms) : dst;
+    PD_CUDA(ctx, pd::launch_profiles(dp.dptr<double>(L.red), dp.dptr<double>(L.lat_sums),
+                                     dp.dptr<PdClassDev>(L.cls), dp.dptr<PdPairDev>(L.pairs),
+                                     P.n_cls, P.red, P.nv, P.n_frames, dp.dptr<double>(L.qv),
+                                     dp.dptr<PdFrameDev>(L.frames), dp.dptr<double>(L.ffA),
+                                     P.has_exc ? dp.dptr<double>(L.ffC) : nullptr,
+                                     P.has_hyd ? dp.dptr<double>(L.ffW) : nullptr, add_exact,
+                                     terms, st));
+    ctx->launches += 2;
     if (P.n_frames > 1) {
         PD_CUDA(ctx, pd::launch_frame_mean(dp.dptr<double>(L.terms), dp.dptr<double>(L.fw),
                                            P.n_frames, P.nq, dst, st, !dp.frame_sum));
         ctx->launches += 1;
-    } else {
-        PD_CUDA(ctx, cudaMemcpyAsync(dst, dp.dptr<double>(L.terms),
-                                     static_cast<size_t>(6) * P.nq * 8,
-                                     cudaMemcpyDeviceToDevice, st));
     }
     return PD_OK;
 }
@@ -556,13 +571,21 @@ int pack_devplan(pd_ctx *ctx, DevPlan &dp, cudaStream_t st) {
     NvtxRange nvtx("pd pack");
     const Plan &P = dp.P;
     const Layout &L = dp.L;
-    PD_CUDA(ctx, pd::launch_centroid(dp.xyz_dev, P.n_atoms, P.n_frames, dp.dptr<double>(L.centroid),
-                                     dp.dptr<double>(L.radius), st));
+    PD_CUDA(ctx, cudaMemsetAsync(dp.base + L.ctl, 0, L.ctl_bytes, st));
+    // a streamed trajectory keeps the status of all its batches
+    PD_CUDA(ctx, pd::launch_centroid(dp.xyz_dev, P.n_atoms, P.n_frames,
+                                     dp.dptr<double>(L.cent_part),
+                                     dp.dptr<unsigned int>(L.cent_done),
+                                     dp.dptr<double>(L.centroid),
+                                     dp.frame_sum ? nullptr : dp.dptr<int32_t>(L.status), st));
     PD_CUDA(ctx, pd::launch_pack(dp.xyz_dev, P.has_hyd ? dp.dptr<double>(L.hw) : nullptr,
                                  dp.dptr<int32_t>(L.perm), dp.dptr<double>(L.centroid), P.n_atoms,
                                  P.n_pad, P.n_frames,
                                  P.precision == PD_FP64 ? nullptr : dp.dptr<float4>(L.atoms),
-                                 P.precision == PD_FP64 ? dp.dptr<double4>(L.atoms) : nullptr, st));
+                                 P.precision == PD_FP64 ? dp.dptr<double4>(L.atoms) : nullptr,
+                                 P.mom, dp.dptr<unsigned long long>(L.rad2),
+                                 dp.dptr<unsigned int>(L.pack_done),
+                                 dp.dptr<PdFrameDev>(L.frames), st));
     ctx->launches += 2;
     if (!P.lat.empty()) {
         PD_CUDA(ctx, pd::launch_lattice(dp.xyz_dev, dp.dptr<int32_t>(L.perm),
@@ -593,8 +616,6 @@ int run_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st,
     const Layout &L = dp.L;
     int rc = pack_devplan(ctx, dp, st);
     if (rc) return rc;
-    // a streamed trajectory keeps the status of all its batches
-    if (!dp.frame_sum) PD_CUDA(ctx, cudaMemsetAsync(dp.base + L.status, 0, 8, st));
     if (ev) cudaEventRecord(ev->first, st);
     if (dp.world > 1)  // a frame's slot may be written by another rank's tile only
         PD_CUDA(ctx, cudaMemsetAsync(dp.dptr<double>(L.slots), 0,
@@ -603,7 +624,6 @@ int run_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st,
                                      st));
     if (!P.jobs.empty()) {
         NvtxRange nvtx("pd pair kernel");
-        PD_CUDA(ctx, cudaMemsetAsync(dp.dptr<int>(L.counter), 0, sizeof(int), st));
         PD_CUDA(ctx, pd::launch_pairs(P.precision, P.tun.K, P.tun.NP, P.mode, dp.dptr<PdJob>(L.jobs),
                                       dp.dptr<int>(L.njobs), dp.dptr<PdReqDev>(L.req),
                                       dp.dptr<int>(L.counter),
@@ -1140,7 +1160,8 @@ void worker_main(pd_ctx *ctx) {
                     }
                     free_devplan(ctx, t->dp, sa);
                     std::lock_guard<std::mutex> lk(ctx->qmu);
-                    t->status = t->drained_only ? PD_ECANCELED : rs;
+                    t->status = t->drained_only || t->canceled ? PD_ECANCELED : rs;
+                    if (t->canceled) t->result = {};
                     if (rs == PD_ETIMEOUT) t->err = kExpiredMsg;
                     if (rs == PD_EINVAL) t->err = kLatticeMsg;
                     t->t_done = now_s();
@@ -1676,7 +1697,13 @@ int pd_cancel(pd_ctx *ctx, uint64_t ticket) {
         std::lock_guard<std::mutex> lk(ctx->qmu);
         auto it = ctx->tickets.find(ticket);
         if (it == ctx->tickets.end()) return PD_ENOTFOUND;
-        if (it->second->status == 1) it->second->canceled = true;
+        PdTicket &t = *it->second;
+        if (t.status == 1) {
+            t.canceled = true;
+        } else if (t.status == 0 && !t.taken) {  // finished, not handed out yet
+            t.status = PD_ECANCELED;
+            t.result = {};
+        }
     }
     ctx->qcv.notify_all();
     return PD_OK;

@@ -63,6 +63,52 @@ constexpr int32_t PD_DEV_WAIT_EXPIRED = 1;  // a bounded wait for a bulk copy ga
 // PdReqDev::flags
 constexpr int32_t PD_REQF_TEST_EXPIRE = 1;  // test hook: the launch's first tile skips its copy
 
+// Per-frame constants, written on the device once the frame's radius is known.
+// With n_mom > 0 the frame runs in the moment form: every pair's
+// sinc(q r) is expanded in cos(n φ), sin(φ/2) = r/d, n < n_mom, and the tiles sum
+// the moments instead of the grid points. A tile's nqb jobs are then n_mblk moment
+// blocks times n_parts parts of its j range (job qb: block qb mod n_mblk, part
+// qb / n_mblk; the jobs past n_mblk·n_parts are idle).
+struct PdFrameDev {
+    double radius;   // largest atom distance from the centroid (Å)
+    double d;        // expansion length: a little over 2·radius (Å)
+    double inv_d2;   // 1/d²
+    int32_t n_mom;   // moments, a multiple of 8; 0: the grid points are summed directly
+    int32_t n_mblk;  // moment blocks of pd_moment_block(K) moments
+    int32_t n_parts;
+    int32_t pad_;
+};
+static_assert(sizeof(PdFrameDev) == 40, "PdFrameDev layout");
+
+// Moments per job of a kernel shape with q-block K: at most K (they share its
+// slots) and what the accumulators of the shape's register budget hold.
+constexpr int pd_moment_block(int K) {
+    return K >= 128 ? 128 : (K >= 64 ? 64 : (K >= 32 ? 32 : 16));
+}
+// The moment form is bounded to this many moments (q_max·d up to about 900).
+constexpr int PD_MAX_MOMENTS = 512;
+
+// When a frame may run in the moment form (block = 0: never).
+struct PdMomentRule {
+    double qmax;          // last grid point
+    int32_t block;        // moments per job, pd_moment_block(K)
+    int32_t nqb;          // jobs per tile
+    int32_t max_moments;  // beyond this the grid points are cheaper (or do not fit)
+    int32_t fp64;
+};
+
+// Sizes of the slot reduction and the profile kernel.
+struct PdReduceShape {
+    int32_t n_pairs, nq, K, nqb;
+    int32_t block;        // moments per job
+    int32_t width;        // row length of the sums: grid points or moments
+    int32_t n_z;          // 128-value blocks per row
+    int32_t n_chunk;      // blocks that share a slot list
+    int32_t max_moments;
+    int32_t pad_;
+    int64_t slots_per_frame;
+};
+
 // Per-request descriptor read by the pair kernels.
 struct PdReqDev {
     const float4 *atoms32;    // [n_frames][n_pad] (FP32 form)
@@ -70,7 +116,7 @@ struct PdReqDev {
     const int32_t *gvalid;    // [n_pad / 32] valid atoms per granule
     const double *qv;         // [nq] grid (FP64 form reads it directly)
     double *slots;            // [n_slots][nv][K]
-    const double *radius;     // [n_frames] largest atom distance from the centroid
+    const PdFrameDev *frames; // [n_frames]
     int32_t *status;          // PD_DEV_* bits, OR-ed in by the pair kernel
     double qmin, dq;          // grid origin and step
     int32_t n_pad;
@@ -95,6 +141,8 @@ struct PdClassDev {
 // (sinc = 1 for every pair): count, Σ w_i, Σ w_j, Σ w_i w_j.
 struct PdPairDev {
     int32_t a, b;
+    int32_t lat;   // lattice set whose pair counts give this self pair sum, or -1
+    int32_t pad;
     double q0[4];
 };
 

@@ -35,6 +35,7 @@
 
 #include "pd_common.h"
 #include "pd_kernels.h"
+#include "pd_moments.cuh"
 #include "pripps_debye.h"
 
 namespace pd {
@@ -750,6 +751,48 @@ constexpr int fp32_min_blocks(int K, int MODE, int NP) {
 constexpr int PD_WAIT_POLLS = 1 << 22;
 constexpr int PD_TEST_WAIT_POLLS = 1 << 10;
 
+// Class-mode flush: the warp sums of acc, added to the warp's FP64 partials
+// part[0 .. 2·NT) in the order of the values.
+template <int NT>
+__device__ __forceinline__ void flush_class(float2 (&acc)[NT], double *__restrict__ part, int lane,
+                                            bool first) {
+    if constexpr (NT % 32 == 0) {
+        // reduce-scatter: lane l ends with the sums of values [l·NT/16, (l+1)·NT/16)
+        warp_reduce_scatter<NT>(acc, lane);
+#pragma unroll
+        for (int m = 0; m < NT / 16; ++m) {
+            double &d = part[lane * (NT / 16) + m];
+            const float sum = (m & 1) ? acc[m >> 1].y : acc[m >> 1].x;
+            d = (first ? 0.0 : d) + static_cast<double>(sum);
+        }
+    } else {
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+            const float v0 = warp_sum(acc[t].x);
+            const float v1 = warp_sum(acc[t].y);
+            if (lane == ((2 * t) & 31))
+                part[2 * t] = (first ? 0.0 : part[2 * t]) + static_cast<double>(v0);
+            if (lane == ((2 * t + 1) & 31))
+                part[2 * t + 1] = (first ? 0.0 : part[2 * t + 1]) + static_cast<double>(v1);
+        }
+    }
+}
+
+// The j range and moment block of a moment-form job (see PdFrameDev): part
+// qb / n_mblk of the tile's range, cut at multiples of 32 atoms from its start.
+struct MomJob {
+    int j0, j1, mb;
+};
+__device__ __forceinline__ MomJob moment_job(int j0, int j1, int qb, int n_mblk, int n_parts) {
+    const int part = qb / n_mblk;
+    const int len = ((j1 - j0 + n_parts - 1) / n_parts + 31) & ~31;
+    MomJob m;
+    m.mb = qb - part * n_mblk;
+    m.j0 = min(j1, j0 + part * len);
+    m.j1 = part < n_parts ? min(j1, m.j0 + len) : m.j0;
+    return m;
+}
+
 // Weighted-mode flush of one accumulator array: the warp sums of acc and of
 // w_i·acc, reduce-scattered (lane l ends with grid points
 // [l·K/32, (l+1)·K/32)) and added to part[k] and part[K + k].
@@ -806,6 +849,7 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
     constexpr int NACC = (MODE == PD_MODE_WEIGHTED) ? 2 : 1;
     constexpr int NV = (MODE == PD_MODE_WEIGHTED) ? 4 : 1;  // FP64 values per q in a slot
     constexpr bool PACKED = (MODE == PD_MODE_CLASS);
+    constexpr bool HAS_MOMENTS = (MODE == PD_MODE_CLASS);
     constexpr bool PACKED_W =
         (MODE == PD_MODE_WEIGHTED) && PD_WEIGHTED_X2 && (K / 2) % 32 == 0 && NP % 2 == 0;
     __shared__ int s_job;
@@ -823,6 +867,7 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
     // in its status word. This state lives in shared memory, not registers,
     // so that it adds nothing to the register pressure of the steps.
     __shared__ int s_dead, s_polls, s_skip;
+    __shared__ int s_empty;  // the job has no pairs: its slots are zeros
     __shared__ uint32_t s_inflight, s_par;  // thread 0: copies in flight, their parities
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -844,8 +889,18 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
         const PdJob jb = jobs[jid];
         const PdReqDev rq = reqs[jb.req];
         const int kq0 = jb.qb * K;
-        const double radius = rq.radius[jb.frame];
-        const bool resid = kq0 < rq.nq && residual_q(rq.qv[kq0], radius);
+        const PdFrameDev fr = rq.frames[jb.frame];
+        const double radius = fr.radius;
+        // moment form: this job's part of the j range and its moment block
+        const bool moments = HAS_MOMENTS && fr.n_mom > 0;
+        int tj0 = jb.j0, tj1 = jb.j1, mblk = 0;
+        if (HAS_MOMENTS && moments) {
+            const MomJob mj = moment_job(jb.j0, jb.j1, jb.qb, fr.n_mblk, fr.n_parts);
+            tj0 = mj.j0;
+            tj1 = mj.j1;
+            mblk = mj.mb;
+        }
+        const bool resid = !moments && kq0 < rq.nq && residual_q(rq.qv[kq0], radius);
         int nres = 0;  // leading grid points of the block in the residual form
         if (resid) {
             for (int base = 0; base < K; base += PD_THREADS) {
@@ -868,6 +923,7 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
             s_polls = s_skip ? PD_TEST_WAIT_POLLS : PD_WAIT_POLLS;
             s_inflight = 0;
             s_par = 0;
+            s_empty = tj1 <= tj0;
         }
         __syncthreads();  // s_qres and the tile state ready; every thread has read s_job
         const float4 *__restrict__ at = rq.atoms32 + static_cast<size_t>(jb.frame) * rq.n_pad;
@@ -882,21 +938,21 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
         // Every pair distance is at most 2·radius (positions are centred):
         // below π/4 for the step angle Δq·r the seeds skip its reduction.
         const bool general_step = rq.dq * (2.0 * radius) > 0.78;
-        const int nstage = s_dead ? 0 : (jb.j1 - jb.j0 + PD_JSTAGE - 1) / PD_JSTAGE;
+        const int nstage = s_dead ? 0 : (tj1 - tj0 + PD_JSTAGE - 1) / PD_JSTAGE;
         if (threadIdx.x == 0 && nstage > 0 && !s_skip) {
-            bulk_copy_to_shared(s_atoms[0], at + jb.j0,
-                                static_cast<uint32_t>(min(jb.j1 - jb.j0, PD_JSTAGE)) * 16,
+            bulk_copy_to_shared(s_atoms[0], at + tj0,
+                                static_cast<uint32_t>(min(tj1 - tj0, PD_JSTAGE)) * 16,
                                 &s_bar[0]);
             s_inflight = 1u;
             s_par = phase & 1u;
         }
         for (int stg = 0; stg < nstage; ++stg) {
-            const int jss = jb.j0 + stg * PD_JSTAGE;
-            const int jse = min(jb.j1, jss + PD_JSTAGE);
+            const int jss = tj0 + stg * PD_JSTAGE;
+            const int jse = min(tj1, jss + PD_JSTAGE);
             if (threadIdx.x == 0 && stg + 1 < nstage) {  // its buffer was released at stg - 1
                 const int nb = (stg + 1) & 1;
                 bulk_copy_to_shared(s_atoms[nb], at + jse,
-                                    static_cast<uint32_t>(min(jb.j1 - jse, PD_JSTAGE)) * 16,
+                                    static_cast<uint32_t>(min(tj1 - jse, PD_JSTAGE)) * 16,
                                     &s_bar[nb]);
                 s_inflight |= 1u << nb;
                 s_par = (s_par & ~(1u << nb)) | (phase & (1u << nb));
@@ -912,8 +968,18 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
             {
                 for (int js = jss; js < jse; js += PD_JFLUSH) {
                     const int je = min(jse, js + PD_JFLUSH);
-                    const bool first = js == jb.j0;
-                    if constexpr (PACKED) {
+                    const bool first = js == tj0;
+                    if (HAS_MOMENTS && moments) {
+                        constexpr int KM = pd_moment_block(K);
+                        float2 acc[KM / 2];
+#pragma unroll
+                        for (int t = 0; t < KM / 2; ++t) acc[t] = make_float2(0.0f, 0.0f);
+                        const int nj = min(KM, fr.n_mom - mblk * KM) >> 3;
+                        constexpr int DBL = KM == 128 ? 4 : (KM == 64 ? 3 : 2);
+                        moments_range<KM>(chunk, jss, pi, i, ivalid, js, je,
+                                          static_cast<float>(fr.inv_d2), nj, mblk, DBL, acc);
+                        flush_class<KM / 2>(acc, part, lane, first);
+                    } else if constexpr (PACKED) {
                         const float2 *q2 = reinterpret_cast<const float2 *>(s_qres);
                         // 16-point chunks of this block that lie on the grid.
                         // The small-q residual blocks (the first of a grid)
@@ -946,28 +1012,7 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
                         }
                         // Warp-reduce and add into this warp's partial sums,
                         // in sub-chunk order (one warp owns them).
-                        if constexpr (PD_FLUSH_RS && (K / 2) % 32 == 0) {
-                        // reduce-scatter: lane l ends with the warp sums of
-                        // grid points [l·K/32, (l+1)·K/32)
-                        warp_reduce_scatter<K / 2>(acc, lane);
-#pragma unroll
-                        for (int m = 0; m < K / 32; ++m) {
-                            double &d = part[lane * (K / 32) + m];
-                            const float sum = (m & 1) ? acc[m >> 1].y : acc[m >> 1].x;
-                            d = (first ? 0.0 : d) + static_cast<double>(sum);
-                        }
-                        } else {
-#pragma unroll
-                        for (int t = 0; t < K / 2; ++t) {
-                            const float v0 = warp_sum(acc[t].x);
-                            const float v1 = warp_sum(acc[t].y);
-                            if (lane == ((2 * t) & 31))
-                                part[2 * t] = (first ? 0.0 : part[2 * t]) + static_cast<double>(v0);
-                            if (lane == ((2 * t + 1) & 31))
-                                part[2 * t + 1] =
-                                    (first ? 0.0 : part[2 * t + 1]) + static_cast<double>(v1);
-                        }
-                        }
+                        flush_class<K / 2>(acc, part, lane, first);
                     } else if constexpr (PACKED_W) {
                         const float2 *q2 = reinterpret_cast<const float2 *>(s_qres);
                         const int nchunk =
@@ -1072,8 +1117,7 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
                         mbar_wait(&s_bar[b], (s_par >> b) & 1u, PD_WAIT_POLLS);
                 atomicOr(rq2->status, PD_DEV_WAIT_EXPIRED);
             }
-            merge_tile_slots(s_part, NV * K, slot_word, rq2->slots, dead,
-                             jobs[jid2].j1 <= jobs[jid2].j0 && !dead);
+            merge_tile_slots(s_part, NV * K, slot_word, rq2->slots, dead, s_empty && !dead);
         }
         __syncthreads();  // s_qres, s_part, s_job and the tile state are rewritten next
     }
@@ -1158,15 +1202,26 @@ __global__ void __launch_bounds__(PD_THREADS) pd_pairs_fp64(const PdJob *__restr
 }
 
 // ------------------------------------------------------- pack and centroid
-// Per-frame centroid of the input positions (FP64, fixed-order tree) and the
-// largest distance of an atom from it.
-__global__ void pd_centroid(const double *__restrict__ xyz, int64_t n_atoms,
-                            double *__restrict__ centroid, double *__restrict__ radius) {
-    __shared__ double red[3][256];
-    const int f = blockIdx.x;
+// Per-frame centroid of the input positions, FP64: every block adds a fixed
+// run of atoms in a fixed tree and the frame's last block adds the blocks'
+// sums in block order, so the centroid does not depend on which block ends
+// last. One block per frame of up to PD_CENT_RUN atoms, more for larger frames (a
+// single block took 150 µs to read 100,000 atoms twice; now 8 µs).
+constexpr int PD_CENT_THREADS = 256;
+constexpr int64_t PD_CENT_RUN = 2048;
+
+__global__ void __launch_bounds__(PD_CENT_THREADS)
+    pd_centroid(const double *__restrict__ xyz, int64_t n_atoms, int32_t n_blk,
+                double *__restrict__ part, unsigned int *__restrict__ done,
+                double *__restrict__ centroid, int32_t *__restrict__ status) {
+    __shared__ double red[3][PD_CENT_THREADS];
+    __shared__ bool s_last;
+    const int f = blockIdx.x / n_blk, b = blockIdx.x % n_blk;
     const double *p = xyz + static_cast<size_t>(f) * n_atoms * 3;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && status) *status = 0;
+    const int64_t i0 = n_atoms * b / n_blk, i1 = n_atoms * (b + 1) / n_blk;
     double sx = 0, sy = 0, sz = 0;
-    for (int64_t i = threadIdx.x; i < n_atoms; i += blockDim.x) {
+    for (int64_t i = i0 + threadIdx.x; i < i1; i += PD_CENT_THREADS) {
         sx += p[3 * i];
         sy += p[3 * i + 1];
         sz += p[3 * i + 2];
@@ -1175,7 +1230,7 @@ __global__ void pd_centroid(const double *__restrict__ xyz, int64_t n_atoms,
     red[1][threadIdx.x] = sy;
     red[2][threadIdx.x] = sz;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
+    for (int s = PD_CENT_THREADS / 2; s > 0; s >>= 1) {
         if (threadIdx.x < s) {
             red[0][threadIdx.x] += red[0][threadIdx.x + s];
             red[1][threadIdx.x] += red[1][threadIdx.x + s];
@@ -1183,174 +1238,387 @@ __global__ void pd_centroid(const double *__restrict__ xyz, int64_t n_atoms,
         }
         __syncthreads();
     }
-    const double cx = red[0][0] / static_cast<double>(n_atoms);
-    const double cy = red[1][0] / static_cast<double>(n_atoms);
-    const double cz = red[2][0] / static_cast<double>(n_atoms);
-    __syncthreads();
     if (threadIdx.x == 0) {
-        centroid[3 * f] = cx;
-        centroid[3 * f + 1] = cy;
-        centroid[3 * f + 2] = cz;
+        for (int a = 0; a < 3; ++a) part[3 * blockIdx.x + a] = red[a][0];
+        __threadfence();
+        s_last = atomicAdd(&done[f], 1u) == static_cast<unsigned>(n_blk - 1);
     }
-    double rm = 0.0;
-    for (int64_t i = threadIdx.x; i < n_atoms; i += blockDim.x) {
-        const double dx = p[3 * i] - cx, dy = p[3 * i + 1] - cy, dz = p[3 * i + 2] - cz;
-        rm = fmax(rm, dx * dx + dy * dy + dz * dz);
-    }
-    red[0][threadIdx.x] = rm;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[0][threadIdx.x] = fmax(red[0][threadIdx.x], red[0][threadIdx.x + s]);
-        __syncthreads();
+    if (s_last && threadIdx.x < 3) {
+        __threadfence();
+        const volatile double *q = part + 3 * static_cast<size_t>(f) * n_blk + threadIdx.x;
+        double s = 0;
+        for (int k = 0; k < n_blk; ++k) s += q[3 * k];
+        centroid[3 * f + threadIdx.x] = s / static_cast<double>(n_atoms);
     }
-    if (threadIdx.x == 0) radius[f] = sqrt(red[0][0]);
 }
 
 // Gather positions into the class-sorted, padded layout, centred per frame.
-__global__ void pd_pack(const double *__restrict__ xyz, const double *__restrict__ weights,
-                        const int32_t *__restrict__ perm, const double *__restrict__ centroid,
-                        int64_t n_atoms, int32_t n_pad, int32_t n_frames,
-                        float4 *__restrict__ out32, double4 *__restrict__ out64) {
-    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (t >= static_cast<int64_t>(n_pad) * n_frames) return;
-    const int f = static_cast<int>(t / n_pad);
-    const int p = static_cast<int>(t % n_pad);
-    const int src = perm[p];
-    double x = 0, y = 0, z = 0, w = 0;
-    if (src >= 0) {
-        const double *s = xyz + (static_cast<size_t>(f) * n_atoms + src) * 3;
-        x = s[0] - centroid[3 * f];
-        y = s[1] - centroid[3 * f + 1];
-        z = s[2] - centroid[3 * f + 2];
-        w = weights ? weights[src] : 0.0;
+// The largest distance from the centroid is collected on the way, and the
+// frame's last block turns it into the frame's constants (PdFrameDev): whether
+// its pairs are summed in the moment form, and the expansion's size.
+constexpr int PD_PACK_THREADS = 256;
+
+__global__ void __launch_bounds__(PD_PACK_THREADS)
+    pd_pack(const double *__restrict__ xyz, const double *__restrict__ weights,
+            const int32_t *__restrict__ perm, const double *__restrict__ centroid,
+            int64_t n_atoms, int32_t n_pad, int32_t n_blk, float4 *__restrict__ out32,
+            double4 *__restrict__ out64, PdMomentRule rule, unsigned long long *__restrict__ rad2,
+            unsigned int *__restrict__ done, PdFrameDev *__restrict__ frames) {
+    __shared__ double s_max[PD_PACK_THREADS / 32];
+    const int f = blockIdx.x / n_blk, b = blockIdx.x % n_blk;
+    const int p = b * PD_PACK_THREADS + threadIdx.x;
+    double r2 = 0.0;
+    if (p < n_pad) {
+        const int src = perm[p];
+        double x = 0, y = 0, z = 0, w = 0;
+        if (src >= 0) {
+            const double *s = xyz + (static_cast<size_t>(f) * n_atoms + src) * 3;
+            x = s[0] - centroid[3 * f];
+            y = s[1] - centroid[3 * f + 1];
+            z = s[2] - centroid[3 * f + 2];
+            w = weights ? weights[src] : 0.0;
+            r2 = x * x + y * y + z * z;
+        }
+        const size_t t = static_cast<size_t>(f) * n_pad + p;
+        if (out32) out32[t] = make_float4(static_cast<float>(x), static_cast<float>(y),
+                                          static_cast<float>(z), static_cast<float>(w));
+        if (out64) out64[t] = make_double4(x, y, z, w);
     }
-    if (out32) out32[t] = make_float4(static_cast<float>(x), static_cast<float>(y),
-                                      static_cast<float>(z), static_cast<float>(w));
-    if (out64) out64[t] = make_double4(x, y, z, w);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) r2 = fmax(r2, __shfl_xor_sync(0xffffffffu, r2, o));
+    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = r2;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int k = 1; k < PD_PACK_THREADS / 32; ++k) r2 = fmax(r2, s_max[k]);
+    // non-negative doubles order as their bit patterns; the maximum is exact
+    atomicMax(&rad2[f], static_cast<unsigned long long>(__double_as_longlong(r2)));
+    __threadfence();
+    if (atomicAdd(&done[f], 1u) != static_cast<unsigned>(n_blk - 1)) return;
+    __threadfence();
+    PdFrameDev fr{};
+    fr.radius = sqrt(__longlong_as_double(
+        static_cast<long long>(atomicMax(&rad2[f], 0ull))));
+    fr.d = fmax(2.0 * PD_MOM_STRETCH * fr.radius, 1e-6);
+    fr.inv_d2 = 1.0 / (fr.d * fr.d);
+    if (rule.block > 0) {
+        const int m8 = (moments_needed(rule.qmax * fr.d, rule.fp64 != 0) + 7) & ~7;
+        const int blocks = (m8 + rule.block - 1) / rule.block;
+        if (m8 <= rule.max_moments && blocks <= rule.nqb) {
+            fr.n_mom = m8;
+            fr.n_mblk = blocks;
+            fr.n_parts = rule.nqb / blocks;
+        }
+    }
+    frames[f] = fr;
 }
 
 // ------------------------------------------------------------ reductions
-// Sum the slots of every (frame, class pair, q) in list order, then turn the
-// Σ sin(q r)/r partials into Σ sinc(q r) by dividing by q; q = 0 takes the
-// exact pair sums. pairsum is [frame][nv][n_pairs][nq].
+// Sums the slots of every (frame, class pair) in a fixed order. A block owns
+// 128 values (grid points, or moments) of one class pair: its groups of 128
+// threads, and the n_chunk blocks along y, each add a contiguous run of the
+// slot list, and the runs' sums are added in run order (by the block that ends
+// last where there are several).
+//  - grid points: the slots hold Σ sin(q r)/r; the sums are divided by q,
+//    and the residual form and q = 0 take their exact pair sums;
+//  - moments: value e of block mb collects the lists of all the parts.
+// red is [frame][pair][nv][width].
+constexpr int PD_RED_GROUPS = 4;
+constexpr int PD_RED_THREADS = 128 * PD_RED_GROUPS;
+
 template <int NV>
-__global__ void pd_reduce_pairs(const double *__restrict__ slots, const int64_t *__restrict__ lptr,
-                                const int64_t *__restrict__ lidx, const PdPairDev *__restrict__ pairs,
-                                const double *__restrict__ qv, int32_t n_pairs, int32_t nq,
-                                int32_t K, int32_t /*nv: the template's NV*/, int32_t n_frames,
-                                int64_t slots_per_frame, const double *__restrict__ radius,
-                                double qmin, double dq, int32_t residual_form, int32_t add_exact,
-                                double *__restrict__ pairsum) {
-    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    const int64_t per_frame = static_cast<int64_t>(n_pairs) * nq;
-    if (t >= per_frame * n_frames) return;
-    const int f = static_cast<int>(t / per_frame);
-    const int rem = static_cast<int>(t % per_frame);
-    const int p = rem / nq;
-    const int q = rem % nq;
-    const int nqb = (nq + K - 1) / K;
-    const int qb = q / K, kk = q % K;
-    const double qval = qv[q];
-    constexpr int nv = NV;  // values per slot entry: 1 (class) or 4 (weighted)
-    double s[4] = {0, 0, 0, 0};
-    if (qval > 0.0) {
-        const int64_t e0 = lptr[p * nqb + qb], e1 = lptr[p * nqb + qb + 1];
-        const int64_t fbase = static_cast<int64_t>(f) * slots_per_frame;
-        const int64_t stride = static_cast<int64_t>(nv) * K;
-        // eight slots in flight per thread, added in list order (the same
-        // order, and so the same rounding, as one slot at a time)
-        int64_t e = e0;
-        for (; e + 8 <= e1; e += 8) {
-            double x[8][4];
+__device__ __forceinline__ void sum_slots(const double *__restrict__ slots,
+                                          const int64_t *__restrict__ lidx, int64_t e0, int64_t e1,
+                                          int64_t fbase, int64_t stride, int K, int kk,
+                                          double (&s)[NV]) {
+    int64_t e = e0;
+    for (; e + 8 <= e1; e += 8) {  // eight slots in flight, added in list order
+        double x[8][NV];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const double *sl = slots + (fbase + lidx[e + u]) * stride + kk;
-                for (int v = 0; v < nv; ++v) x[u][v] = sl[v * K];
-            }
+        for (int u = 0; u < 8; ++u) {
+            const double *sl = slots + (fbase + lidx[e + u]) * stride + kk;
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
-                for (int v = 0; v < nv; ++v) s[v] += x[u][v];
+            for (int v = 0; v < NV; ++v) x[u][v] = sl[v * K];
         }
-        for (; e < e1; ++e) {
-            const double *sl = slots + (fbase + lidx[e]) * stride + kk;
-            for (int v = 0; v < nv; ++v) s[v] += sl[v * K];
-        }
-        for (int v = 0; v < nv; ++v) s[v] /= qval;
-        if (add_exact && residual_form && residual_q(qval, radius[f]))
-            for (int v = 0; v < nv; ++v) s[v] += pairs[p].q0[v];
-    } else if (add_exact) {
-        for (int v = 0; v < 4; ++v) s[v] = pairs[p].q0[v];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+#pragma unroll
+            for (int v = 0; v < NV; ++v) s[v] += x[u][v];
     }
-    const int64_t ob = static_cast<int64_t>(f) * nv * per_frame;
-    for (int v = 0; v < nv; ++v) pairsum[ob + static_cast<int64_t>(v) * per_frame + rem] = s[v];
+    for (; e < e1; ++e) {
+        const double *sl = slots + (fbase + lidx[e]) * stride + kk;
+#pragma unroll
+        for (int v = 0; v < NV; ++v) s[v] += sl[v * K];
+    }
 }
 
-// Six profiles per (frame, q) from the class-pair sums, in FP64.
-__global__ void pd_combine_terms(const double *__restrict__ pairsum,
-                                 const PdClassDev *__restrict__ cls,
-                                 const PdPairDev *__restrict__ pairs, int32_t n_cls,
-                                 int32_t n_pairs, int32_t nq, int32_t nv, int32_t n_frames,
-                                 const double *__restrict__ ffA, const double *__restrict__ ffC,
-                                 const double *__restrict__ ffW, int32_t add_diag,
-                                 double *__restrict__ terms) {
-    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (t >= static_cast<int64_t>(nq) * n_frames) return;
-    const int f = static_cast<int>(t / nq);
-    const int q = static_cast<int>(t % nq);
-    const double fw = ffW ? ffW[q] : 0.0;
-    const bool weighted = (nv == 4);
+template <int NV>
+__global__ void __launch_bounds__(PD_RED_THREADS)
+    pd_reduce_pairs(const double *__restrict__ slots, const int64_t *__restrict__ lptr,
+                    const int64_t *__restrict__ lidx, const PdPairDev *__restrict__ pairs,
+                    const double *__restrict__ qv, const PdFrameDev *__restrict__ frames,
+                    PdReduceShape sh, int32_t residual_form, int32_t add_exact,
+                    double *__restrict__ chunk_sums, unsigned int *__restrict__ done,
+                    double *__restrict__ red) {
+    __shared__ double s_run[PD_RED_GROUPS][NV][128];
+    __shared__ bool s_last;
+    const int z = blockIdx.x % sh.n_z;
+    const int p = blockIdx.x / sh.n_z % sh.n_pairs;
+    const int f = blockIdx.x / sh.n_z / sh.n_pairs;
+    const int tl = threadIdx.x & 127, grp = threadIdx.x >> 7;
+    const int k = z * 128 + tl;
+    const PdFrameDev fr = frames[f];
+    const bool moments = fr.n_mom > 0;
+    if (z * 128 >= (moments ? fr.n_mom : sh.nq)) return;
+    const int64_t fbase = static_cast<int64_t>(f) * sh.slots_per_frame;
+    const int64_t stride = static_cast<int64_t>(NV) * sh.K;
+    const int run = blockIdx.y * PD_RED_GROUPS + grp, n_runs = gridDim.y * PD_RED_GROUPS;
+    double s[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) s[v] = 0.0;
+    const double qval = (!moments && k < sh.nq) ? qv[k] : 0.0;
+    if (moments) {
+        if (k < fr.n_mom) {
+            const int mb = k / sh.block, kk = k - mb * sh.block;
+            for (int part = 0; part < fr.n_parts; ++part) {
+                const int64_t *lp = lptr + p * sh.nqb + part * fr.n_mblk + mb;
+                const int64_t l0 = lp[0], len = lp[1] - l0;
+                sum_slots<NV>(slots, lidx, l0 + len * run / n_runs, l0 + len * (run + 1) / n_runs,
+                              fbase, stride, sh.K, kk, s);
+            }
+        }
+    } else if (qval > 0.0) {
+        const int64_t *lp = lptr + p * sh.nqb + k / sh.K;
+        const int64_t l0 = lp[0], len = lp[1] - l0;
+        sum_slots<NV>(slots, lidx, l0 + len * run / n_runs, l0 + len * (run + 1) / n_runs, fbase,
+                      stride, sh.K, k % sh.K, s);
+    }
+#pragma unroll
+    for (int v = 0; v < NV; ++v) s_run[grp][v][tl] = s[v];
+    __syncthreads();
+    if (grp == 0) {
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+#pragma unroll
+            for (int g = 1; g < PD_RED_GROUPS; ++g) s[v] += s_run[g][v][tl];
+    }
+    if (gridDim.y > 1) {
+        // [block][chunk][nv][128]
+        double *cs = chunk_sums + static_cast<size_t>(blockIdx.x) * gridDim.y * NV * 128;
+        if (grp == 0) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) cs[(blockIdx.y * NV + v) * 128 + tl] = s[v];
+            __threadfence();
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            s_last = atomicAdd(&done[blockIdx.x], 1u) == gridDim.y - 1;
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        if (grp == 0) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) {
+                const volatile double *c = cs + v * 128 + tl;
+                double t = 0.0;
+                for (unsigned y = 0; y < gridDim.y; ++y) t += c[y * NV * 128];
+                s[v] = t;
+            }
+        }
+    }
+    if (grp != 0 || k >= sh.width) return;
+    if (!moments) {
+        if (k >= sh.nq) return;
+        if (qval > 0.0) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) s[v] /= qval;
+            if (add_exact && residual_form && residual_q(qval, fr.radius))
+#pragma unroll
+                for (int v = 0; v < NV; ++v) s[v] += pairs[p].q0[v];
+        } else {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) s[v] = add_exact ? pairs[p].q0[v] : 0.0;
+        }
+    }
+    double *o = red + (static_cast<int64_t>(f) * sh.n_pairs + p) * NV * sh.width + k;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) o[static_cast<int64_t>(v) * sh.width] = s[v];
+}
+
+// c_n(z)·z/4 (c_0·z/2) unnormalised for n < n_mom into coef[n·stride], z = q·d (see
+// pd_moments.cuh); returns the factor that makes them c_n. J_ν(z) by Miller's
+// downward recurrence, normalised with J_0 + 2ΣJ_2k = 1; it starts a few terms
+// beyond the moments z needs, where the value it drops is below the last bit.
+__device__ double moment_coefficients(double z, int n_mom, double *__restrict__ coef, int stride) {
+    if (!(z > 1e-8)) {  // sinc = 1 to the last bit
+        for (int n = 0; n < n_mom; ++n) coef[n * stride] = n == 0 ? 1.0 : 0.0;
+        return 1.0;
+    }
+    const double tz = 2.0 / z;
+    const int top = min(moments_needed(z, true) + 4, n_mom + 8);
+    for (int n = top + 1; n < n_mom; ++n) coef[n * stride] = 0.0;
+    double hi = 0.0, cur = 1e-200;  // J_{ν+1}, J_ν at ν = 2·top + 1
+    double even = 0.0, odd = 0.0;   // ΣJ_2k (k >= 1), ΣJ_{2k+1}
+    for (int n = top; n > 0; --n) {
+        odd += cur;  // ν = 2n + 1
+        if (n < n_mom) coef[n * stride] = odd;
+        const double nu = 2.0 * n;
+        const double lower = fma((nu + 1.0) * tz, cur, -hi);  // J_2n
+        even += lower;
+        cur = fma(nu * tz, lower, -cur);                      // J_{2n−1}
+        hi = lower;
+    }
+    odd += cur;
+    coef[0] = 0.5 * odd;
+    const double j0 = fma(tz, cur, -hi);
+    return 2.0 * tz / fma(2.0, even, j0);
+}
+
+// Six profiles of PD_PROF_Q grid points of one frame: the class-pair sums
+// Σ sinc(q r) (read, or formed from the moments), times the class factors, all
+// in FP64. 32 groups of eight threads (one per grid point) share the class
+// pairs, and where there are fewer pairs than groups also the moments; their
+// partial profiles are added in a fixed order.
+constexpr int PD_PROF_Q = 8;
+constexpr int PD_PROF_THREADS = 256;
+constexpr int PD_PROF_GROUPS = PD_PROF_THREADS / PD_PROF_Q;
+
+template <int NV>
+__global__ void __launch_bounds__(PD_PROF_THREADS)
+    pd_profiles(const double *__restrict__ red, const double *__restrict__ lat_sums,
+                const PdClassDev *__restrict__ cls, const PdPairDev *__restrict__ pairs,
+                int32_t n_cls, PdReduceShape sh, const double *__restrict__ qv,
+                const PdFrameDev *__restrict__ frames, const double *__restrict__ ffA,
+                const double *__restrict__ ffC, const double *__restrict__ ffW, int32_t add_diag,
+                double *__restrict__ terms) {
+    extern __shared__ double s_coef[];  // [n_mom][PD_PROF_Q]
+    __shared__ double s_c0[PD_PROF_Q], s_scale[PD_PROF_Q];
+    __shared__ double s_sum[PD_PROF_THREADS / 32][6][PD_PROF_Q];
+    const int n_qt = (sh.nq + PD_PROF_Q - 1) / PD_PROF_Q;
+    const int f = blockIdx.x / n_qt;
+    const int ql = threadIdx.x % PD_PROF_Q, g = threadIdx.x / PD_PROF_Q;
+    const int q = (blockIdx.x % n_qt) * PD_PROF_Q + ql;
+    const bool ok = q < sh.nq;
+    const PdFrameDev fr = frames[f];
+    const int M = fr.n_mom;
+    const double qval = ok ? qv[q] : 0.0;
+    if (M > 0) {
+        if (threadIdx.x < PD_PROF_Q) {
+            s_scale[ql] = moment_coefficients(qval * fr.d, M, s_coef + ql, PD_PROF_Q);
+            s_c0[ql] = s_coef[ql] * s_scale[ql];
+        }
+        __syncthreads();
+        // the factors of the tiles' sums e = 8j + 2t + {0, 1}, Σ X·vx and Σ Y·vy:
+        // (c_lo + c_hi)/2 and (c_hi − c_lo)/2 of the moments lo = 8j + 3 − t and
+        // hi = 8j + 4 + t
+        for (int j = g; j < M / 8; j += PD_PROF_GROUPS) {
+            double c[8];
+#pragma unroll
+            for (int n = 0; n < 8; ++n)
+                c[n] = 0.5 * s_scale[ql] * s_coef[(8 * j + n) * PD_PROF_Q + ql];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                s_coef[(8 * j + 2 * t) * PD_PROF_Q + ql] = c[3 - t] + c[4 + t];
+                s_coef[(8 * j + 2 * t + 1) * PD_PROF_Q + ql] = c[4 + t] - c[3 - t];
+            }
+        }
+        __syncthreads();
+    }
     double AA = 0, CC = 0, BB = 0, AC = 0, AB = 0, CB = 0;
-    for (int c = 0; c < (add_diag ? n_cls : 0); ++c) {  // i = j terms
-        const double fa = ffA[static_cast<int64_t>(cls[c].species) * nq + q];
-        const double ca = ffC ? ffC[static_cast<int64_t>(cls[c].species) * nq + q] : 0.0;
-        const double n = cls[c].n;
-        AA += n * fa * fa;
-        CC += n * ca * ca;
-        AC += n * fa * ca;
-        if (weighted) {
-            BB += fw * fw * cls[c].w2;
-            AB += fa * fw * cls[c].w1;
-            CB += ca * fw * cls[c].w1;
-        } else {
-            const double b = cls[c].w * fw;
-            BB += n * b * b;
-            AB += n * fa * b;
-            CB += n * ca * b;
+    const double fw = (ok && ffW) ? ffW[q] : 0.0;
+    constexpr bool weighted = NV == 4;
+    if (ok && add_diag) {  // i = j terms
+        for (int c = g; c < n_cls; c += PD_PROF_GROUPS) {
+            const PdClassDev cl = cls[c];
+            const double fa = ffA[static_cast<int64_t>(cl.species) * sh.nq + q];
+            const double ca = ffC ? ffC[static_cast<int64_t>(cl.species) * sh.nq + q] : 0.0;
+            AA += cl.n * fa * fa;
+            CC += cl.n * ca * ca;
+            AC += cl.n * fa * ca;
+            if (weighted) {
+                BB += fw * fw * cl.w2;
+                AB += fa * fw * cl.w1;
+                CB += ca * fw * cl.w1;
+            } else {
+                const double b = cl.w * fw;
+                BB += cl.n * b * b;
+                AB += cl.n * fa * b;
+                CB += cl.n * ca * b;
+            }
         }
     }
-    const int64_t per_frame = static_cast<int64_t>(n_pairs) * nq;
-    const double *ps = pairsum + static_cast<int64_t>(f) * nv * per_frame;
-    for (int p = 0; p < n_pairs; ++p) {  // i < j terms
-        const int a = pairs[p].a, b = pairs[p].b;
-        const double fa = ffA[static_cast<int64_t>(cls[a].species) * nq + q];
-        const double fb = ffA[static_cast<int64_t>(cls[b].species) * nq + q];
-        const double ca = ffC ? ffC[static_cast<int64_t>(cls[a].species) * nq + q] : 0.0;
-        const double cb = ffC ? ffC[static_cast<int64_t>(cls[b].species) * nq + q] : 0.0;
-        const double s0 = ps[static_cast<int64_t>(p) * nq + q];
-        AA += 2.0 * fa * fb * s0;
-        CC += 2.0 * ca * cb * s0;
-        AC += (fa * cb + ca * fb) * s0;
-        if (weighted) {
-            const double si = ps[per_frame + static_cast<int64_t>(p) * nq + q];
-            const double sj = ps[2 * per_frame + static_cast<int64_t>(p) * nq + q];
-            const double sij = ps[3 * per_frame + static_cast<int64_t>(p) * nq + q];
-            BB += 2.0 * fw * fw * sij;
-            AB += fw * (fa * sj + fb * si);
-            CB += fw * (ca * sj + cb * si);
+    // groups per class pair (they share its moments)
+    const int per = sh.n_pairs >= PD_PROF_GROUPS ? 1 : PD_PROF_GROUPS / sh.n_pairs;
+    const int sub = g % per;
+    for (int p = g / per; ok && p < sh.n_pairs; p += PD_PROF_GROUPS / per) {
+        const PdPairDev pr = pairs[p];
+        const double *r = red + (static_cast<int64_t>(f) * sh.n_pairs + p) * NV * sh.width;
+        double s[NV];
+        if (pr.lat >= 0) {  // from the lattice set's pair counts (class mode, one frame)
+            s[0] = sub == 0 ? lat_sums[static_cast<int64_t>(pr.lat) * sh.nq + q] : 0.0;
+        } else if (M == 0) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v)
+                s[v] = sub == 0 ? r[static_cast<int64_t>(v) * sh.width + q] : 0.0;
         } else {
-            const double ba = cls[a].w * fw, bb = cls[b].w * fw;
-            BB += 2.0 * ba * bb * s0;
-            AB += (fa * bb + ba * fb) * s0;
-            CB += (ca * bb + ba * cb) * s0;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) s[v] = 0.0;
+            if (qval > 0.0) {
+#pragma unroll 8
+                for (int e = sub; e < M; e += per) {
+                    const double c = s_coef[e * PD_PROF_Q + ql];
+#pragma unroll
+                    for (int v = 0; v < NV; ++v)
+                        s[v] = fma(c, r[static_cast<int64_t>(v) * sh.width + e], s[v]);
+                }
+            }
+            if (sub == 0) {
+                // the zeroth moment is the exact pair sum at q = 0, not the
+                // tiles' rounded (Σ X·vx − Σ Y·vy)/2
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    const double *rv = r + static_cast<int64_t>(v) * sh.width;
+                    const double m0 = add_diag ? pr.q0[v] : 0.0;
+                    s[v] = qval > 0.0 ? fma(s_c0[ql], m0 - 0.5 * (rv[6] - rv[7]), s[v]) : m0;
+                }
+            }
+        }
+        const PdClassDev cla = cls[pr.a], clb = cls[pr.b];
+        const int64_t sa = static_cast<int64_t>(cla.species) * sh.nq + q;
+        const int64_t sb = static_cast<int64_t>(clb.species) * sh.nq + q;
+        const double fa = ffA[sa], fb = ffA[sb];
+        const double ca = ffC ? ffC[sa] : 0.0, cb = ffC ? ffC[sb] : 0.0;
+        AA += 2.0 * fa * fb * s[0];
+        CC += 2.0 * ca * cb * s[0];
+        AC += (fa * cb + ca * fb) * s[0];
+        if constexpr (weighted) {
+            BB += 2.0 * fw * fw * s[3];
+            AB += fw * (fa * s[2] + fb * s[1]);
+            CB += fw * (ca * s[2] + cb * s[1]);
+        } else {
+            const double ba = cla.w * fw, bb = clb.w * fw;
+            BB += 2.0 * ba * bb * s[0];
+            AB += (fa * bb + ba * fb) * s[0];
+            CB += (ca * bb + ba * cb) * s[0];
         }
     }
-    double *o = terms + static_cast<int64_t>(f) * 6 * nq;
-    o[q] = AA;
-    o[nq + q] = CC;
-    o[2 * nq + q] = BB;
-    o[3 * nq + q] = AC;
-    o[4 * nq + q] = AB;
-    o[5 * nq + q] = CB;
+    double out[6] = {AA, CC, BB, AC, AB, CB};
+#pragma unroll
+    for (int t = 0; t < 6; ++t) {
+        out[t] += __shfl_xor_sync(0xffffffffu, out[t], 8);
+        out[t] += __shfl_xor_sync(0xffffffffu, out[t], 16);
+    }
+    if ((threadIdx.x & 31) < PD_PROF_Q)
+#pragma unroll
+        for (int t = 0; t < 6; ++t) s_sum[threadIdx.x >> 5][t][ql] = out[t];
+    __syncthreads();
+    if (threadIdx.x < 6 * PD_PROF_Q) {
+        const int t = threadIdx.x / PD_PROF_Q;
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < PD_PROF_THREADS / 32; ++w) v += s_sum[w][t][ql];
+        if (ok) terms[(static_cast<int64_t>(f) * 6 + t) * sh.nq + q] = v;
+    }
 }
 
 // ------------------------------------------------------------ lattice sets
@@ -1424,15 +1692,14 @@ __global__ void __launch_bounds__(128) pd_lattice_hist(const PdLatTile *__restri
 // Σ_{i<j} sinc(q r_ij) = Σ_n count(n)·sinc(q·spacing·√n), FP64, one CTA per
 // (q, lattice); each thread adds the bins n ≡ thread (mod 256) in ascending
 // order and a fixed tree adds the threads, so the sum is deterministic. The
-// value overwrites the class pair's entry of `pairsum` (the pair tiles skip
-// those pairs). Only the rank that adds the exact terms writes a sum; the
-// others write 0. *err set: NaN.
+// values are sums[lattice][q] (the pair tiles skip those pairs). Only the rank
+// that adds the exact terms writes a sum; the others write 0. *err set: NaN.
 __global__ void __launch_bounds__(256) pd_lattice_sums(const unsigned long long *__restrict__ hist,
                                                        const PdLatDev *__restrict__ lat,
                                                        const double *__restrict__ qv, int32_t nq,
                                                        int32_t add_exact,
                                                        const int *__restrict__ err,
-                                                       double *__restrict__ pairsum) {
+                                                       double *__restrict__ sums) {
     __shared__ double s_part[256];
     const int q = blockIdx.x;
     const PdLatDev d = lat[blockIdx.y];
@@ -1455,7 +1722,7 @@ __global__ void __launch_bounds__(256) pd_lattice_sums(const unsigned long long 
     if (threadIdx.x == 0) {
         double v = add_exact ? s_part[0] : 0.0;
         if (*err) v = __longlong_as_double(0x7ff8000000000000ll);  // NaN
-        pairsum[static_cast<int64_t>(d.pair) * nq + q] = v;
+        sums[static_cast<int64_t>(blockIdx.y) * nq + q] = v;
     }
 }
 
@@ -2018,48 +2285,68 @@ cudaError_t prepare_pair_kernels() {
     return cudaSuccess;
 }
 
-cudaError_t launch_centroid(const double *xyz, int64_t n_atoms, int n_frames, double *centroid,
-                            double *radius, cudaStream_t st) {
-    pd_centroid<<<n_frames, 256, 0, st>>>(xyz, n_atoms, centroid, radius);
+int32_t centroid_blocks(int64_t n_atoms) {
+    return static_cast<int32_t>(
+        std::min<int64_t>(std::max<int64_t>((n_atoms + PD_CENT_RUN - 1) / PD_CENT_RUN, 1), 256));
+}
+
+cudaError_t launch_centroid(const double *xyz, int64_t n_atoms, int n_frames, double *part,
+                            unsigned int *done, double *centroid, int32_t *status,
+                            cudaStream_t st) {
+    const int32_t nb = centroid_blocks(n_atoms);
+    pd_centroid<<<static_cast<unsigned>(n_frames) * nb, PD_CENT_THREADS, 0, st>>>(
+        xyz, n_atoms, nb, part, done, centroid, status);
     return cudaGetLastError();
 }
 
 cudaError_t launch_pack(const double *xyz, const double *weights, const int32_t *perm,
                         const double *centroid, int64_t n_atoms, int32_t n_pad, int32_t n_frames,
-                        float4 *out32, double4 *out64, cudaStream_t st) {
-    const int64_t total = static_cast<int64_t>(n_pad) * n_frames;
-    const int grid = static_cast<int>((total + 255) / 256);
-    pd_pack<<<grid, 256, 0, st>>>(xyz, weights, perm, centroid, n_atoms, n_pad, n_frames, out32,
-                                  out64);
+                        float4 *out32, double4 *out64, const PdMomentRule &rule,
+                        unsigned long long *rad2, unsigned int *done, PdFrameDev *frames,
+                        cudaStream_t st) {
+    const int64_t nb = (static_cast<int64_t>(n_pad) + PD_PACK_THREADS - 1) / PD_PACK_THREADS;
+    if (nb * n_frames > 0x7fffffffLL) return cudaErrorInvalidValue;
+    pd_pack<<<static_cast<unsigned>(nb * n_frames), PD_PACK_THREADS, 0, st>>>(
+        xyz, weights, perm, centroid, n_atoms, n_pad, static_cast<int32_t>(nb), out32, out64, rule,
+        rad2, done, frames);
     return cudaGetLastError();
 }
 
 cudaError_t launch_reduce(const double *slots, const int64_t *lptr, const int64_t *lidx,
-                          const PdPairDev *pairs, const double *qv, int32_t n_pairs, int32_t nq,
-                          int32_t K, int32_t nv, int32_t n_frames, int64_t slots_per_frame,
-                          const double *radius, double qmin, double dq, int residual_form,
-                          int add_exact, double *pairsum, cudaStream_t st) {
-    const int64_t total = static_cast<int64_t>(n_pairs) * nq * n_frames;
-    const int grid = static_cast<int>((total + 127) / 128);
+                          const PdPairDev *pairs, const double *qv, const PdFrameDev *frames,
+                          const PdReduceShape &sh, int32_t nv, int32_t n_frames, int residual_form,
+                          int add_exact, double *chunk_sums, unsigned int *done, double *red,
+                          cudaStream_t st) {
+    const int64_t blocks = static_cast<int64_t>(n_frames) * sh.n_pairs * sh.n_z;
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+    const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(sh.n_chunk));
     if (nv == 4)
-        pd_reduce_pairs<4><<<grid, 128, 0, st>>>(slots, lptr, lidx, pairs, qv, n_pairs, nq, K,
-                                                 nv, n_frames, slots_per_frame, radius, qmin, dq,
-                                                 residual_form, add_exact, pairsum);
+        pd_reduce_pairs<4><<<grid, PD_RED_THREADS, 0, st>>>(slots, lptr, lidx, pairs, qv, frames,
+                                                            sh, residual_form, add_exact,
+                                                            chunk_sums, done, red);
     else
-        pd_reduce_pairs<1><<<grid, 128, 0, st>>>(slots, lptr, lidx, pairs, qv, n_pairs, nq, K,
-                                                 nv, n_frames, slots_per_frame, radius, qmin, dq,
-                                                 residual_form, add_exact, pairsum);
+        pd_reduce_pairs<1><<<grid, PD_RED_THREADS, 0, st>>>(slots, lptr, lidx, pairs, qv, frames,
+                                                            sh, residual_form, add_exact,
+                                                            chunk_sums, done, red);
     return cudaGetLastError();
 }
 
-cudaError_t launch_combine(const double *pairsum, const PdClassDev *cls, const PdPairDev *pairs,
-                           int32_t n_cls, int32_t n_pairs, int32_t nq, int32_t nv,
-                           int32_t n_frames, const double *ffA, const double *ffC,
-                           const double *ffW, int add_diag, double *terms, cudaStream_t st) {
-    const int64_t total = static_cast<int64_t>(nq) * n_frames;
-    const int grid = static_cast<int>((total + 127) / 128);
-    pd_combine_terms<<<grid, 128, 0, st>>>(pairsum, cls, pairs, n_cls, n_pairs, nq, nv, n_frames,
-                                           ffA, ffC, ffW, add_diag, terms);
+cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdClassDev *cls,
+                            const PdPairDev *pairs, int32_t n_cls, const PdReduceShape &sh,
+                            int32_t nv, int32_t n_frames, const double *qv,
+                            const PdFrameDev *frames, const double *ffA, const double *ffC,
+                            const double *ffW, int add_diag, double *terms, cudaStream_t st) {
+    const int64_t blocks =
+        static_cast<int64_t>(n_frames) * ((sh.nq + PD_PROF_Q - 1) / PD_PROF_Q);
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+    // coefficients of the most moments a frame may have: at most 32 KB
+    const size_t smem = static_cast<size_t>(sh.max_moments) * PD_PROF_Q * sizeof(double);
+    if (nv == 4)
+        pd_profiles<4><<<static_cast<unsigned>(blocks), PD_PROF_THREADS, smem, st>>>(
+            red, lat_sums, cls, pairs, n_cls, sh, qv, frames, ffA, ffC, ffW, add_diag, terms);
+    else
+        pd_profiles<1><<<static_cast<unsigned>(blocks), PD_PROF_THREADS, smem, st>>>(
+            red, lat_sums, cls, pairs, n_cls, sh, qv, frames, ffA, ffC, ffW, add_diag, terms);
     return cudaGetLastError();
 }
 
@@ -2102,9 +2389,9 @@ cudaError_t launch_lattice(const double *xyz, const int32_t *perm, const PdLatDe
 
 cudaError_t launch_lattice_sums(const unsigned long long *hist, const PdLatDev *lat, int n_lat,
                                 const double *qv, int32_t nq, int add_exact, const int *err,
-                                double *pairsum, cudaStream_t st) {
+                                double *sums, cudaStream_t st) {
     if (n_lat == 0) return cudaSuccess;
-    pd_lattice_sums<<<dim3(nq, n_lat), 256, 0, st>>>(hist, lat, qv, nq, add_exact, err, pairsum);
+    pd_lattice_sums<<<dim3(nq, n_lat), 256, 0, st>>>(hist, lat, qv, nq, add_exact, err, sums);
     return cudaGetLastError();
 }
 

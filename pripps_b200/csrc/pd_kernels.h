@@ -21,30 +21,39 @@ cudaError_t prepare_pair_kernels();
 cudaError_t launch_pairs(int precision, int K, int NP, int mode, const PdJob *jobs,
                          const int *n_jobs, const PdReqDev *reqs, int *counter, int grid,
                          cudaStream_t st);
-cudaError_t launch_centroid(const double *xyz, int64_t n_atoms, int n_frames, double *centroid,
-                            double *radius, cudaStream_t st);
+// Blocks per frame of the centroid kernel (3 partial sums each).
+int32_t centroid_blocks(int64_t n_atoms);
+// `done` (one counter per frame) must be zero; `status`, if given, is cleared.
+cudaError_t launch_centroid(const double *xyz, int64_t n_atoms, int n_frames, double *part,
+                            unsigned int *done, double *centroid, int32_t *status,
+                            cudaStream_t st);
+// rad2 and done (one per frame) must be zero; writes the frames' constants.
 cudaError_t launch_pack(const double *xyz, const double *weights, const int32_t *perm,
                         const double *centroid, int64_t n_atoms, int32_t n_pad, int32_t n_frames,
-                        float4 *out32, double4 *out64, cudaStream_t st);
+                        float4 *out32, double4 *out64, const PdMomentRule &rule,
+                        unsigned long long *rad2, unsigned int *done, PdFrameDev *frames,
+                        cudaStream_t st);
+// Slot sums (red: [frame][pair][nv][width]); with n_chunk > 1, chunk_sums holds
+// 128·nv·n_chunk doubles and done one zeroed counter per (frame, pair, n_z).
 cudaError_t launch_reduce(const double *slots, const int64_t *lptr, const int64_t *lidx,
-                          const PdPairDev *pairs, const double *qv, int32_t n_pairs, int32_t nq,
-                          int32_t K, int32_t nv, int32_t n_frames, int64_t slots_per_frame,
-                          const double *radius, double qmin, double dq, int residual_form,
-                          int add_exact, double *pairsum, cudaStream_t st);
-cudaError_t launch_combine(const double *pairsum, const PdClassDev *cls, const PdPairDev *pairs,
-                           int32_t n_cls, int32_t n_pairs, int32_t nq, int32_t nv,
-                           int32_t n_frames, const double *ffA, const double *ffC,
-                           const double *ffW, int add_diag, double *terms, cudaStream_t st);
+                          const PdPairDev *pairs, const double *qv, const PdFrameDev *frames,
+                          const PdReduceShape &sh, int32_t nv, int32_t n_frames, int residual_form,
+                          int add_exact, double *chunk_sums, unsigned int *done, double *red,
+                          cudaStream_t st);
+cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdClassDev *cls,
+                            const PdPairDev *pairs, int32_t n_cls, const PdReduceShape &sh,
+                            int32_t nv, int32_t n_frames, const double *qv,
+                            const PdFrameDev *frames, const double *ffA, const double *ffC,
+                            const double *ffW, int add_diag, double *terms, cudaStream_t st);
 // Lattice sets: integer coordinates of their points and the exact pair count
-// per squared offset (after pack), then their self pair sums (after the slot
-// reduction, overwriting those class pairs' entries of pairsum).
+// per squared offset (after pack), then their self pair sums, sums[lattice][q].
 cudaError_t launch_lattice(const double *xyz, const int32_t *perm, const PdLatDev *lat_dev,
                            const PdLatDev *lat_host, int n_lat, const PdLatTile *tiles,
                            int64_t n_tiles, int4 *idx, unsigned long long *hist, int64_t n_bins,
                            int *err, cudaStream_t st);
 cudaError_t launch_lattice_sums(const unsigned long long *hist, const PdLatDev *lat, int n_lat,
                                 const double *qv, int32_t nq, int add_exact, const int *err,
-                                double *pairsum, cudaStream_t st);
+                                double *sums, cudaStream_t st);
 cudaError_t launch_frame_mean(const double *terms, const double *fw, int32_t n_frames, int32_t nq,
                               double *out, cudaStream_t st, bool normalize = true);
 // Direct transform: (Re A, Im A, |A|², Σ_m |F_m|²) per q-vector for points

@@ -385,6 +385,7 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
             PdPairDev pd{};
             pd.a = a;
             pd.b = b;
+            pd.lat = a == b ? lat_of_cls[a] : -1;
             const double na = P.cls[a].n, nb = P.cls[b].n;
             if (a != b) {
                 pd.q0[0] = na * nb;
@@ -573,7 +574,46 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
             }
         }
     }
+    set_reduction(P);
     return PD_OK;
+}
+
+void set_reduction(Plan &P) {
+    PdMomentRule &m = P.mom;
+    m = PdMomentRule{};
+    m.qmax = P.qmax;
+    m.nqb = P.nqb;
+    m.fp64 = P.precision == PD_FP64 ? 1 : 0;
+    if (P.precision == PD_FP32_FP64RED && P.mode == PD_MODE_CLASS) {
+        m.block = pd_moment_block(P.tun.K);
+        // Lane operations per pair: 1.5 per moment and about 42 for the
+        // sequences, against 3 per grid point and 55 for each q-block's seeds.
+        m.max_moments = static_cast<int32_t>(
+            std::min<int64_t>({PD_MAX_MOMENTS, static_cast<int64_t>(P.nqb) * m.block,
+                               2 * static_cast<int64_t>(P.nq) + 8 * P.nqb}) & ~int64_t{7});
+        if (m.max_moments < 8) m.block = 0;
+    }
+    PdReduceShape &r = P.red;
+    r = PdReduceShape{};
+    r.n_pairs = P.n_pairs;
+    r.nq = P.nq;
+    r.K = P.tun.K;
+    r.nqb = P.nqb;
+    r.block = m.block;
+    r.max_moments = m.block ? m.max_moments : 0;
+    r.width = std::max(P.nq, r.max_moments);
+    r.n_z = (r.width + 127) / 128;
+    // A block adds its share of a class pair's slot list serially: lists of
+    // more than a few hundred entries are shared by up to 16 blocks (one
+    // frame; the frames of a batch fill the GPU by themselves).
+    int64_t longest = 0;
+    for (int p = 0; p < P.n_pairs; ++p)
+        longest = std::max(longest, P.lptr[static_cast<size_t>(p + 1) * P.nqb] -
+                                        P.lptr[static_cast<size_t>(p) * P.nqb]);
+    r.n_chunk = P.n_frames > 1 ? 1
+                               : static_cast<int32_t>(
+                                     std::min<int64_t>(std::max<int64_t>(longest / 256, 1), 16));
+    r.slots_per_frame = P.slots_per_frame;
 }
 
 int shard_plan(const Plan &full, uint32_t rank, uint32_t world, Plan &out) {
@@ -617,6 +657,7 @@ int shard_plan(const Plan &full, uint32_t rank, uint32_t world, Plan &out) {
         }
         out.lptr[e + 1] = static_cast<int64_t>(out.lidx.size());
     }
+    set_reduction(out);
     return PD_OK;
 }
 

@@ -59,6 +59,8 @@ struct Plan {
     int nqb = 0;
     std::vector<int64_t> lptr;  // [n_pairs * nqb + 1]
     std::vector<int64_t> lidx;  // slot indices within a frame
+    PdMomentRule mom{};     // when a frame takes the moment form
+    PdReduceShape red{};    // sizes of the slot reduction
     uint64_t pairs_covered = 0; // per frame, unordered pairs over all tiles
 
     // lattice sets (class mode, one frame): their self pairs are counted per
@@ -76,6 +78,10 @@ Tuning default_tuning(int64_t n_atoms, int64_t nq, int precision, int64_t n_fram
 // The instantiated kernel shape a requested one runs as in a mode (the q
 // block and pairs per thread adjusted where that shape has no kernel).
 Tuning fit_tuning(int precision, int mode, Tuning t);
+
+// The moment rule and reduction sizes of a plan whose tiles and lists stand
+// (again after a shard cut them).
+void set_reduction(Plan &P);
 
 // A rank's share of a plan for a tile-sharded solve: every world-th tile of
 // the cost-ordered job list, with only the slots those tiles write (numbered

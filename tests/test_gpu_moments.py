@@ -1,0 +1,101 @@
+"""The moment form of the pair sum at the sizes where it can go wrong.
+
+Every pair's sinc(q r) is expanded in cos(n φ), sin(φ/2) = r/d; the number of
+moments grows with q_max·d, they are summed in blocks of the kernel shape's
+size, and the q-block jobs of a tile become parts of its j range. The cases
+put the moment count below, at and above a block for every block size, leave
+jobs idle (more q-blocks than blocks × parts use), and reach the bounds of the
+rule (few grid points on a long range: the grid points are summed directly).
+
+Tolerances are those of the two forms: FP64 1e-10 and FP32 1e-5 of the
+compensated oracle, self profiles relative and cross profiles normalised (an
+FP32 moment carries rounding errors of at most n·6e-8 per pair with random
+signs, n <= 512; the worst single pair, two atoms at the largest distance, is
+below 512·6e-8/(z/2) <= 4e-7 of its value's scale).
+"""
+import numpy as np
+import pytest
+
+from conftest import term_errors
+from oracle import oracle as O
+from pripps_b200 import _lib
+from pripps_b200.debye import DebyeRequest, solve
+
+pytestmark = pytest.mark.gpu
+TOL = {"fp64": 1e-10, "fp32": 1e-5}
+
+
+def _request(xyz, nq, qmin, qmax, precision, mode, seed):
+    rng = np.random.default_rng(seed)
+    n = len(xyz)
+    sp = rng.integers(0, 3, n)
+    ff = rng.uniform(1, 8, (3, nq))
+    if mode == "vacuum":
+        return DebyeRequest(xyz, sp, ff, None, None, None, qmin, qmax, nq, None, precision)
+    w = rng.uniform(0, 2, n) if mode == "weighted" else np.where(rng.random(n) < 0.5, 1.25, 0.0)
+    return DebyeRequest(xyz, sp, ff, rng.uniform(0.2, 3, (3, nq)), w, rng.uniform(5, 10, nq),
+                        qmin, qmax, nq, None, precision)
+
+
+def _check(req, ctx, precision):
+    t = solve(req, ctx)
+    qi = np.unique(np.concatenate([np.arange(min(4, req.nq)), [req.nq // 2],
+                                   np.arange(max(0, req.nq - 2), req.nq)]))
+    ref = O.terms_for_request(req, q_index=qi, precise=True)
+    err = term_errors(t[:, qi], ref)
+    assert np.all(err < TOL[precision]), err
+
+
+# radius × qmax sets z = q_max·d ≈ 2.06·radius·qmax, so about z/2 + 5·z^(1/3) moments:
+# 8, 24, 32/33 (a block of 32), 64, 128 (one block of 128), 145 (two), 300 and
+# 500 (several; with nq = 90 more than the rule allows)
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("mode", ["vacuum", "class", "weighted"])
+@pytest.mark.parametrize("radius,qmax,nq", [(1.0, 0.3, 40), (16.0, 0.5, 61), (18.0, 0.98, 100),
+                                            (18.0, 1.02, 100), (40.0, 1.02, 257), (60.0, 1.5, 300),
+                                            (60.0, 2.1, 129), (90.0, 2.9, 400), (150.0, 3.0, 600),
+                                            (150.0, 3.0, 90)])
+def test_moment_counts(gpu_ctx, precision, mode, radius, qmax, nq):
+    rng = np.random.default_rng(int(radius * 100 + nq))
+    n = 333
+    v = rng.normal(size=(n, 3))
+    xyz = radius * v / np.linalg.norm(v, axis=1)[:, None] * rng.random((n, 1)) ** (1 / 3)
+    _check(_request(xyz, nq, 0.02 if nq == 61 else 0.0, qmax, precision, mode, nq), gpu_ctx,
+           precision)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("shape", [(32, 4), (64, 2), (64, 4), (96, 2), (128, 1), (128, 4),
+                                   (160, 1), (192, 1)])
+@pytest.mark.parametrize("tj", [32, 96, 512])
+def test_moment_blocks_of_every_shape(precision, shape, tj):
+    """Moment block and slot stride differ between the shapes, and a part of a
+    short j range may be empty."""
+    K, NP = shape
+    if precision == "fp64":
+        K, NP = (16 if K == 32 else 32), 1
+    ctx = _lib.Context(0)
+    try:
+        rng = np.random.default_rng(K + tj)
+        n, nq = 700, 290
+        _lib.check(_lib.lib().pd_set_tuning(ctx.handle, n, nq, _lib.PRECISIONS[precision], K, tj,
+                                            NP), ctx.handle)
+        xyz = rng.uniform(-20, 20, (n, 3))
+        _check(_request(xyz, nq, 0.0, 1.2, precision, "class", K), ctx, precision)
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("name", ["one", "pair", "coincident", "all_coincident", "line", "far"])
+def test_moment_extreme_distances(gpu_ctx, precision, name):
+    """Distances at the ends of the expansion: r = 0 (also with a zero radius),
+    and r = 2·radius, the largest φ."""
+    rng = np.random.default_rng(5)
+    xyz = {"one": np.zeros((1, 3)),
+           "pair": np.array([[0, 0, 0], [37.0, 0, 0]]),
+           "coincident": np.array([[1, 2, 3], [1, 2, 3], [9.0, -2, 4]]),
+           "all_coincident": np.full((40, 3), 2.5),
+           "line": np.stack([np.linspace(-60, 60, 131), np.zeros(131), np.zeros(131)], axis=1),
+           "far": np.concatenate([rng.normal(size=(60, 3)), rng.normal(size=(60, 3)) + 150.0])}
+    _check(_request(xyz[name], 200, 0.0, 0.8, precision, "vacuum", 3), gpu_ctx, precision)

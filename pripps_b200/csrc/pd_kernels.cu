@@ -794,26 +794,17 @@ __device__ __forceinline__ MomJob moment_job(int j0, int j1, int qb, int n_mblk,
 }
 
 // Weighted-mode flush of one accumulator array: the warp sums of acc and of
-// w_i·acc, reduce-scattered (lane l ends with grid points
-// [l·K/32, (l+1)·K/32)) and added to part[k] and part[K + k].
+// w_i·acc, added to part[k] and part[stride + k].
 template <int K>
-__device__ __forceinline__ void flush_weighted_rs(float2 (&acc)[K / 2], float wi,
-                                                  double *__restrict__ part, int lane,
-                                                  bool first) {
+__device__ __forceinline__ void flush_weighted(float2 (&acc)[K / 2], float wi,
+                                               double *__restrict__ part, int stride, int lane,
+                                               bool first) {
     const float2 wi2 = make_float2(wi, wi);
     float2 tw[K / 2];
 #pragma unroll
     for (int t = 0; t < K / 2; ++t) tw[t] = __fmul2_rn(wi2, acc[t]);
-    warp_reduce_scatter<K / 2>(acc, lane);
-    warp_reduce_scatter<K / 2>(tw, lane);
-#pragma unroll
-    for (int m = 0; m < K / 32; ++m) {
-        const int k = lane * (K / 32) + m;
-        const float s = (m & 1) ? acc[m >> 1].y : acc[m >> 1].x;
-        const float sw = (m & 1) ? tw[m >> 1].y : tw[m >> 1].x;
-        part[k] = (first ? 0.0 : part[k]) + static_cast<double>(s);
-        part[K + k] = (first ? 0.0 : part[K + k]) + static_cast<double>(sw);
-    }
+    flush_class<K / 2>(acc, part, lane, first);
+    flush_class<K / 2>(tw, part + stride, lane, first);
 }
 
 // End of a tile: the warps' FP64 partial sums (part[w·nvk + e], e < nvk) of
@@ -849,7 +840,6 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
     constexpr int NACC = (MODE == PD_MODE_WEIGHTED) ? 2 : 1;
     constexpr int NV = (MODE == PD_MODE_WEIGHTED) ? 4 : 1;  // FP64 values per q in a slot
     constexpr bool PACKED = (MODE == PD_MODE_CLASS);
-    constexpr bool HAS_MOMENTS = (MODE == PD_MODE_CLASS);
     constexpr bool PACKED_W =
         (MODE == PD_MODE_WEIGHTED) && PD_WEIGHTED_X2 && (K / 2) % 32 == 0 && NP % 2 == 0;
     __shared__ int s_job;
@@ -892,9 +882,9 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
         const PdFrameDev fr = rq.frames[jb.frame];
         const double radius = fr.radius;
         // moment form: this job's part of the j range and its moment block
-        const bool moments = HAS_MOMENTS && fr.n_mom > 0;
+        const bool moments = fr.n_mom > 0;
         int tj0 = jb.j0, tj1 = jb.j1, mblk = 0;
-        if (HAS_MOMENTS && moments) {
+        if (moments) {
             const MomJob mj = moment_job(jb.j0, jb.j1, jb.qb, fr.n_mblk, fr.n_parts);
             tj0 = mj.j0;
             tj1 = mj.j1;
@@ -969,16 +959,28 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
                 for (int js = jss; js < jse; js += PD_JFLUSH) {
                     const int je = min(jse, js + PD_JFLUSH);
                     const bool first = js == tj0;
-                    if (HAS_MOMENTS && moments) {
+                    if (moments) {
                         constexpr int KM = pd_moment_block(K);
-                        float2 acc[KM / 2];
-#pragma unroll
-                        for (int t = 0; t < KM / 2; ++t) acc[t] = make_float2(0.0f, 0.0f);
-                        const int nj = min(KM, fr.n_mom - mblk * KM) >> 3;
                         constexpr int DBL = KM == 128 ? 4 : (KM == 64 ? 3 : 2);
-                        moments_range<KM>(chunk, jss, pi, i, ivalid, js, je,
-                                          static_cast<float>(fr.inv_d2), nj, mblk, DBL, acc);
-                        flush_class<KM / 2>(acc, part, lane, first);
+                        const int nj = min(KM, fr.n_mom - mblk * KM) >> 3;
+                        const float inv_d2 = static_cast<float>(fr.inv_d2);
+                        float2 acc0[KM / 2];
+#pragma unroll
+                        for (int t = 0; t < KM / 2; ++t) acc0[t] = make_float2(0.0f, 0.0f);
+                        if constexpr (MODE == PD_MODE_CLASS) {
+                            moments_range<KM>(chunk, jss, pi, i, ivalid, js, je, inv_d2, nj, mblk,
+                                              DBL, acc0);
+                            flush_class<KM / 2>(acc0, part, lane, first);
+                        } else {
+                            float2 acc1[KM / 2];
+#pragma unroll
+                            for (int t = 0; t < KM / 2; ++t) acc1[t] = make_float2(0.0f, 0.0f);
+                            moments_range_w<KM>(chunk, jss, pi, i, ivalid, js, je, inv_d2, nj,
+                                                mblk, DBL, acc0, acc1);
+                            const float wi = ivalid ? pi.w : 0.0f;
+                            flush_weighted<KM>(acc0, wi, part, K, lane, first);
+                            flush_weighted<KM>(acc1, wi, part + 2 * K, K, lane, first);
+                        }
                     } else if constexpr (PACKED) {
                         const float2 *q2 = reinterpret_cast<const float2 *>(s_qres);
                         // 16-point chunks of this block that lie on the grid.
@@ -1045,8 +1047,8 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
                         // the four warp sums of each grid point: Σ acc0,
                         // Σ w_i·acc0, Σ acc1, Σ w_i·acc1
                         const float wi = ivalid ? pi.w : 0.0f;
-                        flush_weighted_rs<K>(acc0, wi, part, lane, first);
-                        flush_weighted_rs<K>(acc1, wi, part + 2 * K, lane, first);
+                        flush_weighted<K>(acc0, wi, part, K, lane, first);
+                        flush_weighted<K>(acc1, wi, part + 2 * K, K, lane, first);
                     } else {
                         const float wi = ivalid ? pi.w : 0.0f;
                         float acc[NACC][K];
@@ -1125,7 +1127,7 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
 
 // ---------------------------------------------------------------- K2 (FP64)
 template <int K, int MODE>
-__global__ void __launch_bounds__(PD_THREADS) pd_pairs_fp64(const PdJob *__restrict__ jobs,
+__global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(const PdJob *__restrict__ jobs,
                                                             const int *__restrict__ n_jobs_ptr,
                                                             const PdReqDev *__restrict__ reqs,
                                                             int *__restrict__ counter) {
@@ -1161,7 +1163,21 @@ __global__ void __launch_bounds__(PD_THREADS) pd_pairs_fp64(const PdJob *__restr
 #pragma unroll
             for (int k = 0; k < K; ++k) acc[a][k] = 0.0;
 
-        for (int j = jb.j0; j < jb.j1; ++j) {
+        const PdFrameDev fr = rq.frames[jb.frame];
+        if (fr.n_mom > 0) {  // moment form: this job's part of the j range and its block
+            constexpr int DBL = K == 64 ? 3 : (K == 32 ? 2 : 1);
+            const MomJob mj = moment_job(jb.j0, jb.j1, jb.qb, fr.n_mblk, fr.n_parts);
+            const int nj = min(K, fr.n_mom - mj.mb * K) >> 3;
+            if constexpr (MODE == PD_MODE_WEIGHTED) {
+                moments_range_f64<K, true>(at, pi, i, ivalid, mj.j0, mj.j1, fr.inv_d2, nj, mj.mb,
+                                           DBL, acc[0], acc[1]);
+            } else {
+                double none[1];
+                moments_range_f64<K, false>(at, pi, i, ivalid, mj.j0, mj.j1, fr.inv_d2, nj, mj.mb,
+                                            DBL, acc[0], none);
+            }
+        }
+        for (int j = fr.n_mom > 0 ? jb.j1 : jb.j0; j < jb.j1; ++j) {
             const double4 pj = at[j];
             const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
             double r2 = dx * dx + dy * dy + dz * dz;
@@ -2229,14 +2245,15 @@ static int occupancy_fp64() {
 // (K, NP) shapes instantiated for the FP32 form; the weighted mode (two
 // accumulators per q) only up to K = 64 to stay within 255 registers.
 bool valid_shape(int precision, int mode, int K, int NP) {
-    if (precision == 1) return (K == 16 || K == 32) && NP == 1;
+    // FP64: weighted mode up to K = 32 (two FP64 accumulators per value)
+    if (precision == 1) return (K == 16 || K == 32 || (K == 64 && mode == PD_MODE_CLASS)) && NP == 1;
     if (mode == PD_MODE_WEIGHTED) return (K == 32 && NP == 2) || (K == 64 && (NP == 2 || NP == 4));
     return (K == 32 && NP == 4) || (K == 64 && NP >= 1 && NP != 3) || (K == 96 && NP == 2) ||
            (K == 128 && NP >= 1 && NP != 3) || ((K == 160 || K == 192) && NP == 1);
 }
 
 bool valid_q_block(int precision, int K) {
-    if (precision == 1) return K == 16 || K == 32;
+    if (precision == 1) return K == 16 || K == 32 || K == 64;
     return K == 32 || K == 64 || K == 96 || K == 128 || K == 160 || K == 192;
 }
 
@@ -2250,7 +2267,7 @@ cudaError_t launch_pairs(int precision, int K_, int NP_, int mode, const PdJob *
                          const int *n_jobs, const PdReqDev *reqs, int *counter, int grid,
                          cudaStream_t st) {
     if (precision == 1) {
-        PD_F64(16, 0) PD_F64(16, 1) PD_F64(32, 0) PD_F64(32, 1)
+        PD_F64(16, 0) PD_F64(16, 1) PD_F64(32, 0) PD_F64(32, 1) PD_F64(64, 0)
         return cudaErrorInvalidValue;
     }
     PD_F32(32, 0, 4) PD_F32(64, 0, 1) PD_F32(64, 0, 2) PD_F32(64, 0, 4) PD_F32(96, 0, 2)
@@ -2266,7 +2283,7 @@ cudaError_t launch_pairs(int precision, int K_, int NP_, int mode, const PdJob *
 
 int pairs_blocks_per_sm(int precision, int K_, int NP_, int mode) {
     if (precision == 1) {
-        PD_O64(16, 0) PD_O64(16, 1) PD_O64(32, 0) PD_O64(32, 1)
+        PD_O64(16, 0) PD_O64(16, 1) PD_O64(32, 0) PD_O64(32, 1) PD_O64(64, 0)
         return 0;
     }
     PD_O32(32, 0, 4) PD_O32(64, 0, 1) PD_O32(64, 0, 2) PD_O32(64, 0, 4) PD_O32(96, 0, 2)

@@ -163,4 +163,125 @@ __device__ __forceinline__ void moments_range(const float4 *__restrict__ at, int
     }
 }
 
+// Weighted mode: the same moments in acc0, and weighted by the j atom's
+// hydration weight in acc1 (16 lane operations per eight moments and the turn's 4).
+template <int KM>
+__device__ __forceinline__ void moments_range_w(const float4 *__restrict__ at, int jbase,
+                                                float4 pi, int i, bool ivalid, int j0, int j1,
+                                                float inv_d2, int nj, int rep, int dbl,
+                                                float2 (&acc0)[KM / 2], float2 (&acc1)[KM / 2]) {
+    const float2 M1 = mom_f2(-1.0f);
+    for (int j = j0; j < j1; j += 2) {
+        const bool inb = j + 1 < j1;
+        const float4 pa = at[j - jbase], pb = at[(inb ? j + 1 : j) - jbase];
+        const float2 dx = __ffma2_rn(make_float2(pa.x, pb.x), M1, mom_f2(pi.x));
+        const float2 dy = __ffma2_rn(make_float2(pa.y, pb.y), M1, mom_f2(pi.y));
+        const float2 dz = __ffma2_rn(make_float2(pa.z, pb.z), M1, mom_f2(pi.z));
+        const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+        MomPair2 P;
+        mom_seed_x2(r2, inv_d2, rep, dbl, P);
+        const bool va = ivalid && j > i, vb = ivalid && inb && j + 1 > i;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const bool v = h ? vb : va;
+            const float w = h ? pb.w : pa.w;
+            float2 U = h ? make_float2(P.X.y, P.Y.y) : make_float2(P.X.x, P.Y.x);
+            U = make_float2(v ? U.x : 0.0f, v ? U.y : 0.0f);
+            const float c8 = h ? P.c8.y : P.c8.x, t1 = h ? P.t1.y : P.t1.x,
+                        t2 = h ? P.t2.y : P.t2.x;
+            float2 V[4], WV[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                V[t] = h ? make_float2(P.vx[t].y, P.vy[t].y) : make_float2(P.vx[t].x, P.vy[t].x);
+                WV[t] = __fmul2_rn(mom_f2(w), V[t]);
+            }
+#pragma unroll
+            for (int jj = 0; jj < KM / 8; ++jj) {
+                if (jj >= nj) break;
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    acc0[4 * jj + t] = __ffma2_rn(U, V[t], acc0[4 * jj + t]);
+                    acc1[4 * jj + t] = __ffma2_rn(U, WV[t], acc1[4 * jj + t]);
+                }
+                const float x = fmaf(U.x, c8, -(U.y * t1));
+                U.y = fmaf(U.y, c8, U.x * t2);
+                U.x = x;
+            }
+        }
+    }
+}
+
+// FP64 form: the same sequences in double, one pair at a time;
+// acc[8·jj + 2t + {0, 1}] = Σ X·vx, Σ Y·vy (and weighted by w_j in accw).
+template <int KM, bool WEIGHTED>
+__device__ __forceinline__ void moments_range_f64(const double4 *__restrict__ at, double4 pi, int i,
+                                                  bool ivalid, int j0, int j1, double inv_d2,
+                                                  int nj, int rep, int dbl, double (&acc)[KM],
+                                                  double (&accw)[WEIGHTED ? KM : 1]) {
+    for (int j = j0; j < j1; ++j) {
+        const double4 pj = at[j];
+        const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+        const double s2 = (dx * dx + dy * dy + dz * dz) * inv_d2;
+        const double e = 1.0 - s2, na = -4.0 * s2, nq = na * e;
+        const double C1 = fma(-2.0, s2, 1.0);
+        const double c1q = C1 * C1;
+        const double c2 = c1q + nq;
+        const double c4 = fma(c2, c2, 4.0 * nq * c1q);
+        const double w4 = 4.0 * C1 * c2;
+        double c8 = fma(c4, c4, nq * w4 * w4);
+        double u8 = 2.0 * w4 * c4;
+        double vx[4], vy[4];
+        vy[0] = -2.0 * s2;
+        vx[0] = 1.0 + C1;
+        vy[1] = fma(na, C1, vy[0]);
+        const double C2 = C1 + vy[1];
+        vx[1] = C1 + C2;
+        vy[2] = fma(na, C2, vy[1]);
+        const double C3 = C2 + vy[2];
+        vx[2] = C2 + C3;
+        vy[3] = fma(na, C3, vy[2]);
+        vx[3] = C3 + (C3 + vy[3]);
+        const bool valid = ivalid && j > i;
+        const double c13 = C1 + C3;
+        double X = fma(2.0, c13 - C2, -1.0), Y = fma(2.0, c13 + C2, 1.0);
+        const double ts = 2.0 * s2, te = 2.0 * e;
+        const double t1 = ts * u8, t2 = te * u8, cc = c8;
+        if (rep > 0) {
+            for (int k = 0; k < dbl; ++k) {
+                const double uu = u8 * u8;
+                u8 = 2.0 * c8 * u8;
+                c8 = fma(c8, c8, nq * uu);
+            }
+            const double T1 = ts * u8, T2 = te * u8;
+            for (int k = 0; k < rep; ++k) {
+                const double x = fma(X, c8, -(Y * T1));
+                Y = fma(Y, c8, X * T2);
+                X = x;
+            }
+        }
+        X = valid ? X : 0.0;
+        Y = valid ? Y : 0.0;
+#pragma unroll
+        for (int jj = 0; jj < KM / 8; ++jj) {
+            if (jj >= nj) break;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                if constexpr (WEIGHTED) {
+                    const double px = X * vx[t], py = Y * vy[t];
+                    acc[8 * jj + 2 * t] += px;
+                    acc[8 * jj + 2 * t + 1] += py;
+                    accw[8 * jj + 2 * t] = fma(pj.w, px, accw[8 * jj + 2 * t]);
+                    accw[8 * jj + 2 * t + 1] = fma(pj.w, py, accw[8 * jj + 2 * t + 1]);
+                } else {
+                    acc[8 * jj + 2 * t] = fma(X, vx[t], acc[8 * jj + 2 * t]);
+                    acc[8 * jj + 2 * t + 1] = fma(Y, vy[t], acc[8 * jj + 2 * t + 1]);
+                }
+            }
+            const double x = fma(X, cc, -(Y * t1));
+            Y = fma(Y, cc, X * t2);
+            X = x;
+        }
+    }
+}
+
 }  // namespace pd

@@ -159,6 +159,7 @@ Tuning fit_tuning(int precision, int mode, Tuning t) {
     // pair per pass.
     if (precision == PD_FP64) {
         t.NP = 1;
+        if (mode == PD_MODE_WEIGHTED && t.K > 32) t.K = 32;
     } else if (!valid_shape(precision, mode, t.K, t.NP)) {
         if (mode == PD_MODE_WEIGHTED) {
             t.K = t.K > 32 ? 64 : 32;
@@ -173,7 +174,8 @@ Tuning fit_tuning(int precision, int mode, Tuning t) {
 Tuning default_tuning(int64_t n_atoms, int64_t nq, int precision, int64_t n_frames) {
     Tuning t;
     if (precision == PD_FP64) {
-        t.K = 32;
+        // K = 64 holds the moments of q_max·d up to 85 in one block
+        t.K = nq > 32 ? 64 : 32;
         t.NP = 1;
         t.TJ = std::clamp(next_pow2(n_atoms / 16), 256, 4096);
         return t;
@@ -584,15 +586,16 @@ void set_reduction(Plan &P) {
     m.qmax = P.qmax;
     m.nqb = P.nqb;
     m.fp64 = P.precision == PD_FP64 ? 1 : 0;
-    if (P.precision == PD_FP32_FP64RED && P.mode == PD_MODE_CLASS) {
-        m.block = pd_moment_block(P.tun.K);
-        // Lane operations per pair: 1.5 per moment and about 42 for the
-        // sequences, against 3 per grid point and 55 for each q-block's seeds.
-        m.max_moments = static_cast<int32_t>(
-            std::min<int64_t>({PD_MAX_MOMENTS, static_cast<int64_t>(P.nqb) * m.block,
-                               2 * static_cast<int64_t>(P.nq) + 8 * P.nqb}) & ~int64_t{7});
-        if (m.max_moments < 8) m.block = 0;
-    }
+    m.block = pd_moment_block(P.tun.K);
+    // FP32 lane operations per pair: 1.5 per moment and about 42 for the
+    // sequences, against 3 per grid point and 55 for each q-block's seeds (weighted
+    // mode: 2.5 against 4); so up to two moments per grid point are cheaper.
+    // FP64: a grid point costs a double sin, some 25 moments' worth.
+    const int64_t per_q = m.fp64 ? 16 : 2;
+    m.max_moments = static_cast<int32_t>(
+        std::min<int64_t>({PD_MAX_MOMENTS, static_cast<int64_t>(P.nqb) * m.block,
+                           per_q * P.nq + 8 * P.nqb}) & ~int64_t{7});
+    if (m.max_moments < 8) m.block = 0;
     PdReduceShape &r = P.red;
     r = PdReduceShape{};
     r.n_pairs = P.n_pairs;

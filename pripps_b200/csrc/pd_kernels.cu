@@ -727,6 +727,13 @@ __device__ __forceinline__ void pairs_range_x2w(const float4 *__restrict__ at, i
 #ifndef PD_JFLUSH
 #define PD_JFLUSH 512
 #endif
+// The same for the moments: their low orders are sums of nearly equal terms at
+// every grid point, so the rounding of long runs shows at the deep minima of a
+// profile (10,000 atoms, 512 pairs: 3.0e-5 of the minimum; 128 pairs: 9.5e-6, for
+// 3 % of the pair kernel's time).
+#ifndef PD_MOM_FLUSH
+#define PD_MOM_FLUSH 128
+#endif
 // j atoms per bulk copy into shared memory (two buffers of PD_JSTAGE float4,
 // 64 KB of dynamic shared memory per CTA); a multiple of PD_JFLUSH. One CTA
 // barrier per stage releases the buffer for the next copy.
@@ -734,7 +741,8 @@ __device__ __forceinline__ void pairs_range_x2w(const float4 *__restrict__ at, i
 #define PD_JSTAGE_ATOMS 2048
 #endif
 constexpr int PD_JSTAGE = PD_JSTAGE_ATOMS;
-static_assert(PD_JSTAGE % PD_JFLUSH == 0, "stage must hold whole sub-chunks");
+static_assert(PD_JSTAGE % PD_JFLUSH == 0 && PD_JSTAGE % PD_MOM_FLUSH == 0,
+              "stage must hold whole sub-chunks");
 constexpr size_t PD_FP32_DYN_SMEM = 2 * PD_JSTAGE * sizeof(float4);
 
 // Resident CTAs per SM each FP32 shape is compiled for (register budget
@@ -956,8 +964,9 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
             // below: no branch around the steps.
             const float4 *chunk = s_atoms[b];
             {
-                for (int js = jss; js < jse; js += PD_JFLUSH) {
-                    const int je = min(jse, js + PD_JFLUSH);
+                const int run = moments ? PD_MOM_FLUSH : PD_JFLUSH;
+                for (int js = jss; js < jse; js += run) {
+                    const int je = min(jse, js + run);
                     const bool first = js == tj0;
                     if (moments) {
                         constexpr int KM = pd_moment_block(K);
@@ -968,15 +977,16 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
 #pragma unroll
                         for (int t = 0; t < KM / 2; ++t) acc0[t] = make_float2(0.0f, 0.0f);
                         if constexpr (MODE == PD_MODE_CLASS) {
-                            moments_range<KM>(chunk, jss, pi, i, ivalid, js, je, inv_d2, nj, mblk,
-                                              DBL, acc0);
+                            float2 none[1];
+                            moments_range<KM, false>(chunk, jss, pi, i, ivalid, js, je, inv_d2, nj,
+                                                     mblk, DBL, acc0, none);
                             flush_class<KM / 2>(acc0, part, lane, first);
                         } else {
                             float2 acc1[KM / 2];
 #pragma unroll
                             for (int t = 0; t < KM / 2; ++t) acc1[t] = make_float2(0.0f, 0.0f);
-                            moments_range_w<KM>(chunk, jss, pi, i, ivalid, js, je, inv_d2, nj,
-                                                mblk, DBL, acc0, acc1);
+                            moments_range<KM, true>(chunk, jss, pi, i, ivalid, js, je, inv_d2, nj,
+                                                    mblk, DBL, acc0, acc1);
                             const float wi = ivalid ? pi.w : 0.0f;
                             flush_weighted<KM>(acc0, wi, part, K, lane, first);
                             flush_weighted<KM>(acc1, wi, part + 2 * K, K, lane, first);
@@ -1315,8 +1325,11 @@ __global__ void __launch_bounds__(PD_PACK_THREADS)
     PdFrameDev fr{};
     fr.radius = sqrt(__longlong_as_double(
         static_cast<long long>(atomicMax(&rad2[f], 0ull))));
+    // d follows the FP32 value of 1/d² that the pairs are scaled with: rounding
+    // 1/d² alone would stretch every distance by the same 1 + 3e-8
     fr.d = fmax(2.0 * PD_MOM_STRETCH * fr.radius, 1e-6);
-    fr.inv_d2 = 1.0 / (fr.d * fr.d);
+    fr.inv_d2 = static_cast<double>(static_cast<float>(1.0 / (fr.d * fr.d)));
+    fr.d = 1.0 / sqrt(fr.inv_d2);
     if (rule.block > 0) {
         const int m8 = (moments_needed(rule.qmax * fr.d, rule.fp64 != 0) + 7) & ~7;
         const int blocks = (m8 + rule.block - 1) / rule.block;
@@ -1529,9 +1542,11 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
         // hi = 8j + 4 + t
         for (int j = g; j < M / 8; j += PD_PROF_GROUPS) {
             double c[8];
+            // the tiles' sums carry the signs + + − − of their group within the block
+            const double sg = (j % (sh.block / 8)) & 2 ? -0.5 : 0.5;
 #pragma unroll
             for (int n = 0; n < 8; ++n)
-                c[n] = 0.5 * s_scale[ql] * s_coef[(8 * j + n) * PD_PROF_Q + ql];
+                c[n] = sg * s_scale[ql] * s_coef[(8 * j + n) * PD_PROF_Q + ql];
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 s_coef[(8 * j + 2 * t) * PD_PROF_Q + ql] = c[3 - t] + c[4 + t];

@@ -49,170 +49,114 @@ __device__ __forceinline__ int moments_needed(double z, bool fp64) {
 // determines φ poorly, at the price of 3 % more moments.
 constexpr double PD_MOM_STRETCH = 1.03;
 
-// A pair's sequences: X = cos(cφ)/cos(φ/2), Y = sin(cφ)/sin(φ/2) at the first c
-// of the block; (c8, t1, t2) turn (X, Y) by 8φ: X' = X·c8 − Y·t1,
-// Y' = Y·c8 + X·t2; vx[t] = 2cos((t+½)φ)cos(φ/2), vy[t] = −2sin((t+½)φ)sin(φ/2).
-// Then X·vx = m_{c+b} + m_{c−b} and Y·vy = m_{c+b} − m_{c−b}.
-struct MomPair2 {  // two pairs, one in each half
-    float2 X, Y, c8, t1, t2, vx[4], vy[4];
+// A pair's sequences. U_j = (cos(cφ)/cos(φ/2), sin(cφ)/sin(φ/2)) at c = 8j + 3.5
+// follows the three-term recurrence U_{j+1} = 2cos(8φ)·U_j − U_{j−1}. It is kept
+// as W_j = s_j·U_j with the signs s = + + − − + + − − …, which turns every step into one
+// multiply-add, W_{j+1} = ±2cos(8φ)·W_j + W_{j−1} (+ for even j): no negation, no
+// half swapped, the older of the two registers overwritten. V_t = (2cos((t+½)φ)cos(φ/2),
+// −2sin((t+½)φ)sin(φ/2)), so that U.x·V.x = m_{c+b} + m_{c−b}, U.y·V.y =
+// m_{c+b} − m_{c−b}.
+struct MomPair {
+    float2 w0, w1;  // W at the first two j of the block
+    float cc;       // 2cos(8φ)
+    float2 v[4];
 };
 
-__device__ __forceinline__ float2 mom_f2(float a) { return make_float2(a, a); }
-
-// `turns` = 8-fold blocks before this one (moment block × groups per block); a
-// later block starts from X, Y turned by 8·turns·φ: the turn by 8φ is doubled
-// `dbl` times and applied `rep` times, turns = rep·2^dbl.
-__device__ __forceinline__ void mom_seed_x2(float2 r2, float inv_d2, int rep, int dbl,
-                                            MomPair2 &P) {
-    const float2 one = mom_f2(1.0f), two = mom_f2(2.0f), M1 = mom_f2(-1.0f), M2 = mom_f2(-2.0f);
-    const float2 s2 = __fmul2_rn(r2, mom_f2(inv_d2));
-    const float2 e = __ffma2_rn(s2, M1, one);   // cos²(φ/2)
-    const float2 c1 = __ffma2_rn(s2, M2, one);  // cos φ
-    const float2 na = __fmul2_rn(s2, mom_f2(-4.0f));
-    const float2 nq = __fmul2_rn(na, e);        // −sin²φ
-    // doublings of φ with sin(nφ) = u_n·sin φ
-    const float2 c1q = __fmul2_rn(c1, c1);
-    const float2 c2 = __fadd2_rn(c1q, nq);
-    const float2 c4 = __ffma2_rn(c2, c2, __fmul2_rn(__fmul2_rn(mom_f2(4.0f), nq), c1q));
-    const float2 w = __fmul2_rn(c1, c2);        // u_4/4
-    const float2 w4 = __fmul2_rn(mom_f2(4.0f), w);
-    float2 c8 = __ffma2_rn(c4, c4, __fmul2_rn(__fmul2_rn(nq, w4), w4));
-    float2 u8 = __fmul2_rn(__fmul2_rn(two, w4), c4);
-    // cos tφ by Reinsch differences d_{t+1} = d_t − α cos tφ
-    float2 d = __fmul2_rn(s2, M2);
-    const float2 C1 = c1;
-    P.vy[0] = d;
-    P.vx[0] = __fadd2_rn(one, C1);
-    d = __ffma2_rn(na, C1, d);
-    const float2 C2 = __fadd2_rn(C1, d);
-    P.vy[1] = d;
-    P.vx[1] = __fadd2_rn(C1, C2);
-    d = __ffma2_rn(na, C2, d);
-    const float2 C3 = __fadd2_rn(C2, d);
-    P.vy[2] = d;
-    P.vx[2] = __fadd2_rn(C2, C3);
-    d = __ffma2_rn(na, C3, d);
-    const float2 C4 = __fadd2_rn(C3, d);
-    P.vy[3] = d;
-    P.vx[3] = __fadd2_rn(C3, C4);
-    // c = 3.5: cos(3.5φ)/cos(φ/2) and sin(3.5φ)/sin(φ/2)
-    const float2 c13 = __fadd2_rn(C1, C3);
-    P.X = __ffma2_rn(two, __ffma2_rn(C2, M1, c13), M1);
-    P.Y = __ffma2_rn(two, __fadd2_rn(c13, C2), one);
-    const float2 ts = __fmul2_rn(two, s2), te = __fmul2_rn(two, e);
-    P.c8 = c8;
-    P.t1 = __fmul2_rn(ts, u8);
-    P.t2 = __fmul2_rn(te, u8);
-    if (rep > 0) {
-        for (int k = 0; k < dbl; ++k) {
-            const float2 uu = __fmul2_rn(u8, u8);
-            u8 = __fmul2_rn(__fmul2_rn(two, c8), u8);
-            c8 = __ffma2_rn(c8, c8, __fmul2_rn(nq, uu));
-        }
-        const float2 T1 = __fmul2_rn(ts, u8), T2 = __fmul2_rn(te, u8);
-        for (int k = 0; k < rep; ++k) {
-            const float2 x = __ffma2_rn(P.X, c8, __fmul2_rn(__fmul2_rn(P.Y, T1), M1));
-            P.Y = __ffma2_rn(P.Y, c8, __fmul2_rn(P.X, T2));
-            P.X = x;
-        }
+// U at the first c of a later moment block: turned by the angle of `rep` blocks,
+// 8·2^dbl·φ each. (xx, yy) → turned, from sin(nφ) = u_n sin φ and cos(nφ) = c_n at n = 8.
+__device__ __forceinline__ void mom_later_block(float c8, float u8, float nq, float ts, float te,
+                                                int rep, int dbl, float &X, float &Y) {
+    for (int k = 0; k < dbl; ++k) {
+        const float uu = u8 * u8;
+        u8 = 2.0f * c8 * u8;
+        c8 = fmaf(c8, c8, nq * uu);
+    }
+    const float T1 = ts * u8, T2 = te * u8;
+    for (int k = 0; k < rep; ++k) {
+        const float x = fmaf(X, c8, -(Y * T1));
+        Y = fmaf(Y, c8, X * T2);
+        X = x;
     }
 }
 
+// Scalar operations throughout: they cost the FP32 pipe the same lane slots as
+// packed ones over two pairs would, and write the halves of the packed operands in place
+// (packed over two pairs, the transposition was 90 register moves per pair:
+// 20,000 atoms, 72 moments: 2.05 ms, FMA pipe 41 % and ALU pipe 48 % busy).
+__device__ __forceinline__ void mom_seed(float r2, float inv_d2, int rep, int dbl, bool valid,
+                                         MomPair &P) {
+    const float s2 = r2 * inv_d2;          // sin²(φ/2)
+    const float e = 1.0f - s2;             // cos²(φ/2)
+    const float na = -4.0f * s2;           // −α
+    const float nq = na * e;               // −sin²φ
+    const float d1 = -2.0f * s2;
+    const float C1 = 1.0f + d1;            // cos φ
+    // cos(nφ), u_n = sin(nφ)/sin φ for n = 2, 4, 8
+    const float c1q = C1 * C1;
+    const float c2 = c1q + nq;
+    const float c4 = fmaf(c2, c2, 4.0f * nq * c1q);
+    const float w4 = 4.0f * (C1 * c2);
+    const float c8 = fmaf(c4, c4, nq * w4 * w4);
+    const float u8 = 2.0f * (w4 * c4);
+    // cos tφ by Reinsch differences d_{t+1} = d_t − α cos tφ
+    const float d2 = fmaf(na, C1, d1), C2 = C1 + d2;
+    const float d3 = fmaf(na, C2, d2), C3 = C2 + d3;
+    const float d4 = fmaf(na, C3, d3);
+    P.v[0] = make_float2(1.0f + C1, d1);
+    P.v[1] = make_float2(C1 + C2, d2);
+    P.v[2] = make_float2(C2 + C3, d3);
+    P.v[3] = make_float2(C3 + (C3 + d4), d4);
+    // c = 3.5: cos(3.5φ)/cos(φ/2) and sin(3.5φ)/sin(φ/2)
+    const float c13 = C1 + C3;
+    float X = fmaf(2.0f, c13 - C2, -1.0f), Y = fmaf(2.0f, c13 + C2, 1.0f);
+    const float ts = s2 + s2, te = e + e;
+    if (rep > 0) mom_later_block(c8, u8, nq, ts, te, rep, dbl, X, Y);
+    X = valid ? X : 0.0f;
+    Y = valid ? Y : 0.0f;
+    P.w0 = make_float2(X, Y);
+    P.w1 = make_float2(fmaf(X, c8, -(Y * (ts * u8))), fmaf(Y, c8, X * (te * u8)));
+    P.cc = c8 + c8;
+}
+
 // Moments of the pairs (i, j), j0 <= j < j1, j > i, of one thread's i into
-// acc[4·jj + t] = (Σ X·vx, Σ Y·vy), for the first nj groups of eight of the block.
-// `at` holds the atoms [jbase, ...) in shared memory.
-template <int KM>
+// acc[4·jj + t] = s_jj·(Σ U.x·V.x, Σ U.y·V.y), for the first nj groups of eight of
+// the block. `at` holds the atoms [jbase, ...) in shared memory. Weighted mode
+// (WEIGHTED): the sums weighted by the j atom's w in accw as well.
+template <int KM, bool WEIGHTED>
 __device__ __forceinline__ void moments_range(const float4 *__restrict__ at, int jbase, float4 pi,
                                               int i, bool ivalid, int j0, int j1, float inv_d2,
-                                              int nj, int rep, int dbl, float2 (&acc)[KM / 2]) {
-    const float2 M1 = mom_f2(-1.0f);
-    for (int j = j0; j < j1; j += 2) {
-        const bool inb = j + 1 < j1;
-        const float4 pa = at[j - jbase], pb = at[(inb ? j + 1 : j) - jbase];
-        const float2 dx = __ffma2_rn(make_float2(pa.x, pb.x), M1, mom_f2(pi.x));
-        const float2 dy = __ffma2_rn(make_float2(pa.y, pb.y), M1, mom_f2(pi.y));
-        const float2 dz = __ffma2_rn(make_float2(pa.z, pb.z), M1, mom_f2(pi.z));
-        const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-        MomPair2 P;
-        mom_seed_x2(r2, inv_d2, rep, dbl, P);
-        const bool va = ivalid && j > i, vb = ivalid && inb && j + 1 > i;
-        float2 Ua = make_float2(va ? P.X.x : 0.0f, va ? P.Y.x : 0.0f);
-        float2 Ub = make_float2(vb ? P.X.y : 0.0f, vb ? P.Y.y : 0.0f);
-        float2 Va[4], Vb[4];
+                                              int nj, int rep, int dbl, float2 (&acc)[KM / 2],
+                                              float2 (&accw)[WEIGHTED ? KM / 2 : 1]) {
+    for (int j = j0; j < j1; ++j) {
+        const float4 pj = at[j - jbase];
+        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        MomPair P;
+        mom_seed(r2, inv_d2, rep, dbl, ivalid && j > i, P);
+        const float2 cp = make_float2(P.cc, P.cc), cn = make_float2(-P.cc, -P.cc);
+        float2 W[2] = {P.w0, P.w1};
+        float2 WV[WEIGHTED ? 4 : 1];
+        if constexpr (WEIGHTED)
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
-            Va[t] = make_float2(P.vx[t].x, P.vy[t].x);
-            Vb[t] = make_float2(P.vx[t].y, P.vy[t].y);
-        }
+            for (int t = 0; t < 4; ++t) WV[t] = __fmul2_rn(make_float2(pj.w, pj.w), P.v[t]);
 #pragma unroll
         for (int jj = 0; jj < KM / 8; ++jj) {
             if (jj >= nj) break;
 #pragma unroll
-            for (int t = 0; t < 4; ++t) acc[4 * jj + t] = __ffma2_rn(Ua, Va[t], acc[4 * jj + t]);
-#pragma unroll
-            for (int t = 0; t < 4; ++t) acc[4 * jj + t] = __ffma2_rn(Ub, Vb[t], acc[4 * jj + t]);
-            if (jj + 1 < KM / 8) {
-                const float xa = fmaf(Ua.x, P.c8.x, -(Ua.y * P.t1.x));
-                Ua.y = fmaf(Ua.y, P.c8.x, Ua.x * P.t2.x);
-                Ua.x = xa;
-                const float xb = fmaf(Ub.x, P.c8.y, -(Ub.y * P.t1.y));
-                Ub.y = fmaf(Ub.y, P.c8.y, Ub.x * P.t2.y);
-                Ub.x = xb;
-            }
-        }
-    }
-}
-
-// Weighted mode: the same moments in acc0, and weighted by the j atom's
-// hydration weight in acc1 (16 lane operations per eight moments and the turn's 4).
-template <int KM>
-__device__ __forceinline__ void moments_range_w(const float4 *__restrict__ at, int jbase,
-                                                float4 pi, int i, bool ivalid, int j0, int j1,
-                                                float inv_d2, int nj, int rep, int dbl,
-                                                float2 (&acc0)[KM / 2], float2 (&acc1)[KM / 2]) {
-    const float2 M1 = mom_f2(-1.0f);
-    for (int j = j0; j < j1; j += 2) {
-        const bool inb = j + 1 < j1;
-        const float4 pa = at[j - jbase], pb = at[(inb ? j + 1 : j) - jbase];
-        const float2 dx = __ffma2_rn(make_float2(pa.x, pb.x), M1, mom_f2(pi.x));
-        const float2 dy = __ffma2_rn(make_float2(pa.y, pb.y), M1, mom_f2(pi.y));
-        const float2 dz = __ffma2_rn(make_float2(pa.z, pb.z), M1, mom_f2(pi.z));
-        const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-        MomPair2 P;
-        mom_seed_x2(r2, inv_d2, rep, dbl, P);
-        const bool va = ivalid && j > i, vb = ivalid && inb && j + 1 > i;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const bool v = h ? vb : va;
-            const float w = h ? pb.w : pa.w;
-            float2 U = h ? make_float2(P.X.y, P.Y.y) : make_float2(P.X.x, P.Y.x);
-            U = make_float2(v ? U.x : 0.0f, v ? U.y : 0.0f);
-            const float c8 = h ? P.c8.y : P.c8.x, t1 = h ? P.t1.y : P.t1.x,
-                        t2 = h ? P.t2.y : P.t2.x;
-            float2 V[4], WV[4];
-#pragma unroll
             for (int t = 0; t < 4; ++t) {
-                V[t] = h ? make_float2(P.vx[t].y, P.vy[t].y) : make_float2(P.vx[t].x, P.vy[t].x);
-                WV[t] = __fmul2_rn(mom_f2(w), V[t]);
+                acc[4 * jj + t] = __ffma2_rn(W[jj & 1], P.v[t], acc[4 * jj + t]);
+                if constexpr (WEIGHTED)
+                    accw[4 * jj + t] = __ffma2_rn(W[jj & 1], WV[t], accw[4 * jj + t]);
             }
-#pragma unroll
-            for (int jj = 0; jj < KM / 8; ++jj) {
-                if (jj >= nj) break;
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    acc0[4 * jj + t] = __ffma2_rn(U, V[t], acc0[4 * jj + t]);
-                    acc1[4 * jj + t] = __ffma2_rn(U, WV[t], acc1[4 * jj + t]);
-                }
-                const float x = fmaf(U.x, c8, -(U.y * t1));
-                U.y = fmaf(U.y, c8, U.x * t2);
-                U.x = x;
-            }
+            // W_{jj+2} = ±2cos(8φ)·W_{jj+1} + W_jj
+            if (jj + 2 < KM / 8)
+                W[jj & 1] = __ffma2_rn((jj & 1) ? cp : cn, W[(jj & 1) ^ 1], W[jj & 1]);
         }
     }
 }
 
-// FP64 form: the same sequences in double, one pair at a time;
-// acc[8·jj + 2t + {0, 1}] = Σ X·vx, Σ Y·vy (and weighted by w_j in accw).
+// FP64 form: the same sequences in double;
+// acc[8·jj + 2t + {0, 1}] = s_jj·(Σ U.x·V.x, Σ U.y·V.y) (and weighted by w_j in accw).
 template <int KM, bool WEIGHTED>
 __device__ __forceinline__ void moments_range_f64(const double4 *__restrict__ at, double4 pi, int i,
                                                   bool ivalid, int j0, int j1, double inv_d2,
@@ -259,27 +203,34 @@ __device__ __forceinline__ void moments_range_f64(const double4 *__restrict__ at
                 X = x;
             }
         }
-        X = valid ? X : 0.0;
-        Y = valid ? Y : 0.0;
+        double WX[2], WY[2];
+        WX[0] = valid ? X : 0.0;
+        WY[0] = valid ? Y : 0.0;
+        WX[1] = fma(WX[0], cc, -(WY[0] * t1));
+        WY[1] = fma(WY[0], cc, WX[0] * t2);
+        const double c2x = 2.0 * cc;
 #pragma unroll
         for (int jj = 0; jj < KM / 8; ++jj) {
             if (jj >= nj) break;
+            const double wx = WX[jj & 1], wy = WY[jj & 1];
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 if constexpr (WEIGHTED) {
-                    const double px = X * vx[t], py = Y * vy[t];
+                    const double px = wx * vx[t], py = wy * vy[t];
                     acc[8 * jj + 2 * t] += px;
                     acc[8 * jj + 2 * t + 1] += py;
                     accw[8 * jj + 2 * t] = fma(pj.w, px, accw[8 * jj + 2 * t]);
                     accw[8 * jj + 2 * t + 1] = fma(pj.w, py, accw[8 * jj + 2 * t + 1]);
                 } else {
-                    acc[8 * jj + 2 * t] = fma(X, vx[t], acc[8 * jj + 2 * t]);
-                    acc[8 * jj + 2 * t + 1] = fma(Y, vy[t], acc[8 * jj + 2 * t + 1]);
+                    acc[8 * jj + 2 * t] = fma(wx, vx[t], acc[8 * jj + 2 * t]);
+                    acc[8 * jj + 2 * t + 1] = fma(wy, vy[t], acc[8 * jj + 2 * t + 1]);
                 }
             }
-            const double x = fma(X, cc, -(Y * t1));
-            Y = fma(Y, cc, X * t2);
-            X = x;
+            if (jj + 2 < KM / 8) {
+                const double sc = (jj & 1) ? c2x : -c2x;
+                WX[jj & 1] = fma(sc, WX[(jj & 1) ^ 1], wx);
+                WY[jj & 1] = fma(sc, WY[(jj & 1) ^ 1], wy);
+            }
         }
     }
 }

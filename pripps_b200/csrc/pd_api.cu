@@ -64,15 +64,16 @@ struct NvtxRange {
 // copy; the rest is device-only scratch.
 struct Layout {
     uint64_t qv, ffA, ffC, ffW, hw, fw, cls, pairs, perm, gvalid, jobs, lptr, lidx, req, njobs,
-        xyz, lat, lat_tiles;
+        xyz, lat, lat_tiles, chunks, cls_ptr, cls_chunk;
     uint64_t upload_bytes;
     uint64_t hres;         // host-only: pinned landing area of the [6][nq] result
     uint64_t stage_bytes;  // pinned image size (upload + result area)
     uint64_t centroid, cent_part, frames, atoms, slots, red, chunk_sums, terms, out;
     uint64_t status;  // int32 device status of the pair kernel, right after out
     // counters and maxima that every execution starts from zero (one memset)
-    uint64_t ctl, counter, cent_done, pack_done, rad2, red_done, ctl_bytes;
+    uint64_t ctl, counter, cent_done, pack_done, rad2, red_done, dir_done, ctl_bytes;
     uint64_t lat_sums;
+    uint64_t dirs, dir_part;  // direction form: table, the groups' averages
     uint64_t lat_idx, hist, lat_err;  // lattice sets: coordinates, pair counts, error flag
     uint64_t total;
 };
@@ -104,6 +105,9 @@ Layout make_layout(const Plan &P, bool host_xyz) {
     L.xyz = take(host_xyz ? static_cast<uint64_t>(P.n_atoms) * 3 * P.n_frames * 8 : 0);
     L.lat = take(P.lat.size() * sizeof(PdLatDev));
     L.lat_tiles = take(P.lat_tiles.size() * sizeof(PdLatTile));
+    L.chunks = take(P.chunks.size() * sizeof(PdChunk));
+    L.cls_ptr = take(P.cls_ptr.size() * 4);
+    L.cls_chunk = take(P.cls_chunk.size() * 4);
     L.upload_bytes = o;
     L.hres = o;
     L.stage_bytes = align_up(o + 6 * nq * 8 + 8, 256);  // result and status land here
@@ -113,7 +117,9 @@ Layout make_layout(const Plan &P, bool host_xyz) {
     L.frames = take(F * sizeof(PdFrameDev));
     L.atoms = take(static_cast<uint64_t>(P.n_pad) * P.n_frames *
                    (P.precision == PD_FP64 ? sizeof(double4) : sizeof(float4)));
-    L.slots = take(static_cast<uint64_t>(P.slots_per_frame) * P.n_frames * P.nv * P.tun.K * 8);
+    // one region for the tiles' slots or the direction form's chunk sums
+    L.slots = take(std::max(static_cast<uint64_t>(P.slots_per_frame) * P.nv * P.tun.K,
+                            static_cast<uint64_t>(P.amp.slot_cap)) * F * 8);
     const PdReduceShape &sh = P.red;
     const uint64_t red_rows = F * static_cast<uint64_t>(P.n_pairs);
     L.red = take(red_rows * P.nv * sh.width * 8);
@@ -128,7 +134,13 @@ Layout make_layout(const Plan &P, bool host_xyz) {
     L.cent_done = take(F * 4);
     L.pack_done = take(F * 4);
     L.red_done = take(sh.n_chunk > 1 ? red_rows * sh.n_z * 4 : 0);
+    const uint64_t n_nt =
+        P.amp.dir_cap ? (P.amp.node_cap + P.amp.node_tile - 1) / P.amp.node_tile : 0;
+    L.dir_done = take(F * n_nt * 4);
     L.ctl_bytes = o - L.ctl;
+    L.dirs = take(F * P.amp.dir_cap * sizeof(double4));
+    L.dir_part = take(F * P.amp.grp_cap * static_cast<uint64_t>(P.n_pairs) * P.nv *
+                      P.amp.node_cap * 8);
     L.lat_sums = take(P.lat.size() * nq * 8);
     L.lat_idx = take(P.lat.empty() ? 0 : static_cast<uint64_t>(P.n_pad) * sizeof(int4));
     L.hist = take(static_cast<uint64_t>(P.lat_bins) * 8);
@@ -435,6 +447,9 @@ void stage_structure(DevPlan &dp) {
         std::memcpy(dp.hptr<char>(L.lat_tiles), P.lat_tiles.data(),
                     P.lat_tiles.size() * sizeof(PdLatTile));
     }
+    std::memcpy(dp.hptr<char>(L.chunks), P.chunks.data(), P.chunks.size() * sizeof(PdChunk));
+    std::memcpy(dp.hptr<char>(L.cls_ptr), P.cls_ptr.data(), P.cls_ptr.size() * 4);
+    std::memcpy(dp.hptr<char>(L.cls_chunk), P.cls_chunk.data(), P.cls_chunk.size() * 4);
     PdReqDev rd{};
     if (P.precision == PD_FP64)
         rd.atoms64 = dp.dptr<double4>(L.atoms);
@@ -444,6 +459,9 @@ void stage_structure(DevPlan &dp) {
     rd.qv = dp.dptr<double>(L.qv);
     rd.slots = dp.dptr<double>(L.slots);
     rd.frames = dp.dptr<PdFrameDev>(L.frames);
+    rd.dirs = dp.dptr<double4>(L.dirs);
+    rd.chunks = dp.dptr<PdChunk>(L.chunks);
+    rd.amp = P.amp;
     rd.status = dp.dptr<int32_t>(L.status);
     rd.flags = P.test_expire ? PD_REQF_TEST_EXPIRE : 0;
     rd.qmin = P.qmin;
@@ -457,21 +475,31 @@ void stage_structure(DevPlan &dp) {
     std::memcpy(dp.hptr<char>(L.njobs), &nj, sizeof(int));
 }
 
+// Radius hint of a validated request with host coordinates.
+double host_radius(const pd_request *req) {
+    return pd::max_radius(req->xyz, static_cast<int64_t>(req->n_atoms),
+                          static_cast<int64_t>(req->n_frames ? req->n_frames : 1));
+}
+
 constexpr int kBudgetWait = -100;  // internal: does not fit the budget right now
 
 // Host planning only: tiles, lists and the device layout.
 int plan_host(pd_ctx *ctx, const pd_request *req, const uint32_t *species, const double *weights,
-              bool host_xyz, DevPlan &dp, const Tuning *force = nullptr) {
+              bool host_xyz, double radius_hint, DevPlan &dp, const Tuning *force = nullptr) {
     NvtxRange nvtx("pd plan (host)");
     std::string msg;
     const Tuning tun = force ? *force : tuning_for_request(ctx, req, species, weights);
-    int rc = pd::build_plan(req, species, weights, tun, dp.P, msg);
+    int rc = pd::build_plan(req, species, weights, tun, dp.P, msg, false, radius_hint);
     if (rc != PD_OK) {
         ctx->set_error(msg);
         return rc;
     }
     dp.host_xyz = host_xyz;
     dp.L = make_layout(dp.P, host_xyz);
+    if (dp.L.total > ctx->budget) {  // the pair form alone may fit
+        pd::drop_directions(dp.P);
+        dp.L = make_layout(dp.P, host_xyz);
+    }
     if (dp.L.total > ctx->budget) {
         ctx->set_error("request needs " + std::to_string(dp.L.total) +
                        " device bytes, the budget is " + std::to_string(ctx->budget));
@@ -520,9 +548,9 @@ int plan_device(pd_ctx *ctx, const pd_request *req, DevPlan &dp, cudaStream_t st
 }
 
 int create_devplan(pd_ctx *ctx, const pd_request *req, const uint32_t *species,
-                   const double *weights, bool host_xyz, DevPlan &dp, cudaStream_t st,
-                   const Tuning *force = nullptr) {
-    int rc = plan_host(ctx, req, species, weights, host_xyz, dp, force);
+                   const double *weights, bool host_xyz, double radius_hint, DevPlan &dp,
+                   cudaStream_t st, const Tuning *force = nullptr) {
+    int rc = plan_host(ctx, req, species, weights, host_xyz, radius_hint, dp, force);
     if (rc) return rc;
     return plan_device(ctx, req, dp, st, false);
 }
@@ -540,12 +568,22 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st) {
                                    P.nv, P.n_frames, P.precision == PD_FP32_FP64RED ? 1 : 0,
                                    add_exact, dp.dptr<double>(L.chunk_sums),
                                    dp.dptr<unsigned int>(L.red_done), dp.dptr<double>(L.red), st));
+    if (P.amp.dir_cap > 0) {
+        PD_CUDA(ctx, pd::launch_direction_sums(
+                         dp.dptr<double>(L.slots), dp.dptr<double4>(L.dirs),
+                         dp.dptr<PdFrameDev>(L.frames), P.amp, P.qmax, P.n_frames,
+                         dp.dptr<PdClassDev>(L.cls), dp.dptr<PdPairDev>(L.pairs), P.n_pairs,
+                         dp.dptr<int32_t>(L.cls_ptr), dp.dptr<int32_t>(L.cls_chunk), P.red.width,
+                         add_exact, dp.dptr<double>(L.dir_part),
+                         dp.dptr<unsigned int>(L.dir_done), dp.dptr<double>(L.red), st));
+        ctx->launches += 1;
+    }
     if (!P.lat.empty()) {
         PD_CUDA(ctx, pd::launch_lattice_sums(
                          reinterpret_cast<const unsigned long long *>(dp.dptr<char>(L.hist)),
                          dp.dptr<PdLatDev>(L.lat), static_cast<int>(P.lat.size()),
                          dp.dptr<double>(L.qv), P.nq, add_exact, dp.dptr<int>(L.lat_err),
-                         dp.dptr<double>(L.lat_sums), st));
+                         dp.dptr<PdFrameDev>(L.frames), dp.dptr<double>(L.lat_sums), st));
         ctx->launches += 1;
     }
     double *dst = out_dev ? out_dev : dp.dptr<double>(L.out);
@@ -556,6 +594,7 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st) {
                                      dp.dptr<PdFrameDev>(L.frames), dp.dptr<double>(L.ffA),
                                      P.has_exc ? dp.dptr<double>(L.ffC) : nullptr,
                                      P.has_hyd ? dp.dptr<double>(L.ffW) : nullptr, add_exact,
+                                     P.qmax, P.lat.empty() ? nullptr : dp.dptr<int>(L.lat_err),
                                      terms, st));
     ctx->launches += 2;
     if (P.n_frames > 1) {
@@ -585,7 +624,7 @@ int pack_devplan(pd_ctx *ctx, DevPlan &dp, cudaStream_t st) {
                                  P.precision == PD_FP64 ? dp.dptr<double4>(L.atoms) : nullptr,
                                  P.mom, dp.dptr<unsigned long long>(L.rad2),
                                  dp.dptr<unsigned int>(L.pack_done),
-                                 dp.dptr<PdFrameDev>(L.frames), st));
+                                 dp.dptr<PdFrameDev>(L.frames), dp.dptr<double4>(L.dirs), st));
     ctx->launches += 2;
     if (!P.lat.empty()) {
         PD_CUDA(ctx, pd::launch_lattice(dp.xyz_dev, dp.dptr<int32_t>(L.perm),
@@ -595,7 +634,8 @@ int pack_devplan(pd_ctx *ctx, DevPlan &dp, cudaStream_t st) {
                                         static_cast<int64_t>(P.lat_tiles.size()),
                                         dp.dptr<int4>(L.lat_idx),
                                         reinterpret_cast<unsigned long long *>(dp.dptr<char>(L.hist)),
-                                        P.lat_bins, dp.dptr<int>(L.lat_err), st));
+                                        P.lat_bins, dp.dptr<int>(L.lat_err),
+                                        dp.dptr<PdFrameDev>(L.frames), st));
         ctx->launches += P.lat_tiles.empty() ? 1 : 2;
     }
     return PD_OK;
@@ -781,7 +821,8 @@ void planner_main(pd_ctx *ctx) {
         int rc = PD_OK;
         std::string m;
         if (!t->canceled) {
-            rc = plan_host(ctx, &t->req, t->req.species, t->req.hyd_weights, true, t->dp);
+            rc = plan_host(ctx, &t->req, t->req.species, t->req.hyd_weights, true,
+                           host_radius(&t->req), t->dp);
             if (rc != PD_OK) {
                 std::lock_guard<std::mutex> g(ctx->mu);
                 m = ctx->errors[std::this_thread::get_id()];
@@ -1248,6 +1289,7 @@ int pd_ctx_create(int device, uint64_t mem_budget_bytes, pd_ctx **out) {
     cudaMemGetInfo(&free_b, &total_b);
     ctx->budget = mem_budget_bytes ? mem_budget_bytes : static_cast<uint64_t>(free_b * 0.9);
     e = pd::prepare_pair_kernels();
+    if (e == cudaSuccess) e = pd::prepare_direction_rules();
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
         cudaMemPoolProps pp{};
@@ -1343,7 +1385,8 @@ int pd_solve(pd_ctx *ctx, const pd_request *req, double *out_terms) {
     std::lock_guard<std::mutex> g(ctx->solve_mu);
     cudaSetDevice(ctx->device);
     DevPlan dp;
-    rc = create_devplan(ctx, req, req->species, req->hyd_weights, true, dp, ctx->stream);
+    rc = create_devplan(ctx, req, req->species, req->hyd_weights, true, host_radius(req), dp,
+                        ctx->stream);
     if (rc) return rc;
     rc = run_devplan(ctx, dp, nullptr, ctx->stream);
     if (rc == PD_OK) {
@@ -1394,7 +1437,9 @@ int plan_create_impl(pd_ctx *ctx, const pd_request *req, pd_plan **out, const Tu
     std::lock_guard<std::mutex> g(ctx->solve_mu);
     cudaSetDevice(ctx->device);
     auto *p = new pd_plan();
-    rc = create_devplan(ctx, &r, r.species, r.hyd_weights, false, p->dp, ctx->stream, force);
+    // executions bring other frames of the topology: room for a radius 15 % larger
+    const double hint = req->xyz ? 1.15 * host_radius(&r) : -1.0;
+    rc = create_devplan(ctx, &r, r.species, r.hyd_weights, false, hint, p->dp, ctx->stream, force);
     if (rc == PD_OK) {
         cudaError_t e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) rc = cuda_fail(ctx, e, "pd_plan_create");
@@ -2074,6 +2119,7 @@ int pd_request_device_bytes(pd_ctx *ctx, const pd_request *req, int host_coordin
         if (ctx) ctx->set_error(msg);
         return rc;
     }
+    pd::drop_directions(P);
     *device_bytes = make_layout(P, host_coordinates != 0).total;
     return PD_OK;
 }
@@ -2478,7 +2524,7 @@ extern "C" int pd_stream_open(pd_ctx *ctx, const pd_request *req, uint32_t frame
         stream_free(ctx, s);
         return cuda_fail(ctx, e, "pd_stream_open: streams");
     }
-    rc = create_devplan(ctx, &r, r.species, r.hyd_weights, false, s->dp, s->cs);
+    rc = create_devplan(ctx, &r, r.species, r.hyd_weights, false, -1.0, s->dp, s->cs);
     if (rc) {
         stream_free(ctx, s);
         return rc;
@@ -2694,6 +2740,7 @@ NoallocDevice *noalloc_device(int dev, int *rc) {
     nd->ctx->device = dev;
     nd->ctx->sm_count = sms;
     e = pd::prepare_pair_kernels();  // launch attributes, before any capture
+    if (e == cudaSuccess) e = pd::prepare_direction_rules();
     if (e != cudaSuccess) {
         *rc = noalloc_fail(PD_EDEVICE, std::string("pd_solve_noalloc: kernel set-up failed: ") +
                                            cudaGetErrorString(e));
@@ -2718,6 +2765,10 @@ extern "C" int pd_solve_noalloc(const pd_request *req, const double *xyz_dev,
     rc = pd::build_plan(&r, r.species, r.hyd_weights, tun, dp.P, msg);
     if (rc) return noalloc_fail(rc, "pd_solve_noalloc: " + msg);
     dp.L = make_layout(dp.P, false);
+    if (dp.L.total > PD_NOALLOC_SCRATCH_BYTES) {  // the pair form alone may fit
+        pd::drop_directions(dp.P);
+        dp.L = make_layout(dp.P, false);
+    }
     if (dp.L.total > PD_NOALLOC_SCRATCH_BYTES)
         return noalloc_fail(PD_EBUDGET,
                             "pd_solve_noalloc: the request needs " + std::to_string(dp.L.total) +

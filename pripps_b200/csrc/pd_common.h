@@ -52,8 +52,10 @@ struct PdJob {
     // Warps of one class share a slot; slot numbers follow the first warp
     // of each class, so warp 0 always has relative slot 0.
     int64_t slot;
+    int32_t ord;    // ordinal among the frame's jobs (direction form)
+    int32_t n_ord;  // jobs of the frame
 };
-static_assert(sizeof(PdJob) == 32, "PdJob layout");
+static_assert(sizeof(PdJob) == 40, "PdJob layout");
 constexpr int PD_SLOT_MAP_SHIFT = 48;
 constexpr int64_t PD_SLOT_MASK = (int64_t{1} << PD_SLOT_MAP_SHIFT) - 1;
 
@@ -64,21 +66,39 @@ constexpr int32_t PD_DEV_WAIT_EXPIRED = 1;  // a bounded wait for a bulk copy ga
 constexpr int32_t PD_REQF_TEST_EXPIRE = 1;  // test hook: the launch's first tile skips its copy
 
 // Per-frame constants, written on the device once the frame's radius is known.
-// With n_mom > 0 the frame runs in the moment form: every pair's
-// sinc(q r) is expanded in cos(n φ), sin(φ/2) = r/d, n < n_mom, and the tiles sum
-// the moments instead of the grid points. A tile's nqb jobs are then n_mblk moment
-// blocks times n_parts parts of its j range (job qb: block qb mod n_mblk, part
-// qb / n_mblk; the jobs past n_mblk·n_parts are idle).
+//
+// n_grp > 0: the frame runs in the direction form (amplitudes over a
+// quadrature of the sphere, pd_moments.cuh). Its work units are (atom chunk,
+// moment block, group of 32 directions); the request's jobs share them by
+// ordinal.
+//
+// Else n_mom > 0: moment form of the pairs. Every pair's sinc(q r) is expanded in
+// cos(n φ), sin(φ/2) = r/d, n < n_mom, and the tiles sum the moments instead of the
+// grid points. A tile's nqb jobs are then n_mblk moment blocks times n_parts
+// parts of its j range (job qb: block qb mod n_mblk, part qb / n_mblk; the jobs
+// past n_mblk·n_parts are idle).
+//
+// Else the grid points are summed directly.
 struct PdFrameDev {
     double radius;   // largest atom distance from the centroid (Å)
-    double d;        // expansion length: a little over 2·radius (Å)
+    double d;        // pairs: expansion length, a little over 2·radius (Å)
     double inv_d2;   // 1/d²
-    int32_t n_mom;   // moments, a multiple of 8; 0: the grid points are summed directly
+    double r1;       // directions: expansion length, a little over the radius (Å)
+    int32_t n_mom;   // moments, a multiple of 8; 0: no moment form
     int32_t n_mblk;  // moment blocks of pd_moment_block(K) moments
     int32_t n_parts;
+    int32_t n_grp;   // this rank's groups of 32 directions; 0: no direction form
+    int32_t n_amp;   // moments of the direction form, a multiple of 8
+    int32_t n_ablk;  // their blocks
+    int32_t n_node;  // Chebyshev nodes of the q range (direction form)
     int32_t pad_;
 };
-static_assert(sizeof(PdFrameDev) == 40, "PdFrameDev layout");
+static_assert(sizeof(PdFrameDev) == 64, "PdFrameDev layout");
+
+// Atoms [j0, j1) (padded indices) of one class: a work unit of the direction form.
+struct PdChunk {
+    int32_t cls, j0, j1, pad_;
+};
 
 // Moments per job of a kernel shape with q-block K: at most K (they share its
 // slots) and what the accumulators of the shape's register budget hold.
@@ -88,6 +108,11 @@ constexpr int pd_moment_block(int K) {
 // The moment form is bounded to this many moments (q_max·d up to about 900).
 constexpr int PD_MAX_MOMENTS = 512;
 
+// The direction form: at most this many moments (q_max·radius up to about 220),
+// and the shared memory of the kernel that sums the class pairs.
+constexpr int PD_MAX_DIR_MOMENTS = 256;
+constexpr int PD_DIR_SMEM = 200 * 1024;
+
 // When a frame may run in the moment form (block = 0: never).
 struct PdMomentRule {
     double qmax;          // last grid point
@@ -95,6 +120,25 @@ struct PdMomentRule {
     int32_t nqb;          // jobs per tile
     int32_t max_moments;  // beyond this the grid points are cheaper (or do not fit)
     int32_t fp64;
+    // direction form (dir_cap = 0: never)
+    int32_t dir_cap;      // directions the frame's table holds (a multiple of 32)
+    int32_t grp_cap;      // direction groups of this rank that the sums hold
+    int32_t amp_cap;      // moments
+    int32_t node_cap;     // Chebyshev nodes
+    int32_t n_chunk, n_cls, nv2;  // nv2: 1, or 2 with sums weighted by w (weighted mode)
+    int32_t rank, world;
+    int64_t slot_cap;     // doubles per frame for the chunks' sums
+    int64_t n_atoms;
+    int32_t nq;
+};
+
+// Sizes the direction kernels share.
+struct PdAmpShape {
+    int32_t n_chunk, n_cls, nv2, nq;
+    int32_t dir_cap, grp_cap, amp_cap, node_cap;
+    int32_t node_tile;  // nodes per block of the sums' kernel
+    int32_t rank, world, block;
+    int64_t slot_cap;
 };
 
 // Sizes of the slot reduction and the profile kernel.
@@ -117,6 +161,8 @@ struct PdReqDev {
     const double *qv;         // [nq] grid (FP64 form reads it directly)
     double *slots;            // [n_slots][nv][K]
     const PdFrameDev *frames; // [n_frames]
+    const double4 *dirs;      // [n_frames][dir_cap] direction/(2·r1) and quadrature weight
+    const PdChunk *chunks;    // [n_chunk]
     int32_t *status;          // PD_DEV_* bits, OR-ed in by the pair kernel
     double qmin, dq;          // grid origin and step
     int32_t n_pad;
@@ -125,6 +171,7 @@ struct PdReqDev {
     int32_t mode;
     int32_t flags;            // PD_REQF_* bits
     int32_t pad_;
+    PdAmpShape amp;
 };
 
 // Per-class constants for the combine kernel.

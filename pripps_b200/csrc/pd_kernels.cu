@@ -31,7 +31,10 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <cmath>
 #include <cstdio>
+#include <mutex>
+#include <vector>
 
 #include "pd_common.h"
 #include "pd_kernels.h"
@@ -801,6 +804,74 @@ __device__ __forceinline__ MomJob moment_job(int j0, int j1, int qb, int n_mblk,
     return m;
 }
 
+// Atoms a warp sums in FP32 for its directions before the sums go into the CTA's
+// FP64 partial sums.
+#ifndef PD_DIR_RUN
+#define PD_DIR_RUN 512
+#endif
+
+// Direction form: the job's work units (see direction_unit), one at a time. The
+// CTA's four warps share the unit's atoms, each lane one of its 32 directions;
+// part (FP64, [v][moment sum][32]) collects the warps' runs in warp order, so the
+// sums do not depend on timing.
+template <int K, int MODE>
+__device__ __forceinline__ void direction_units(const PdJob &jb, const PdReqDev &rq,
+                                                const PdFrameDev &fr, double *__restrict__ part,
+                                                int warp, int lane) {
+    constexpr int KM = pd_moment_block(K);
+    constexpr int DBL = KM == 128 ? 4 : (KM == 64 ? 3 : 2);
+    constexpr bool W = MODE == PD_MODE_WEIGHTED;
+    const float4 *__restrict__ at = rq.atoms32 + static_cast<size_t>(jb.frame) * rq.n_pad;
+    const int64_t n_units = static_cast<int64_t>(rq.amp.n_chunk) * fr.n_ablk * fr.n_grp;
+    for (int64_t u = jb.ord; u < n_units; u += jb.n_ord) {
+        const DirUnit un = direction_unit(u, fr, rq.amp.n_chunk);
+        const PdChunk ck = rq.chunks[un.chunk];
+        const double4 D = rq.dirs[static_cast<int64_t>(jb.frame) * rq.amp.dir_cap +
+                                  (static_cast<int64_t>(un.grp) * rq.amp.world + rq.amp.rank) * 32 +
+                                  lane];
+        const float3 dv = make_float3(static_cast<float>(D.x), static_cast<float>(D.y),
+                                      static_cast<float>(D.z));
+        const int per = (ck.j1 - ck.j0 + PD_WARPS - 1) / PD_WARPS;
+        const int w0 = min(ck.j1, ck.j0 + warp * per), w1 = min(ck.j1, w0 + per);
+        const int nj = min(KM, fr.n_amp - un.mb * KM) >> 3;
+        for (int run = 0; run < per; run += PD_DIR_RUN) {
+            float2 acc[KM / 2], accw[W ? KM / 2 : 1];
+#pragma unroll
+            for (int t = 0; t < KM / 2; ++t) {
+                acc[t] = make_float2(0.0f, 0.0f);
+                if constexpr (W) accw[t] = make_float2(0.0f, 0.0f);
+            }
+            direction_range<KM, W>(at, dv, min(w1, w0 + run), min(w1, w0 + run + PD_DIR_RUN), nj,
+                                   un.mb, DBL, acc, accw);
+            for (int w = 0; w < PD_WARPS; ++w) {
+                if (warp == w) {
+                    const bool first = run == 0 && w == 0;
+#pragma unroll
+                    for (int t = 0; t < KM / 2; ++t) {
+                        if (t >= 4 * nj) break;
+                        double *p = part + 2 * t * 32 + lane;
+                        p[0] = (first ? 0.0 : p[0]) + static_cast<double>(acc[t].x);
+                        p[32] = (first ? 0.0 : p[32]) + static_cast<double>(acc[t].y);
+                        if constexpr (W) {
+                            p += KM * 32;
+                            p[0] = (first ? 0.0 : p[0]) + static_cast<double>(accw[t].x);
+                            p[32] = (first ? 0.0 : p[32]) + static_cast<double>(accw[t].y);
+                        }
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        double *out = rq.slots + static_cast<int64_t>(jb.frame) * rq.amp.slot_cap;
+        direction_store(part, nj, un.mb * KM,
+                        out + direction_slot(un.chunk, 0, un.grp, rq.amp.nv2, fr));
+        if constexpr (W)
+            direction_store(part + KM * 32, nj, un.mb * KM,
+                            out + direction_slot(un.chunk, 1, un.grp, rq.amp.nv2, fr));
+        __syncthreads();  // part is rewritten by the next unit
+    }
+}
+
 // Weighted-mode flush of one accumulator array: the warp sums of acc and of
 // w_i·acc, added to part[k] and part[stride + k].
 template <int K>
@@ -888,6 +959,12 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
         const PdReqDev rq = reqs[jb.req];
         const int kq0 = jb.qb * K;
         const PdFrameDev fr = rq.frames[jb.frame];
+        if (fr.n_grp > 0) {
+            direction_units<K, MODE>(jb, rq, fr, reinterpret_cast<double *>(pd_dyn_atoms), warp,
+                                     lane);
+            __syncthreads();  // every thread has read s_job
+            continue;
+        }
         const double radius = fr.radius;
         // moment form: this job's part of the j range and its moment block
         const bool moments = fr.n_mom > 0;
@@ -1136,6 +1213,53 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
 }
 
 // ---------------------------------------------------------------- K2 (FP64)
+// direction_units in FP64 (one run per unit).
+template <int K, int MODE>
+__device__ __forceinline__ void direction_units_f64(const PdJob &jb, const PdReqDev &rq,
+                                                    const PdFrameDev &fr,
+                                                    double *__restrict__ part, int warp, int lane) {
+    constexpr int DBL = K == 64 ? 3 : (K == 32 ? 2 : 1);
+    constexpr bool W = MODE == PD_MODE_WEIGHTED;
+    const double4 *__restrict__ at = rq.atoms64 + static_cast<size_t>(jb.frame) * rq.n_pad;
+    const int64_t n_units = static_cast<int64_t>(rq.amp.n_chunk) * fr.n_ablk * fr.n_grp;
+    for (int64_t u = jb.ord; u < n_units; u += jb.n_ord) {
+        const DirUnit un = direction_unit(u, fr, rq.amp.n_chunk);
+        const PdChunk ck = rq.chunks[un.chunk];
+        const double4 D = rq.dirs[static_cast<int64_t>(jb.frame) * rq.amp.dir_cap +
+                                  (static_cast<int64_t>(un.grp) * rq.amp.world + rq.amp.rank) * 32 +
+                                  lane];
+        const int per = (ck.j1 - ck.j0 + PD_WARPS - 1) / PD_WARPS;
+        const int w0 = min(ck.j1, ck.j0 + warp * per), w1 = min(ck.j1, w0 + per);
+        const int nj = min(K, fr.n_amp - un.mb * K) >> 3;
+        double acc[K], accw[W ? K : 1];
+#pragma unroll
+        for (int e = 0; e < K; ++e) {
+            acc[e] = 0.0;
+            if constexpr (W) accw[e] = 0.0;
+        }
+        direction_range_f64<K, W>(at, D, w0, w1, nj, un.mb, DBL, acc, accw);
+        for (int w = 0; w < PD_WARPS; ++w) {
+            if (warp == w) {
+#pragma unroll
+                for (int e = 0; e < K; ++e) {
+                    if (e >= 8 * nj) break;
+                    double *p = part + e * 32 + lane;
+                    p[0] = (w == 0 ? 0.0 : p[0]) + acc[e];
+                    if constexpr (W) p[K * 32] = (w == 0 ? 0.0 : p[K * 32]) + accw[e];
+                }
+            }
+            __syncthreads();
+        }
+        double *out = rq.slots + static_cast<int64_t>(jb.frame) * rq.amp.slot_cap;
+        direction_store(part, nj, un.mb * K,
+                        out + direction_slot(un.chunk, 0, un.grp, rq.amp.nv2, fr));
+        if constexpr (W)
+            direction_store(part + K * 32, nj, un.mb * K,
+                            out + direction_slot(un.chunk, 1, un.grp, rq.amp.nv2, fr));
+        __syncthreads();  // part is rewritten by the next unit
+    }
+}
+
 template <int K, int MODE>
 __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(const PdJob *__restrict__ jobs,
                                                             const int *__restrict__ n_jobs_ptr,
@@ -1146,6 +1270,7 @@ __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(con
     __shared__ int s_job;
     __shared__ double s_q[K];
     __shared__ double s_part[PD_WARPS * NV * K];
+    __shared__ double s_dir[NACC * K * 32];  // direction form: sums of the CTA's directions
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int n_jobs = *n_jobs_ptr;
@@ -1157,6 +1282,12 @@ __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(con
         if (jid >= n_jobs) break;
         const PdJob jb = jobs[jid];
         const PdReqDev rq = reqs[jb.req];
+        const PdFrameDev fr = rq.frames[jb.frame];
+        if (fr.n_grp > 0) {
+            direction_units_f64<K, MODE>(jb, rq, fr, s_dir, warp, lane);
+            __syncthreads();  // every thread has read s_job
+            continue;
+        }
         if (threadIdx.x < K) {
             const int kq = jb.qb * K + threadIdx.x;
             s_q[threadIdx.x] = kq < rq.nq ? rq.qv[kq] : 0.0;
@@ -1173,7 +1304,6 @@ __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(con
 #pragma unroll
             for (int k = 0; k < K; ++k) acc[a][k] = 0.0;
 
-        const PdFrameDev fr = rq.frames[jb.frame];
         if (fr.n_mom > 0) {  // moment form: this job's part of the j range and its block
             constexpr int DBL = K == 64 ? 3 : (K == 32 ? 2 : 1);
             const MomJob mj = moment_job(jb.j0, jb.j1, jb.qb, fr.n_mblk, fr.n_parts);
@@ -1281,17 +1411,31 @@ __global__ void __launch_bounds__(PD_CENT_THREADS)
 
 // Gather positions into the class-sorted, padded layout, centred per frame.
 // The largest distance from the centroid is collected on the way, and the
-// frame's last block turns it into the frame's constants (PdFrameDev): whether
-// its pairs are summed in the moment form, and the expansion's size.
+// frame's last block turns it into the frame's constants (PdFrameDev): which form
+// its pairs are summed in, the expansion's size and the direction table.
+//
+// The rule counts FP32 lane operations. A pair, or an atom in one direction, costs
+// about 44 for its sequences (in each moment block) and 1.25 per moment; a
+// direction also n_cls·M terms per node in FP64. Measured on both
+// sides of the line (FP32, nq 200, R 16·(N/1000)^{1/3}): pairs are the faster form below about
+// 300 atoms, directions above.
 constexpr int PD_PACK_THREADS = 256;
+
+__device__ __forceinline__ int ring_points(double z_sin, bool fp64) {
+    return max(4, static_cast<int>(direction_order(z_sin, fp64)) + 1);
+}
 
 __global__ void __launch_bounds__(PD_PACK_THREADS)
     pd_pack(const double *__restrict__ xyz, const double *__restrict__ weights,
             const int32_t *__restrict__ perm, const double *__restrict__ centroid,
             int64_t n_atoms, int32_t n_pad, int32_t n_blk, float4 *__restrict__ out32,
             double4 *__restrict__ out64, PdMomentRule rule, unsigned long long *__restrict__ rad2,
-            unsigned int *__restrict__ done, PdFrameDev *__restrict__ frames) {
+            unsigned int *__restrict__ done, PdFrameDev *__restrict__ frames,
+            double4 *__restrict__ dirs) {
     __shared__ double s_max[PD_PACK_THREADS / 32];
+    __shared__ bool s_last;
+    __shared__ double s_radius;
+    __shared__ int s_off[PD_GL_MAX + 1];  // first direction of each ring
     const int f = blockIdx.x / n_blk, b = blockIdx.x % n_blk;
     const int p = b * PD_PACK_THREADS + threadIdx.x;
     double r2 = 0.0;
@@ -1315,31 +1459,108 @@ __global__ void __launch_bounds__(PD_PACK_THREADS)
     for (int o = 16; o > 0; o >>= 1) r2 = fmax(r2, __shfl_xor_sync(0xffffffffu, r2, o));
     if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = r2;
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    for (int k = 1; k < PD_PACK_THREADS / 32; ++k) r2 = fmax(r2, s_max[k]);
-    // non-negative doubles order as their bit patterns; the maximum is exact
-    atomicMax(&rad2[f], static_cast<unsigned long long>(__double_as_longlong(r2)));
-    __threadfence();
-    if (atomicAdd(&done[f], 1u) != static_cast<unsigned>(n_blk - 1)) return;
-    __threadfence();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < PD_PACK_THREADS / 32; ++k) r2 = fmax(r2, s_max[k]);
+        // non-negative doubles order as their bit patterns; the maximum is exact
+        atomicMax(&rad2[f], static_cast<unsigned long long>(__double_as_longlong(r2)));
+        __threadfence();
+        s_last = atomicAdd(&done[f], 1u) == static_cast<unsigned>(n_blk - 1);
+        if (s_last) {
+            __threadfence();
+            s_radius = sqrt(__longlong_as_double(
+                static_cast<long long>(atomicMax(&rad2[f], 0ull))));
+        }
+    }
+    __syncthreads();
+    if (!s_last) return;
+
+    const double radius = s_radius;
+    const bool fp64 = rule.fp64 != 0;
     PdFrameDev fr{};
-    fr.radius = sqrt(__longlong_as_double(
-        static_cast<long long>(atomicMax(&rad2[f], 0ull))));
+    fr.radius = radius;
     // d follows the FP32 value of 1/d² that the pairs are scaled with: rounding
     // 1/d² alone would stretch every distance by the same 1 + 3e-8
-    fr.d = fmax(2.0 * PD_MOM_STRETCH * fr.radius, 1e-6);
+    fr.d = fmax(2.0 * PD_MOM_STRETCH * radius, 1e-6);
     fr.inv_d2 = static_cast<double>(static_cast<float>(1.0 / (fr.d * fr.d)));
     fr.d = 1.0 / sqrt(fr.inv_d2);
+    fr.r1 = fmax(PD_MOM_STRETCH * radius, 1e-6);
+    double pair_cost = 1e300;
     if (rule.block > 0) {
-        const int m8 = (moments_needed(rule.qmax * fr.d, rule.fp64 != 0) + 7) & ~7;
+        const int m8 = (moments_needed(rule.qmax * fr.d, fp64) + 7) & ~7;
         const int blocks = (m8 + rule.block - 1) / rule.block;
         if (m8 <= rule.max_moments && blocks <= rule.nqb) {
             fr.n_mom = m8;
             fr.n_mblk = blocks;
             fr.n_parts = rule.nqb / blocks;
+            pair_cost = 0.5 * static_cast<double>(rule.n_atoms) * rule.n_atoms *
+                        (44.0 * blocks + 1.25 * m8);
         }
     }
-    frames[f] = fr;
+    // ---- directions: 2h Gauss rings (upper half: h), enough points on each
+    if (rule.dir_cap == 0) {
+        if (threadIdx.x == 0) frames[f] = fr;
+        return;
+    }
+    const double z = 2.0 * radius * rule.qmax;
+    const double order = direction_order(z, fp64);
+    const int h = order < 4.0 * PD_GL_MAX - 4.0 ? static_cast<int>(order * 0.25) + 1 : 0;
+    const double2 *gl = pd_gl_rules + h * (h - 1) / 2;
+    if (threadIdx.x < h) {
+        const double x = gl[threadIdx.x].x;
+        s_off[threadIdx.x + 1] = ring_points(z * sqrt(1.0 - x * x), fp64);
+    }
+    __syncthreads();
+    for (int o = 1; o < h; o <<= 1) {  // inclusive scan of s_off[1 .. h]
+        const int k = threadIdx.x + 1;
+        const int v = (k <= h && k > o) ? s_off[k - o] : 0;
+        __syncthreads();
+        if (k <= h) s_off[k] += v;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) s_off[0] = 0;
+    __syncthreads();
+    const int S = h > 0 ? s_off[h] : 0;
+    const int groups = (S + 31) / 32;
+    const int mine = rule.rank < groups ? (groups - rule.rank + rule.world - 1) / rule.world : 0;
+    const double mo = direction_order(fr.r1 * rule.qmax, fp64);
+    const int m8 = mo < 1e6 ? ((static_cast<int>(mo) + 8) & ~7) : 1000000;
+    const int ablk = (m8 + rule.block - 1) / max(rule.block, 1);
+    const int nodes = moments_needed(2.0 * fr.r1 * rule.qmax, true);
+    const double dir_cost =
+        static_cast<double>(S) * (static_cast<double>(rule.n_atoms) * (44.0 * ablk + 1.25 * m8) +
+                                  4.0 * rule.n_cls * m8 * nodes);
+    const bool use = S > 0 && rule.block > 0 && groups * 32 <= rule.dir_cap && mine > 0 &&
+                     (groups + rule.world - 1) / rule.world <= rule.grp_cap &&
+                     m8 <= rule.amp_cap && nodes <= rule.node_cap &&
+                     static_cast<int64_t>(rule.n_chunk) * rule.nv2 *
+                             ((groups + rule.world - 1) / rule.world) * m8 * 32 <= rule.slot_cap &&
+                     groups >= rule.world && dir_cost < pair_cost;
+    if (use) {
+        fr.n_grp = mine;
+        fr.n_amp = m8;
+        fr.n_ablk = ablk;
+        fr.n_node = nodes;
+        const double sc = 0.5 / fr.r1;
+        double4 *o = dirs + static_cast<int64_t>(f) * rule.dir_cap;
+        for (int s = threadIdx.x; s < groups * 32; s += PD_PACK_THREADS) {
+            double4 d = make_double4(0.0, 0.0, 0.0, 0.0);
+            if (s < S) {
+                int lo = 0, hi = h;  // ring with s_off[lo] <= s < s_off[lo + 1]
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (s_off[mid] <= s) lo = mid; else hi = mid;
+                }
+                const double2 nw = gl[lo];
+                const int n = s_off[lo + 1] - s_off[lo];
+                const double st = sqrt(1.0 - nw.x * nw.x) * sc;
+                double sn, cs;
+                sincospi(2.0 * (s - s_off[lo]) / n, &sn, &cs);
+                d = make_double4(st * cs, st * sn, nw.x * sc, nw.y / n);
+            }
+            o[s] = d;
+        }
+    }
+    if (threadIdx.x == 0) frames[f] = fr;
 }
 
 // ------------------------------------------------------------ reductions
@@ -1398,6 +1619,7 @@ __global__ void __launch_bounds__(PD_RED_THREADS)
     const int k = z * 128 + tl;
     const PdFrameDev fr = frames[f];
     const bool moments = fr.n_mom > 0;
+    if (fr.n_grp > 0) return;  // direction form
     if (z * 128 >= (moments ? fr.n_mom : sh.nq)) return;
     const int64_t fbase = static_cast<int64_t>(f) * sh.slots_per_frame;
     const int64_t stride = static_cast<int64_t>(NV) * sh.K;
@@ -1474,6 +1696,168 @@ __global__ void __launch_bounds__(PD_RED_THREADS)
     for (int v = 0; v < NV; ++v) o[static_cast<int64_t>(v) * sh.width] = s[v];
 }
 
+// Direction form: class-pair sums at Chebyshev nodes of the q range.
+//
+// S_ab(q) = Σ sinc(q r) is an even entire function of q whose expansion in
+// T_2k(q/q_max) ends, like the moments, at k ≈ q_max·d/2 + …: its values at that many
+// nodes q_k = q_max·cos((2k+1)π/4M) give every grid point by interpolation (pd_profiles), so
+// the amplitudes are formed at 30 to 120 nodes instead of 200 to 1,000 grid
+// points. A block takes 32 directions and PD_DNODE_T nodes (fewer where many
+// classes share its memory): E_c = Σ_n g_n(q_k r1)·m_n, g_n = i^n (2 − δ_n0) J_n, of every class in
+// FP64 — the sums of the class's chunks added in chunk order, the zeroth
+// moment the exact atom count or weight sum — then Σ w·Re(E_a E_b*) over the directions
+// of every class pair. The frame's last block of these nodes adds the groups in
+// group order and takes the i = j terms out of the self sums.
+constexpr int PD_DNODE_T = 16;
+constexpr int PD_DSUM_THREADS = 256;
+constexpr int PD_DSUM_WARPS = PD_DSUM_THREADS / 32;
+
+// (2 − δ_n0)·J_n(y)·(sign of i^n) for n < n_mom, unnormalised, into g[n·stride];
+// returns the factor that normalises them (J_0 + 2ΣJ_2k = 1, Miller's recurrence).
+__device__ double direction_coefficients(double y, int n_mom, double *__restrict__ g, int stride) {
+    if (!(y > 1e-8)) {
+        for (int n = 0; n < n_mom; ++n) g[n * stride] = n == 0 ? 1.0 : 0.0;
+        return 1.0;
+    }
+    const double ty = 2.0 / y;
+    const int top = static_cast<int>(bessel_order(y, 14.0, 8.0)) | 1;
+    for (int n = top + 1; n < n_mom; ++n) g[n * stride] = 0.0;
+    double hi = 0.0, cur = 1e-200, even = 0.0;
+    for (int n = top; n > 0; --n) {  // cur = J_n
+        if (n < n_mom) g[n * stride] = (n & 2) ? -2.0 * cur : 2.0 * cur;
+        if (!(n & 1)) even += cur;
+        const double lower = fma(n * ty, cur, -hi);
+        hi = cur;
+        cur = lower;
+    }
+    g[0] = cur;
+    return 1.0 / fma(2.0, even, cur);
+}
+
+// Node k of n on the q range [0, qmax]: q = qmax·cos((2k+1)π/4n).
+__device__ __forceinline__ double direction_node(int k, int n, double qmax) {
+    return qmax * cospi((2 * k + 1) / (4.0 * n));
+}
+
+template <int NV2>
+__global__ void __launch_bounds__(PD_DSUM_THREADS)
+    pd_direction_sums(const double *__restrict__ slots, const double4 *__restrict__ dirs,
+                      const PdFrameDev *__restrict__ frames, PdAmpShape sh, double qmax,
+                      const PdClassDev *__restrict__ cls, const PdPairDev *__restrict__ pairs,
+                      int32_t n_pairs, const int32_t *__restrict__ cls_ptr,
+                      const int32_t *__restrict__ cls_chunk, int32_t width, int32_t add_exact,
+                      double *__restrict__ part, unsigned int *__restrict__ done,
+                      double *__restrict__ red) {
+    extern __shared__ double s_dyn[];
+    __shared__ double s_scale[PD_DNODE_T];
+    __shared__ bool s_last;
+    const int f = blockIdx.y;
+    const PdFrameDev fr = frames[f];
+    const int NT = sh.node_tile;
+    const int n_nt = (sh.node_cap + NT - 1) / NT;
+    const int tile = blockIdx.x % n_nt, grp = blockIdx.x / n_nt;
+    if (grp >= fr.n_grp || tile * NT >= fr.n_node) return;
+    const int M = fr.n_amp, nn = min(NT, fr.n_node - tile * NT);
+    double *s_g = s_dyn;                        // [M][NT]
+    double *s_m = s_g + sh.amp_cap * NT;        // [M][32]
+    double *s_e = s_m + sh.amp_cap * 32;        // [n_cls][NV2][NT][2][32]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < nn)
+        s_scale[threadIdx.x] = direction_coefficients(
+            direction_node(tile * NT + threadIdx.x, fr.n_node, qmax) * fr.r1, M, s_g + threadIdx.x,
+            NT);
+    const double *sl = slots + static_cast<int64_t>(f) * sh.slot_cap;
+    for (int cv = 0; cv < sh.n_cls * NV2; ++cv) {
+        const int c = cv / NV2, v = cv % NV2;
+        const int e0 = cls_ptr[c], e1 = cls_ptr[c + 1];
+        __syncthreads();  // the previous class's moments are read
+        for (int k = threadIdx.x; k < M * 32; k += PD_DSUM_THREADS) {
+            double m = 0.0;
+            for (int e = e0; e < e1; ++e)
+                m += sl[direction_slot(cls_chunk[e], v, grp, NV2, fr) + k];
+            s_m[k] = k < 32 ? (v ? cls[c].w1 : cls[c].n) : m;
+        }
+        __syncthreads();
+        for (int t = warp; t < nn; t += 2 * PD_DSUM_WARPS) {  // two nodes at a time
+            const int t2 = min(t + PD_DSUM_WARPS, nn - 1);
+            double er = 0, ei = 0, fr2 = 0, fi2 = 0;
+            const double *ga = s_g + t, *gb = s_g + t2;
+#pragma unroll 4
+            for (int n = 0; n < M; n += 2) {  // M is a multiple of 8
+                const double m0 = s_m[n * 32 + lane], m1 = s_m[(n + 1) * 32 + lane];
+                er = fma(ga[n * NT], m0, er);
+                ei = fma(ga[(n + 1) * NT], m1, ei);
+                fr2 = fma(gb[n * NT], m0, fr2);
+                fi2 = fma(gb[(n + 1) * NT], m1, fi2);
+            }
+            double *o = s_e + (cv * NT + t) * 64 + lane;
+            o[0] = er * s_scale[t];
+            o[32] = ei * s_scale[t];
+            if (t + PD_DSUM_WARPS < nn) {
+                o = s_e + (cv * NT + t2) * 64 + lane;
+                o[0] = fr2 * s_scale[t2];
+                o[32] = fi2 * s_scale[t2];
+            }
+        }
+    }
+    __syncthreads();
+    const double w = dirs[static_cast<int64_t>(f) * sh.dir_cap +
+                          (static_cast<int64_t>(grp) * sh.world + sh.rank) * 32 + lane].w;
+    constexpr int NV = NV2 == 2 ? 4 : 1;
+    // [frame][group][pair][nv][node]
+    const int64_t row = static_cast<int64_t>(n_pairs) * NV * sh.node_cap;
+    double *pt = part + (static_cast<int64_t>(f) * sh.grp_cap + grp) * row;
+    for (int k = warp; k < n_pairs * nn; k += PD_DSUM_WARPS) {
+        const int p = k / nn, t = k - p * nn;
+        const int a = pairs[p].a, b = pairs[p].b;
+        const double *Ea = s_e + (a * NV2 * NT + t) * 64 + lane;
+        const double *Eb = s_e + (b * NV2 * NT + t) * 64 + lane;
+        double x[NV];
+        x[0] = w * (Ea[0] * Eb[0] + Ea[32] * Eb[32]);
+        if constexpr (NV == 4) {  // Fa, Fb: weighted amplitudes
+            const double *Fa = Ea + NT * 64, *Fb = Eb + NT * 64;
+            x[1] = w * (Fa[0] * Eb[0] + Fa[32] * Eb[32]);
+            x[2] = w * (Ea[0] * Fb[0] + Ea[32] * Fb[32]);
+            x[3] = w * (Fa[0] * Fb[0] + Fa[32] * Fb[32]);
+        }
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+            x[v] = warp_sum(x[v]);
+            if (lane == 0)
+                pt[(static_cast<int64_t>(p) * NV + v) * sh.node_cap + tile * NT + t] = x[v];
+        }
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0)
+        s_last = atomicAdd(&done[f * n_nt + tile], 1u) == static_cast<unsigned>(fr.n_grp - 1);
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const double *p0 = part + static_cast<int64_t>(f) * sh.grp_cap * row;
+    for (int k = threadIdx.x; k < n_pairs * NV * nn; k += PD_DSUM_THREADS) {
+        const int pv = k / nn, t = k - pv * nn, p = pv / NV, v = pv % NV;
+        const double *q = p0 + static_cast<int64_t>(pv) * sh.node_cap + tile * NT + t;
+        double s = 0.0;
+        int g = 0;
+        for (; g + 8 <= fr.n_grp; g += 8) {
+            double x[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) x[u] = __ldcg(q + (g + u) * row);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) s += x[u];
+        }
+        for (; g < fr.n_grp; ++g) s += __ldcg(q + g * row);
+        const PdPairDev pr = pairs[p];
+        if (pr.a == pr.b) {  // all (i, j) of the class: i < j is half of the rest
+            const PdClassDev cl = cls[pr.a];
+            const double diag = v == 0 ? cl.n : (v == 3 ? cl.w2 : cl.w1);
+            s = 0.5 * (s - (add_exact ? diag : 0.0));
+        }
+        red[(static_cast<int64_t>(f) * n_pairs * NV + pv) * width + tile * NT + t] = s;
+    }
+}
+
 // c_n(z)·z/4 (c_0·z/2) unnormalised for n < n_mom into coef[n·stride], z = q·d (see
 // pd_moments.cuh); returns the factor that makes them c_n. J_ν(z) by Miller's
 // downward recurrence, normalised with J_0 + 2ΣJ_2k = 1; it starts a few terms
@@ -1519,7 +1903,7 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
                 int32_t n_cls, PdReduceShape sh, const double *__restrict__ qv,
                 const PdFrameDev *__restrict__ frames, const double *__restrict__ ffA,
                 const double *__restrict__ ffC, const double *__restrict__ ffW, int32_t add_diag,
-                double *__restrict__ terms) {
+                double qmax, const int *__restrict__ err, double *__restrict__ terms) {
     extern __shared__ double s_coef[];  // [n_mom][PD_PROF_Q]
     __shared__ double s_c0[PD_PROF_Q], s_scale[PD_PROF_Q];
     __shared__ double s_sum[PD_PROF_THREADS / 32][6][PD_PROF_Q];
@@ -1529,9 +1913,50 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
     const int q = (blockIdx.x % n_qt) * PD_PROF_Q + ql;
     const bool ok = q < sh.nq;
     const PdFrameDev fr = frames[f];
-    const int M = fr.n_mom;
+    const bool nodes = fr.n_grp > 0;
+    const int M = nodes ? fr.n_node : fr.n_mom;
     const double qval = ok ? qv[q] : 0.0;
-    if (M > 0) {
+    if (nodes) {
+        // interpolation from the Chebyshev nodes y_k = cos((2k+1)π/2M) of
+        // y = 2(q/qmax)² − 1, barycentric form
+        const double y = qmax > 0.0 ? 2.0 * (qval / qmax) * (qval / qmax) - 1.0 : -1.0;
+        double sum = 0.0;
+        int hit = 0;
+        for (int k = g; k < M; k += PD_PROF_GROUPS) {
+            double sn, cs;
+            sincospi((2 * k + 1) / (2.0 * M), &sn, &cs);
+            const double dy = y - cs;
+            const double l = dy != 0.0 ? ((k & 1) ? -sn : sn) / dy : 0.0;
+            if (dy == 0.0) hit = k + 1;
+            s_coef[k * PD_PROF_Q + ql] = l;
+            sum += l;
+        }
+        sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+        hit = max(hit, __shfl_xor_sync(0xffffffffu, hit, 8));
+        hit = max(hit, __shfl_xor_sync(0xffffffffu, hit, 16));
+        if ((threadIdx.x & 31) < PD_PROF_Q) {
+            s_sum[threadIdx.x >> 5][0][ql] = sum;
+            s_sum[threadIdx.x >> 5][1][ql] = hit;
+        }
+        __syncthreads();
+        if (threadIdx.x < PD_PROF_Q) {
+            double v = 0.0, h = 0.0;
+            for (int w = 0; w < PD_PROF_THREADS / 32; ++w) {
+                v += s_sum[w][0][ql];
+                h = fmax(h, s_sum[w][1][ql]);
+            }
+            s_scale[ql] = 1.0 / v;
+            s_c0[ql] = h;  // the grid point's own node + 1, or 0
+        }
+        __syncthreads();
+        hit = static_cast<int>(s_c0[ql]);
+        for (int k = g; k < M; k += PD_PROF_GROUPS) {
+            double &c = s_coef[k * PD_PROF_Q + ql];
+            c = hit ? (k + 1 == hit ? 1.0 : 0.0) : c * s_scale[ql];
+        }
+        __syncthreads();
+    } else if (M > 0) {
         if (threadIdx.x < PD_PROF_Q) {
             s_scale[ql] = moment_coefficients(qval * fr.d, M, s_coef + ql, PD_PROF_Q);
             s_c0[ql] = s_coef[ql] * s_scale[ql];
@@ -1585,7 +2010,7 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
         const PdPairDev pr = pairs[p];
         const double *r = red + (static_cast<int64_t>(f) * sh.n_pairs + p) * NV * sh.width;
         double s[NV];
-        if (pr.lat >= 0) {  // from the lattice set's pair counts (class mode, one frame)
+        if (!nodes && pr.lat >= 0) {  // from the lattice set's pair counts (class mode, one frame)
             s[0] = sub == 0 ? lat_sums[static_cast<int64_t>(pr.lat) * sh.nq + q] : 0.0;
         } else if (M == 0) {
 #pragma unroll
@@ -1603,7 +2028,11 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
                         s[v] = fma(c, r[static_cast<int64_t>(v) * sh.width + e], s[v]);
                 }
             }
-            if (sub == 0) {
+            if (nodes) {
+                if (!(qval > 0.0))
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) s[v] = (add_diag && sub == 0) ? pr.q0[v] : 0.0;
+            } else if (sub == 0) {
                 // the zeroth moment is the exact pair sum at q = 0, not the
                 // tiles' rounded (Σ X·vx − Σ Y·vy)/2
 #pragma unroll
@@ -1648,6 +2077,7 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
         double v = 0.0;
 #pragma unroll
         for (int w = 0; w < PD_PROF_THREADS / 32; ++w) v += s_sum[w][t][ql];
+        if (err && *err) v = __longlong_as_double(0x7ff8000000000000ll);  // a point off its lattice
         if (ok) terms[(static_cast<int64_t>(f) * 6 + t) * sh.nq + q] = v;
     }
 }
@@ -1690,8 +2120,10 @@ __global__ void __launch_bounds__(128) pd_lattice_hist(const PdLatTile *__restri
                                                        const PdLatDev *__restrict__ lat,
                                                        const int4 *__restrict__ idx,
                                                        unsigned long long *__restrict__ hist,
+                                                       const PdFrameDev *__restrict__ frames,
                                                        int shared_bins) {
     extern __shared__ unsigned int s_hist[];
+    if (frames[0].n_grp > 0) return;  // direction form: no pairs are counted
     const PdLatTile t = tiles[blockIdx.x];
     const PdLatDev d = lat[t.lat];
     const bool use_shared = shared_bins > 0;
@@ -1730,8 +2162,10 @@ __global__ void __launch_bounds__(256) pd_lattice_sums(const unsigned long long 
                                                        const double *__restrict__ qv, int32_t nq,
                                                        int32_t add_exact,
                                                        const int *__restrict__ err,
+                                                       const PdFrameDev *__restrict__ frames,
                                                        double *__restrict__ sums) {
     __shared__ double s_part[256];
+    if (frames[0].n_grp > 0) return;  // direction form
     const int q = blockIdx.x;
     const PdLatDev d = lat[blockIdx.y];
     const double qval = qv[q];
@@ -2335,13 +2769,97 @@ cudaError_t launch_pack(const double *xyz, const double *weights, const int32_t 
                         const double *centroid, int64_t n_atoms, int32_t n_pad, int32_t n_frames,
                         float4 *out32, double4 *out64, const PdMomentRule &rule,
                         unsigned long long *rad2, unsigned int *done, PdFrameDev *frames,
-                        cudaStream_t st) {
+                        double4 *dirs, cudaStream_t st) {
     const int64_t nb = (static_cast<int64_t>(n_pad) + PD_PACK_THREADS - 1) / PD_PACK_THREADS;
     if (nb * n_frames > 0x7fffffffLL) return cudaErrorInvalidValue;
     pd_pack<<<static_cast<unsigned>(nb * n_frames), PD_PACK_THREADS, 0, st>>>(
         xyz, weights, perm, centroid, n_atoms, n_pad, static_cast<int32_t>(nb), out32, out64, rule,
-        rad2, done, frames);
+        rad2, done, frames, dirs);
     return cudaGetLastError();
+}
+
+// Gauss–Legendre rules: Newton's method on P_2h from Tricomi's estimate, in
+// long double, once per process; copied to each device that asks.
+cudaError_t prepare_direction_rules() {
+    static std::mutex mu;
+    static std::vector<double2> rules;
+    static uint64_t done = 0;
+    std::lock_guard<std::mutex> g(mu);
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = dev < 64 ? (uint64_t{1} << dev) : 0;
+    if (bit && (done & bit)) return cudaSuccess;
+    if (rules.empty()) {
+        rules.resize(PD_GL_MAX * (PD_GL_MAX + 1) / 2);
+        for (int h = 1; h <= PD_GL_MAX; ++h) {
+            const int n = 2 * h;
+            for (int i = 0; i < h; ++i) {  // i-th largest node
+                long double x = cosl(3.14159265358979323846264L * (i + 0.75L) / (n + 0.5L));
+                long double dp = 1.0L;
+                for (int it = 0; it < 6; ++it) {
+                    long double p0 = 1.0L, p1 = x;
+                    for (int k = 2; k <= n; ++k) {
+                        const long double p2 = ((2 * k - 1) * x * p1 - (k - 1) * p0) / k;
+                        p0 = p1;
+                        p1 = p2;
+                    }
+                    dp = n * (x * p1 - p0) / (x * x - 1.0L);
+                    const long double dx = p1 / dp;
+                    x -= dx;
+                    if (fabsl(dx) < 1e-12L) break;  // quadratic: the next step is below the last bit
+                }
+                {
+                    long double p0 = 1.0L, p1 = x;
+                    for (int k = 2; k <= n; ++k) {
+                        const long double p2 = ((2 * k - 1) * x * p1 - (k - 1) * p0) / k;
+                        p0 = p1;
+                        p1 = p2;
+                    }
+                    dp = n * (x * p1 - p0) / (x * x - 1.0L);
+                }
+                double2 &r = rules[h * (h - 1) / 2 + (h - 1 - i)];
+                r.x = static_cast<double>(x);
+                r.y = static_cast<double>(2.0L / ((1.0L - x * x) * dp * dp));
+            }
+            long double sum = 0.0L;
+            for (int i = 0; i < h; ++i) sum += rules[h * (h - 1) / 2 + i].y;
+            for (int i = 0; i < h; ++i)
+                rules[h * (h - 1) / 2 + i].y = static_cast<double>(rules[h * (h - 1) / 2 + i].y / sum);
+        }
+    }
+    const cudaError_t e =
+        cudaMemcpyToSymbol(pd_gl_rules, rules.data(), rules.size() * sizeof(double2));
+    if (e == cudaSuccess) done |= bit;
+    return e;
+}
+
+cudaError_t launch_direction_sums(const double *slots, const double4 *dirs,
+                                  const PdFrameDev *frames, const PdAmpShape &sh, double qmax,
+                                  int32_t n_frames, const PdClassDev *cls, const PdPairDev *pairs,
+                                  int32_t n_pairs, const int32_t *cls_ptr,
+                                  const int32_t *cls_chunk, int32_t width, int add_exact,
+                                  double *part, unsigned int *done, double *red, cudaStream_t st) {
+    const size_t smem = (static_cast<size_t>(sh.amp_cap) * (sh.node_tile + 32) +
+                         static_cast<size_t>(sh.n_cls) * sh.nv2 * sh.node_tile * 64) *
+                        sizeof(double);
+    auto kern = sh.nv2 == 2 ? pd_direction_sums<2> : pd_direction_sums<1>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         PD_DIR_SMEM);
+    if (e != cudaSuccess) return e;
+    if (smem > PD_DIR_SMEM) return cudaErrorInvalidValue;
+    const int64_t n_nt = (sh.node_cap + sh.node_tile - 1) / sh.node_tile;
+    const int64_t nv = sh.nv2 == 2 ? 4 : 1;
+    for (int32_t f0 = 0; f0 < n_frames; f0 += 65535) {  // grid.y limit
+        const dim3 grid(static_cast<unsigned>(n_nt * sh.grp_cap),
+                        static_cast<unsigned>(std::min(n_frames - f0, 65535)));
+        kern<<<grid, PD_DSUM_THREADS, smem, st>>>(
+            slots + f0 * sh.slot_cap, dirs + static_cast<int64_t>(f0) * sh.dir_cap, frames + f0, sh,
+            qmax, cls, pairs, n_pairs, cls_ptr, cls_chunk, width, add_exact,
+            part + f0 * static_cast<int64_t>(sh.grp_cap) * n_pairs * nv * sh.node_cap,
+            done + f0 * n_nt, red + f0 * static_cast<int64_t>(n_pairs) * nv * width);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_reduce(const double *slots, const int64_t *lptr, const int64_t *lidx,
@@ -2367,7 +2885,8 @@ cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdC
                             const PdPairDev *pairs, int32_t n_cls, const PdReduceShape &sh,
                             int32_t nv, int32_t n_frames, const double *qv,
                             const PdFrameDev *frames, const double *ffA, const double *ffC,
-                            const double *ffW, int add_diag, double *terms, cudaStream_t st) {
+                            const double *ffW, int add_diag, double qmax, const int *err,
+                            double *terms, cudaStream_t st) {
     const int64_t blocks =
         static_cast<int64_t>(n_frames) * ((sh.nq + PD_PROF_Q - 1) / PD_PROF_Q);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
@@ -2375,17 +2894,19 @@ cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdC
     const size_t smem = static_cast<size_t>(sh.max_moments) * PD_PROF_Q * sizeof(double);
     if (nv == 4)
         pd_profiles<4><<<static_cast<unsigned>(blocks), PD_PROF_THREADS, smem, st>>>(
-            red, lat_sums, cls, pairs, n_cls, sh, qv, frames, ffA, ffC, ffW, add_diag, terms);
+            red, lat_sums, cls, pairs, n_cls, sh, qv, frames, ffA, ffC, ffW, add_diag, qmax,
+            err, terms);
     else
         pd_profiles<1><<<static_cast<unsigned>(blocks), PD_PROF_THREADS, smem, st>>>(
-            red, lat_sums, cls, pairs, n_cls, sh, qv, frames, ffA, ffC, ffW, add_diag, terms);
+            red, lat_sums, cls, pairs, n_cls, sh, qv, frames, ffA, ffC, ffW, add_diag, qmax,
+            err, terms);
     return cudaGetLastError();
 }
 
 cudaError_t launch_lattice(const double *xyz, const int32_t *perm, const PdLatDev *lat_dev,
                            const PdLatDev *lat_host, int n_lat, const PdLatTile *tiles,
                            int64_t n_tiles, int4 *idx, unsigned long long *hist, int64_t n_bins,
-                           int *err, cudaStream_t st) {
+                           int *err, const PdFrameDev *frames, cudaStream_t st) {
     if (n_lat == 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(hist, 0, static_cast<size_t>(n_bins) * 8, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(int), st);
@@ -2415,15 +2936,16 @@ cudaError_t launch_lattice(const double *xyz, const int32_t *perm, const PdLatDe
         }
     }
     pd_lattice_hist<<<static_cast<unsigned>(n_tiles), 128, smem, st>>>(tiles, lat_dev, idx, hist,
-                                                                        shared_bins);
+                                                                        frames, shared_bins);
     return cudaGetLastError();
 }
 
 cudaError_t launch_lattice_sums(const unsigned long long *hist, const PdLatDev *lat, int n_lat,
                                 const double *qv, int32_t nq, int add_exact, const int *err,
-                                double *sums, cudaStream_t st) {
+                                const PdFrameDev *frames, double *sums, cudaStream_t st) {
     if (n_lat == 0) return cudaSuccess;
-    pd_lattice_sums<<<dim3(nq, n_lat), 256, 0, st>>>(hist, lat, qv, nq, add_exact, err, sums);
+    pd_lattice_sums<<<dim3(nq, n_lat), 256, 0, st>>>(hist, lat, qv, nq, add_exact, err, frames,
+                                                       sums);
     return cudaGetLastError();
 }
 

@@ -32,7 +32,19 @@ cudaError_t launch_pack(const double *xyz, const double *weights, const int32_t 
                         const double *centroid, int64_t n_atoms, int32_t n_pad, int32_t n_frames,
                         float4 *out32, double4 *out64, const PdMomentRule &rule,
                         unsigned long long *rad2, unsigned int *done, PdFrameDev *frames,
-                        cudaStream_t st);
+                        double4 *dirs, cudaStream_t st);
+// The quadrature rules of the direction form on the current device (before any
+// launch_pack there, and before a stream capture).
+cudaError_t prepare_direction_rules();
+// Direction form: class-pair sums at the nodes, from the chunks' moments, into
+// red (does nothing for frames in the other forms). part holds grp_cap·pairs·nv·
+// node_cap doubles per frame, done one zeroed counter per node tile and frame.
+cudaError_t launch_direction_sums(const double *slots, const double4 *dirs,
+                                  const PdFrameDev *frames, const PdAmpShape &sh, double qmax,
+                                  int32_t n_frames, const PdClassDev *cls, const PdPairDev *pairs,
+                                  int32_t n_pairs, const int32_t *cls_ptr,
+                                  const int32_t *cls_chunk, int32_t width, int add_exact,
+                                  double *part, unsigned int *done, double *red, cudaStream_t st);
 // Slot sums (red: [frame][pair][nv][width]); with n_chunk > 1, chunk_sums holds
 // 128·nv·n_chunk doubles and done one zeroed counter per (frame, pair, n_z).
 cudaError_t launch_reduce(const double *slots, const int64_t *lptr, const int64_t *lidx,
@@ -44,16 +56,17 @@ cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdC
                             const PdPairDev *pairs, int32_t n_cls, const PdReduceShape &sh,
                             int32_t nv, int32_t n_frames, const double *qv,
                             const PdFrameDev *frames, const double *ffA, const double *ffC,
-                            const double *ffW, int add_diag, double *terms, cudaStream_t st);
+                            const double *ffW, int add_diag, double qmax, const int *err,
+                            double *terms, cudaStream_t st);
 // Lattice sets: integer coordinates of their points and the exact pair count
 // per squared offset (after pack), then their self pair sums, sums[lattice][q].
 cudaError_t launch_lattice(const double *xyz, const int32_t *perm, const PdLatDev *lat_dev,
                            const PdLatDev *lat_host, int n_lat, const PdLatTile *tiles,
                            int64_t n_tiles, int4 *idx, unsigned long long *hist, int64_t n_bins,
-                           int *err, cudaStream_t st);
+                           int *err, const PdFrameDev *frames, cudaStream_t st);
 cudaError_t launch_lattice_sums(const unsigned long long *hist, const PdLatDev *lat, int n_lat,
                                 const double *qv, int32_t nq, int add_exact, const int *err,
-                                double *sums, cudaStream_t st);
+                                const PdFrameDev *frames, double *sums, cudaStream_t st);
 cudaError_t launch_frame_mean(const double *terms, const double *fw, int32_t n_frames, int32_t nq,
                               double *out, cudaStream_t st, bool normalize = true);
 // Direct transform: (Re A, Im A, |A|², Σ_m |F_m|²) per q-vector for points

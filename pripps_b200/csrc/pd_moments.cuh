@@ -27,6 +27,20 @@
 // grid point in the direct form. The sines and cosines are kept divided by
 // sin(φ/2) and cos(φ/2) in the long sequence (X, Y) and multiplied by them in
 // the short one, which removes both square roots.
+//
+// Direction form. The sum over all pairs is an average over directions,
+//
+//   Σ_ij a_i b_j sinc(q r_ij) = <A(q n) B*(q n)>,  A(k) = Σ_i a_i e^{i k·r_i},
+//
+// and the integrand is a polynomial of degree ~2·q·radius on the sphere up to a tail
+// that falls off like J_ν: a Gauss–Legendre × equispaced rule with S ≈
+// (2 q_max·radius)²/4·0.7 + … directions on a hemisphere integrates it to the same
+// accuracy as above. The phase k·r expands in the same way,
+// e^{i q x} = Σ_n i^n (2 − δ_n0) J_n(q r1) T_n(x/r1), |x| <= radius < r1, so that a
+// thread sums T_n(x/r1) = cos(nφ), cos φ = x/r1, over the atoms for its
+// direction with the same sequences as for the pairs, N·S of them instead of
+// N²/2. The amplitudes come out relative to themselves, not to N²: at the
+// deep minima of a profile this form is the more accurate one.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -35,19 +49,34 @@
 
 namespace pd {
 
+// First ν beyond which J_ν(z) stays below the bound: ν − z = a·(z/2)^{1/3} + b on
+// the Airy tail; a and b were fitted to the exact tails for z from 0.01 to 900.
+__device__ __forceinline__ double bessel_order(double z, double a, double b) {
+    return z + a * cbrt(0.5 * z) + b;
+}
+
 // Moments that q_max·d = z needs: the tail Σ_{n>=M} |c_n| is below 1e-11 (FP32
 // form, whose terms are rounded to 6e-8 each) or 1e-15 (FP64 form).
-// ν − z = a·(z/2)^{1/3} is where the Airy tail of J_ν(z) reaches the bound; a and
-// the constant were fitted to the exact tails for z from 0.01 to 900.
 __device__ __forceinline__ int moments_needed(double z, bool fp64) {
-    const double a = fp64 ? 13.0 : 9.7, b = fp64 ? 3.0 : 3.5;
-    const double m = 0.5 * (z + a * cbrt(0.5 * z) + b);
+    const double m = 0.5 * (fp64 ? bessel_order(z, 13.0, 3.0) : bessel_order(z, 9.7, 3.5));
     return m < 1e6 ? static_cast<int>(m) + 1 : 1000000;
 }
 
 // d = PD_MOM_STRETCH · 2·radius keeps φ away from π (φ <= 152°), where r²
-// determines φ poorly, at the price of 3 % more moments.
+// determines φ poorly, at the price of 3 % more moments; likewise r1.
 constexpr double PD_MOM_STRETCH = 1.03;
+
+// Direction form: orders kept of the rule and of the expansion; the tails are
+// below 1e-9 (FP32 form) and 1e-14 (FP64 form) of one pair's or atom's term.
+__device__ __forceinline__ double direction_order(double z, bool fp64) {
+    return fp64 ? bessel_order(z, 13.0, 3.0) : bessel_order(z, 8.0, 2.0);
+}
+
+// Nodes and weights of the 2h-point Gauss–Legendre rules, upper half
+// (x > 0, ascending), h = 1 … PD_GL_MAX: rule h at h·(h − 1)/2. The weights of
+// a half add up to 1. Filled once per device (prepare_direction_rules).
+constexpr int PD_GL_MAX = 128;
+__device__ double2 pd_gl_rules[PD_GL_MAX * (PD_GL_MAX + 1) / 2];
 
 // A pair's sequences. U_j = (cos(cφ)/cos(φ/2), sin(cφ)/sin(φ/2)) at c = 8j + 3.5
 // follows the three-term recurrence U_{j+1} = 2cos(8φ)·U_j − U_{j−1}. It is kept
@@ -83,9 +112,8 @@ __device__ __forceinline__ void mom_later_block(float c8, float u8, float nq, fl
 // packed ones over two pairs would, and write the halves of the packed operands in place
 // (packed over two pairs, the transposition was 90 register moves per pair:
 // 20,000 atoms, 72 moments: 2.05 ms, FMA pipe 41 % and ALU pipe 48 % busy).
-__device__ __forceinline__ void mom_seed(float r2, float inv_d2, int rep, int dbl, bool valid,
-                                         MomPair &P) {
-    const float s2 = r2 * inv_d2;          // sin²(φ/2)
+// s2 = sin²(φ/2).
+__device__ __forceinline__ void mom_seed(float s2, int rep, int dbl, bool valid, MomPair &P) {
     const float e = 1.0f - s2;             // cos²(φ/2)
     const float na = -4.0f * s2;           // −α
     const float nq = na * e;               // −sin²φ
@@ -118,6 +146,31 @@ __device__ __forceinline__ void mom_seed(float r2, float inv_d2, int rep, int db
     P.cc = c8 + c8;
 }
 
+template <int KM, bool WEIGHTED>
+__device__ __forceinline__ void mom_accumulate(const MomPair &P, float w, int nj,
+                                               float2 (&acc)[KM / 2],
+                                               float2 (&accw)[WEIGHTED ? KM / 2 : 1]) {
+    const float2 cp = make_float2(P.cc, P.cc), cn = make_float2(-P.cc, -P.cc);
+    float2 W[2] = {P.w0, P.w1};
+    float2 WV[WEIGHTED ? 4 : 1];
+    if constexpr (WEIGHTED)
+#pragma unroll
+        for (int t = 0; t < 4; ++t) WV[t] = __fmul2_rn(make_float2(w, w), P.v[t]);
+#pragma unroll
+    for (int jj = 0; jj < KM / 8; ++jj) {
+        if (jj >= nj) break;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            acc[4 * jj + t] = __ffma2_rn(W[jj & 1], P.v[t], acc[4 * jj + t]);
+            if constexpr (WEIGHTED)
+                accw[4 * jj + t] = __ffma2_rn(W[jj & 1], WV[t], accw[4 * jj + t]);
+        }
+        // W_{jj+2} = ±2cos(8φ)·W_{jj+1} + W_jj
+        if (jj + 2 < KM / 8)
+            W[jj & 1] = __ffma2_rn((jj & 1) ? cp : cn, W[(jj & 1) ^ 1], W[jj & 1]);
+    }
+}
+
 // Moments of the pairs (i, j), j0 <= j < j1, j > i, of one thread's i into
 // acc[4·jj + t] = s_jj·(Σ U.x·V.x, Σ U.y·V.y), for the first nj groups of eight of
 // the block. `at` holds the atoms [jbase, ...) in shared memory. Weighted mode
@@ -132,31 +185,104 @@ __device__ __forceinline__ void moments_range(const float4 *__restrict__ at, int
         const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
         const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
         MomPair P;
-        mom_seed(r2, inv_d2, rep, dbl, ivalid && j > i, P);
-        const float2 cp = make_float2(P.cc, P.cc), cn = make_float2(-P.cc, -P.cc);
-        float2 W[2] = {P.w0, P.w1};
-        float2 WV[WEIGHTED ? 4 : 1];
-        if constexpr (WEIGHTED)
+        mom_seed(r2 * inv_d2, rep, dbl, ivalid && j > i, P);
+        mom_accumulate<KM, WEIGHTED>(P, pj.w, nj, acc, accw);
+    }
+}
+
+// Direction form: the atoms [j0, j1) of a warp, for the thread's direction
+// dv = n/(2·r1); same layout of the sums.
+template <int KM, bool WEIGHTED>
+__device__ __forceinline__ void direction_range(const float4 *__restrict__ at, float3 dv, int j0,
+                                                int j1, int nj, int rep, int dbl,
+                                                float2 (&acc)[KM / 2],
+                                                float2 (&accw)[WEIGHTED ? KM / 2 : 1]) {
+    if (j0 >= j1) return;
+    float4 next = __ldg(at + j0);
+    for (int j = j0; j < j1; ++j) {
+        const float4 pj = next;
+        next = __ldg(at + min(j + 1, j1 - 1));
+        // sin²(φ/2) = (1 − x/r1)/2
+        const float s2 = fmaf(-dv.x, pj.x, fmaf(-dv.y, pj.y, fmaf(-dv.z, pj.z, 0.5f)));
+        MomPair P;
+        mom_seed(s2, rep, dbl, true, P);
+        mom_accumulate<KM, WEIGHTED>(P, pj.w, nj, acc, accw);
+    }
+}
+
+// FP64 form: the same sequences in double for one s2 = sin²(φ/2);
+// acc[8·jj + 2t + {0, 1}] = s_jj·(Σ U.x·V.x, Σ U.y·V.y) (and weighted by w in accw).
+template <int KM, bool WEIGHTED>
+__device__ __forceinline__ void mom_accumulate_f64(double s2, bool valid, double w, int nj,
+                                                   int rep, int dbl, double (&acc)[KM],
+                                                   double (&accw)[WEIGHTED ? KM : 1]) {
+    const double e = 1.0 - s2, na = -4.0 * s2, nq = na * e;
+    const double C1 = fma(-2.0, s2, 1.0);
+    const double c1q = C1 * C1;
+    const double c2 = c1q + nq;
+    const double c4 = fma(c2, c2, 4.0 * nq * c1q);
+    const double w4 = 4.0 * C1 * c2;
+    double c8 = fma(c4, c4, nq * w4 * w4);
+    double u8 = 2.0 * w4 * c4;
+    double vx[4], vy[4];
+    vy[0] = -2.0 * s2;
+    vx[0] = 1.0 + C1;
+    vy[1] = fma(na, C1, vy[0]);
+    const double C2 = C1 + vy[1];
+    vx[1] = C1 + C2;
+    vy[2] = fma(na, C2, vy[1]);
+    const double C3 = C2 + vy[2];
+    vx[2] = C2 + C3;
+    vy[3] = fma(na, C3, vy[2]);
+    vx[3] = C3 + (C3 + vy[3]);
+    const double c13 = C1 + C3;
+    double X = fma(2.0, c13 - C2, -1.0), Y = fma(2.0, c13 + C2, 1.0);
+    const double ts = 2.0 * s2, te = 2.0 * e;
+    const double t1 = ts * u8, t2 = te * u8, cc = c8;
+    if (rep > 0) {
+        for (int k = 0; k < dbl; ++k) {
+            const double uu = u8 * u8;
+            u8 = 2.0 * c8 * u8;
+            c8 = fma(c8, c8, nq * uu);
+        }
+        const double T1 = ts * u8, T2 = te * u8;
+        for (int k = 0; k < rep; ++k) {
+            const double x = fma(X, c8, -(Y * T1));
+            Y = fma(Y, c8, X * T2);
+            X = x;
+        }
+    }
+    double WX[2], WY[2];
+    WX[0] = valid ? X : 0.0;
+    WY[0] = valid ? Y : 0.0;
+    WX[1] = fma(WX[0], cc, -(WY[0] * t1));
+    WY[1] = fma(WY[0], cc, WX[0] * t2);
+    const double c2x = 2.0 * cc;
 #pragma unroll
-            for (int t = 0; t < 4; ++t) WV[t] = __fmul2_rn(make_float2(pj.w, pj.w), P.v[t]);
+    for (int jj = 0; jj < KM / 8; ++jj) {
+        if (jj >= nj) break;
+        const double wx = WX[jj & 1], wy = WY[jj & 1];
 #pragma unroll
-        for (int jj = 0; jj < KM / 8; ++jj) {
-            if (jj >= nj) break;
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                acc[4 * jj + t] = __ffma2_rn(W[jj & 1], P.v[t], acc[4 * jj + t]);
-                if constexpr (WEIGHTED)
-                    accw[4 * jj + t] = __ffma2_rn(W[jj & 1], WV[t], accw[4 * jj + t]);
+        for (int t = 0; t < 4; ++t) {
+            if constexpr (WEIGHTED) {
+                const double px = wx * vx[t], py = wy * vy[t];
+                acc[8 * jj + 2 * t] += px;
+                acc[8 * jj + 2 * t + 1] += py;
+                accw[8 * jj + 2 * t] = fma(w, px, accw[8 * jj + 2 * t]);
+                accw[8 * jj + 2 * t + 1] = fma(w, py, accw[8 * jj + 2 * t + 1]);
+            } else {
+                acc[8 * jj + 2 * t] = fma(wx, vx[t], acc[8 * jj + 2 * t]);
+                acc[8 * jj + 2 * t + 1] = fma(wy, vy[t], acc[8 * jj + 2 * t + 1]);
             }
-            // W_{jj+2} = ±2cos(8φ)·W_{jj+1} + W_jj
-            if (jj + 2 < KM / 8)
-                W[jj & 1] = __ffma2_rn((jj & 1) ? cp : cn, W[(jj & 1) ^ 1], W[jj & 1]);
+        }
+        if (jj + 2 < KM / 8) {
+            const double sc = (jj & 1) ? c2x : -c2x;
+            WX[jj & 1] = fma(sc, WX[(jj & 1) ^ 1], wx);
+            WY[jj & 1] = fma(sc, WY[(jj & 1) ^ 1], wy);
         }
     }
 }
 
-// FP64 form: the same sequences in double;
-// acc[8·jj + 2t + {0, 1}] = s_jj·(Σ U.x·V.x, Σ U.y·V.y) (and weighted by w_j in accw).
 template <int KM, bool WEIGHTED>
 __device__ __forceinline__ void moments_range_f64(const double4 *__restrict__ at, double4 pi, int i,
                                                   bool ivalid, int j0, int j1, double inv_d2,
@@ -165,73 +291,56 @@ __device__ __forceinline__ void moments_range_f64(const double4 *__restrict__ at
     for (int j = j0; j < j1; ++j) {
         const double4 pj = at[j];
         const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-        const double s2 = (dx * dx + dy * dy + dz * dz) * inv_d2;
-        const double e = 1.0 - s2, na = -4.0 * s2, nq = na * e;
-        const double C1 = fma(-2.0, s2, 1.0);
-        const double c1q = C1 * C1;
-        const double c2 = c1q + nq;
-        const double c4 = fma(c2, c2, 4.0 * nq * c1q);
-        const double w4 = 4.0 * C1 * c2;
-        double c8 = fma(c4, c4, nq * w4 * w4);
-        double u8 = 2.0 * w4 * c4;
-        double vx[4], vy[4];
-        vy[0] = -2.0 * s2;
-        vx[0] = 1.0 + C1;
-        vy[1] = fma(na, C1, vy[0]);
-        const double C2 = C1 + vy[1];
-        vx[1] = C1 + C2;
-        vy[2] = fma(na, C2, vy[1]);
-        const double C3 = C2 + vy[2];
-        vx[2] = C2 + C3;
-        vy[3] = fma(na, C3, vy[2]);
-        vx[3] = C3 + (C3 + vy[3]);
-        const bool valid = ivalid && j > i;
-        const double c13 = C1 + C3;
-        double X = fma(2.0, c13 - C2, -1.0), Y = fma(2.0, c13 + C2, 1.0);
-        const double ts = 2.0 * s2, te = 2.0 * e;
-        const double t1 = ts * u8, t2 = te * u8, cc = c8;
-        if (rep > 0) {
-            for (int k = 0; k < dbl; ++k) {
-                const double uu = u8 * u8;
-                u8 = 2.0 * c8 * u8;
-                c8 = fma(c8, c8, nq * uu);
-            }
-            const double T1 = ts * u8, T2 = te * u8;
-            for (int k = 0; k < rep; ++k) {
-                const double x = fma(X, c8, -(Y * T1));
-                Y = fma(Y, c8, X * T2);
-                X = x;
-            }
-        }
-        double WX[2], WY[2];
-        WX[0] = valid ? X : 0.0;
-        WY[0] = valid ? Y : 0.0;
-        WX[1] = fma(WX[0], cc, -(WY[0] * t1));
-        WY[1] = fma(WY[0], cc, WX[0] * t2);
-        const double c2x = 2.0 * cc;
-#pragma unroll
-        for (int jj = 0; jj < KM / 8; ++jj) {
-            if (jj >= nj) break;
-            const double wx = WX[jj & 1], wy = WY[jj & 1];
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                if constexpr (WEIGHTED) {
-                    const double px = wx * vx[t], py = wy * vy[t];
-                    acc[8 * jj + 2 * t] += px;
-                    acc[8 * jj + 2 * t + 1] += py;
-                    accw[8 * jj + 2 * t] = fma(pj.w, px, accw[8 * jj + 2 * t]);
-                    accw[8 * jj + 2 * t + 1] = fma(pj.w, py, accw[8 * jj + 2 * t + 1]);
-                } else {
-                    acc[8 * jj + 2 * t] = fma(wx, vx[t], acc[8 * jj + 2 * t]);
-                    acc[8 * jj + 2 * t + 1] = fma(wy, vy[t], acc[8 * jj + 2 * t + 1]);
-                }
-            }
-            if (jj + 2 < KM / 8) {
-                const double sc = (jj & 1) ? c2x : -c2x;
-                WX[jj & 1] = fma(sc, WX[(jj & 1) ^ 1], wx);
-                WY[jj & 1] = fma(sc, WY[(jj & 1) ^ 1], wy);
-            }
-        }
+        mom_accumulate_f64<KM, WEIGHTED>((dx * dx + dy * dy + dz * dz) * inv_d2, ivalid && j > i,
+                                         pj.w, nj, rep, dbl, acc, accw);
+    }
+}
+
+template <int KM, bool WEIGHTED>
+__device__ __forceinline__ void direction_range_f64(const double4 *__restrict__ at, double4 dv,
+                                                    int j0, int j1, int nj, int rep, int dbl,
+                                                    double (&acc)[KM],
+                                                    double (&accw)[WEIGHTED ? KM : 1]) {
+    for (int j = j0; j < j1; ++j) {
+        const double4 pj = at[j];
+        const double s2 = fma(-dv.x, pj.x, fma(-dv.y, pj.y, fma(-dv.z, pj.z, 0.5)));
+        mom_accumulate_f64<KM, WEIGHTED>(s2, true, pj.w, nj, rep, dbl, acc, accw);
+    }
+}
+
+// A work unit of the direction form, u-th of the frame's n_chunk·n_ablk·n_grp: the
+// longest chunks first, direction groups innermost.
+struct DirUnit {
+    int chunk, mb, grp;
+    bool ok;
+};
+__device__ __forceinline__ DirUnit direction_unit(int64_t u, const PdFrameDev &fr, int n_chunk) {
+    DirUnit d;
+    d.grp = static_cast<int>(u % fr.n_grp);
+    const int64_t r = u / fr.n_grp;
+    d.mb = static_cast<int>(r % fr.n_ablk);
+    d.chunk = static_cast<int>(r / fr.n_ablk);
+    d.ok = d.chunk < n_chunk;
+    return d;
+}
+
+// Where a unit's sums go: [chunk][v][group][moment][32 directions].
+__device__ __forceinline__ int64_t direction_slot(int chunk, int v, int grp, int nv2,
+                                                  const PdFrameDev &fr) {
+    return ((static_cast<int64_t>(chunk) * nv2 + v) * fr.n_grp + grp) * fr.n_amp * 32;
+}
+
+// The CTA's sums part[e·32 + lane] (FP64, e as in the accumulators) of one block
+// written as the moments of cos(nφ): m = s_jj·(x ± y)/2.
+__device__ __forceinline__ void direction_store(const double *__restrict__ part, int nj, int n0,
+                                                double *__restrict__ out) {
+    for (int k = threadIdx.x; k < nj * 128; k += PD_THREADS) {
+        const int lane = k & 31, t = (k >> 5) & 3, jj = k >> 7;
+        const double x = part[(8 * jj + 2 * t) * 32 + lane];
+        const double y = part[(8 * jj + 2 * t + 1) * 32 + lane];
+        const double h = (jj & 2) ? -0.5 : 0.5;
+        out[static_cast<int64_t>(n0 + 8 * jj + 4 + t) * 32 + lane] = h * (x + y);
+        out[static_cast<int64_t>(n0 + 8 * jj + 3 - t) * 32 + lane] = h * (x - y);
     }
 }
 

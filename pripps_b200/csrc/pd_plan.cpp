@@ -266,8 +266,10 @@ static void species_class_keys(int64_t n, const uint32_t *species, int32_t n_spe
 }
 
 int build_plan(const pd_request *req, const uint32_t *species, const double *w,
-               const Tuning &tun, Plan &P, std::string &msg, bool count_pairs) {
+               const Tuning &tun, Plan &P, std::string &msg, bool count_pairs,
+               double radius_hint) {
     P = Plan();
+    P.radius_hint = radius_hint;
     P.n_atoms = static_cast<int64_t>(req->n_atoms);
     P.nq = static_cast<int32_t>(req->nq);
     P.n_frames = static_cast<int32_t>(req->n_frames ? req->n_frames : 1);
@@ -434,6 +436,31 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
         P.lat_bins = off;
     }
 
+    // ---- atom chunks of the direction form: about 1/6 of the atoms each (so
+    // that a few direction groups already fill the GPU, and the CTA's FP64 merge
+    // of a chunk stays a small part of it), longest first
+    {
+        const int64_t len = std::clamp<int64_t>(next_pow2(n / 6), 256, 16384);
+        for (int k = 0; k < c; ++k) {
+            const int64_t nk = static_cast<int64_t>(members[k].size());
+            const int64_t parts = (nk + len - 1) / len;
+            for (int64_t t = 0; t < parts; ++t)
+                P.chunks.push_back(PdChunk{k, P.cls_start[k] + static_cast<int32_t>(nk * t / parts),
+                                           P.cls_start[k] +
+                                               static_cast<int32_t>(nk * (t + 1) / parts),
+                                           0});
+        }
+        std::stable_sort(P.chunks.begin(), P.chunks.end(), [](const PdChunk &x, const PdChunk &y) {
+            return x.j1 - x.j0 > y.j1 - y.j0;
+        });
+        P.cls_ptr.assign(c + 1, 0);
+        for (int k = 0; k < c; ++k) {
+            for (size_t t = 0; t < P.chunks.size(); ++t)
+                if (P.chunks[t].cls == k) P.cls_chunk.push_back(static_cast<int32_t>(t));
+            P.cls_ptr[k + 1] = static_cast<int32_t>(P.cls_chunk.size());
+        }
+    }
+
     // ---- tiles of one frame, in creation order
     const int K = P.tun.K, TJ = P.tun.TJ;
     P.nqb = (P.nq + K - 1) / K;
@@ -571,6 +598,8 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
             for (int f = 0; f < P.n_frames; ++f) {
                 PdJob jb = frame_jobs[o * P.nqb + qb];
                 jb.frame = f;
+                jb.ord = static_cast<int32_t>(P.jobs.size() / P.n_frames);
+                jb.n_ord = static_cast<int32_t>(P.jobs_per_frame);
                 jb.slot += static_cast<int64_t>(f) * P.slots_per_frame;
                 P.jobs.push_back(jb);
             }
@@ -578,6 +607,80 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
     }
     set_reduction(P);
     return PD_OK;
+}
+
+double max_radius(const double *xyz, int64_t n, int64_t n_frames) {
+    double best = 0.0;
+    for (int64_t f = 0; f < n_frames; ++f) {
+        const double *p = xyz + 3 * n * f;
+        double s[3] = {0, 0, 0};
+        for (int64_t i = 0; i < n; ++i)
+            for (int a = 0; a < 3; ++a) s[a] += p[3 * i + a];
+        for (double &v : s) v /= static_cast<double>(n);
+        for (int64_t i = 0; i < n; ++i) {
+            const double x = p[3 * i] - s[0], y = p[3 * i + 1] - s[1], z = p[3 * i + 2] - s[2];
+            best = std::max(best, x * x + y * y + z * z);
+        }
+    }
+    return std::sqrt(best);
+}
+
+// Sizes of the direction form for frames of up to the hinted radius (pd_pack
+// decides per frame, with the same formulas, whether it fits and pays).
+static void set_directions(Plan &P) {
+    P.amp = PdAmpShape{};
+    P.amp.nq = P.nq;
+    P.amp.block = P.mom.block;
+    P.amp.rank = static_cast<int32_t>(P.rank);
+    P.amp.world = static_cast<int32_t>(P.world);
+    P.amp.n_cls = P.n_cls;
+    P.amp.nv2 = P.mode == PD_MODE_WEIGHTED ? 2 : 1;
+    P.amp.n_chunk = static_cast<int32_t>(P.chunks.size());
+    // Below 150 atoms the pairs are always fewer than the directions. The jobs
+    // carry the work units, so every rank needs jobs of every frame. The test
+    // hook needs the pair tiles.
+    if (P.n_atoms < 150 || P.jobs_per_frame < 2 * static_cast<int64_t>(P.world) ||
+        (P.world > 1 && P.n_frames > 1) || P.mom.block == 0 || P.test_expire)
+        return;
+    // unknown coordinates: 20 cubic Angstrom per atom, elongated up to about 2.5 : 1
+    const double radius =
+        P.radius_hint >= 0.0
+            ? P.radius_hint
+            : 1.9 * std::cbrt(static_cast<double>(P.n_atoms) * 20.0 * 3.0 / (4.0 * M_PI));
+    const bool fp64 = P.precision == PD_FP64;
+    auto order = [&](double z) {
+        return fp64 ? z + 13.0 * std::cbrt(0.5 * z) + 3.0 : z + 8.0 * std::cbrt(0.5 * z) + 2.0;
+    };
+    const double z = 2.0 * radius * P.qmax;
+    const double top = order(z), mo = order(1.03 * radius * P.qmax);
+    if (!(top < 500.0) || !(mo < PD_MAX_DIR_MOMENTS - 8.0)) return;
+    const int h = static_cast<int>(top * 0.25) + 1;
+    int64_t S = 0;
+    for (int i = 0; i < h; ++i)  // rings at nearly the Gauss angles, one point to spare each
+        S += std::max(4, static_cast<int>(order(z * std::sin(M_PI * (i + 0.75) / (2 * h + 0.5)))) + 2);
+    const int64_t groups = (S + 31) / 32, mine = (groups + P.world - 1) / P.world;
+    const int64_t m8 = (static_cast<int64_t>(mo) + 8) & ~int64_t{7};
+    const double zn = 2.0 * 1.03 * radius * P.qmax;
+    const int64_t nodes = static_cast<int64_t>(0.5 * (zn + 13.0 * std::cbrt(0.5 * zn) + 3.0)) + 1;
+    // amplitudes of every class at a tile of nodes, 32 directions each
+    const int64_t room = PD_DIR_SMEM / 8 - m8 * (16 + 32);
+    const int64_t tile = std::min<int64_t>(16, room / (P.n_cls * P.amp.nv2 * 64));
+    if (tile < 1) return;
+    const int64_t slots = P.amp.n_chunk * P.amp.nv2 * mine * m8 * 32;
+    if (slots * 8 * P.n_frames > (int64_t{4} << 30)) return;
+    P.amp.dir_cap = static_cast<int32_t>(groups * 32);
+    P.amp.grp_cap = static_cast<int32_t>(mine);
+    P.amp.amp_cap = static_cast<int32_t>(std::min<int64_t>(m8, PD_MAX_DIR_MOMENTS));
+    P.amp.node_cap = static_cast<int32_t>(nodes);
+    P.amp.node_tile = static_cast<int32_t>(tile);
+    P.amp.slot_cap = slots;
+}
+
+void drop_directions(Plan &P) {
+    P.amp.dir_cap = P.amp.grp_cap = P.amp.amp_cap = P.amp.node_cap = 0;
+    P.amp.slot_cap = 0;
+    P.mom.dir_cap = P.mom.grp_cap = P.mom.amp_cap = P.mom.node_cap = 0;
+    P.mom.slot_cap = 0;
 }
 
 void set_reduction(Plan &P) {
@@ -596,6 +699,19 @@ void set_reduction(Plan &P) {
         std::min<int64_t>({PD_MAX_MOMENTS, static_cast<int64_t>(P.nqb) * m.block,
                            per_q * P.nq + 8 * P.nqb}) & ~int64_t{7});
     if (m.max_moments < 8) m.block = 0;
+    set_directions(P);
+    m.dir_cap = P.amp.dir_cap;
+    m.grp_cap = P.amp.grp_cap;
+    m.amp_cap = P.amp.amp_cap;
+    m.node_cap = P.amp.node_cap;
+    m.n_chunk = P.amp.n_chunk;
+    m.n_cls = P.amp.n_cls;
+    m.nv2 = P.amp.nv2;
+    m.rank = P.amp.rank;
+    m.world = P.amp.world;
+    m.slot_cap = P.amp.slot_cap;
+    m.n_atoms = P.n_atoms;
+    m.nq = P.nq;
     PdReduceShape &r = P.red;
     r = PdReduceShape{};
     r.n_pairs = P.n_pairs;
@@ -604,8 +720,9 @@ void set_reduction(Plan &P) {
     r.nqb = P.nqb;
     r.block = m.block;
     r.max_moments = m.block ? m.max_moments : 0;
+    r.n_z = (std::max(P.nq, r.max_moments) + 127) / 128;
+    r.max_moments = std::max(r.max_moments, P.amp.node_cap);
     r.width = std::max(P.nq, r.max_moments);
-    r.n_z = (r.width + 127) / 128;
     // A block adds its share of a class pair's slot list serially: lists of
     // more than a few hundred entries are shared by up to 16 blocks (one
     // frame; the frames of a batch fill the GPU by themselves).
@@ -634,6 +751,8 @@ int shard_plan(const Plan &full, uint32_t rank, uint32_t world, Plan &out) {
             n = std::max(n, 1 + static_cast<int>((jb.slot >> (PD_SLOT_MAP_SHIFT + 2 * w)) & 3));
         return n;
     };
+    out.rank = rank;
+    out.world = world;
     out.jobs.clear();
     for (size_t t = rank; t < full.jobs.size(); t += world) {
         const PdJob &jb = full.jobs[t];
@@ -660,6 +779,10 @@ int shard_plan(const Plan &full, uint32_t rank, uint32_t world, Plan &out) {
         }
         out.lptr[e + 1] = static_cast<int64_t>(out.lidx.size());
     }
+    // ordinals among the rank's own jobs of each frame
+    std::vector<int32_t> count(static_cast<size_t>(out.n_frames), 0);
+    for (PdJob &jb : out.jobs) jb.ord = count[static_cast<size_t>(jb.frame)]++;
+    for (PdJob &jb : out.jobs) jb.n_ord = count[static_cast<size_t>(jb.frame)];
     set_reduction(out);
     return PD_OK;
 }

@@ -61,6 +61,13 @@ struct Plan {
     std::vector<int64_t> lidx;  // slot indices within a frame
     PdMomentRule mom{};     // when a frame takes the moment form
     PdReduceShape red{};    // sizes of the slot reduction
+    // direction form: atom chunks (longest first), the chunks of each class in
+    // chunk order, and the sizes its device arrays are given
+    std::vector<PdChunk> chunks;
+    std::vector<int32_t> cls_ptr, cls_chunk;
+    PdAmpShape amp{};
+    double radius_hint = -1.0;  // largest distance from the centroid, < 0: not known
+    uint32_t rank = 0, world = 1;
     uint64_t pairs_covered = 0; // per frame, unordered pairs over all tiles
 
     // lattice sets (class mode, one frame): their self pairs are counted per
@@ -90,8 +97,17 @@ int shard_plan(const Plan &full, uint32_t rank, uint32_t world, Plan &out);
 
 // Build the plan from host-side species and weights (hyd may be NULL).
 // count_pairs fills Plan::pairs_covered (an O(N · tiles per block) host loop
-// that only pd_plan_inspect needs).
+// that only pd_plan_inspect needs). radius_hint sizes the direction form's arrays: the
+// largest distance of an atom from its frame's centroid, or < 0 when the
+// coordinates are not known yet (a generous estimate from the atom count).
 int build_plan(const pd_request *req, const uint32_t *species_host, const double *weights_host,
-               const Tuning &tun, Plan &plan, std::string &msg, bool count_pairs = false);
+               const Tuning &tun, Plan &plan, std::string &msg, bool count_pairs = false,
+               double radius_hint = -1.0);
+
+// Largest distance of an atom from its frame's centroid (host coordinates).
+double max_radius(const double *xyz, int64_t n_atoms, int64_t n_frames);
+
+// Give up the direction form's arrays (a request that only fits without them).
+void drop_directions(Plan &P);
 
 }  // namespace pd

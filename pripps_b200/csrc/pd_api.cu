@@ -230,6 +230,7 @@ struct pd_ctx {
     std::condition_variable plan_cv;
     std::map<uint64_t, std::shared_ptr<PdTicket>> tickets;
     uint64_t next_ticket = 1;
+    double last_small = -1e9;  // submission time of the latest small request
     bool stop = false;
     std::thread worker;
     std::vector<std::thread> planners;  // host planning, PD_PLANNERS threads
@@ -701,6 +702,7 @@ struct PdTicket {
     bool taken = false;               // result copied out by pd_wait
     size_t next_job = 0;              // first tile not yet issued
     bool express_wait = false;        // small: waits for a free express lane
+    bool small = false;               // by its pair·q count: goes before larger ones
     bool finish_issued = false;       // reduction (or, if cancelled, the drain) enqueued
     bool drained_only = false;        // cancelled after admission: no reduction was run
     uint32_t used_streams = 0;        // lane streams that ran some of its tiles
@@ -754,6 +756,15 @@ constexpr double EXPRESS_COST = PD_EXPRESS_COST;
 #define PD_EXPRESS_MAX_WAIT 0.25
 #endif
 constexpr double EXPRESS_MAX_WAIT = PD_EXPRESS_MAX_WAIT;
+// Larger requests leave the GPU to a burst of small ones: while a small request
+// is queued, and for this long (s) after one was submitted, the steps issue
+// nothing of a larger request that was admitted less than EXPRESS_MAX_WAIT
+// ago. (A 25,000-atom request takes under a millisecond, less than it takes a
+// client to submit a burst; without this it would run between its members.)
+#ifndef PD_SMALL_GRACE
+#define PD_SMALL_GRACE 0.5e-3
+#endif
+constexpr double SMALL_GRACE = PD_SMALL_GRACE;
 constexpr int EXPRESS = STEP_BUFS;  // row of the express lanes
 static_assert((STEP_BUFS + 1) * STEP_LANES <= 32, "lane bits of PdTicket::used_streams");
 
@@ -892,6 +903,7 @@ void worker_main(pd_ctx *ctx) {
     size_t rr = 0;
     for (;;) {
         std::vector<std::shared_ptr<PdTicket>> head;  // planned front of the queue
+        bool hold_large = false;
         {
             std::unique_lock<std::mutex> lk(ctx->qmu);
             bool waiting_device = false;
@@ -914,6 +926,8 @@ void worker_main(pd_ctx *ctx) {
                     ++it;
                 }
             }
+            hold_large = now_s() - ctx->last_small < SMALL_GRACE;
+            for (uint64_t id : ctx->pending) hold_large |= ctx->tickets[id]->small;
             for (uint64_t id : ctx->pending) {
                 auto t = ctx->tickets[id];
                 if (t->plan_state == 0) break;  // FIFO: wait for its planning
@@ -1065,8 +1079,11 @@ void worker_main(pd_ctx *ctx) {
         // requests (rotating start), each request's tiles into the lane of
         // its kernel variant; up to STEP_LANES variants per step.
         std::vector<std::shared_ptr<PdTicket>> cand;
+        for (auto &t : active) hold_large |= t->small && t->express_wait;
+        const double t_step = now_s();
         for (auto &t : active)
-            if (!t->canceled && !t->express_wait && t->next_job < t->dp.P.jobs.size())
+            if (!t->canceled && !t->express_wait && t->next_job < t->dp.P.jobs.size() &&
+                (t->small || !hold_large || t_step - t->t_admit > EXPRESS_MAX_WAIT))
                 cand.push_back(t);
         Lane *step = lanes[cur];
         std::tuple<int, int, int, int> lane_key[STEP_LANES];
@@ -1673,8 +1690,12 @@ int pd_submit(pd_ctx *ctx, const pd_request *req, uint64_t *ticket) {
     t->req.ff_water = req->hyd_weights ? t->ffW.data() : nullptr;
     t->req.frame_weights = req->frame_weights ? t->fw.data() : nullptr;
     t->t_submit = now_s();
+    t->small = 0.5 * static_cast<double>(n) * static_cast<double>(n) * static_cast<double>(nq) *
+                   static_cast<double>(nf) * (req->precision == PD_FP64 ? 24.0 : 1.0) <=
+               EXPRESS_COST;
     {
         std::lock_guard<std::mutex> lk(ctx->qmu);
+        if (t->small) ctx->last_small = t->t_submit;
         if (!ctx->worker_started) {
             ctx->worker = std::thread(worker_main, ctx);
             const unsigned hw = std::max(1u, std::thread::hardware_concurrency());

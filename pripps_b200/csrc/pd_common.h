@@ -136,8 +136,9 @@ struct PdMomentRule {
 struct PdAmpShape {
     int32_t n_chunk, n_cls, nv2, nq;
     int32_t dir_cap, grp_cap, amp_cap, node_cap;
-    int32_t node_tile;  // nodes per block of the sums' kernel
-    int32_t rank, world, block;
+    int32_t node_tile;  // nodes per block of the sums' kernel (a multiple of 4)
+    int32_t sum_smem;   // its shared memory in doubles
+    int32_t rank, world, block, pad_;
     int64_t slot_cap;
 };
 

@@ -804,71 +804,101 @@ __device__ __forceinline__ MomJob moment_job(int j0, int j1, int qb, int n_mblk,
     return m;
 }
 
-// Atoms a warp sums in FP32 for its directions before the sums go into the CTA's
-// FP64 partial sums.
+// Atoms a thread sums in FP32 for its direction before the CTA's sums go, in FP64,
+// into the unit's slot.
 #ifndef PD_DIR_RUN
 #define PD_DIR_RUN 512
 #endif
 
-// Direction form: the job's work units (see direction_unit), one at a time. The
-// CTA's four warps share the unit's atoms, each lane one of its 32 directions;
-// part (FP64, [v][moment sum][32]) collects the warps' runs in warp order, so the
-// sums do not depend on timing.
-template <int K, int MODE>
-__device__ __forceinline__ void direction_units(const PdJob &jb, const PdReqDev &rq,
-                                                const PdFrameDev &fr, double *__restrict__ part,
-                                                int warp, int lane) {
-    constexpr int KM = pd_moment_block(K);
+// Direction form: one work unit. A lane is one of 8 directions for every 16th atom
+// of the chunk, so 128 threads share 8·n_amp sums: few enough units fill the GPU
+// with short loops on small structures, and the slots stay small. A run's FP32 sums
+// of the 16 atom lanes meet in shared memory (buf) and are added in lane order
+// in FP64.
+template <int KM, bool W, bool ILP>
+__device__ __forceinline__ void direction_unit_run(const float4 *__restrict__ at, const PdChunk &ck,
+                                                   float3 dv, const DirUnit &un, int n_amp,
+                                                   float *__restrict__ buf,
+                                                   double *__restrict__ out0,
+                                                   double *__restrict__ out1) {
     constexpr int DBL = KM == 128 ? 4 : (KM == 64 ? 3 : 2);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int al = threadIdx.x / PD_DIR_DIRS;
+    const int nj = min(KM, n_amp - un.mb * KM) >> 3;
+    constexpr int RUN = PD_DIR_RUN * PD_DIR_LANES;
+    for (int r0 = ck.j0; r0 < ck.j1; r0 += RUN) {
+        float2 acc[KM / 2], accw[W ? KM / 2 : 1];
+#pragma unroll
+        for (int t = 0; t < KM / 2; ++t) {
+            acc[t] = make_float2(0.0f, 0.0f);
+            if constexpr (W) accw[t] = make_float2(0.0f, 0.0f);
+        }
+        direction_range<KM, W, ILP>(at, dv, r0 + al, min(ck.j1, r0 + RUN), nj, un.mb, DBL, acc,
+                                    accw);
+        // [v][warp][e][32 lanes], each row turned by 8·e lanes: reads of one
+        // atom lane's 8 directions at four consecutive e touch all banks once
+        float *b = buf + warp * KM * 32;
+#pragma unroll
+        for (int t = 0; t < KM / 2; ++t) {
+            if (t >= 4 * nj) break;
+            b[(2 * t) * 32 + ((lane + 16 * t) & 31)] = acc[t].x;
+            b[(2 * t + 1) * 32 + ((lane + 16 * t + 8) & 31)] = acc[t].y;
+            if constexpr (W) {
+                float *bw = b + PD_WARPS * KM * 32;
+                bw[(2 * t) * 32 + ((lane + 16 * t) & 31)] = accw[t].x;
+                bw[(2 * t + 1) * 32 + ((lane + 16 * t + 8) & 31)] = accw[t].y;
+            }
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < nj * 4 * PD_DIR_DIRS; k += PD_THREADS) {
+            const int dir = k % PD_DIR_DIRS, i = k / PD_DIR_DIRS;  // i = 4·jj + t
+#pragma unroll
+            for (int v = 0; v < (W ? 2 : 1); ++v) {
+                double x = 0.0, y = 0.0;
+#pragma unroll
+                for (int w = 0; w < PD_WARPS; ++w) {
+                    const float *c = buf + ((v * PD_WARPS + w) * KM + 2 * i) * 32;
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) {
+                        x += static_cast<double>(c[(a * 8 + dir + 16 * i) & 31]);
+                        y += static_cast<double>(c[32 + ((a * 8 + dir + 16 * i + 8) & 31)]);
+                    }
+                }
+                direction_put(v ? out1 : out0, un.mb * KM, i >> 2, i & 3, dir, x, y, r0 == ck.j0);
+            }
+        }
+        __syncthreads();  // buf is rewritten by the next run
+    }
+}
+
+// The job's work units (see direction_unit), one after another.
+template <int K, int MODE>
+__device__ __noinline__ void direction_units(const PdJob &jb, const PdReqDev &rq,
+                                             const PdFrameDev &fr, float *__restrict__ buf) {
+    constexpr int KM = pd_moment_block(K);
     constexpr bool W = MODE == PD_MODE_WEIGHTED;
+    const int lane = threadIdx.x & 31;
     const float4 *__restrict__ at = rq.atoms32 + static_cast<size_t>(jb.frame) * rq.n_pad;
-    const int64_t n_units = static_cast<int64_t>(rq.amp.n_chunk) * fr.n_ablk * fr.n_grp;
+    const int64_t n_units = static_cast<int64_t>(rq.amp.n_chunk) * fr.n_ablk * fr.n_grp *
+                            (32 / PD_DIR_DIRS);
+    double *slots = rq.slots + static_cast<int64_t>(jb.frame) * rq.amp.slot_cap;
     for (int64_t u = jb.ord; u < n_units; u += jb.n_ord) {
-        const DirUnit un = direction_unit(u, fr, rq.amp.n_chunk);
+        const DirUnit un = direction_unit(u, fr);
         const PdChunk ck = rq.chunks[un.chunk];
         const double4 D = rq.dirs[static_cast<int64_t>(jb.frame) * rq.amp.dir_cap +
                                   (static_cast<int64_t>(un.grp) * rq.amp.world + rq.amp.rank) * 32 +
-                                  lane];
+                                  un.sub * PD_DIR_DIRS + lane % PD_DIR_DIRS];
         const float3 dv = make_float3(static_cast<float>(D.x), static_cast<float>(D.y),
                                       static_cast<float>(D.z));
-        const int per = (ck.j1 - ck.j0 + PD_WARPS - 1) / PD_WARPS;
-        const int w0 = min(ck.j1, ck.j0 + warp * per), w1 = min(ck.j1, w0 + per);
-        const int nj = min(KM, fr.n_amp - un.mb * KM) >> 3;
-        for (int run = 0; run < per; run += PD_DIR_RUN) {
-            float2 acc[KM / 2], accw[W ? KM / 2 : 1];
-#pragma unroll
-            for (int t = 0; t < KM / 2; ++t) {
-                acc[t] = make_float2(0.0f, 0.0f);
-                if constexpr (W) accw[t] = make_float2(0.0f, 0.0f);
-            }
-            direction_range<KM, W>(at, dv, min(w1, w0 + run), min(w1, w0 + run + PD_DIR_RUN), nj,
-                                   un.mb, DBL, acc, accw);
-            for (int w = 0; w < PD_WARPS; ++w) {
-                if (warp == w) {
-                    const bool first = run == 0 && w == 0;
-#pragma unroll
-                    for (int t = 0; t < KM / 2; ++t) {
-                        if (t >= 4 * nj) break;
-                        double *p = part + 2 * t * 32 + lane;
-                        p[0] = (first ? 0.0 : p[0]) + static_cast<double>(acc[t].x);
-                        p[32] = (first ? 0.0 : p[32]) + static_cast<double>(acc[t].y);
-                        if constexpr (W) {
-                            p += KM * 32;
-                            p[0] = (first ? 0.0 : p[0]) + static_cast<double>(accw[t].x);
-                            p[32] = (first ? 0.0 : p[32]) + static_cast<double>(accw[t].y);
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-        }
-        double *out = rq.slots + static_cast<int64_t>(jb.frame) * rq.amp.slot_cap;
-        direction_store(part, nj, un.mb * KM,
-                        out + direction_slot(un.chunk, 0, un.grp, rq.amp.nv2, fr));
-        if constexpr (W)
-            direction_store(part + KM * 32, nj, un.mb * KM,
-                            out + direction_slot(un.chunk, 1, un.grp, rq.amp.nv2, fr));
-        __syncthreads();  // part is rewritten by the next unit
+        double *out0 = slots + direction_slot(un.chunk, 0, un.grp, rq.amp.nv2, fr) +
+                       un.sub * PD_DIR_DIRS;
+        double *out1 = W ? slots + direction_slot(un.chunk, 1, un.grp, rq.amp.nv2, fr) +
+                               un.sub * PD_DIR_DIRS
+                         : out0;
+        if (KM > 64 && fr.n_amp <= 64)  // half the accumulators: two atoms at a time
+            direction_unit_run<64, W, true>(at, ck, dv, un, fr.n_amp, buf, out0, out1);
+        else
+            direction_unit_run<KM, W, KM <= 64 && !W>(at, ck, dv, un, fr.n_amp, buf, out0, out1);
     }
 }
 
@@ -960,8 +990,7 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
         const int kq0 = jb.qb * K;
         const PdFrameDev fr = rq.frames[jb.frame];
         if (fr.n_grp > 0) {
-            direction_units<K, MODE>(jb, rq, fr, reinterpret_cast<double *>(pd_dyn_atoms), warp,
-                                     lane);
+            direction_units<K, MODE>(jb, rq, fr, reinterpret_cast<float *>(pd_dyn_atoms));
             __syncthreads();  // every thread has read s_job
             continue;
         }
@@ -1213,23 +1242,25 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
 }
 
 // ---------------------------------------------------------------- K2 (FP64)
-// direction_units in FP64 (one run per unit).
+// direction_units in FP64 (one run per unit; the atom lanes of a warp meet by
+// shuffles, the warps in shared memory, part[v][warp][e][8]).
 template <int K, int MODE>
-__device__ __forceinline__ void direction_units_f64(const PdJob &jb, const PdReqDev &rq,
-                                                    const PdFrameDev &fr,
-                                                    double *__restrict__ part, int warp, int lane) {
+__device__ __noinline__ void direction_units_f64(const PdJob &jb, const PdReqDev &rq,
+                                                 const PdFrameDev &fr, double *__restrict__ part) {
     constexpr int DBL = K == 64 ? 3 : (K == 32 ? 2 : 1);
     constexpr bool W = MODE == PD_MODE_WEIGHTED;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int al = threadIdx.x / PD_DIR_DIRS;
     const double4 *__restrict__ at = rq.atoms64 + static_cast<size_t>(jb.frame) * rq.n_pad;
-    const int64_t n_units = static_cast<int64_t>(rq.amp.n_chunk) * fr.n_ablk * fr.n_grp;
+    const int64_t n_units = static_cast<int64_t>(rq.amp.n_chunk) * fr.n_ablk * fr.n_grp *
+                            (32 / PD_DIR_DIRS);
+    double *slots = rq.slots + static_cast<int64_t>(jb.frame) * rq.amp.slot_cap;
     for (int64_t u = jb.ord; u < n_units; u += jb.n_ord) {
-        const DirUnit un = direction_unit(u, fr, rq.amp.n_chunk);
+        const DirUnit un = direction_unit(u, fr);
         const PdChunk ck = rq.chunks[un.chunk];
         const double4 D = rq.dirs[static_cast<int64_t>(jb.frame) * rq.amp.dir_cap +
                                   (static_cast<int64_t>(un.grp) * rq.amp.world + rq.amp.rank) * 32 +
-                                  lane];
-        const int per = (ck.j1 - ck.j0 + PD_WARPS - 1) / PD_WARPS;
-        const int w0 = min(ck.j1, ck.j0 + warp * per), w1 = min(ck.j1, w0 + per);
+                                  un.sub * PD_DIR_DIRS + lane % PD_DIR_DIRS];
         const int nj = min(K, fr.n_amp - un.mb * K) >> 3;
         double acc[K], accw[W ? K : 1];
 #pragma unroll
@@ -1237,25 +1268,39 @@ __device__ __forceinline__ void direction_units_f64(const PdJob &jb, const PdReq
             acc[e] = 0.0;
             if constexpr (W) accw[e] = 0.0;
         }
-        direction_range_f64<K, W>(at, D, w0, w1, nj, un.mb, DBL, acc, accw);
-        for (int w = 0; w < PD_WARPS; ++w) {
-            if (warp == w) {
+        direction_range_f64<K, W>(at, D, ck.j0 + al, ck.j1, nj, un.mb, DBL, acc, accw);
 #pragma unroll
-                for (int e = 0; e < K; ++e) {
-                    if (e >= 8 * nj) break;
-                    double *p = part + e * 32 + lane;
-                    p[0] = (w == 0 ? 0.0 : p[0]) + acc[e];
-                    if constexpr (W) p[K * 32] = (w == 0 ? 0.0 : p[K * 32]) + accw[e];
-                }
+        for (int e = 0; e < K; ++e) {
+            if (e >= 8 * nj) break;
+            double a = acc[e];
+            a += __shfl_xor_sync(0xffffffffu, a, 8);
+            a += __shfl_xor_sync(0xffffffffu, a, 16);
+            if (lane < PD_DIR_DIRS) part[(warp * K + e) * PD_DIR_DIRS + lane] = a;
+            if constexpr (W) {
+                double b = accw[e];
+                b += __shfl_xor_sync(0xffffffffu, b, 8);
+                b += __shfl_xor_sync(0xffffffffu, b, 16);
+                if (lane < PD_DIR_DIRS)
+                    part[((PD_WARPS + warp) * K + e) * PD_DIR_DIRS + lane] = b;
             }
-            __syncthreads();
         }
-        double *out = rq.slots + static_cast<int64_t>(jb.frame) * rq.amp.slot_cap;
-        direction_store(part, nj, un.mb * K,
-                        out + direction_slot(un.chunk, 0, un.grp, rq.amp.nv2, fr));
-        if constexpr (W)
-            direction_store(part + K * 32, nj, un.mb * K,
-                            out + direction_slot(un.chunk, 1, un.grp, rq.amp.nv2, fr));
+        __syncthreads();
+        for (int k = threadIdx.x; k < nj * 4 * PD_DIR_DIRS; k += PD_THREADS) {
+            const int dir = k % PD_DIR_DIRS, i = k / PD_DIR_DIRS;
+#pragma unroll
+            for (int v = 0; v < (W ? 2 : 1); ++v) {
+                double x = 0.0, y = 0.0;
+#pragma unroll
+                for (int w = 0; w < PD_WARPS; ++w) {
+                    const double *c = part + ((v * PD_WARPS + w) * K + 2 * i) * PD_DIR_DIRS + dir;
+                    x += c[0];
+                    y += c[PD_DIR_DIRS];
+                }
+                direction_put(slots + direction_slot(un.chunk, v, un.grp, rq.amp.nv2, fr) +
+                                  un.sub * PD_DIR_DIRS,
+                              un.mb * K, i >> 2, i & 3, dir, x, y, true);
+            }
+        }
         __syncthreads();  // part is rewritten by the next unit
     }
 }
@@ -1270,7 +1315,7 @@ __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(con
     __shared__ int s_job;
     __shared__ double s_q[K];
     __shared__ double s_part[PD_WARPS * NV * K];
-    __shared__ double s_dir[NACC * K * 32];  // direction form: sums of the CTA's directions
+    __shared__ double s_dir[NACC * PD_WARPS * K * PD_DIR_DIRS];  // direction form
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int n_jobs = *n_jobs_ptr;
@@ -1284,7 +1329,7 @@ __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(con
         const PdReqDev rq = reqs[jb.req];
         const PdFrameDev fr = rq.frames[jb.frame];
         if (fr.n_grp > 0) {
-            direction_units_f64<K, MODE>(jb, rq, fr, s_dir, warp, lane);
+            direction_units_f64<K, MODE>(jb, rq, fr, s_dir);
             __syncthreads();  // every thread has read s_job
             continue;
         }
@@ -1758,45 +1803,61 @@ __global__ void __launch_bounds__(PD_DSUM_THREADS)
     const int tile = blockIdx.x % n_nt, grp = blockIdx.x / n_nt;
     if (grp >= fr.n_grp || tile * NT >= fr.n_node) return;
     const int M = fr.n_amp, nn = min(NT, fr.n_node - tile * NT);
+    const int ncv = sh.n_cls * NV2;             // class sums (plain, weighted)
     double *s_g = s_dyn;                        // [M][NT]
-    double *s_m = s_g + sh.amp_cap * NT;        // [M][32]
-    double *s_e = s_m + sh.amp_cap * 32;        // [n_cls][NV2][NT][2][32]
+    double *s_e = s_g + M * NT;                 // [n_cls][NV2][NT][2][32]
+    double *s_m = s_e + ncv * NT * 64;          // [batch][M][32]
+    const int batch = min(ncv, (sh.sum_smem - M * NT - ncv * NT * 64) / (M * 32));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x < nn)
-        s_scale[threadIdx.x] = direction_coefficients(
-            direction_node(tile * NT + threadIdx.x, fr.n_node, qmax) * fr.r1, M, s_g + threadIdx.x,
-            NT);
+    if (warp == PD_DSUM_WARPS - 1 && lane < nn)
+        s_scale[lane] = direction_coefficients(
+            direction_node(tile * NT + lane, fr.n_node, qmax) * fr.r1, M, s_g + lane, NT);
     const double *sl = slots + static_cast<int64_t>(f) * sh.slot_cap;
-    for (int cv = 0; cv < sh.n_cls * NV2; ++cv) {
-        const int c = cv / NV2, v = cv % NV2;
-        const int e0 = cls_ptr[c], e1 = cls_ptr[c + 1];
-        __syncthreads();  // the previous class's moments are read
-        for (int k = threadIdx.x; k < M * 32; k += PD_DSUM_THREADS) {
+    for (int c0 = 0; c0 < ncv; c0 += batch) {  // as many classes at once as fit
+        const int nb = min(batch, ncv - c0);
+        if (c0) __syncthreads();  // the previous classes' moments are read
+        // two moments' rows of 32 directions per warp and step, all loads of a
+        // warp in flight together
+        for (int k = threadIdx.x; k < nb * M * 32; k += PD_DSUM_THREADS) {
+            const int cb = k / (M * 32), i = k - cb * (M * 32);
+            const int c = (c0 + cb) / NV2, v = (c0 + cb) % NV2;
+            const int e1 = cls_ptr[c + 1];
             double m = 0.0;
-            for (int e = e0; e < e1; ++e)
-                m += sl[direction_slot(cls_chunk[e], v, grp, NV2, fr) + k];
-            s_m[k] = k < 32 ? (v ? cls[c].w1 : cls[c].n) : m;
+            for (int e = cls_ptr[c]; e < e1; e += 4) {
+                double x[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    x[u] = e + u < e1
+                               ? __ldg(sl + direction_slot(cls_chunk[e + u], v, grp, NV2, fr) + i)
+                               : 0.0;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) m += x[u];
+            }
+            s_m[k] = i < 32 ? (v ? cls[c].w1 : cls[c].n) : m;
         }
         __syncthreads();
-        for (int t = warp; t < nn; t += 2 * PD_DSUM_WARPS) {  // two nodes at a time
-            const int t2 = min(t + PD_DSUM_WARPS, nn - 1);
-            double er = 0, ei = 0, fr2 = 0, fi2 = 0;
-            const double *ga = s_g + t, *gb = s_g + t2;
-#pragma unroll 4
+        // (class, four nodes) per warp and step
+        const int n4 = (nn + 3) / 4;
+        for (int k = warp; k < nb * n4; k += PD_DSUM_WARPS) {
+            const int cb = k / n4, t0 = (k - cb * n4) * 4;
+            const double *mm = s_m + cb * (M * 32) + lane;
+            const double *g = s_g + t0;
+            double er[4] = {0, 0, 0, 0}, ei[4] = {0, 0, 0, 0};
+#pragma unroll 2
             for (int n = 0; n < M; n += 2) {  // M is a multiple of 8
-                const double m0 = s_m[n * 32 + lane], m1 = s_m[(n + 1) * 32 + lane];
-                er = fma(ga[n * NT], m0, er);
-                ei = fma(ga[(n + 1) * NT], m1, ei);
-                fr2 = fma(gb[n * NT], m0, fr2);
-                fi2 = fma(gb[(n + 1) * NT], m1, fi2);
+                const double m0 = mm[n * 32], m1 = mm[(n + 1) * 32];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {  // NT is a multiple of 4: rows past nn are unused
+                    er[t] = fma(g[n * NT + t], m0, er[t]);
+                    ei[t] = fma(g[(n + 1) * NT + t], m1, ei[t]);
+                }
             }
-            double *o = s_e + (cv * NT + t) * 64 + lane;
-            o[0] = er * s_scale[t];
-            o[32] = ei * s_scale[t];
-            if (t + PD_DSUM_WARPS < nn) {
-                o = s_e + (cv * NT + t2) * 64 + lane;
-                o[0] = fr2 * s_scale[t2];
-                o[32] = fi2 * s_scale[t2];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                if (t0 + t >= nn) break;
+                double *o = s_e + ((c0 + cb) * NT + t0 + t) * 64 + lane;
+                o[0] = er[t] * s_scale[t0 + t];
+                o[32] = ei[t] * s_scale[t0 + t];
             }
         }
     }
@@ -2839,9 +2900,7 @@ cudaError_t launch_direction_sums(const double *slots, const double4 *dirs,
                                   int32_t n_pairs, const int32_t *cls_ptr,
                                   const int32_t *cls_chunk, int32_t width, int add_exact,
                                   double *part, unsigned int *done, double *red, cudaStream_t st) {
-    const size_t smem = (static_cast<size_t>(sh.amp_cap) * (sh.node_tile + 32) +
-                         static_cast<size_t>(sh.n_cls) * sh.nv2 * sh.node_tile * 64) *
-                        sizeof(double);
+    const size_t smem = static_cast<size_t>(sh.sum_smem) * sizeof(double);
     auto kern = sh.nv2 == 2 ? pd_direction_sums<2> : pd_direction_sums<1>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          PD_DIR_SMEM);

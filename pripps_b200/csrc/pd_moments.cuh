@@ -171,6 +171,44 @@ __device__ __forceinline__ void mom_accumulate(const MomPair &P, float w, int nj
     }
 }
 
+// The same for two terms at once.
+template <int KM, bool WEIGHTED>
+__device__ __forceinline__ void mom_accumulate2(const MomPair &A, const MomPair &C, float wa,
+                                                float wc, int nj, float2 (&acc)[KM / 2],
+                                                float2 (&accw)[WEIGHTED ? KM / 2 : 1]) {
+    const float2 ap = make_float2(A.cc, A.cc), an = make_float2(-A.cc, -A.cc);
+    const float2 bp = make_float2(C.cc, C.cc), bn = make_float2(-C.cc, -C.cc);
+    float2 U[2] = {A.w0, A.w1}, W[2] = {C.w0, C.w1};
+    float2 UV[WEIGHTED ? 4 : 1], WV[WEIGHTED ? 4 : 1];
+    if constexpr (WEIGHTED) {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            UV[t] = __fmul2_rn(make_float2(wa, wa), A.v[t]);
+            WV[t] = __fmul2_rn(make_float2(wc, wc), C.v[t]);
+        }
+    }
+#pragma unroll
+    for (int jj = 0; jj < KM / 8; ++jj) {
+        if (jj >= nj) break;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            acc[4 * jj + t] = __ffma2_rn(U[jj & 1], A.v[t], acc[4 * jj + t]);
+            if constexpr (WEIGHTED)
+                accw[4 * jj + t] = __ffma2_rn(U[jj & 1], UV[t], accw[4 * jj + t]);
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            acc[4 * jj + t] = __ffma2_rn(W[jj & 1], C.v[t], acc[4 * jj + t]);
+            if constexpr (WEIGHTED)
+                accw[4 * jj + t] = __ffma2_rn(W[jj & 1], WV[t], accw[4 * jj + t]);
+        }
+        if (jj + 2 < KM / 8) {
+            U[jj & 1] = __ffma2_rn((jj & 1) ? ap : an, U[(jj & 1) ^ 1], U[jj & 1]);
+            W[jj & 1] = __ffma2_rn((jj & 1) ? bp : bn, W[(jj & 1) ^ 1], W[jj & 1]);
+        }
+    }
+}
+
 // Moments of the pairs (i, j), j0 <= j < j1, j > i, of one thread's i into
 // acc[4·jj + t] = s_jj·(Σ U.x·V.x, Σ U.y·V.y), for the first nj groups of eight of
 // the block. `at` holds the atoms [jbase, ...) in shared memory. Weighted mode
@@ -190,23 +228,39 @@ __device__ __forceinline__ void moments_range(const float4 *__restrict__ at, int
     }
 }
 
-// Direction form: the atoms [j0, j1) of a warp, for the thread's direction
-// dv = n/(2·r1); same layout of the sums.
-template <int KM, bool WEIGHTED>
+// Direction form: a thread's atoms j0, j0 + PD_DIR_LANES, … < j1 for its direction
+// dv = n/(2·r1); same layout of the sums. With room in registers (ILP) two atoms
+// at a time: their sequences' dependency chains overlap.
+constexpr int PD_DIR_DIRS = 8;                           // directions of a work unit
+constexpr int PD_DIR_LANES = PD_THREADS / PD_DIR_DIRS;   // atoms it takes at once
+
+template <int KM, bool WEIGHTED, bool ILP>
 __device__ __forceinline__ void direction_range(const float4 *__restrict__ at, float3 dv, int j0,
                                                 int j1, int nj, int rep, int dbl,
                                                 float2 (&acc)[KM / 2],
                                                 float2 (&accw)[WEIGHTED ? KM / 2 : 1]) {
     if (j0 >= j1) return;
-    float4 next = __ldg(at + j0);
-    for (int j = j0; j < j1; ++j) {
-        const float4 pj = next;
-        next = __ldg(at + min(j + 1, j1 - 1));
+    constexpr int STEP = ILP ? 2 * PD_DIR_LANES : PD_DIR_LANES;
+    const int last = j1 - 1;
+    float4 na = __ldg(at + j0), nb;
+    if constexpr (ILP) nb = __ldg(at + min(j0 + PD_DIR_LANES, last));
+    for (int j = j0; j < j1; j += STEP) {
+        const float4 pa = na;
+        na = __ldg(at + min(j + STEP, last));
         // sin²(φ/2) = (1 − x/r1)/2
-        const float s2 = fmaf(-dv.x, pj.x, fmaf(-dv.y, pj.y, fmaf(-dv.z, pj.z, 0.5f)));
-        MomPair P;
-        mom_seed(s2, rep, dbl, true, P);
-        mom_accumulate<KM, WEIGHTED>(P, pj.w, nj, acc, accw);
+        const float sa = fmaf(-dv.x, pa.x, fmaf(-dv.y, pa.y, fmaf(-dv.z, pa.z, 0.5f)));
+        MomPair A;
+        mom_seed(sa, rep, dbl, true, A);
+        if constexpr (ILP) {
+            const float4 pb = nb;
+            nb = __ldg(at + min(j + STEP + PD_DIR_LANES, last));
+            const float sb = fmaf(-dv.x, pb.x, fmaf(-dv.y, pb.y, fmaf(-dv.z, pb.z, 0.5f)));
+            MomPair C;
+            mom_seed(sb, rep, dbl, j + PD_DIR_LANES < j1, C);
+            mom_accumulate2<KM, WEIGHTED>(A, C, pa.w, pb.w, nj, acc, accw);
+        } else {
+            mom_accumulate<KM, WEIGHTED>(A, pa.w, nj, acc, accw);
+        }
     }
 }
 
@@ -301,47 +355,47 @@ __device__ __forceinline__ void direction_range_f64(const double4 *__restrict__ 
                                                     int j0, int j1, int nj, int rep, int dbl,
                                                     double (&acc)[KM],
                                                     double (&accw)[WEIGHTED ? KM : 1]) {
-    for (int j = j0; j < j1; ++j) {
+    for (int j = j0; j < j1; j += PD_DIR_LANES) {
         const double4 pj = at[j];
         const double s2 = fma(-dv.x, pj.x, fma(-dv.y, pj.y, fma(-dv.z, pj.z, 0.5)));
         mom_accumulate_f64<KM, WEIGHTED>(s2, true, pj.w, nj, rep, dbl, acc, accw);
     }
 }
 
-// A work unit of the direction form, u-th of the frame's n_chunk·n_ablk·n_grp: the
-// longest chunks first, direction groups innermost.
+// A work unit of the direction form, u-th of the frame's n_chunk·n_ablk·4·n_grp: one
+// chunk and moment block in 8 directions (a quarter of a group). The longest
+// chunks come first, the directions are innermost.
 struct DirUnit {
-    int chunk, mb, grp;
-    bool ok;
+    int chunk, mb, grp, sub;
 };
-__device__ __forceinline__ DirUnit direction_unit(int64_t u, const PdFrameDev &fr, int n_chunk) {
+__device__ __forceinline__ DirUnit direction_unit(int64_t u, const PdFrameDev &fr) {
+    constexpr int PER = 32 / PD_DIR_DIRS;
     DirUnit d;
-    d.grp = static_cast<int>(u % fr.n_grp);
-    const int64_t r = u / fr.n_grp;
+    const int n8 = fr.n_grp * PER;
+    const int g8 = static_cast<int>(u % n8);
+    const int64_t r = u / n8;
+    d.grp = g8 / PER;
+    d.sub = g8 % PER;
     d.mb = static_cast<int>(r % fr.n_ablk);
     d.chunk = static_cast<int>(r / fr.n_ablk);
-    d.ok = d.chunk < n_chunk;
     return d;
 }
 
-// Where a unit's sums go: [chunk][v][group][moment][32 directions].
+// Where the sums go: [chunk][v][group][moment][32 directions].
 __device__ __forceinline__ int64_t direction_slot(int chunk, int v, int grp, int nv2,
                                                   const PdFrameDev &fr) {
     return ((static_cast<int64_t>(chunk) * nv2 + v) * fr.n_grp + grp) * fr.n_amp * 32;
 }
 
-// The CTA's sums part[e·32 + lane] (FP64, e as in the accumulators) of one block
-// written as the moments of cos(nφ): m = s_jj·(x ± y)/2.
-__device__ __forceinline__ void direction_store(const double *__restrict__ part, int nj, int n0,
-                                                double *__restrict__ out) {
-    for (int k = threadIdx.x; k < nj * 128; k += PD_THREADS) {
-        const int lane = k & 31, t = (k >> 5) & 3, jj = k >> 7;
-        const double x = part[(8 * jj + 2 * t) * 32 + lane];
-        const double y = part[(8 * jj + 2 * t + 1) * 32 + lane];
-        const double h = (jj & 2) ? -0.5 : 0.5;
-        out[static_cast<int64_t>(n0 + 8 * jj + 4 + t) * 32 + lane] = h * (x + y);
-        out[static_cast<int64_t>(n0 + 8 * jj + 3 - t) * 32 + lane] = h * (x - y);
-    }
+// x = s_jj·Σ U.x·V.x and y of group jj, element t, direction dir of a unit: the
+// moments of cos(nφ), s_jj·(x ± y)/2, stored or added to what earlier runs left.
+__device__ __forceinline__ void direction_put(double *__restrict__ out, int n0, int jj, int t,
+                                              int dir, double x, double y, bool first) {
+    const double h = (jj & 2) ? -0.5 : 0.5;
+    double *hi = out + static_cast<int64_t>(n0 + 8 * jj + 4 + t) * 32 + dir;
+    double *lo = out + static_cast<int64_t>(n0 + 8 * jj + 3 - t) * 32 + dir;
+    *hi = (first ? 0.0 : *hi) + h * (x + y);
+    *lo = (first ? 0.0 : *lo) + h * (x - y);
 }
 
 }  // namespace pd

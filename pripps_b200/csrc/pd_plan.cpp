@@ -436,11 +436,11 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
         P.lat_bins = off;
     }
 
-    // ---- atom chunks of the direction form: about 1/6 of the atoms each (so
-    // that a few direction groups already fill the GPU, and the CTA's FP64 merge
-    // of a chunk stays a small part of it), longest first
+    // ---- atom chunks of the direction form: at most 1/6 of the atoms each (a few
+    // direction groups then fill the GPU already; shorter chunks mean more sums
+    // to hold and to add up), longest first
     {
-        const int64_t len = std::clamp<int64_t>(next_pow2(n / 6), 256, 16384);
+        const int64_t len = std::clamp<int64_t>(n / 6, 256, 16384);
         for (int k = 0; k < c; ++k) {
             const int64_t nk = static_cast<int64_t>(members[k].size());
             const int64_t parts = (nk + len - 1) / len;
@@ -662,10 +662,18 @@ static void set_directions(Plan &P) {
     const int64_t m8 = (static_cast<int64_t>(mo) + 8) & ~int64_t{7};
     const double zn = 2.0 * 1.03 * radius * P.qmax;
     const int64_t nodes = static_cast<int64_t>(0.5 * (zn + 13.0 * std::cbrt(0.5 * zn) + 3.0)) + 1;
-    // amplitudes of every class at a tile of nodes, 32 directions each
-    const int64_t room = PD_DIR_SMEM / 8 - m8 * (16 + 32);
-    const int64_t tile = std::min<int64_t>(16, room / (P.n_cls * P.amp.nv2 * 64));
-    if (tile < 1) return;
+    // The sums' kernel: a block's shared memory holds the coefficients and the
+    // amplitudes of every class at a tile of nodes (16, or fewer while that leaves
+    // SMs without a block), and the moments of as many classes as fit; up to
+    // 110 KB (two blocks per SM) unless one class's moments need more.
+    const int64_t ncv = static_cast<int64_t>(P.n_cls) * P.amp.nv2;
+    int64_t tile = 16;
+    while (tile > 4 && (S + 31) / 32 * ((nodes + tile - 1) / tile) * P.n_frames < 296) tile /= 2;
+    while (tile > 4 && m8 * (tile + 32) + ncv * tile * 64 > PD_DIR_SMEM / 8) tile -= 4;
+    const int64_t least = m8 * (tile + 32) + ncv * tile * 64;
+    if (least > PD_DIR_SMEM / 8) return;
+    P.amp.sum_smem = static_cast<int32_t>(std::max(
+        least, std::min<int64_t>(110 * 1024 / 8, m8 * tile + ncv * (tile * 64 + m8 * 32))));
     const int64_t slots = P.amp.n_chunk * P.amp.nv2 * mine * m8 * 32;
     if (slots * 8 * P.n_frames > (int64_t{4} << 30)) return;
     P.amp.dir_cap = static_cast<int32_t>(groups * 32);

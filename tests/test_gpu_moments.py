@@ -99,3 +99,56 @@ def test_moment_extreme_distances(gpu_ctx, precision, name):
            "line": np.stack([np.linspace(-60, 60, 131), np.zeros(131), np.zeros(131)], axis=1),
            "far": np.concatenate([rng.normal(size=(60, 3)), rng.normal(size=(60, 3)) + 150.0])}
     _check(_request(xyz[name], 200, 0.0, 0.8, precision, "vacuum", 3), gpu_ctx, precision)
+
+
+# The direction form (amplitudes over a quadrature of the sphere) runs where
+# there are more atoms than directions: sizes around the chunk length (256), a
+# chunk of one atom, several chunks of a class; z = 2·radius·qmax of a few rings,
+# of 33/64/65 directions' worth of moments, and past one moment block; 49 grid
+# points that hit an interpolation node (qmin = qmax·cos(π/4M) is not on the grid:
+# q = 0 and the ends are the exact cases).
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("mode", ["vacuum", "class", "weighted"])
+@pytest.mark.parametrize("n,qmax,nq,qmin", [(700, 0.15, 30, 0.0), (1025, 0.4, 49, 0.02),
+                                            (1536, 0.5, 65, 0.5), (1300, 1.2, 129, 0.0),
+                                            (2100, 2.3, 140, 0.0)])
+def test_direction_form(gpu_ctx, precision, mode, n, qmax, nq, qmin):
+    from pripps_b200 import synth
+    rng = np.random.default_rng(n)
+    r = synth.sphere_radius_for(n)
+    xyz = synth.rsa_points(n, (r, r, r), rng)
+    req = _request(xyz, nq, qmin, qmax, precision, mode, n)
+    req.species[:] = rng.choice(3, size=n, p=[0.6, 0.4 - 1.0 / n, 1.0 / n])
+    _check(req, gpu_ctx, precision)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_direction_form_shards_add_up(precision):
+    """Ranks take whole groups of directions; three ranks' partial profiles (run
+    one after another) add up to the whole solve."""
+    import ctypes as C
+
+    import torch
+    lib = _lib.lib()
+    ctx = _lib.Context(0)
+    try:
+        rng = np.random.default_rng(8)
+        xyz = rng.uniform(-22, 22, (2500, 3))
+        req = _request(xyz, 150, 0.0, 0.7, precision, "class", 8)
+        r = req.c_struct()
+        whole = solve(req, ctx)
+        dev = torch.from_numpy(req.xyz).cuda()
+        total = np.zeros((6, req.nq))
+        for rank in range(3):
+            p = C.c_void_p()
+            _lib.check(lib.pd_plan_create(ctx.handle, C.byref(r), C.byref(p)), ctx.handle)
+            _lib.check(lib.pd_plan_set_shard(ctx.handle, p, rank, 3), ctx.handle)
+            out = torch.empty((6, req.nq), dtype=torch.float64, device="cuda")
+            _lib.check(lib.pd_plan_execute(ctx.handle, p, dev.data_ptr(), out.data_ptr(),
+                                           torch.cuda.current_stream().cuda_stream), ctx.handle)
+            torch.cuda.synchronize()
+            total += out.cpu().numpy()
+            lib.pd_plan_destroy(ctx.handle, p)
+        assert np.all(term_errors(total, whole) < 1e-12)
+    finally:
+        ctx.close()

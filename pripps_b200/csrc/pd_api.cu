@@ -130,7 +130,7 @@ Layout make_layout(const Plan &P, bool host_xyz) {
     L.status = L.out + 6 * nq * 8;
     L.ctl = o;
     L.rad2 = take(F * 8);
-    L.counter = take(sizeof(int));
+    L.counter = take(2 * sizeof(int));  // next job, next direction unit
     L.cent_done = take(F * 4);
     L.pack_done = take(F * 4);
     L.red_done = take(sh.n_chunk > 1 ? red_rows * sh.n_z * 4 : 0);
@@ -667,7 +667,7 @@ int run_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st,
         NvtxRange nvtx("pd pair kernel");
         PD_CUDA(ctx, pd::launch_pairs(P.precision, P.tun.K, P.tun.NP, P.mode, dp.dptr<PdJob>(L.jobs),
                                       dp.dptr<int>(L.njobs), dp.dptr<PdReqDev>(L.req),
-                                      dp.dptr<int>(L.counter),
+                                      dp.dptr<int>(L.counter), P.n_frames,
                                       persistent_grid(ctx, P, static_cast<int64_t>(P.jobs.size())),
                                       st));
         ctx->launches += 1;
@@ -798,7 +798,7 @@ int lane_graph(pd_ctx *ctx, Lane &ln, int precision, int K, int NP, int mode,
     cudaMemcpyAsync(ln.d_jobs, ln.h_jobs, STEP_MAX_JOBS * sizeof(PdJob), cudaMemcpyHostToDevice,
                     ln.st);
     cudaMemsetAsync(ln.d_counter, 0, sizeof(int), ln.st);
-    pd::launch_pairs(precision, K, NP, mode, ln.d_jobs, ln.d_n, ln.d_reqs, ln.d_counter, grid,
+    pd::launch_pairs(precision, K, NP, mode, ln.d_jobs, ln.d_n, ln.d_reqs, ln.d_counter, 0, grid,
                      ln.st);
     PD_CUDA(ctx, cudaStreamEndCapture(ln.st, &g));
     cudaGraphExec_t ge = nullptr;

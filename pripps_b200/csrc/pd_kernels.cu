@@ -810,96 +810,143 @@ __device__ __forceinline__ MomJob moment_job(int j0, int j1, int qb, int n_mblk,
 #define PD_DIR_RUN 512
 #endif
 
+// Atoms staged at once: two buffers of 16 KB, filled by asynchronous copies (a
+// thread's pass is shorter than a read from L2, and the pair kernels' shared
+// memory leaves little L1).
+constexpr int PD_DIR_BLOCK = 1024;
+static_assert(PD_DIR_RUN * PD_DIR_LANES % PD_DIR_BLOCK == 0, "a run is whole blocks");
+static_assert(2 * PD_DIR_BLOCK * sizeof(float4) + PD_WARPS * 128 * PD_DIR_DIRS * sizeof(float) <=
+                  2 * PD_JSTAGE_ATOMS * sizeof(float4),
+              "blocks and sums share the staging memory");
+
+__device__ __forceinline__ void direction_stage(float4 *dst, const float4 *__restrict__ at, int j0,
+                                                int j1) {
+    for (int k = threadIdx.x; k < j1 - j0; k += PD_THREADS)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst + k)),
+                     "l"(at + j0 + k)
+                     : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+// The sums of a warp's four atom lanes (lane / 8), reduce-scattered: afterwards
+// atom lane a holds acc[t], a·NT/4 <= t < (a + 1)·NT/4, in acc[0 .. NT/4).
+template <int NT>
+__device__ __forceinline__ void direction_scatter(float2 (&v)[NT], int lane) {
+#pragma unroll
+    for (int lev = 0; lev < 2; ++lev) {
+        const int o = 16 >> lev, h = (NT >> lev) / 2;
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const float2 lo = v[k], hi = v[k + h];
+            const float2 keep = up ? hi : lo;
+            const float2 send = up ? lo : hi;
+            v[k] = __fadd2_rn(keep, make_float2(__shfl_xor_sync(0xffffffffu, send.x, o),
+                                                __shfl_xor_sync(0xffffffffu, send.y, o)));
+        }
+    }
+}
+
 // Direction form: one work unit. A lane is one of 8 directions for every 16th atom
 // of the chunk, so 128 threads share 8·n_amp sums: few enough units fill the GPU
 // with short loops on small structures, and the slots stay small. A run's FP32 sums
-// of the 16 atom lanes meet in shared memory (buf) and are added in lane order
-// in FP64.
+// of the 16 atom lanes meet by shuffles and in shared memory and are added to
+// the slot in warp order, in FP64.
 template <int KM, bool W, bool ILP>
 __device__ __forceinline__ void direction_unit_run(const float4 *__restrict__ at, const PdChunk &ck,
                                                    float3 dv, const DirUnit &un, int n_amp,
-                                                   float *__restrict__ buf,
+                                                   float4 *__restrict__ buf,
                                                    double *__restrict__ out0,
                                                    double *__restrict__ out1) {
     constexpr int DBL = KM == 128 ? 4 : (KM == 64 ? 3 : 2);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int al = threadIdx.x / PD_DIR_DIRS;
+    constexpr int NT = KM / 2, RUN = PD_DIR_RUN * PD_DIR_LANES;
+    float *sums = reinterpret_cast<float *>(buf + 2 * PD_DIR_BLOCK);  // [v][warp][e][8]
     const int nj = min(KM, n_amp - un.mb * KM) >> 3;
-    constexpr int RUN = PD_DIR_RUN * PD_DIR_LANES;
+    int b = 0;
+    direction_stage(buf, at, ck.j0, min(ck.j1, ck.j0 + PD_DIR_BLOCK));
     for (int r0 = ck.j0; r0 < ck.j1; r0 += RUN) {
-        float2 acc[KM / 2], accw[W ? KM / 2 : 1];
+        float2 acc[NT], accw[W ? NT : 1];
 #pragma unroll
-        for (int t = 0; t < KM / 2; ++t) {
+        for (int t = 0; t < NT; ++t) {
             acc[t] = make_float2(0.0f, 0.0f);
             if constexpr (W) accw[t] = make_float2(0.0f, 0.0f);
         }
-        direction_range<KM, W, ILP>(at, dv, r0 + al, min(ck.j1, r0 + RUN), nj, un.mb, DBL, acc,
-                                    accw);
-        // [v][warp][e][32 lanes], each row turned by 8·e lanes: reads of one
-        // atom lane's 8 directions at four consecutive e touch all banks once
-        float *b = buf + warp * KM * 32;
+        for (int j0 = r0; j0 < min(ck.j1, r0 + RUN); j0 += PD_DIR_BLOCK, b ^= 1) {
+            const int j1 = min(ck.j1, j0 + PD_DIR_BLOCK);
+            direction_stage(buf + (b ^ 1) * PD_DIR_BLOCK, at, j1, min(ck.j1, j1 + PD_DIR_BLOCK));
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+            __syncthreads();
+            direction_range<KM, W, ILP>(buf + b * PD_DIR_BLOCK, dv,
+                                        static_cast<int>(threadIdx.x) / PD_DIR_DIRS, j1 - j0, nj,
+                                        un.mb, DBL, acc, accw);
+            __syncthreads();  // the block is read before its buffer is refilled
+        }
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const int dir = lane % PD_DIR_DIRS, a = lane / PD_DIR_DIRS;
 #pragma unroll
-        for (int t = 0; t < KM / 2; ++t) {
-            if (t >= 4 * nj) break;
-            b[(2 * t) * 32 + ((lane + 16 * t) & 31)] = acc[t].x;
-            b[(2 * t + 1) * 32 + ((lane + 16 * t + 8) & 31)] = acc[t].y;
-            if constexpr (W) {
-                float *bw = b + PD_WARPS * KM * 32;
-                bw[(2 * t) * 32 + ((lane + 16 * t) & 31)] = accw[t].x;
-                bw[(2 * t + 1) * 32 + ((lane + 16 * t + 8) & 31)] = accw[t].y;
+        for (int v = 0; v < (W ? 2 : 1); ++v) {
+            float2 *x = acc;
+            if constexpr (W)
+                if (v) x = accw;
+            float *o = sums + (v * PD_WARPS + warp) * KM * PD_DIR_DIRS + dir;
+            if (v == 0) direction_scatter<NT>(acc, lane);
+            if constexpr (W)
+                if (v == 1) direction_scatter<NT>(accw, lane);
+#pragma unroll
+            for (int t = 0; t < NT / 4; ++t) {
+                // row e ^ a: the four atom lanes write different banks
+                const int e = 2 * (a * (NT / 4) + t);
+                o[(e ^ a) * PD_DIR_DIRS] = x[t].x;
+                o[((e + 1) ^ a) * PD_DIR_DIRS] = x[t].y;
             }
         }
         __syncthreads();
         for (int k = threadIdx.x; k < nj * 4 * PD_DIR_DIRS; k += PD_THREADS) {
-            const int dir = k % PD_DIR_DIRS, i = k / PD_DIR_DIRS;  // i = 4·jj + t
+            const int d = k % PD_DIR_DIRS, i = k / PD_DIR_DIRS, al = i / (NT / 4);  // i = 4·jj + t
 #pragma unroll
             for (int v = 0; v < (W ? 2 : 1); ++v) {
                 double x = 0.0, y = 0.0;
 #pragma unroll
                 for (int w = 0; w < PD_WARPS; ++w) {
-                    const float *c = buf + ((v * PD_WARPS + w) * KM + 2 * i) * 32;
-#pragma unroll
-                    for (int a = 0; a < 4; ++a) {
-                        x += static_cast<double>(c[(a * 8 + dir + 16 * i) & 31]);
-                        y += static_cast<double>(c[32 + ((a * 8 + dir + 16 * i + 8) & 31)]);
-                    }
+                    const float *c = sums + (v * PD_WARPS + w) * KM * PD_DIR_DIRS + d;
+                    x += static_cast<double>(c[((2 * i) ^ al) * PD_DIR_DIRS]);
+                    y += static_cast<double>(c[((2 * i + 1) ^ al) * PD_DIR_DIRS]);
                 }
-                direction_put(v ? out1 : out0, un.mb * KM, i >> 2, i & 3, dir, x, y, r0 == ck.j0);
+                direction_put(v ? out1 : out0, un.mb * KM, i >> 2, i & 3, d, x, y, r0 == ck.j0);
             }
         }
-        __syncthreads();  // buf is rewritten by the next run
+        __syncthreads();  // sums are rewritten by the next run
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");  // (the last, empty block)
 }
 
-// The job's work units (see direction_unit), one after another.
+// Units of a frame.
+__device__ __forceinline__ int64_t direction_unit_count(const PdReqDev &rq, const PdFrameDev &fr) {
+    return static_cast<int64_t>(rq.amp.n_chunk) * fr.n_ablk * fr.n_grp * (32 / PD_DIR_DIRS);
+}
+
+// Work unit u of a frame (see direction_unit).
 template <int K, int MODE>
-__device__ __noinline__ void direction_units(const PdJob &jb, const PdReqDev &rq,
-                                             const PdFrameDev &fr, float *__restrict__ buf) {
+__device__ __noinline__ void direction_unit_f32(int frame, int64_t u, const PdReqDev &rq,
+                                                const PdFrameDev &fr, float4 *__restrict__ buf) {
     constexpr int KM = pd_moment_block(K);
     constexpr bool W = MODE == PD_MODE_WEIGHTED;
     const int lane = threadIdx.x & 31;
-    const float4 *__restrict__ at = rq.atoms32 + static_cast<size_t>(jb.frame) * rq.n_pad;
-    const int64_t n_units = static_cast<int64_t>(rq.amp.n_chunk) * fr.n_ablk * fr.n_grp *
-                            (32 / PD_DIR_DIRS);
-    double *slots = rq.slots + static_cast<int64_t>(jb.frame) * rq.amp.slot_cap;
-    for (int64_t u = jb.ord; u < n_units; u += jb.n_ord) {
-        const DirUnit un = direction_unit(u, fr);
-        const PdChunk ck = rq.chunks[un.chunk];
-        const double4 D = rq.dirs[static_cast<int64_t>(jb.frame) * rq.amp.dir_cap +
-                                  (static_cast<int64_t>(un.grp) * rq.amp.world + rq.amp.rank) * 32 +
-                                  un.sub * PD_DIR_DIRS + lane % PD_DIR_DIRS];
-        const float3 dv = make_float3(static_cast<float>(D.x), static_cast<float>(D.y),
-                                      static_cast<float>(D.z));
-        double *out0 = slots + direction_slot(un.chunk, 0, un.grp, rq.amp.nv2, fr) +
-                       un.sub * PD_DIR_DIRS;
-        double *out1 = W ? slots + direction_slot(un.chunk, 1, un.grp, rq.amp.nv2, fr) +
-                               un.sub * PD_DIR_DIRS
-                         : out0;
-        if (KM > 64 && fr.n_amp <= 64)  // half the accumulators: two atoms at a time
-            direction_unit_run<64, W, true>(at, ck, dv, un, fr.n_amp, buf, out0, out1);
-        else
-            direction_unit_run<KM, W, KM <= 64 && !W>(at, ck, dv, un, fr.n_amp, buf, out0, out1);
-    }
+    const float4 *__restrict__ at = rq.atoms32 + static_cast<size_t>(frame) * rq.n_pad;
+    const DirUnit un = direction_unit(u, fr);
+    const PdChunk ck = rq.chunks[un.chunk];
+    const double4 D = rq.dirs[static_cast<int64_t>(frame) * rq.amp.dir_cap +
+                              (static_cast<int64_t>(un.grp) * rq.amp.world + rq.amp.rank) * 32 +
+                              un.sub * PD_DIR_DIRS + lane % PD_DIR_DIRS];
+    const float3 dv = make_float3(static_cast<float>(D.x), static_cast<float>(D.y),
+                                  static_cast<float>(D.z));
+    double *slots = rq.slots + static_cast<int64_t>(frame) * rq.amp.slot_cap + un.sub * PD_DIR_DIRS;
+    double *out0 = slots + direction_slot(un.chunk, 0, un.grp, rq.amp.nv2, fr);
+    double *out1 = W ? slots + direction_slot(un.chunk, 1, un.grp, rq.amp.nv2, fr) : out0;
+    if (KM > 64 && fr.n_amp <= 64)  // half the accumulators: two atoms at a time
+        direction_unit_run<64, W, true>(at, ck, dv, un, fr.n_amp, buf, out0, out1);
+    else
+        direction_unit_run<KM, W, KM <= 64 && !W>(at, ck, dv, un, fr.n_amp, buf, out0, out1);
 }
 
 // Weighted-mode flush of one accumulator array: the warp sums of acc and of
@@ -945,7 +992,7 @@ __device__ __forceinline__ void merge_tile_slots(const double *__restrict__ part
 template <int K, int MODE, int NP>
 __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
     pd_pairs_fp32(const PdJob *__restrict__ jobs, const int *__restrict__ n_jobs_ptr,
-                  const PdReqDev *__restrict__ reqs, int *__restrict__ counter) {
+                  const PdReqDev *__restrict__ reqs, int *__restrict__ counter, int plan_frames) {
     constexpr int NACC = (MODE == PD_MODE_WEIGHTED) ? 2 : 1;
     constexpr int NV = (MODE == PD_MODE_WEIGHTED) ? 4 : 1;  // FP64 values per q in a slot
     constexpr bool PACKED = (MODE == PD_MODE_CLASS);
@@ -980,6 +1027,37 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
     __syncthreads();
     uint32_t phase = 0;  // bit b: parity of buffer b's next completion
     double *part = s_part + warp * NV * K;
+    // The whole plan of one request: the CTAs take its direction frames' units by
+    // number, without the job list (an idle job costs a chain of four dependent
+    // loads), and the list runs only if some frame sums pairs. The next number
+    // is fetched while a unit is computed.
+    if (plan_frames > 0) {
+        const PdReqDev rq = reqs[0];
+        bool pairs = false;
+        int64_t base = 0;  // units of the frames before f
+        if (threadIdx.x == 0) s_job = atomicAdd(&counter[1], 1);
+        __syncthreads();
+        int64_t cur = s_job;
+        for (int f = 0; f < plan_frames; ++f) {
+            const PdFrameDev fr = rq.frames[f];
+            if (fr.n_grp == 0) {
+                pairs = true;
+                continue;
+            }
+            const int64_t n_units = direction_unit_count(rq, fr);
+            while (cur < base + n_units) {
+                __syncthreads();  // s_job is read
+                if (threadIdx.x == 0) s_job = atomicAdd(&counter[1], 1);
+                const int64_t u = cur - base;
+                direction_unit_f32<K, MODE>(f, u, rq, fr, pd_dyn_atoms);
+                __syncthreads();
+                cur = s_job;
+            }
+            base += n_units;
+        }
+        if (!pairs) return;
+        __syncthreads();
+    }
     for (;;) {
         if (threadIdx.x == 0) s_job = atomicAdd(counter, 1);
         __syncthreads();
@@ -990,7 +1068,10 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
         const int kq0 = jb.qb * K;
         const PdFrameDev fr = rq.frames[jb.frame];
         if (fr.n_grp > 0) {
-            direction_units<K, MODE>(jb, rq, fr, reinterpret_cast<float *>(pd_dyn_atoms));
+            // (the whole plan's units are done already)
+            const int64_t n_units = plan_frames ? 0 : direction_unit_count(rq, fr);
+            for (int64_t u = jb.ord; u < n_units; u += jb.n_ord)
+                direction_unit_f32<K, MODE>(jb.frame, u, rq, fr, pd_dyn_atoms);
             __syncthreads();  // every thread has read s_job
             continue;
         }
@@ -1242,74 +1323,69 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
 }
 
 // ---------------------------------------------------------------- K2 (FP64)
-// direction_units in FP64 (one run per unit; the atom lanes of a warp meet by
+// direction_unit_f32 in FP64 (one run per unit; the atom lanes of a warp meet by
 // shuffles, the warps in shared memory, part[v][warp][e][8]).
 template <int K, int MODE>
-__device__ __noinline__ void direction_units_f64(const PdJob &jb, const PdReqDev &rq,
-                                                 const PdFrameDev &fr, double *__restrict__ part) {
+__device__ __noinline__ void direction_unit_f64(int frame, int64_t u, const PdReqDev &rq,
+                                                const PdFrameDev &fr, double *__restrict__ part) {
     constexpr int DBL = K == 64 ? 3 : (K == 32 ? 2 : 1);
     constexpr bool W = MODE == PD_MODE_WEIGHTED;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int al = threadIdx.x / PD_DIR_DIRS;
-    const double4 *__restrict__ at = rq.atoms64 + static_cast<size_t>(jb.frame) * rq.n_pad;
-    const int64_t n_units = static_cast<int64_t>(rq.amp.n_chunk) * fr.n_ablk * fr.n_grp *
-                            (32 / PD_DIR_DIRS);
-    double *slots = rq.slots + static_cast<int64_t>(jb.frame) * rq.amp.slot_cap;
-    for (int64_t u = jb.ord; u < n_units; u += jb.n_ord) {
-        const DirUnit un = direction_unit(u, fr);
-        const PdChunk ck = rq.chunks[un.chunk];
-        const double4 D = rq.dirs[static_cast<int64_t>(jb.frame) * rq.amp.dir_cap +
-                                  (static_cast<int64_t>(un.grp) * rq.amp.world + rq.amp.rank) * 32 +
-                                  un.sub * PD_DIR_DIRS + lane % PD_DIR_DIRS];
-        const int nj = min(K, fr.n_amp - un.mb * K) >> 3;
-        double acc[K], accw[W ? K : 1];
+    const double4 *__restrict__ at = rq.atoms64 + static_cast<size_t>(frame) * rq.n_pad;
+    const DirUnit un = direction_unit(u, fr);
+    const PdChunk ck = rq.chunks[un.chunk];
+    const double4 D = rq.dirs[static_cast<int64_t>(frame) * rq.amp.dir_cap +
+                              (static_cast<int64_t>(un.grp) * rq.amp.world + rq.amp.rank) * 32 +
+                              un.sub * PD_DIR_DIRS + lane % PD_DIR_DIRS];
+    const int nj = min(K, fr.n_amp - un.mb * K) >> 3;
+    double acc[K], accw[W ? K : 1];
 #pragma unroll
-        for (int e = 0; e < K; ++e) {
-            acc[e] = 0.0;
-            if constexpr (W) accw[e] = 0.0;
-        }
-        direction_range_f64<K, W>(at, D, ck.j0 + al, ck.j1, nj, un.mb, DBL, acc, accw);
-#pragma unroll
-        for (int e = 0; e < K; ++e) {
-            if (e >= 8 * nj) break;
-            double a = acc[e];
-            a += __shfl_xor_sync(0xffffffffu, a, 8);
-            a += __shfl_xor_sync(0xffffffffu, a, 16);
-            if (lane < PD_DIR_DIRS) part[(warp * K + e) * PD_DIR_DIRS + lane] = a;
-            if constexpr (W) {
-                double b = accw[e];
-                b += __shfl_xor_sync(0xffffffffu, b, 8);
-                b += __shfl_xor_sync(0xffffffffu, b, 16);
-                if (lane < PD_DIR_DIRS)
-                    part[((PD_WARPS + warp) * K + e) * PD_DIR_DIRS + lane] = b;
-            }
-        }
-        __syncthreads();
-        for (int k = threadIdx.x; k < nj * 4 * PD_DIR_DIRS; k += PD_THREADS) {
-            const int dir = k % PD_DIR_DIRS, i = k / PD_DIR_DIRS;
-#pragma unroll
-            for (int v = 0; v < (W ? 2 : 1); ++v) {
-                double x = 0.0, y = 0.0;
-#pragma unroll
-                for (int w = 0; w < PD_WARPS; ++w) {
-                    const double *c = part + ((v * PD_WARPS + w) * K + 2 * i) * PD_DIR_DIRS + dir;
-                    x += c[0];
-                    y += c[PD_DIR_DIRS];
-                }
-                direction_put(slots + direction_slot(un.chunk, v, un.grp, rq.amp.nv2, fr) +
-                                  un.sub * PD_DIR_DIRS,
-                              un.mb * K, i >> 2, i & 3, dir, x, y, true);
-            }
-        }
-        __syncthreads();  // part is rewritten by the next unit
+    for (int e = 0; e < K; ++e) {
+        acc[e] = 0.0;
+        if constexpr (W) accw[e] = 0.0;
     }
+    direction_range_f64<K, W>(at, D, ck.j0 + static_cast<int>(threadIdx.x) / PD_DIR_DIRS, ck.j1, nj,
+                              un.mb, DBL, acc, accw);
+#pragma unroll
+    for (int e = 0; e < K; ++e) {
+        if (e >= 8 * nj) break;
+        double a = acc[e];
+        a += __shfl_xor_sync(0xffffffffu, a, 8);
+        a += __shfl_xor_sync(0xffffffffu, a, 16);
+        if (lane < PD_DIR_DIRS) part[(warp * K + e) * PD_DIR_DIRS + lane] = a;
+        if constexpr (W) {
+            double b = accw[e];
+            b += __shfl_xor_sync(0xffffffffu, b, 8);
+            b += __shfl_xor_sync(0xffffffffu, b, 16);
+            if (lane < PD_DIR_DIRS) part[((PD_WARPS + warp) * K + e) * PD_DIR_DIRS + lane] = b;
+        }
+    }
+    __syncthreads();
+    double *slots = rq.slots + static_cast<int64_t>(frame) * rq.amp.slot_cap + un.sub * PD_DIR_DIRS;
+    for (int k = threadIdx.x; k < nj * 4 * PD_DIR_DIRS; k += PD_THREADS) {
+        const int dir = k % PD_DIR_DIRS, i = k / PD_DIR_DIRS;
+#pragma unroll
+        for (int v = 0; v < (W ? 2 : 1); ++v) {
+            double x = 0.0, y = 0.0;
+#pragma unroll
+            for (int w = 0; w < PD_WARPS; ++w) {
+                const double *c = part + ((v * PD_WARPS + w) * K + 2 * i) * PD_DIR_DIRS + dir;
+                x += c[0];
+                y += c[PD_DIR_DIRS];
+            }
+            direction_put(slots + direction_slot(un.chunk, v, un.grp, rq.amp.nv2, fr), un.mb * K,
+                          i >> 2, i & 3, dir, x, y, true);
+        }
+    }
+    __syncthreads();  // part is rewritten by the next unit
 }
 
 template <int K, int MODE>
 __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(const PdJob *__restrict__ jobs,
                                                             const int *__restrict__ n_jobs_ptr,
                                                             const PdReqDev *__restrict__ reqs,
-                                                            int *__restrict__ counter) {
+                                                            int *__restrict__ counter,
+                                                            int plan_frames) {
     constexpr int NACC = (MODE == PD_MODE_WEIGHTED) ? 2 : 1;
     constexpr int NV = (MODE == PD_MODE_WEIGHTED) ? 4 : 1;
     __shared__ int s_job;
@@ -1320,6 +1396,37 @@ __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(con
     const int warp = threadIdx.x >> 5;
     const int n_jobs = *n_jobs_ptr;
     double *part = s_part + warp * NV * K;
+    // The whole plan of one request: the CTAs take its direction frames' units by
+    // number, without the job list (an idle job costs a chain of four dependent
+    // loads), and the list runs only if some frame sums pairs. The next number
+    // is fetched while a unit is computed.
+    if (plan_frames > 0) {
+        const PdReqDev rq = reqs[0];
+        bool pairs = false;
+        int64_t base = 0;  // units of the frames before f
+        if (threadIdx.x == 0) s_job = atomicAdd(&counter[1], 1);
+        __syncthreads();
+        int64_t cur = s_job;
+        for (int f = 0; f < plan_frames; ++f) {
+            const PdFrameDev fr = rq.frames[f];
+            if (fr.n_grp == 0) {
+                pairs = true;
+                continue;
+            }
+            const int64_t n_units = direction_unit_count(rq, fr);
+            while (cur < base + n_units) {
+                __syncthreads();  // s_job is read
+                if (threadIdx.x == 0) s_job = atomicAdd(&counter[1], 1);
+                const int64_t u = cur - base;
+                direction_unit_f64<K, MODE>(f, u, rq, fr, s_dir);
+                __syncthreads();
+                cur = s_job;
+            }
+            base += n_units;
+        }
+        if (!pairs) return;
+        __syncthreads();
+    }
     for (;;) {
         if (threadIdx.x == 0) s_job = atomicAdd(counter, 1);
         __syncthreads();
@@ -1329,7 +1436,9 @@ __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(con
         const PdReqDev rq = reqs[jb.req];
         const PdFrameDev fr = rq.frames[jb.frame];
         if (fr.n_grp > 0) {
-            direction_units_f64<K, MODE>(jb, rq, fr, s_dir);
+            const int64_t n_units = plan_frames ? 0 : direction_unit_count(rq, fr);
+            for (int64_t u = jb.ord; u < n_units; u += jb.n_ord)
+                direction_unit_f64<K, MODE>(jb.frame, u, rq, fr, s_dir);
             __syncthreads();  // every thread has read s_job
             continue;
         }
@@ -1816,24 +1925,23 @@ __global__ void __launch_bounds__(PD_DSUM_THREADS)
     for (int c0 = 0; c0 < ncv; c0 += batch) {  // as many classes at once as fit
         const int nb = min(batch, ncv - c0);
         if (c0) __syncthreads();  // the previous classes' moments are read
-        // two moments' rows of 32 directions per warp and step, all loads of a
-        // warp in flight together
-        for (int k = threadIdx.x; k < nb * M * 32; k += PD_DSUM_THREADS) {
-            const int cb = k / (M * 32), i = k - cb * (M * 32);
+        // (class, 8 moments) per warp and step: the rows of 32 directions of one
+        // chunk are 8 independent loads
+        const int n8 = M / 8;
+        for (int k = warp; k < nb * n8; k += PD_DSUM_WARPS) {
+            const int cb = k / n8, r0 = (k - cb * n8) * 8;
             const int c = (c0 + cb) / NV2, v = (c0 + cb) % NV2;
-            const int e1 = cls_ptr[c + 1];
-            double m = 0.0;
-            for (int e = cls_ptr[c]; e < e1; e += 4) {
-                double x[4];
+            double m[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            for (int e = cls_ptr[c]; e < cls_ptr[c + 1]; ++e) {
+                const double *src =
+                    sl + direction_slot(cls_chunk[e], v, grp, NV2, fr) + r0 * 32 + lane;
 #pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    x[u] = e + u < e1
-                               ? __ldg(sl + direction_slot(cls_chunk[e + u], v, grp, NV2, fr) + i)
-                               : 0.0;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) m += x[u];
+                for (int u = 0; u < 8; ++u) m[u] += __ldg(src + u * 32);
             }
-            s_m[k] = i < 32 ? (v ? cls[c].w1 : cls[c].n) : m;
+            if (r0 == 0) m[0] = v ? cls[c].w1 : cls[c].n;
+            double *dst = s_m + (cb * M + r0) * 32 + lane;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) dst[u * 32] = m[u];
         }
         __syncthreads();
         // (class, four nodes) per warp and step
@@ -2724,17 +2832,17 @@ static cudaError_t fp32_smem_attr() {
 }
 template <int K, int MODE, int NP>
 static cudaError_t launch_fp32_t(const PdJob *jobs, const int *n_jobs, const PdReqDev *reqs,
-                                 int *counter, int grid, cudaStream_t st) {
+                                 int *counter, int plan_frames, int grid, cudaStream_t st) {
     cudaError_t e = fp32_smem_attr<K, MODE, NP>();
     if (e != cudaSuccess) return e;
-    pd_pairs_fp32<K, MODE, NP><<<grid, PD_THREADS, PD_FP32_DYN_SMEM, st>>>(jobs, n_jobs, reqs,
-                                                                           counter);
+    pd_pairs_fp32<K, MODE, NP><<<grid, PD_THREADS, PD_FP32_DYN_SMEM, st>>>(
+        jobs, n_jobs, reqs, counter, plan_frames);
     return cudaGetLastError();
 }
 template <int K, int MODE>
 static cudaError_t launch_fp64_t(const PdJob *jobs, const int *n_jobs, const PdReqDev *reqs,
-                                 int *counter, int grid, cudaStream_t st) {
-    pd_pairs_fp64<K, MODE><<<grid, PD_THREADS, 0, st>>>(jobs, n_jobs, reqs, counter);
+                                 int *counter, int plan_frames, int grid, cudaStream_t st) {
+    pd_pairs_fp64<K, MODE><<<grid, PD_THREADS, 0, st>>>(jobs, n_jobs, reqs, counter, plan_frames);
     return cudaGetLastError();
 }
 template <int K, int MODE, int NP>
@@ -2769,13 +2877,13 @@ bool valid_q_block(int precision, int K) {
 
 #define PD_F32(K, M, NP)                                                                 \
     if (K_ == K && mode == M && NP_ == NP)                                               \
-        return launch_fp32_t<K, M, NP>(jobs, n_jobs, reqs, counter, grid, st);
+        return launch_fp32_t<K, M, NP>(jobs, n_jobs, reqs, counter, plan_frames, grid, st);
 #define PD_F64(K, M) \
-    if (K_ == K && mode == M) return launch_fp64_t<K, M>(jobs, n_jobs, reqs, counter, grid, st);
+    if (K_ == K && mode == M) return launch_fp64_t<K, M>(jobs, n_jobs, reqs, counter, plan_frames, grid, st);
 
 cudaError_t launch_pairs(int precision, int K_, int NP_, int mode, const PdJob *jobs,
-                         const int *n_jobs, const PdReqDev *reqs, int *counter, int grid,
-                         cudaStream_t st) {
+                         const int *n_jobs, const PdReqDev *reqs, int *counter, int plan_frames,
+                         int grid, cudaStream_t st) {
     if (precision == 1) {
         PD_F64(16, 0) PD_F64(16, 1) PD_F64(32, 0) PD_F64(32, 1) PD_F64(64, 0)
         return cudaErrorInvalidValue;

@@ -18,9 +18,12 @@ int pairs_blocks_per_sm(int precision, int K, int NP, int mode);
 cudaError_t prepare_pair_kernels();
 
 // n_jobs points to the tile count in device memory (read once per CTA).
+// plan_frames > 0: the jobs are those of one request (reqs[0]) with that many
+// frames, all of them (counter: two zeroed ints); 0: any jobs of any requests
+// (one).
 cudaError_t launch_pairs(int precision, int K, int NP, int mode, const PdJob *jobs,
-                         const int *n_jobs, const PdReqDev *reqs, int *counter, int grid,
-                         cudaStream_t st);
+                         const int *n_jobs, const PdReqDev *reqs, int *counter, int plan_frames,
+                         int grid, cudaStream_t st);
 // Blocks per frame of the centroid kernel (3 partial sums each).
 int32_t centroid_blocks(int64_t n_atoms);
 // `done` (one counter per frame) must be zero; `status`, if given, is cleared.

@@ -228,9 +228,10 @@ __device__ __forceinline__ void moments_range(const float4 *__restrict__ at, int
     }
 }
 
-// Direction form: a thread's atoms j0, j0 + PD_DIR_LANES, … < j1 for its direction
-// dv = n/(2·r1); same layout of the sums. With room in registers (ILP) two atoms
-// at a time: their sequences' dependency chains overlap.
+// Direction form: a thread's atoms j0, j0 + PD_DIR_LANES, … < j1 of a block staged in
+// shared memory, for its direction dv = n/(2·r1); same layout of the sums. With
+// room in registers (ILP) two atoms at a time: their sequences' dependency
+// chains overlap.
 constexpr int PD_DIR_DIRS = 8;                           // directions of a work unit
 constexpr int PD_DIR_LANES = PD_THREADS / PD_DIR_DIRS;   // atoms it takes at once
 
@@ -239,21 +240,15 @@ __device__ __forceinline__ void direction_range(const float4 *__restrict__ at, f
                                                 int j1, int nj, int rep, int dbl,
                                                 float2 (&acc)[KM / 2],
                                                 float2 (&accw)[WEIGHTED ? KM / 2 : 1]) {
-    if (j0 >= j1) return;
     constexpr int STEP = ILP ? 2 * PD_DIR_LANES : PD_DIR_LANES;
-    const int last = j1 - 1;
-    float4 na = __ldg(at + j0), nb;
-    if constexpr (ILP) nb = __ldg(at + min(j0 + PD_DIR_LANES, last));
     for (int j = j0; j < j1; j += STEP) {
-        const float4 pa = na;
-        na = __ldg(at + min(j + STEP, last));
+        const float4 pa = at[j];
         // sin²(φ/2) = (1 − x/r1)/2
         const float sa = fmaf(-dv.x, pa.x, fmaf(-dv.y, pa.y, fmaf(-dv.z, pa.z, 0.5f)));
         MomPair A;
         mom_seed(sa, rep, dbl, true, A);
         if constexpr (ILP) {
-            const float4 pb = nb;
-            nb = __ldg(at + min(j + STEP + PD_DIR_LANES, last));
+            const float4 pb = at[min(j + PD_DIR_LANES, j1 - 1)];
             const float sb = fmaf(-dv.x, pb.x, fmaf(-dv.y, pb.y, fmaf(-dv.z, pb.z, 0.5f)));
             MomPair C;
             mom_seed(sb, rep, dbl, j + PD_DIR_LANES < j1, C);

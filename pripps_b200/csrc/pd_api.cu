@@ -73,7 +73,7 @@ struct Layout {
     // counters and maxima that every execution starts from zero (one memset)
     uint64_t ctl, counter, cent_done, pack_done, rad2, red_done, dir_done, ctl_bytes;
     uint64_t lat_sums;
-    uint64_t dirs, dir_part;  // direction form: table, the groups' averages
+    uint64_t dirs, nodes, dir_part;  // direction form: tables, the groups' averages
     uint64_t lat_idx, hist, lat_err;  // lattice sets: coordinates, pair counts, error flag
     uint64_t total;
 };
@@ -139,6 +139,7 @@ Layout make_layout(const Plan &P, bool host_xyz) {
     L.dir_done = take(F * n_nt * 4);
     L.ctl_bytes = o - L.ctl;
     L.dirs = take(F * P.amp.dir_cap * sizeof(double4));
+    L.nodes = take(F * P.amp.node_cap * sizeof(double2));
     L.dir_part = take(F * P.amp.grp_cap * static_cast<uint64_t>(P.n_pairs) * P.nv *
                       P.amp.node_cap * 8);
     L.lat_sums = take(P.lat.size() * nq * 8);
@@ -592,8 +593,8 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st) {
     PD_CUDA(ctx, pd::launch_profiles(dp.dptr<double>(L.red), dp.dptr<double>(L.lat_sums),
                                      dp.dptr<PdClassDev>(L.cls), dp.dptr<PdPairDev>(L.pairs),
                                      P.n_cls, P.red, P.nv, P.n_frames, dp.dptr<double>(L.qv),
-                                     dp.dptr<PdFrameDev>(L.frames), dp.dptr<double>(L.ffA),
-                                     P.has_exc ? dp.dptr<double>(L.ffC) : nullptr,
+                                     dp.dptr<PdFrameDev>(L.frames), dp.dptr<double2>(L.nodes),
+                                     dp.dptr<double>(L.ffA), P.has_exc ? dp.dptr<double>(L.ffC) : nullptr,
                                      P.has_hyd ? dp.dptr<double>(L.ffW) : nullptr, add_exact,
                                      P.qmax, P.lat.empty() ? nullptr : dp.dptr<int>(L.lat_err),
                                      terms, st));
@@ -625,7 +626,8 @@ int pack_devplan(pd_ctx *ctx, DevPlan &dp, cudaStream_t st) {
                                  P.precision == PD_FP64 ? dp.dptr<double4>(L.atoms) : nullptr,
                                  P.mom, dp.dptr<unsigned long long>(L.rad2),
                                  dp.dptr<unsigned int>(L.pack_done),
-                                 dp.dptr<PdFrameDev>(L.frames), dp.dptr<double4>(L.dirs), st));
+                                 dp.dptr<PdFrameDev>(L.frames), dp.dptr<double4>(L.dirs),
+                                 dp.dptr<double2>(L.nodes), st));
     ctx->launches += 2;
     if (!P.lat.empty()) {
         PD_CUDA(ctx, pd::launch_lattice(dp.xyz_dev, dp.dptr<int32_t>(L.perm),

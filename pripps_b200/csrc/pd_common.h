@@ -149,8 +149,8 @@ struct PdReduceShape {
     int32_t width;        // row length of the sums: grid points or moments
     int32_t n_z;          // 128-value blocks per row
     int32_t n_chunk;      // blocks that share a slot list
-    int32_t max_moments;
-    int32_t pad_;
+    int32_t max_moments;  // moments or nodes
+    int32_t node_cap;     // nodes (direction form)
     int64_t slots_per_frame;
 };
 

@@ -1531,6 +1531,7 @@ __global__ void __launch_bounds__(PD_CENT_THREADS)
     if (blockIdx.x == 0 && threadIdx.x == 0 && status) *status = 0;
     const int64_t i0 = n_atoms * b / n_blk, i1 = n_atoms * (b + 1) / n_blk;
     double sx = 0, sy = 0, sz = 0;
+#pragma unroll 4
     for (int64_t i = i0 + threadIdx.x; i < i1; i += PD_CENT_THREADS) {
         sx += p[3 * i];
         sy += p[3 * i + 1];
@@ -1554,12 +1555,14 @@ __global__ void __launch_bounds__(PD_CENT_THREADS)
         s_last = atomicAdd(&done[f], 1u) == static_cast<unsigned>(n_blk - 1);
     }
     __syncthreads();
-    if (s_last && threadIdx.x < 3) {
+    if (s_last && threadIdx.x < 96) {  // a warp per axis, lanes added in a fixed tree
         __threadfence();
-        const volatile double *q = part + 3 * static_cast<size_t>(f) * n_blk + threadIdx.x;
+        const int ax = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const double *q = part + 3 * static_cast<size_t>(f) * n_blk + ax;
         double s = 0;
-        for (int k = 0; k < n_blk; ++k) s += q[3 * k];
-        centroid[3 * f + threadIdx.x] = s / static_cast<double>(n_atoms);
+        for (int k = lane; k < n_blk; k += 32) s += __ldcg(q + 3 * k);
+        s = warp_sum(s);
+        if (lane == 0) centroid[3 * f + ax] = s / static_cast<double>(n_atoms);
     }
 }
 
@@ -1585,7 +1588,7 @@ __global__ void __launch_bounds__(PD_PACK_THREADS)
             int64_t n_atoms, int32_t n_pad, int32_t n_blk, float4 *__restrict__ out32,
             double4 *__restrict__ out64, PdMomentRule rule, unsigned long long *__restrict__ rad2,
             unsigned int *__restrict__ done, PdFrameDev *__restrict__ frames,
-            double4 *__restrict__ dirs) {
+            double4 *__restrict__ dirs, double2 *__restrict__ node_tab) {
     __shared__ double s_max[PD_PACK_THREADS / 32];
     __shared__ bool s_last;
     __shared__ double s_radius;
@@ -1694,6 +1697,13 @@ __global__ void __launch_bounds__(PD_PACK_THREADS)
         fr.n_amp = m8;
         fr.n_ablk = ablk;
         fr.n_node = nodes;
+        // Chebyshev nodes of the q range: y_k and the barycentric weight
+        for (int k = threadIdx.x; k < nodes; k += PD_PACK_THREADS) {
+            double sn, cs;
+            sincospi((2 * k + 1) / (2.0 * nodes), &sn, &cs);
+            node_tab[static_cast<int64_t>(f) * rule.node_cap + k] =
+                make_double2(cs, (k & 1) ? -sn : sn);
+        }
         const double sc = 0.5 / fr.r1;
         double4 *o = dirs + static_cast<int64_t>(f) * rule.dir_cap;
         for (int s = threadIdx.x; s < groups * 32; s += PD_PACK_THREADS) {
@@ -1903,7 +1913,7 @@ __global__ void __launch_bounds__(PD_DSUM_THREADS)
                       double *__restrict__ part, unsigned int *__restrict__ done,
                       double *__restrict__ red) {
     extern __shared__ double s_dyn[];
-    __shared__ double s_scale[PD_DNODE_T];
+    __shared__ double s_scale[PD_DNODE_T], s_w[32];
     __shared__ bool s_last;
     const int f = blockIdx.y;
     const PdFrameDev fr = frames[f];
@@ -1918,30 +1928,39 @@ __global__ void __launch_bounds__(PD_DSUM_THREADS)
     double *s_m = s_e + ncv * NT * 64;          // [batch][M][32]
     const int batch = min(ncv, (sh.sum_smem - M * NT - ncv * NT * 64) / (M * 32));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp == PD_DSUM_WARPS - 1 && lane < nn)
-        s_scale[lane] = direction_coefficients(
-            direction_node(tile * NT + lane, fr.n_node, qmax) * fr.r1, M, s_g + lane, NT);
+    constexpr int LOADERS = PD_DSUM_WARPS - 1;
+    if (warp == LOADERS) {  // one warp: the coefficients, while the others load
+        if (lane < nn)
+            s_scale[lane] = direction_coefficients(
+                direction_node(tile * NT + lane, fr.n_node, qmax) * fr.r1, M, s_g + lane, NT);
+        s_w[lane] = dirs[static_cast<int64_t>(f) * sh.dir_cap +
+                         (static_cast<int64_t>(grp) * sh.world + sh.rank) * 32 + lane].w;
+    }
     const double *sl = slots + static_cast<int64_t>(f) * sh.slot_cap;
     for (int c0 = 0; c0 < ncv; c0 += batch) {  // as many classes at once as fit
         const int nb = min(batch, ncv - c0);
         if (c0) __syncthreads();  // the previous classes' moments are read
-        // (class, 8 moments) per warp and step: the rows of 32 directions of one
-        // chunk are 8 independent loads
-        const int n8 = M / 8;
-        for (int k = warp; k < nb * n8; k += PD_DSUM_WARPS) {
-            const int cb = k / n8, r0 = (k - cb * n8) * 8;
+        // (class, 16 moments) per warp and step: the rows of 32 directions of one
+        // chunk are 16 independent loads
+        const int n16 = (M + 15) / 16;
+        for (int k = warp; k < nb * n16 && warp < LOADERS; k += LOADERS) {
+            const int cb = k / n16, r0 = (k - cb * n16) * 16;
             const int c = (c0 + cb) / NV2, v = (c0 + cb) % NV2;
-            double m[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            const int rows = min(16, M - r0);  // 16 or 8
+            double m[16];
+#pragma unroll
+            for (int u = 0; u < 16; ++u) m[u] = 0.0;
             for (int e = cls_ptr[c]; e < cls_ptr[c + 1]; ++e) {
                 const double *src =
                     sl + direction_slot(cls_chunk[e], v, grp, NV2, fr) + r0 * 32 + lane;
 #pragma unroll
-                for (int u = 0; u < 8; ++u) m[u] += __ldg(src + u * 32);
+                for (int u = 0; u < 16; ++u) m[u] += u < rows ? __ldg(src + u * 32) : 0.0;
             }
             if (r0 == 0) m[0] = v ? cls[c].w1 : cls[c].n;
             double *dst = s_m + (cb * M + r0) * 32 + lane;
 #pragma unroll
-            for (int u = 0; u < 8; ++u) dst[u * 32] = m[u];
+            for (int u = 0; u < 16; ++u)
+                if (u < rows) dst[u * 32] = m[u];
         }
         __syncthreads();
         // (class, four nodes) per warp and step
@@ -1970,31 +1989,36 @@ __global__ void __launch_bounds__(PD_DSUM_THREADS)
         }
     }
     __syncthreads();
-    const double w = dirs[static_cast<int64_t>(f) * sh.dir_cap +
-                          (static_cast<int64_t>(grp) * sh.world + sh.rank) * 32 + lane].w;
     constexpr int NV = NV2 == 2 ? 4 : 1;
     // [frame][group][pair][nv][node]
     const int64_t row = static_cast<int64_t>(n_pairs) * NV * sh.node_cap;
     double *pt = part + (static_cast<int64_t>(f) * sh.grp_cap + grp) * row;
-    for (int k = warp; k < n_pairs * nn; k += PD_DSUM_WARPS) {
+    // a thread per (pair, node); each starts at a direction of its own, so that
+    // the 32 reads of a warp touch all banks
+    for (int k = threadIdx.x; k < n_pairs * nn; k += PD_DSUM_THREADS) {
         const int p = k / nn, t = k - p * nn;
         const int a = pairs[p].a, b = pairs[p].b;
-        const double *Ea = s_e + (a * NV2 * NT + t) * 64 + lane;
-        const double *Eb = s_e + (b * NV2 * NT + t) * 64 + lane;
+        const double *Ea = s_e + (a * NV2 * NT + t) * 64, *Eb = s_e + (b * NV2 * NT + t) * 64;
         double x[NV];
-        x[0] = w * (Ea[0] * Eb[0] + Ea[32] * Eb[32]);
-        if constexpr (NV == 4) {  // Fa, Fb: weighted amplitudes
-            const double *Fa = Ea + NT * 64, *Fb = Eb + NT * 64;
-            x[1] = w * (Fa[0] * Eb[0] + Fa[32] * Eb[32]);
-            x[2] = w * (Ea[0] * Fb[0] + Ea[32] * Fb[32]);
-            x[3] = w * (Fa[0] * Fb[0] + Fa[32] * Fb[32]);
+#pragma unroll
+        for (int v = 0; v < NV; ++v) x[v] = 0.0;
+#pragma unroll 4
+        for (int i = 0; i < 32; ++i) {
+            const int d = (i + lane) & 31;
+            const double w = s_w[d];
+            const double ar = w * Ea[d], ai = w * Ea[32 + d], br = Eb[d], bi = Eb[32 + d];
+            x[0] = fma(ar, br, fma(ai, bi, x[0]));
+            if constexpr (NV == 4) {  // weighted amplitudes
+                const double *Fa = Ea + NT * 64, *Fb = Eb + NT * 64;
+                const double fr_ = w * Fa[d], fi_ = w * Fa[32 + d], gr = Fb[d], gi = Fb[32 + d];
+                x[1] = fma(fr_, br, fma(fi_, bi, x[1]));
+                x[2] = fma(ar, gr, fma(ai, gi, x[2]));
+                x[3] = fma(fr_, gr, fma(fi_, gi, x[3]));
+            }
         }
 #pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            x[v] = warp_sum(x[v]);
-            if (lane == 0)
-                pt[(static_cast<int64_t>(p) * NV + v) * sh.node_cap + tile * NT + t] = x[v];
-        }
+        for (int v = 0; v < NV; ++v)
+            pt[(static_cast<int64_t>(p) * NV + v) * sh.node_cap + tile * NT + t] = x[v];
     }
     __threadfence();
     __syncthreads();
@@ -2057,33 +2081,63 @@ __device__ double moment_coefficients(double z, int n_mom, double *__restrict__ 
 }
 
 // Six profiles of PD_PROF_Q grid points of one frame: the class-pair sums
-// Σ sinc(q r) (read, or formed from the moments), times the class factors, all
-// in FP64. 32 groups of eight threads (one per grid point) share the class
-// pairs, and where there are fewer pairs than groups also the moments; their
-// partial profiles are added in a fixed order.
+// Σ sinc(q r) (read, formed from the moments, or interpolated from the nodes),
+// times the class factors, all in FP64. 32 groups of eight threads (one per
+// grid point) share the class pairs, and where there are fewer pairs than
+// groups also the moments; their partial profiles are added in a fixed order. The class
+// factors and the rows of as many pairs as fit are staged in shared memory
+// with all loads in flight.
 constexpr int PD_PROF_Q = 8;
 constexpr int PD_PROF_THREADS = 256;
 constexpr int PD_PROF_GROUPS = PD_PROF_THREADS / PD_PROF_Q;
+constexpr int PD_PROF_ROWS = 2048;  // doubles of pair rows staged at once
 
 template <int NV>
 __global__ void __launch_bounds__(PD_PROF_THREADS)
     pd_profiles(const double *__restrict__ red, const double *__restrict__ lat_sums,
                 const PdClassDev *__restrict__ cls, const PdPairDev *__restrict__ pairs,
                 int32_t n_cls, PdReduceShape sh, const double *__restrict__ qv,
-                const PdFrameDev *__restrict__ frames, const double *__restrict__ ffA,
-                const double *__restrict__ ffC, const double *__restrict__ ffW, int32_t add_diag,
-                double qmax, const int *__restrict__ err, double *__restrict__ terms) {
-    extern __shared__ double s_coef[];  // [n_mom][PD_PROF_Q]
+                const PdFrameDev *__restrict__ frames, const double2 *__restrict__ node_tab,
+                const double *__restrict__ ffA, const double *__restrict__ ffC,
+                const double *__restrict__ ffW, int32_t add_diag, double qmax,
+                const int *__restrict__ err, double *__restrict__ terms) {
+    extern __shared__ double s_dyn[];
     __shared__ double s_c0[PD_PROF_Q], s_scale[PD_PROF_Q];
     __shared__ double s_sum[PD_PROF_THREADS / 32][6][PD_PROF_Q];
+    double *s_row = s_dyn;                                 // [pair][nv][M]
+    double *s_fac = s_row + PD_PROF_ROWS;                  // [class][A, C, B][PD_PROF_Q]
+    double *s_coef = s_fac + n_cls * 3 * PD_PROF_Q;        // [M][PD_PROF_Q]
     const int n_qt = (sh.nq + PD_PROF_Q - 1) / PD_PROF_Q;
     const int f = blockIdx.x / n_qt;
     const int ql = threadIdx.x % PD_PROF_Q, g = threadIdx.x / PD_PROF_Q;
     const int q = (blockIdx.x % n_qt) * PD_PROF_Q + ql;
     const bool ok = q < sh.nq;
+    constexpr bool weighted = NV == 4;
     const PdFrameDev fr = frames[f];
     const bool nodes = fr.n_grp > 0;
     const int M = nodes ? fr.n_node : fr.n_mom;
+    const double *rows = red + static_cast<int64_t>(f) * sh.n_pairs * NV * sh.width;
+    // the rows of pairs [p0, p0 + n): n·NV rows of M
+    const int fit = M > 0 ? min(sh.n_pairs, PD_PROF_ROWS / (NV * M)) : 0;
+    auto stage_rows = [&](int p0, int n) {
+        for (int k = threadIdx.x; k < n * NV * M; k += PD_PROF_THREADS) {
+            const int r = k / M;
+            s_row[k] = __ldg(rows + static_cast<int64_t>(p0 * NV + r) * sh.width + (k - r * M));
+        }
+    };
+    stage_rows(0, fit);
+    for (int k = threadIdx.x; k < n_cls * 3 * PD_PROF_Q; k += PD_PROF_THREADS) {
+        const int c = k / (3 * PD_PROF_Q), w = k / PD_PROF_Q % 3;
+        const int qq = q - ql + k % PD_PROF_Q;
+        double v = 0.0;
+        if (qq < sh.nq) {
+            const int64_t at = static_cast<int64_t>(cls[c].species) * sh.nq + qq;
+            if (w == 0) v = ffA[at];
+            if (w == 1 && ffC) v = ffC[at];
+            if (w == 2 && ffW) v = weighted ? ffW[qq] : cls[c].w * ffW[qq];
+        }
+        s_fac[k] = v;
+    }
     const double qval = ok ? qv[q] : 0.0;
     if (nodes) {
         // interpolation from the Chebyshev nodes y_k = cos((2k+1)π/2M) of
@@ -2092,10 +2146,9 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
         double sum = 0.0;
         int hit = 0;
         for (int k = g; k < M; k += PD_PROF_GROUPS) {
-            double sn, cs;
-            sincospi((2 * k + 1) / (2.0 * M), &sn, &cs);
-            const double dy = y - cs;
-            const double l = dy != 0.0 ? ((k & 1) ? -sn : sn) / dy : 0.0;
+            const double2 nd = __ldg(node_tab + static_cast<int64_t>(f) * sh.node_cap + k);
+            const double dy = y - nd.x;
+            const double l = dy != 0.0 ? nd.y / dy : 0.0;
             if (dy == 0.0) hit = k + 1;
             s_coef[k * PD_PROF_Q + ql] = l;
             sum += l;
@@ -2109,22 +2162,17 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
             s_sum[threadIdx.x >> 5][1][ql] = hit;
         }
         __syncthreads();
-        if (threadIdx.x < PD_PROF_Q) {
-            double v = 0.0, h = 0.0;
-            for (int w = 0; w < PD_PROF_THREADS / 32; ++w) {
-                v += s_sum[w][0][ql];
-                h = fmax(h, s_sum[w][1][ql]);
-            }
-            s_scale[ql] = 1.0 / v;
-            s_c0[ql] = h;  // the grid point's own node + 1, or 0
+        double v = 0.0, h = 0.0;
+#pragma unroll
+        for (int w = 0; w < PD_PROF_THREADS / 32; ++w) {
+            v += s_sum[w][0][ql];
+            h = fmax(h, s_sum[w][1][ql]);  // the grid point's own node + 1, or 0
         }
-        __syncthreads();
-        hit = static_cast<int>(s_c0[ql]);
+        const double scale = 1.0 / v;
         for (int k = g; k < M; k += PD_PROF_GROUPS) {
             double &c = s_coef[k * PD_PROF_Q + ql];
-            c = hit ? (k + 1 == hit ? 1.0 : 0.0) : c * s_scale[ql];
+            c = h > 0.0 ? (k + 1 == static_cast<int>(h) ? 1.0 : 0.0) : c * scale;
         }
-        __syncthreads();
     } else if (M > 0) {
         if (threadIdx.x < PD_PROF_Q) {
             s_scale[ql] = moment_coefficients(qval * fr.d, M, s_coef + ql, PD_PROF_Q);
@@ -2147,89 +2195,85 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
                 s_coef[(8 * j + 2 * t + 1) * PD_PROF_Q + ql] = c[4 + t] - c[3 - t];
             }
         }
-        __syncthreads();
     }
+    __syncthreads();
     double AA = 0, CC = 0, BB = 0, AC = 0, AB = 0, CB = 0;
-    const double fw = (ok && ffW) ? ffW[q] : 0.0;
-    constexpr bool weighted = NV == 4;
-    if (ok && add_diag) {  // i = j terms
+    if (add_diag) {  // i = j terms
         for (int c = g; c < n_cls; c += PD_PROF_GROUPS) {
             const PdClassDev cl = cls[c];
-            const double fa = ffA[static_cast<int64_t>(cl.species) * sh.nq + q];
-            const double ca = ffC ? ffC[static_cast<int64_t>(cl.species) * sh.nq + q] : 0.0;
+            const double *fc = s_fac + c * 3 * PD_PROF_Q + ql;
+            const double fa = fc[0], ca = fc[PD_PROF_Q], b = fc[2 * PD_PROF_Q];
             AA += cl.n * fa * fa;
             CC += cl.n * ca * ca;
             AC += cl.n * fa * ca;
-            if (weighted) {
-                BB += fw * fw * cl.w2;
-                AB += fa * fw * cl.w1;
-                CB += ca * fw * cl.w1;
-            } else {
-                const double b = cl.w * fw;
-                BB += cl.n * b * b;
-                AB += cl.n * fa * b;
-                CB += cl.n * ca * b;
-            }
+            BB += (weighted ? cl.w2 : cl.n) * b * b;
+            AB += (weighted ? cl.w1 : cl.n) * fa * b;
+            CB += (weighted ? cl.w1 : cl.n) * ca * b;
         }
     }
-    // groups per class pair (they share its moments)
-    const int per = sh.n_pairs >= PD_PROF_GROUPS ? 1 : PD_PROF_GROUPS / sh.n_pairs;
-    const int sub = g % per;
-    for (int p = g / per; ok && p < sh.n_pairs; p += PD_PROF_GROUPS / per) {
-        const PdPairDev pr = pairs[p];
-        const double *r = red + (static_cast<int64_t>(f) * sh.n_pairs + p) * NV * sh.width;
-        double s[NV];
-        if (!nodes && pr.lat >= 0) {  // from the lattice set's pair counts (class mode, one frame)
-            s[0] = sub == 0 ? lat_sums[static_cast<int64_t>(pr.lat) * sh.nq + q] : 0.0;
-        } else if (M == 0) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v)
-                s[v] = sub == 0 ? r[static_cast<int64_t>(v) * sh.width + q] : 0.0;
-        } else {
+    for (int p0 = 0; p0 < sh.n_pairs;) {
+        // M = 0 (grid points summed directly): one value per pair, not staged
+        const int n = M > 0 ? min(fit, sh.n_pairs - p0) : sh.n_pairs;
+        if (p0 > 0) {
+            __syncthreads();  // the previous pairs' rows are read
+            stage_rows(p0, n);
+            __syncthreads();
+        }
+        // groups per class pair (they share its moments)
+        const int per = n >= PD_PROF_GROUPS ? 1 : PD_PROF_GROUPS / n;
+        const int sub = g % per;
+        for (int pl = g / per; pl < n; pl += PD_PROF_GROUPS / per) {
+            const int p = p0 + pl;
+            const PdPairDev pr = pairs[p];
+            double s[NV];
 #pragma unroll
             for (int v = 0; v < NV; ++v) s[v] = 0.0;
-            if (qval > 0.0) {
-#pragma unroll 8
+            if (!nodes && pr.lat >= 0) {  // from the lattice set's pair counts (class mode, one frame)
+                if (sub == 0 && ok) s[0] = lat_sums[static_cast<int64_t>(pr.lat) * sh.nq + q];
+            } else if (M == 0) {
+                if (sub == 0 && ok)
+#pragma unroll
+                    for (int v = 0; v < NV; ++v)
+                        s[v] = rows[static_cast<int64_t>(p * NV + v) * sh.width + q];
+            } else if (!(qval > 0.0)) {  // exact pair sums
+                if (sub == 0 && add_diag)
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) s[v] = pr.q0[v];
+            } else {
+                const double *r = s_row + pl * NV * M;
+#pragma unroll 4
                 for (int e = sub; e < M; e += per) {
                     const double c = s_coef[e * PD_PROF_Q + ql];
 #pragma unroll
-                    for (int v = 0; v < NV; ++v)
-                        s[v] = fma(c, r[static_cast<int64_t>(v) * sh.width + e], s[v]);
+                    for (int v = 0; v < NV; ++v) s[v] = fma(c, r[v * M + e], s[v]);
                 }
-            }
-            if (nodes) {
-                if (!(qval > 0.0))
-#pragma unroll
-                    for (int v = 0; v < NV; ++v) s[v] = (add_diag && sub == 0) ? pr.q0[v] : 0.0;
-            } else if (sub == 0) {
                 // the zeroth moment is the exact pair sum at q = 0, not the
                 // tiles' rounded (Σ X·vx − Σ Y·vy)/2
+                if (!nodes && sub == 0)
 #pragma unroll
-                for (int v = 0; v < NV; ++v) {
-                    const double *rv = r + static_cast<int64_t>(v) * sh.width;
-                    const double m0 = add_diag ? pr.q0[v] : 0.0;
-                    s[v] = qval > 0.0 ? fma(s_c0[ql], m0 - 0.5 * (rv[6] - rv[7]), s[v]) : m0;
-                }
+                    for (int v = 0; v < NV; ++v)
+                        s[v] = fma(s_c0[ql],
+                                   (add_diag ? pr.q0[v] : 0.0) - 0.5 * (r[v * M + 6] - r[v * M + 7]),
+                                   s[v]);
+            }
+            const double *fa_ = s_fac + pr.a * 3 * PD_PROF_Q + ql,
+                         *fb_ = s_fac + pr.b * 3 * PD_PROF_Q + ql;
+            const double fa = fa_[0], fb = fb_[0], ca = fa_[PD_PROF_Q], cb = fb_[PD_PROF_Q];
+            const double ba = fa_[2 * PD_PROF_Q], bb = fb_[2 * PD_PROF_Q];
+            AA += 2.0 * fa * fb * s[0];
+            CC += 2.0 * ca * cb * s[0];
+            AC += (fa * cb + ca * fb) * s[0];
+            if constexpr (weighted) {  // ba = bb = F_water
+                BB += 2.0 * ba * ba * s[3];
+                AB += ba * (fa * s[2] + fb * s[1]);
+                CB += ba * (ca * s[2] + cb * s[1]);
+            } else {
+                BB += 2.0 * ba * bb * s[0];
+                AB += (fa * bb + ba * fb) * s[0];
+                CB += (ca * bb + ba * cb) * s[0];
             }
         }
-        const PdClassDev cla = cls[pr.a], clb = cls[pr.b];
-        const int64_t sa = static_cast<int64_t>(cla.species) * sh.nq + q;
-        const int64_t sb = static_cast<int64_t>(clb.species) * sh.nq + q;
-        const double fa = ffA[sa], fb = ffA[sb];
-        const double ca = ffC ? ffC[sa] : 0.0, cb = ffC ? ffC[sb] : 0.0;
-        AA += 2.0 * fa * fb * s[0];
-        CC += 2.0 * ca * cb * s[0];
-        AC += (fa * cb + ca * fb) * s[0];
-        if constexpr (weighted) {
-            BB += 2.0 * fw * fw * s[3];
-            AB += fw * (fa * s[2] + fb * s[1]);
-            CB += fw * (ca * s[2] + cb * s[1]);
-        } else {
-            const double ba = cla.w * fw, bb = clb.w * fw;
-            BB += 2.0 * ba * bb * s[0];
-            AB += (fa * bb + ba * fb) * s[0];
-            CB += (ca * bb + ba * cb) * s[0];
-        }
+        p0 += n;
     }
     double out[6] = {AA, CC, BB, AC, AB, CB};
 #pragma unroll
@@ -2237,6 +2281,7 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
         out[t] += __shfl_xor_sync(0xffffffffu, out[t], 8);
         out[t] += __shfl_xor_sync(0xffffffffu, out[t], 16);
     }
+    __syncthreads();  // s_sum's earlier use is over
     if ((threadIdx.x & 31) < PD_PROF_Q)
 #pragma unroll
         for (int t = 0; t < 6; ++t) s_sum[threadIdx.x >> 5][t][ql] = out[t];
@@ -2938,12 +2983,12 @@ cudaError_t launch_pack(const double *xyz, const double *weights, const int32_t 
                         const double *centroid, int64_t n_atoms, int32_t n_pad, int32_t n_frames,
                         float4 *out32, double4 *out64, const PdMomentRule &rule,
                         unsigned long long *rad2, unsigned int *done, PdFrameDev *frames,
-                        double4 *dirs, cudaStream_t st) {
+                        double4 *dirs, double2 *node_tab, cudaStream_t st) {
     const int64_t nb = (static_cast<int64_t>(n_pad) + PD_PACK_THREADS - 1) / PD_PACK_THREADS;
     if (nb * n_frames > 0x7fffffffLL) return cudaErrorInvalidValue;
     pd_pack<<<static_cast<unsigned>(nb * n_frames), PD_PACK_THREADS, 0, st>>>(
         xyz, weights, perm, centroid, n_atoms, n_pad, static_cast<int32_t>(nb), out32, out64, rule,
-        rad2, done, frames, dirs);
+        rad2, done, frames, dirs, node_tab);
     return cudaGetLastError();
 }
 
@@ -3051,22 +3096,25 @@ cudaError_t launch_reduce(const double *slots, const int64_t *lptr, const int64_
 cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdClassDev *cls,
                             const PdPairDev *pairs, int32_t n_cls, const PdReduceShape &sh,
                             int32_t nv, int32_t n_frames, const double *qv,
-                            const PdFrameDev *frames, const double *ffA, const double *ffC,
-                            const double *ffW, int add_diag, double qmax, const int *err,
+                            const PdFrameDev *frames, const double2 *node_tab, const double *ffA,
+                            const double *ffC, const double *ffW, int add_diag, double qmax, const int *err,
                             double *terms, cudaStream_t st) {
     const int64_t blocks =
         static_cast<int64_t>(n_frames) * ((sh.nq + PD_PROF_Q - 1) / PD_PROF_Q);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-    // coefficients of the most moments a frame may have: at most 32 KB
-    const size_t smem = static_cast<size_t>(sh.max_moments) * PD_PROF_Q * sizeof(double);
-    if (nv == 4)
-        pd_profiles<4><<<static_cast<unsigned>(blocks), PD_PROF_THREADS, smem, st>>>(
-            red, lat_sums, cls, pairs, n_cls, sh, qv, frames, ffA, ffC, ffW, add_diag, qmax,
-            err, terms);
-    else
-        pd_profiles<1><<<static_cast<unsigned>(blocks), PD_PROF_THREADS, smem, st>>>(
-            red, lat_sums, cls, pairs, n_cls, sh, qv, frames, ffA, ffC, ffW, add_diag, qmax,
-            err, terms);
+    // pair rows, class factors, and the coefficients of the most moments a frame
+    // may have: at most 16 + 9 + 32 KB
+    const size_t smem = (PD_PROF_ROWS + static_cast<size_t>(n_cls) * 3 * PD_PROF_Q +
+                         static_cast<size_t>(sh.max_moments) * PD_PROF_Q) * sizeof(double);
+    auto kern = nv == 4 ? pd_profiles<4> : pd_profiles<1>;
+    if (smem > 44 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(
+            kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+        if (e != cudaSuccess) return e;
+    }
+    kern<<<static_cast<unsigned>(blocks), PD_PROF_THREADS, smem, st>>>(
+        red, lat_sums, cls, pairs, n_cls, sh, qv, frames, node_tab, ffA, ffC, ffW, add_diag, qmax,
+        err, terms);
     return cudaGetLastError();
 }
 

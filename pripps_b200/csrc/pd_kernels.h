@@ -35,7 +35,7 @@ cudaError_t launch_pack(const double *xyz, const double *weights, const int32_t 
                         const double *centroid, int64_t n_atoms, int32_t n_pad, int32_t n_frames,
                         float4 *out32, double4 *out64, const PdMomentRule &rule,
                         unsigned long long *rad2, unsigned int *done, PdFrameDev *frames,
-                        double4 *dirs, cudaStream_t st);
+                        double4 *dirs, double2 *node_tab, cudaStream_t st);
 // The quadrature rules of the direction form on the current device (before any
 // launch_pack there, and before a stream capture).
 cudaError_t prepare_direction_rules();
@@ -58,8 +58,8 @@ cudaError_t launch_reduce(const double *slots, const int64_t *lptr, const int64_
 cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdClassDev *cls,
                             const PdPairDev *pairs, int32_t n_cls, const PdReduceShape &sh,
                             int32_t nv, int32_t n_frames, const double *qv,
-                            const PdFrameDev *frames, const double *ffA, const double *ffC,
-                            const double *ffW, int add_diag, double qmax, const int *err,
+                            const PdFrameDev *frames, const double2 *node_tab, const double *ffA,
+                            const double *ffC, const double *ffW, int add_diag, double qmax, const int *err,
                             double *terms, cudaStream_t st);
 // Lattice sets: integer coordinates of their points and the exact pair count
 // per squared offset (after pack), then their self pair sums, sums[lattice][q].

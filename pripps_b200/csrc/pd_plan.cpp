@@ -730,6 +730,7 @@ void set_reduction(Plan &P) {
     r.max_moments = m.block ? m.max_moments : 0;
     r.n_z = (std::max(P.nq, r.max_moments) + 127) / 128;
     r.max_moments = std::max(r.max_moments, P.amp.node_cap);
+    r.node_cap = P.amp.node_cap;
     r.width = std::max(P.nq, r.max_moments);
     // A block adds its share of a class pair's slot list serially: lists of
     // more than a few hundred entries are shared by up to 16 blocks (one

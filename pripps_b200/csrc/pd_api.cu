@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <chrono>
 #include <cmath>
@@ -16,6 +17,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <numeric>
 #include <random>
 #include <string>
 #include <thread>
@@ -2185,7 +2187,8 @@ uint64_t pd_launch_count(pd_ctx *ctx) { return ctx ? ctx->launches.load() : 0; }
 namespace {
 
 // Checks shared by pd_direct and pd_direct_lattice (the q-vectors apart).
-std::string direct_validate(const pd_direct_request *req) {
+// The coordinates may be left to the caller, who checks them while copying.
+std::string direct_validate(const pd_direct_request *req, bool coordinates = true) {
     const uint64_t n = req->n_points, nv = req->n_vectors;
     const uint64_t nm = req->n_molecules ? req->n_molecules : 1;
     if (n == 0 || nv == 0 || req->n_kinds == 0 || !req->xyz || !req->kind || !req->ff ||
@@ -2200,12 +2203,9 @@ std::string direct_validate(const pd_direct_request *req) {
         if (req->kind[i] >= req->n_kinds)
             return "kind " + std::to_string(req->kind[i]) + " at point " + std::to_string(i) +
                    " is >= n_kinds";
-    for (uint64_t i = 0; i < 3 * n; ++i)
-        if (!std::isfinite(req->xyz[i])) return "non-finite coordinate";
-    for (uint64_t i = 0; i < nv * req->n_kinds; ++i)
-        if (!std::isfinite(req->ff[i])) return "non-finite form factor";
-    for (uint64_t i = 0; req->weight && i < n; ++i)
-        if (!std::isfinite(req->weight[i])) return "non-finite point weight";
+    if (coordinates && !pd::all_finite(req->xyz, 3 * n)) return "non-finite coordinate";
+    if (!pd::all_finite(req->ff, nv * req->n_kinds)) return "non-finite form factor";
+    if (req->weight && !pd::all_finite(req->weight, n)) return "non-finite point weight";
     return std::string();
 }
 
@@ -2276,6 +2276,227 @@ int direct_run(pd_ctx *ctx, const pd_direct_request *req, const double *ff, cons
     return PD_OK;
 }
 
+// Lattice vectors as segments of up to LINE_J consecutive ones on lines
+// n0 + j·δ. Lines are the multiples of a primitive direction, or consecutive
+// indices along one axis, whichever cuts the list into fewer segments.
+constexpr int LINE_J = 16;
+struct LineSet {
+    std::vector<PdLine> lines;
+    std::vector<int32_t> index;     // distinct |indices|: axis 0, 1, 2
+    int32_t n_index[3] = {0, 0, 0};
+    std::vector<uint32_t> slot;     // per given vector: j·n_line + line
+};
+
+struct LineKey {
+    int32_t d[3];  // the line: direction (primitive), or the fixed indices
+    int32_t p;     // position on it
+    uint32_t i;    // vector
+};
+
+// Sort keys of the vectors for one kind of line: axis < 0: multiples of a
+// primitive direction; else along that axis.
+void line_keys(const int32_t *hkl, uint64_t nv, int axis, std::vector<LineKey> &keys) {
+    keys.resize(nv);
+    for (uint64_t i = 0; i < nv; ++i) {
+        LineKey &k = keys[i];
+        k.i = static_cast<uint32_t>(i);
+        const int32_t *n = hkl + 3 * i;
+        if (axis < 0) {
+            int32_t g = std::gcd(std::gcd(std::abs(n[0]), std::abs(n[1])), std::abs(n[2]));
+            if (g == 0) g = 1;
+            for (int a = 0; a < 3; ++a) k.d[a] = n[a] / g;
+            k.p = g;
+        } else {
+            for (int a = 0; a < 3; ++a) k.d[a] = a == axis ? 0 : n[a];
+            k.p = n[axis];
+        }
+    }
+    std::sort(keys.begin(), keys.end(), [](const LineKey &x, const LineKey &y) {
+        if (x.d[0] != y.d[0]) return x.d[0] < y.d[0];
+        if (x.d[1] != y.d[1]) return x.d[1] < y.d[1];
+        if (x.d[2] != y.d[2]) return x.d[2] < y.d[2];
+        if (x.p != y.p) return x.p < y.p;
+        return x.i < y.i;
+    });
+}
+
+// Whether b continues the segment of a at the next position.
+bool line_next(const LineKey &a, const LineKey &b) {
+    return a.d[0] == b.d[0] && a.d[1] == b.d[1] && a.d[2] == b.d[2] && b.p == a.p + 1;
+}
+
+uint64_t line_segments(const std::vector<LineKey> &k) {
+    uint64_t n = 0;
+    int len = 0;
+    for (size_t i = 0; i < k.size(); ++i) {
+        if (i == 0 || len == LINE_J || !line_next(k[i - 1], k[i])) {
+            ++n;
+            len = 0;
+        }
+        ++len;
+    }
+    return n;
+}
+
+// False when the vectors lie on no lines worth the segments (fewer than four
+// vectors per segment: the table kernel reads less than the padded lines compute).
+bool find_lines(const int32_t *hkl, uint64_t nv, LineSet &out) {
+    std::vector<LineKey> keys, best;
+    uint64_t fewest = ~uint64_t{0};
+    int best_axis = -1;
+    for (int axis : {-1, 2, 1, 0}) {
+        line_keys(hkl, nv, axis, keys);
+        const uint64_t n = line_segments(keys);
+        if (n < fewest) {
+            fewest = n;
+            best.swap(keys);
+            best_axis = axis;
+        }
+        if (fewest * 10 <= nv) break;  // ten of 16 lanes: good enough to stop looking
+    }
+    if (fewest * 4 > nv || fewest > (uint64_t{1} << 26)) return false;
+    std::vector<std::array<int32_t, 6>> raw;  // start, step
+    out.slot.assign(nv, 0);
+    std::vector<std::pair<uint32_t, uint32_t>> where(nv);  // (segment, j)
+    int len = 0;
+    for (size_t i = 0; i < best.size(); ++i) {
+        const LineKey &k = best[i];
+        if (i == 0 || len == LINE_J || !line_next(best[i - 1], k)) {
+            const int32_t *n = hkl + 3 * static_cast<size_t>(k.i);
+            std::array<int32_t, 6> r{n[0], n[1], n[2], 0, 0, 0};
+            for (int a = 0; a < 3; ++a)
+                r[3 + a] = best_axis < 0 ? k.d[a] : (a == best_axis ? 1 : 0);
+            raw.push_back(r);
+            len = 0;
+        }
+        where[k.i] = {static_cast<uint32_t>(raw.size() - 1), static_cast<uint32_t>(len)};
+        ++len;
+    }
+    const uint32_t n_line = static_cast<uint32_t>(raw.size());
+    for (uint64_t i = 0; i < nv; ++i) out.slot[i] = where[i].second * n_line + where[i].first;
+    out.lines.resize(n_line);
+    for (int a = 0; a < 3; ++a) {
+        std::vector<int32_t> vals;
+        for (const auto &r : raw) {
+            vals.push_back(std::abs(r[a]));
+            vals.push_back(std::abs(r[3 + a]));
+        }
+        std::sort(vals.begin(), vals.end());
+        vals.erase(std::unique(vals.begin(), vals.end()), vals.end());
+        const int32_t base = static_cast<int32_t>(out.index.size());
+        auto at = [&](int32_t n) {
+            const int32_t k = base + static_cast<int32_t>(
+                                         std::lower_bound(vals.begin(), vals.end(), std::abs(n)) -
+                                         vals.begin());
+            return n < 0 ? static_cast<int32_t>(static_cast<uint32_t>(k) | 0x80000000u) : k;
+        };
+        for (uint32_t l = 0; l < n_line; ++l) {
+            PdLine &ln = out.lines[l];
+            (a == 0 ? ln.x : (a == 1 ? ln.y : ln.z)) = at(raw[l][a]);
+            (a == 0 ? ln.sx : (a == 1 ? ln.sy : ln.sz)) = at(raw[l][3 + a]);
+        }
+        out.n_index[a] = static_cast<int32_t>(vals.size());
+        out.index.insert(out.index.end(), vals.begin(), vals.end());
+    }
+    return true;
+}
+
+// Molecules of at least this many points take the line kernel (its chunks lie
+// within one molecule, and each flushes every kind it meets).
+constexpr int64_t LINE_MIN_MOLECULE = 128;
+
+constexpr uint64_t LINE_MAX_KINDS = 32;  // the device sort's counters
+
+// One blocking solve by the line kernel. The inputs go through a pinned image, the
+// coordinates in pieces that are uploaded while the next one is copied and
+// checked; the points are sorted by kind within their molecule on the device.
+int direct_run_lines(pd_ctx *ctx, const pd_direct_request *req, const LineSet &ls,
+                     const double *box, double *out) {
+    const uint64_t n = req->n_points, nv = req->n_vectors, nk = req->n_kinds;
+    const int64_t nm = static_cast<int64_t>(req->n_molecules ? req->n_molecules : 1);
+    const int64_t mol = static_cast<int64_t>(n) / nm;
+    const int32_t n_line = static_cast<int32_t>(ls.lines.size());
+    int64_t chunk = 0, spm = 0;
+    pd::direct_line_layout(static_cast<int64_t>(n), mol, n_line, &chunk, &spm);
+    const uint64_t nvp = static_cast<uint64_t>(n_line) * LINE_J;
+    // image: form factors, lines, indices, kinds, weights, coordinates
+    const uint64_t o_line = align_up(nk * nvp * 8, 256),
+                   o_idx = o_line + align_up(ls.lines.size() * sizeof(PdLine), 256),
+                   o_kind = o_idx + align_up(ls.index.size() * 4, 256),
+                   o_w = o_kind + align_up(n * 4, 256),
+                   o_xyz = o_w + (req->weight ? align_up(n * 8, 256) : 0),
+                   b_up = o_xyz + align_up(n * 24, 256), b_out = nvp * 32;
+    const uint64_t o_kind2 = b_up, o_w2 = o_kind2 + (o_w - o_kind), o_xyz2 = o_w2 + (o_xyz - o_w),
+                   o_part = o_xyz2 + (b_up - o_xyz),
+                   o_out = o_part + static_cast<uint64_t>(nm * spm) * 2 * nvp * 8,
+                   total = o_out + b_out;
+    std::lock_guard<std::mutex> g(ctx->solve_mu);
+    cudaSetDevice(ctx->device);
+    cudaStream_t st = ctx->stream;
+    char *img = nullptr, *base = nullptr;
+    uint64_t cls = 0;
+    cudaError_t e = ctx->pinned.get(b_up + b_out, &img, &cls);
+    if (e == cudaSuccess)
+        e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(&base), total, ctx->pool, st);
+    if (e != cudaSuccess) {
+        if (img) ctx->pinned.put(img, cls);
+        return cuda_fail(ctx, e, "pd_direct_lattice: allocation");
+    }
+    bool finite = true;
+    constexpr uint64_t PIECE = 3 * 16384;
+    for (uint64_t i = 0; i < 3 * n && finite && e == cudaSuccess; i += PIECE) {
+        const uint64_t m = std::min(PIECE, 3 * n - i);
+        finite = pd::all_finite(req->xyz + i, m);
+        std::memcpy(img + o_xyz + i * 8, req->xyz + i, m * 8);
+        e = cudaMemcpyAsync(base + o_xyz + i * 8, img + o_xyz + i * 8, m * 8,
+                            cudaMemcpyHostToDevice, st);
+    }
+    if (finite && e == cudaSuccess) {
+        double *h_ff = reinterpret_cast<double *>(img);
+        std::memset(h_ff, 0, nk * nvp * 8);  // vectors past a segment's end
+        for (uint64_t t = 0; t < nk; ++t)
+            for (uint64_t i = 0; i < nv; ++i) h_ff[t * nvp + ls.slot[i]] = req->ff[t * nv + i];
+        std::memcpy(img + o_line, ls.lines.data(), ls.lines.size() * sizeof(PdLine));
+        std::memcpy(img + o_idx, ls.index.data(), ls.index.size() * 4);
+        std::memcpy(img + o_kind, req->kind, n * 4);
+        if (req->weight) std::memcpy(img + o_w, req->weight, n * 8);
+        e = cudaMemcpyAsync(base, img, o_xyz, cudaMemcpyHostToDevice, st);
+        double *w2 = req->weight ? reinterpret_cast<double *>(base + o_w2) : nullptr;
+        if (e == cudaSuccess)
+            e = pd::launch_direct_sort(
+                reinterpret_cast<double *>(base + o_xyz), reinterpret_cast<uint32_t *>(base + o_kind),
+                req->weight ? reinterpret_cast<double *>(base + o_w) : nullptr,
+                static_cast<int64_t>(n), mol, static_cast<int32_t>(nk),
+                reinterpret_cast<double *>(base + o_xyz2),
+                reinterpret_cast<uint32_t *>(base + o_kind2), w2, st);
+        if (e == cudaSuccess)
+            e = pd::launch_direct_lines(
+                reinterpret_cast<double *>(base + o_xyz2),
+                reinterpret_cast<uint32_t *>(base + o_kind2), w2, reinterpret_cast<double *>(base),
+                reinterpret_cast<PdLine *>(base + o_line),
+                reinterpret_cast<int32_t *>(base + o_idx), ls.n_index, box, n_line,
+                static_cast<int64_t>(n), mol, chunk, spm, reinterpret_cast<double *>(base + o_part),
+                reinterpret_cast<double *>(base + o_out), st);
+        if (e == cudaSuccess) {
+            ctx->launches += 3;
+            e = cudaMemcpyAsync(img + b_up, base + o_out, b_out, cudaMemcpyDeviceToHost, st);
+        }
+    }
+    cudaFreeAsync(base, st);
+    const cudaError_t e2 = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = e2;
+    if (e == cudaSuccess && finite)
+        for (uint64_t i = 0; i < nv; ++i)
+            std::memcpy(out + 4 * i, img + b_up + 32 * static_cast<uint64_t>(ls.slot[i]), 32);
+    ctx->pinned.put(img, cls);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "pd_direct_lattice");
+    if (!finite) {
+        ctx->set_error("non-finite coordinate");
+        return PD_EINVAL;
+    }
+    return PD_OK;
+}
+
 // Lattice indices up to this bound use the phase tables; beyond it a table
 // row costs more than the sincos it saves, and the vectors go to the sincos
 // kernel as q = 2π·hkl/L.
@@ -2298,7 +2519,8 @@ extern "C" int pd_direct(pd_ctx *ctx, const pd_direct_request *req, double *out)
 extern "C" int pd_direct_lattice(pd_ctx *ctx, const pd_direct_request *req, const int32_t *hkl,
                                  const double box[3], double *out) {
     if (!ctx || !req || !out) return PD_EINVAL;
-    std::string msg = (hkl && box) ? direct_validate(req) : "pd_direct_lattice: hkl and box required";
+    std::string msg = (hkl && box) ? direct_validate(req, false)
+                                   : "pd_direct_lattice: hkl and box required";
     for (int a = 0; msg.empty() && a < 3; ++a)
         if (!std::isfinite(box[a]) || !(box[a] > 0.0)) msg = "box sides must be finite and > 0";
     if (!msg.empty()) {
@@ -2309,6 +2531,28 @@ extern "C" int pd_direct_lattice(pd_ctx *ctx, const pd_direct_request *req, cons
     int64_t nmax = 0;
     for (uint64_t i = 0; i < 3 * nv; ++i)
         nmax = std::max<int64_t>(nmax, std::llabs(static_cast<long long>(hkl[i])));
+    // Vectors on lines (a Miller grid, a filled lattice): the line kernel, where
+    // its table of distinct indices leaves room for at least 8 points at once and
+    // its partial amplitudes stay below 8 GiB.
+    const int64_t mol =
+        static_cast<int64_t>(req->n_points / (req->n_molecules ? req->n_molecules : 1));
+    LineSet ls;
+    if (mol >= LINE_MIN_MOLECULE && nk <= LINE_MAX_KINDS && nmax <= kDirectTableMaxIndex &&
+        find_lines(hkl, nv, ls) &&
+        pd::direct_line_points(static_cast<int32_t>(ls.index.size())) >= 8) {
+        int64_t chunk = 0, spm = 0;
+        pd::direct_line_layout(static_cast<int64_t>(req->n_points), mol,
+                               static_cast<int32_t>(ls.lines.size()), &chunk, &spm);
+        const double chunks = static_cast<double>(req->n_points / static_cast<uint64_t>(mol)) * spm;
+        const double vb = std::ceil(static_cast<double>(ls.lines.size()) / 32.0);
+        if (chunks * static_cast<double>(ls.lines.size()) * LINE_J * 16.0 <= 8.0 * (1ull << 30) &&
+            chunks * vb < 2.0e9)
+            return direct_run_lines(ctx, req, ls, box, out);
+    }
+    if (!pd::all_finite(req->xyz, 3 * req->n_points)) {
+        ctx->set_error("non-finite coordinate");
+        return PD_EINVAL;
+    }
     if (nmax > kDirectTableMaxIndex || pd::direct_table_points(static_cast<int32_t>(nmax)) < 1) {
         std::vector<double> q(3 * nv);
         for (uint64_t i = 0; i < nv; ++i)

@@ -215,3 +215,11 @@ struct PdLatTile {
     int32_t lat, i0, j0, j1;
 };
 static_assert(sizeof(PdLatTile) == 16, "PdLatTile layout");
+
+// Direct transform at lattice vectors on lines: a segment of consecutive vectors
+// n0 + j·δ. The members are entries of a point's phase table (the distinct |indices| of
+// each axis): those of the start n0 and of the step δ; the sign bit is set where
+// the index is negative.
+struct PdLine {
+    int32_t x, y, z, sx, sy, sz;
+};

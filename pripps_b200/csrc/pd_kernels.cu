@@ -2688,6 +2688,247 @@ __global__ void __launch_bounds__(PD_DTAB_THREADS, 2)
     }
 }
 
+// Direct transform at lattice vectors that lie on lines n0 + j·δ (the Miller grid's
+// multiples of a direction, or consecutive indices along an axis): a thread owns
+// a segment of PD_DLINE_J vectors of one line and needs, per point, only the
+// phases of its start and step — two products of table entries — instead of three
+// table reads and two complex products per vector (pd_direct_table: the reads
+// bound it, 0.50 ms for 128,000 points × 1,300 vectors; this kernel: see
+// launch_direct_lines). With E = e^{iφ} at the segment's index 4 (and 12) and
+// V_k = e^{ikδ·r}, the vectors ±k around it share four products,
+//   Re = x·c ∓ y·s, Im = y·c ± x·s,
+// accumulated separately: 4.6 FP64 operations per (vector, point). The points of
+// a molecule are sorted by kind, so the form factors enter once per kind of a chunk
+// (flush), not per point. A table holds the distinct |indices| that starts and steps
+// use on each axis. Chunks are slices of one molecule.
+constexpr int PD_DLINE_J = 16;
+constexpr int PD_DLINE_THREADS = 128;
+constexpr int PD_DLINE_MAX_POINTS = 64;
+constexpr int PD_DLINE_TABLE_BYTES = 40 * 1024;
+
+__device__ __forceinline__ double2 csqr(double2 a) {
+    return make_double2(fma(a.x, a.x, -a.y * a.y), 2.0 * a.x * a.y);
+}
+
+__global__ void __launch_bounds__(PD_DLINE_THREADS, 3)
+    pd_direct_lines(const double *__restrict__ xyz, const uint32_t *__restrict__ kind,
+                    const double *__restrict__ weight, const double *__restrict__ ff,
+                    const PdLine *__restrict__ lines, const int32_t *__restrict__ index,
+                    int3 n_index, double lx, double ly, double lz, int32_t npts, int32_t n_line,
+                    int32_t n_vblocks, int64_t mol_size, int64_t chunk_points,
+                    int64_t slices_per_mol, double *__restrict__ part) {
+    constexpr int J = PD_DLINE_J;
+    extern __shared__ __align__(16) double2 pd_dl_tab[];  // [npts][entries], then [J][2][threads]
+    __shared__ double s_w[PD_DLINE_MAX_POINTS], s_u[3 * PD_DLINE_MAX_POINTS];
+    __shared__ uint32_t s_k[PD_DLINE_MAX_POINTS];
+    const int T = blockDim.x, tid = threadIdx.x;
+    const int n_ent = n_index.x + n_index.y + n_index.z;
+    double *s_f = reinterpret_cast<double *>(pd_dl_tab + npts * n_ent);
+    const int64_t c = blockIdx.x / n_vblocks;
+    const int seg = static_cast<int>(blockIdx.x % n_vblocks) * T + tid;
+    const bool ok = seg < n_line;
+    const PdLine ln = lines[ok ? seg : 0];
+    const int64_t m = c / slices_per_mol, sl = c % slices_per_mol;
+    const int64_t p0 = m * mol_size + sl * chunk_points,
+                  p1 = min((m + 1) * mol_size, p0 + chunk_points);
+    // sums over the points of one kind: center h: x, y; pairs ±k: x·c, y·s, y·c,
+    // x·s; index −4: re, im
+    double a[2][16];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 16; ++e) a[h][e] = 0.0;
+    for (int j = 0; j < 2 * J; ++j) s_f[j * T + tid] = 0.0;
+    auto flush = [&](uint32_t k) {
+        const double *f = ff + static_cast<int64_t>(k) * J * n_line + (ok ? seg : 0);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int b = -4; b < 4; ++b) {
+                double re, im;
+                if (b == -4) {
+                    re = a[h][14];
+                    im = a[h][15];
+                } else if (b == 0) {
+                    re = a[h][0];
+                    im = a[h][1];
+                } else {
+                    const int q = 2 + 4 * ((b < 0 ? -b : b) - 1);
+                    re = b > 0 ? a[h][q] - a[h][q + 1] : a[h][q] + a[h][q + 1];
+                    im = b > 0 ? a[h][q + 2] + a[h][q + 3] : a[h][q + 2] - a[h][q + 3];
+                }
+                const int j = 8 * h + 4 + b;
+                const double fj = f[static_cast<int64_t>(j) * n_line];
+                s_f[(2 * j) * T + tid] = fma(fj, re, s_f[(2 * j) * T + tid]);
+                s_f[(2 * j + 1) * T + tid] = fma(fj, im, s_f[(2 * j + 1) * T + tid]);
+            }
+#pragma unroll
+            for (int e = 0; e < 16; ++e) a[h][e] = 0.0;
+        }
+    };
+    uint32_t cur = 0xffffffffu;
+    for (int64_t s0 = p0; s0 < p1; s0 += npts) {
+        const int ns = static_cast<int>(min(static_cast<int64_t>(npts), p1 - s0));
+        __syncthreads();  // the previous stage's table is read
+        for (int t = tid; t < 3 * ns; t += T) {
+            const int ax = t % 3;
+            s_u[t] = xyz[3 * s0 + t] / (ax == 0 ? lx : (ax == 1 ? ly : lz));
+        }
+        __syncthreads();
+        for (int t = tid; t < ns * n_ent; t += T) {
+            const int pt = t / n_ent, e = t - pt * n_ent;
+            const int ax = e < n_index.x ? 0 : (e < n_index.x + n_index.y ? 1 : 2);
+            // n·x/L reduced to half a turn before the multiplication by 2π
+            const double u = static_cast<double>(index[e]) * s_u[3 * pt + ax];
+            double sn, cs;
+            sincospi(2.0 * (u - rint(u)), &sn, &cs);
+            pd_dl_tab[t] = make_double2(cs, sn);
+        }
+        for (int t = tid; t < ns; t += T) {
+            s_w[t] = weight ? weight[s0 + t] : 1.0;
+            s_k[t] = kind[s0 + t];
+        }
+        __syncthreads();
+        for (int pt = 0; pt < ns; ++pt) {
+            const uint32_t k = s_k[pt];
+            if (k != cur) {
+                if (cur != 0xffffffffu) flush(cur);
+                cur = k;
+            }
+            const double2 *row = pd_dl_tab + pt * n_ent;
+            // a negative index is the conjugate entry (sign bit of the member)
+            auto at = [&](int32_t m) {
+                return conj_if(row[m & 0x7fffffff], m & static_cast<int>(0x80000000u));
+            };
+            const double2 st = cmul(cmul(at(ln.sx), at(ln.sy)), at(ln.sz));
+            double2 e0 = cmul(cmul(at(ln.x), at(ln.y)), at(ln.z));
+            if (weight) {
+                const double w = s_w[pt];
+                e0.x *= w;
+                e0.y *= w;
+            }
+            double2 v[4];
+            v[0] = st;
+            v[1] = csqr(st);
+            v[2] = cmul(v[1], st);
+            v[3] = csqr(v[1]);
+            double2 E = cmul(e0, v[3]);
+            const double2 v8 = csqr(v[3]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                a[h][0] += E.x;
+                a[h][1] += E.y;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    a[h][2 + 4 * q] = fma(E.x, v[q].x, a[h][2 + 4 * q]);
+                    a[h][3 + 4 * q] = fma(E.y, v[q].y, a[h][3 + 4 * q]);
+                    a[h][4 + 4 * q] = fma(E.y, v[q].x, a[h][4 + 4 * q]);
+                    a[h][5 + 4 * q] = fma(E.x, v[q].y, a[h][5 + 4 * q]);
+                }
+                a[h][14] = fma(E.x, v[3].x, fma(E.y, v[3].y, a[h][14]));
+                a[h][15] = fma(E.y, v[3].x, fma(-E.x, v[3].y, a[h][15]));
+                if (h == 0) E = cmul(E, v8);
+            }
+        }
+    }
+    if (cur != 0xffffffffu) flush(cur);
+    if (!ok) return;
+    double *o = part + c * 2 * J * n_line + seg;  // [chunk][j][re, im][line]
+    for (int j = 0; j < 2 * J; ++j) o[static_cast<int64_t>(j) * n_line] = s_f[j * T + tid];
+}
+
+// The points of each molecule (a block each) in stable order of their kinds: every
+// thread counts the kinds of a contiguous run, the counts are scanned kind by kind,
+// and the runs are scattered in order.
+constexpr int PD_DSORT_THREADS = 256;
+
+__global__ void __launch_bounds__(PD_DSORT_THREADS)
+    pd_direct_sort(const double *__restrict__ xyz, const uint32_t *__restrict__ kind,
+                   const double *__restrict__ weight, int64_t mol_size, int32_t n_kinds,
+                   double *__restrict__ xyz_out, uint32_t *__restrict__ kind_out,
+                   double *__restrict__ weight_out) {
+    constexpr int T = PD_DSORT_THREADS;
+    extern __shared__ uint32_t s_cnt[];  // [kind][thread]
+    __shared__ uint32_t s_scan[T];
+    const int64_t m0 = static_cast<int64_t>(blockIdx.x) * mol_size;
+    const int t = threadIdx.x;
+    const int64_t i0 = m0 + mol_size * t / T, i1 = m0 + mol_size * (t + 1) / T;
+    for (int k = 0; k < n_kinds; ++k) s_cnt[k * T + t] = 0;
+    for (int64_t i = i0; i < i1; ++i) ++s_cnt[kind[i] * T + t];
+    __syncthreads();
+    // exclusive scan of the flattened counts: n_kinds consecutive ones per thread
+    uint32_t sum = 0;
+    for (int k = 0; k < n_kinds; ++k) sum += s_cnt[t * n_kinds + k];
+    s_scan[t] = sum;
+    __syncthreads();
+    for (int o = 1; o < T; o <<= 1) {
+        const uint32_t v = t >= o ? s_scan[t - o] : 0;
+        __syncthreads();
+        s_scan[t] += v;
+        __syncthreads();
+    }
+    uint32_t at = s_scan[t] - sum;
+    for (int k = 0; k < n_kinds; ++k) {
+        const uint32_t v = s_cnt[t * n_kinds + k];
+        s_cnt[t * n_kinds + k] = at;
+        at += v;
+    }
+    __syncthreads();
+    for (int64_t i = i0; i < i1; ++i) {
+        const uint32_t k = kind[i];
+        const int64_t o = m0 + s_cnt[k * T + t]++;
+        xyz_out[3 * o] = xyz[3 * i];
+        xyz_out[3 * o + 1] = xyz[3 * i + 1];
+        xyz_out[3 * o + 2] = xyz[3 * i + 2];
+        kind_out[o] = k;
+        if (weight) weight_out[o] = weight[i];
+    }
+}
+
+// Per vector of pd_direct_lines (j·n_line + line): the slices of a molecule joined,
+// A = Σ F_m and Σ_m |F_m|². 32 lanes are 32 vectors, the warps 32 fixed runs of
+// molecules, added in run order.
+__global__ void __launch_bounds__(1024)
+    pd_direct_lines_reduce(const double *__restrict__ part, int32_t n_line, int64_t n_mol,
+                           int64_t slices_per_mol, double *__restrict__ out) {
+    __shared__ double s_run[32][3][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int n_vec = PD_DLINE_J * n_line;
+    const int v = blockIdx.x * 32 + lane;
+    const bool ok = v < n_vec;
+    const int j = ok ? v / n_line : 0, l = ok ? v - j * n_line : 0;
+    const int64_t u0 = n_mol * w / 32, u1 = n_mol * (w + 1) / 32;
+    double ar = 0.0, ai = 0.0, self = 0.0;
+    for (int64_t m = u0; ok && m < u1; ++m) {
+        double fr = 0.0, fi = 0.0;
+#pragma unroll 4
+        for (int64_t s = 0; s < slices_per_mol; ++s) {
+            const double *o = part + ((m * slices_per_mol + s) * 2 * PD_DLINE_J + 2 * j) * n_line + l;
+            fr += o[0];
+            fi += o[n_line];
+        }
+        ar += fr;
+        ai += fi;
+        self += fr * fr + fi * fi;
+    }
+    s_run[w][0][lane] = ar;
+    s_run[w][1][lane] = ai;
+    s_run[w][2][lane] = self;
+    __syncthreads();
+    if (w == 0 && ok) {
+        double x = 0.0, y = 0.0, sf = 0.0;
+        for (int r = 0; r < 32; ++r) {
+            x += s_run[r][0][lane];
+            y += s_run[r][1][lane];
+            sf += s_run[r][2][lane];
+        }
+        out[4 * static_cast<int64_t>(v)] = x;
+        out[4 * static_cast<int64_t>(v) + 1] = y;
+        out[4 * static_cast<int64_t>(v) + 2] = x * x + y * y;
+        out[4 * static_cast<int64_t>(v) + 3] = sf;
+    }
+}
+
 // Per q-vector: A = Σ chunks, Σ_m |F_m|² with the slices of a molecule joined
 // first. out[v] = (Re A, Im A, |A|², Σ_m |F_m|²). A block takes 32 vectors (a
 // lane each); its 32 warps sum 32 fixed runs of whole molecules' chunks, each in
@@ -3268,6 +3509,63 @@ cudaError_t launch_direct_table(const double *xyz, const uint32_t *kind, const d
     if (e != cudaSuccess) return e;
     pd_direct_reduce<<<static_cast<unsigned>((n_vec + 31) / 32), 32 * PD_DIRECT_RED_WARPS, 0, st>>>(
         part, n_vec, n_chunks, spm, out);
+    return cudaGetLastError();
+}
+
+int direct_line_points(int32_t n_entries) {
+    return std::min(PD_DLINE_MAX_POINTS, static_cast<int>(PD_DLINE_TABLE_BYTES /
+                                                          (n_entries * sizeof(double2))));
+}
+
+// Slices of a molecule for the line kernel: up to 4 blocks per SM (what its
+// shared memory allows) in one round where the box allows that, slices of 128 to
+// 2,048 points.
+void direct_line_layout(int64_t n_points, int64_t mol_size, int32_t n_line, int64_t *chunk,
+                        int64_t *spm) {
+    const int64_t vblocks = (n_line + PD_DLINE_THREADS - 1) / PD_DLINE_THREADS;
+    const int64_t units = n_points / mol_size * vblocks;
+    *spm = std::clamp<int64_t>(148 * 4 / units, (mol_size + 2047) / 2048,
+                               std::max<int64_t>((mol_size + 127) / 128, 1));
+    *chunk = (mol_size + *spm - 1) / *spm;
+    *spm = (mol_size + *chunk - 1) / *chunk;
+}
+
+cudaError_t launch_direct_sort(const double *xyz, const uint32_t *kind, const double *weight,
+                               int64_t n_points, int64_t mol_size, int32_t n_kinds,
+                               double *xyz_out, uint32_t *kind_out, double *weight_out,
+                               cudaStream_t st) {
+    const size_t smem = static_cast<size_t>(n_kinds) * PD_DSORT_THREADS * sizeof(uint32_t);
+    if (smem > 46 * 1024 || n_points / mol_size > 0x7fffffffLL) return cudaErrorInvalidValue;
+    pd_direct_sort<<<static_cast<unsigned>(n_points / mol_size), PD_DSORT_THREADS, smem, st>>>(
+        xyz, kind, weight, mol_size, n_kinds, xyz_out, kind_out, weight_out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_direct_lines(const double *xyz, const uint32_t *kind, const double *weight,
+                                const double *ff, const PdLine *lines, const int32_t *index,
+                                const int32_t n_index[3], const double box[3], int32_t n_line,
+                                int64_t n_points, int64_t mol_size, int64_t chunk, int64_t spm,
+                                double *part, double *out, cudaStream_t st) {
+    const int n_ent = n_index[0] + n_index[1] + n_index[2];
+    const int npts = direct_line_points(n_ent);
+    if (npts < 1 || n_line < 1) return cudaErrorInvalidValue;
+    const int threads = std::min(PD_DLINE_THREADS, (n_line + 31) / 32 * 32);
+    const int vblocks = (n_line + threads - 1) / threads;
+    const int64_t n_mol = n_points / mol_size, blocks = n_mol * spm * vblocks;
+    if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+    const size_t smem = static_cast<size_t>(npts) * n_ent * sizeof(double2) +
+                        2 * PD_DLINE_J * static_cast<size_t>(threads) * sizeof(double);
+    cudaError_t e = cudaFuncSetAttribute(
+        pd_direct_lines, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        PD_DLINE_TABLE_BYTES + 2 * PD_DLINE_J * PD_DLINE_THREADS * static_cast<int>(sizeof(double)));
+    if (e != cudaSuccess) return e;
+    pd_direct_lines<<<static_cast<unsigned>(blocks), threads, smem, st>>>(
+        xyz, kind, weight, ff, lines, index, make_int3(n_index[0], n_index[1], n_index[2]), box[0],
+        box[1], box[2], npts, n_line, vblocks, mol_size, chunk, spm, part);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    pd_direct_lines_reduce<<<static_cast<unsigned>((PD_DLINE_J * static_cast<int64_t>(n_line) + 31) /
+                                                   32),
+                             1024, 0, st>>>(part, n_line, n_mol, spm, out);
     return cudaGetLastError();
 }
 

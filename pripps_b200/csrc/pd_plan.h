@@ -77,6 +77,9 @@ struct Plan {
     int64_t lat_bins = 0;
 };
 
+// Whether every one of n values is finite (no early exit: a few values per cycle).
+bool all_finite(const double *x, uint64_t n);
+
 // Validate a request; fills msg and returns a PD_E* code on failure.
 int validate_request(const pd_request *req, bool device_pointers, std::string &msg);
 

@@ -168,3 +168,47 @@ def test_lattice_grid_direct_intensity_matches_oracle(gpu_ctx):
     q, ref = grid.group(qn, rows[:, 2:3])
     assert np.array_equal(got.q, q)
     assert np.max(np.abs(got.total - ref[:, 0]) / np.abs(ref[:, 0]).max()) < 1e-12
+
+
+@pytest.mark.parametrize("case", ["miller_17", "miller_1", "axis_runs", "axis_runs_k", "no_lines",
+                                  "weights", "slices", "many_kinds", "duplicates"])
+def test_lines_match_the_sincos_rows(gpu_ctx, case):
+    """pd_direct_lattice's line kernel (segments of 16 consecutive vectors; the
+    points sorted by kind within molecules of at least 128 points) against
+    pd_direct at the same vectors: segments of 1, 16 and 17 vectors, lines along an
+    axis with negative indices and gaps, vectors on no line (the table kernel),
+    weights, molecules cut into several slices, more kinds than the device sort
+    takes, and repeated vectors. 1e-12 of (Σ|w f|)² and of Σ|w f|, the
+    tolerance of the two entry points."""
+    rng = np.random.default_rng(len(case))
+    n_mol, mol, nk = (3, 130, 3) if case != "slices" else (2, 4999, 3)
+    if case == "many_kinds":
+        nk = 40
+    n = n_mol * mol
+    box = np.array([37.0, 41.0, 29.0])
+    xyz = rng.uniform(-60, 60, (n, 3))
+    kind = rng.integers(0, nk, n)
+    if case == "axis_runs":
+        hkl = np.array([(h, k, l) for h in range(-2, 3) for k in (0, 3) for l in range(-20, 21)
+                        if l != 7])
+    elif case == "axis_runs_k":
+        hkl = np.array([(h, k, 5) for h in range(3) for k in range(-33, 30)])
+    elif case == "no_lines":
+        hkl = rng.integers(-30, 31, (60, 3))
+    elif case == "duplicates":
+        hkl = np.concatenate([miller_indices(20), miller_indices(9), np.zeros((2, 3), int)])
+    else:
+        hkl = miller_indices(1 if case == "miller_1" else 17)
+    hkl = hkl[rng.permutation(len(hkl))]
+    qv = 2 * np.pi * hkl / box
+    ff = rng.uniform(-2, 8, (nk, len(hkl)))
+    w = rng.uniform(0, 2, n) if case in ("weights", "slices") else None
+    got = amplitudes(xyz, kind, ff, None, n_mol, w, gpu_ctx, hkl=hkl, box=box)
+    ref = amplitudes(xyz, kind, ff, qv, n_mol, w, gpu_ctx)
+    scale = np.sum(np.abs(ff[kind]) * (1.0 if w is None else w[:, None]), axis=0)
+    assert np.all(np.abs(got[:, :2] - ref[:, :2]) <= 1e-12 * scale[:, None])
+    assert np.all(np.abs(got[:, 2:] - ref[:, 2:]) <= 1e-12 * scale[:, None] ** 2)
+    bad = xyz.copy()
+    bad[n // 2, 1] = np.nan
+    with pytest.raises(Exception, match="non-finite coordinate"):
+        amplitudes(bad, kind, ff, None, n_mol, w, gpu_ctx, hkl=hkl, box=box)

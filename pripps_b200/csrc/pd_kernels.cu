@@ -1994,17 +1994,20 @@ __global__ void __launch_bounds__(PD_DSUM_THREADS)
     const int64_t row = static_cast<int64_t>(n_pairs) * NV * sh.node_cap;
     double *pt = part + (static_cast<int64_t>(f) * sh.grp_cap + grp) * row;
     // a thread per (pair, node); each starts at a direction of its own, so that
-    // the 32 reads of a warp touch all banks
+    // the 32 reads of a warp touch all banks (tiles of 4, 8 or 16 nodes: the
+    // pair's bits reversed). The start depends on the pair and the node alone: the
+    // order of a sum, and so its rounding, does not follow the tile size.
     for (int k = threadIdx.x; k < n_pairs * nn; k += PD_DSUM_THREADS) {
         const int p = k / nn, t = k - p * nn;
         const int a = pairs[p].a, b = pairs[p].b;
         const double *Ea = s_e + (a * NV2 * NT + t) * 64, *Eb = s_e + (b * NV2 * NT + t) * 64;
+        const int rot = tile * NT + t + static_cast<int>(__brev(p) >> 27);
         double x[NV];
 #pragma unroll
         for (int v = 0; v < NV; ++v) x[v] = 0.0;
 #pragma unroll 4
         for (int i = 0; i < 32; ++i) {
-            const int d = (i + lane) & 31;
+            const int d = (i + rot) & 31;
             const double w = s_w[d];
             const double ar = w * Ea[d], ai = w * Ea[32 + d], br = Eb[d], bi = Eb[32 + d];
             x[0] = fma(ar, br, fma(ai, bi, x[0]));

@@ -181,6 +181,7 @@ struct PinnedPool {
             if (it != free_blocks.end() && !it->second.empty()) {
                 *out = it->second.back();
                 it->second.pop_back();
+                kept -= c;
                 *cls = c;
                 return cudaSuccess;
             }
@@ -194,15 +195,27 @@ struct PinnedPool {
         *cls = c;
         return cudaSuccess;
     }
+    // At most KEEP bytes wait for a next use; a block beyond goes back to the system.
+    static constexpr uint64_t KEEP = uint64_t{1} << 30;
+    uint64_t kept = 0;
     void put(char *p, uint64_t cls) {
-        std::lock_guard<std::mutex> g(mu);
-        free_blocks[cls].push_back(p);
+        {
+            std::lock_guard<std::mutex> g(mu);
+            if (kept + cls <= KEEP) {
+                kept += cls;
+                free_blocks[cls].push_back(p);
+                return;
+            }
+            all.erase(std::find(all.begin(), all.end(), p));
+        }
+        cudaFreeHost(p);
     }
     void release() {
         std::lock_guard<std::mutex> g(mu);
         for (char *p : all) cudaFreeHost(p);
         all.clear();
         free_blocks.clear();
+        kept = 0;
     }
 };
 
@@ -489,17 +502,24 @@ constexpr int kBudgetWait = -100;  // internal: does not fit the budget right no
 
 // Host planning only: tiles, lists and the device layout.
 int plan_host(pd_ctx *ctx, const pd_request *req, const uint32_t *species, const double *weights,
-              bool host_xyz, double radius_hint, DevPlan &dp, const Tuning *force = nullptr) {
+              bool host_xyz, double radius_hint, DevPlan &dp, const Tuning *force = nullptr,
+              bool exact_radius = false) {
     NvtxRange nvtx("pd plan (host)");
     std::string msg;
     const Tuning tun = force ? *force : tuning_for_request(ctx, req, species, weights);
-    int rc = pd::build_plan(req, species, weights, tun, dp.P, msg, false, radius_hint);
-    if (rc != PD_OK) {
-        ctx->set_error(msg);
-        return rc;
-    }
     dp.host_xyz = host_xyz;
-    dp.L = make_layout(dp.P, host_xyz);
+    for (bool tiles = !exact_radius;; tiles = true) {
+        int rc = pd::build_plan(req, species, weights, tun, dp.P, msg, false, radius_hint, !tiles);
+        if (rc != PD_OK) {
+            ctx->set_error(msg);
+            return rc;
+        }
+        dp.L = make_layout(dp.P, host_xyz);
+        // without tiles only where their plan would have fitted too
+        if (!dp.P.dir_only || static_cast<double>(dp.L.total) + dp.P.pair_bytes <=
+                                  static_cast<double>(ctx->budget))
+            break;
+    }
     if (dp.L.total > ctx->budget) {  // the pair form alone may fit
         pd::drop_directions(dp.P);
         dp.L = make_layout(dp.P, host_xyz);
@@ -542,7 +562,8 @@ int plan_device(pd_ctx *ctx, const pd_request *req, DevPlan &dp, cudaStream_t st
     }
     stage_plan(ctx, dp, req);
     e = cudaMemcpyAsync(dp.base, dp.stage, dp.L.upload_bytes, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(dp.base + dp.L.status, 0, 8, st);
+    // every execution clears the status, but a streamed trajectory's keep it
+    if (e == cudaSuccess && dp.frame_sum) e = cudaMemsetAsync(dp.base + dp.L.status, 0, 8, st);
     if (e != cudaSuccess) {
         free_devplan(ctx, dp, st);
         return cuda_fail(ctx, e, "plan upload");
@@ -553,8 +574,9 @@ int plan_device(pd_ctx *ctx, const pd_request *req, DevPlan &dp, cudaStream_t st
 
 int create_devplan(pd_ctx *ctx, const pd_request *req, const uint32_t *species,
                    const double *weights, bool host_xyz, double radius_hint, DevPlan &dp,
-                   cudaStream_t st, const Tuning *force = nullptr) {
-    int rc = plan_host(ctx, req, species, weights, host_xyz, radius_hint, dp, force);
+                   cudaStream_t st, const Tuning *force = nullptr, bool exact_radius = false) {
+    int rc = plan_host(ctx, req, species, weights, host_xyz, radius_hint, dp, force,
+                       exact_radius);
     if (rc) return rc;
     return plan_device(ctx, req, dp, st, false);
 }
@@ -566,12 +588,16 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st) {
     const Plan &P = dp.P;
     const Layout &L = dp.L;
     const int add_exact = dp.rank == 0 ? 1 : 0;
-    PD_CUDA(ctx, pd::launch_reduce(dp.dptr<double>(L.slots), dp.dptr<int64_t>(L.lptr),
-                                   dp.dptr<int64_t>(L.lidx), dp.dptr<PdPairDev>(L.pairs),
-                                   dp.dptr<double>(L.qv), dp.dptr<PdFrameDev>(L.frames), P.red,
-                                   P.nv, P.n_frames, P.precision == PD_FP32_FP64RED ? 1 : 0,
-                                   add_exact, dp.dptr<double>(L.chunk_sums),
-                                   dp.dptr<unsigned int>(L.red_done), dp.dptr<double>(L.red), st));
+    if (!P.dir_only) {
+        PD_CUDA(ctx, pd::launch_reduce(dp.dptr<double>(L.slots), dp.dptr<int64_t>(L.lptr),
+                                       dp.dptr<int64_t>(L.lidx), dp.dptr<PdPairDev>(L.pairs),
+                                       dp.dptr<double>(L.qv), dp.dptr<PdFrameDev>(L.frames), P.red,
+                                       P.nv, P.n_frames, P.precision == PD_FP32_FP64RED ? 1 : 0,
+                                       add_exact, dp.dptr<double>(L.chunk_sums),
+                                       dp.dptr<unsigned int>(L.red_done), dp.dptr<double>(L.red),
+                                       st));
+        ctx->launches += 1;
+    }
     if (P.amp.dir_cap > 0) {
         PD_CUDA(ctx, pd::launch_direction_sums(
                          dp.dptr<double>(L.slots), dp.dptr<double4>(L.dirs),
@@ -582,7 +608,7 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st) {
                          dp.dptr<unsigned int>(L.dir_done), dp.dptr<double>(L.red), st));
         ctx->launches += 1;
     }
-    if (!P.lat.empty()) {
+    if (!P.lat.empty() && !P.dir_only) {
         PD_CUDA(ctx, pd::launch_lattice_sums(
                          reinterpret_cast<const unsigned long long *>(dp.dptr<char>(L.hist)),
                          dp.dptr<PdLatDev>(L.lat), static_cast<int>(P.lat.size()),
@@ -600,7 +626,7 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st) {
                                      P.has_hyd ? dp.dptr<double>(L.ffW) : nullptr, add_exact,
                                      P.qmax, P.lat.empty() ? nullptr : dp.dptr<int>(L.lat_err),
                                      terms, st));
-    ctx->launches += 2;
+    ctx->launches += 1;
     if (P.n_frames > 1) {
         PD_CUDA(ctx, pd::launch_frame_mean(dp.dptr<double>(L.terms), dp.dptr<double>(L.fw),
                                            P.n_frames, P.nq, dst, st, !dp.frame_sum));
@@ -774,6 +800,7 @@ static_assert((STEP_BUFS + 1) * STEP_LANES <= 32, "lane bits of PdTicket::used_s
 
 // Relative cost of one pair·q of a tile (FP32 class mode = 1).
 double tile_cost(const Plan &P, const PdJob &jb) {
+    if (P.dir_only) return P.job_cost;
     double c = static_cast<double>(PD_IBLOCK) * (jb.j1 - jb.j0) * P.tun.K;
     if (P.precision == PD_FP64) c *= 24.0;
     if (P.mode == PD_MODE_WEIGHTED) c *= 1.5;
@@ -837,7 +864,7 @@ void planner_main(pd_ctx *ctx) {
         std::string m;
         if (!t->canceled) {
             rc = plan_host(ctx, &t->req, t->req.species, t->req.hyd_weights, true,
-                           host_radius(&t->req), t->dp);
+                           host_radius(&t->req), t->dp, nullptr, /*exact_radius=*/true);
             if (rc != PD_OK) {
                 std::lock_guard<std::mutex> g(ctx->mu);
                 m = ctx->errors[std::this_thread::get_id()];
@@ -984,7 +1011,7 @@ void worker_main(pd_ctx *ctx) {
                     if (cost > EXPRESS_COST) break;
                 }
                 t->express_wait =
-                    !P.jobs.empty() && cost <= EXPRESS_COST && P.jobs.size() <= STEP_MAX_JOBS;
+                    t->small && !P.jobs.empty() && cost <= EXPRESS_COST && P.jobs.size() <= STEP_MAX_JOBS;
             }
             // the device and the pinned image hold the inputs now
             t->xyz = {};
@@ -1407,23 +1434,28 @@ int pd_solve(pd_ctx *ctx, const pd_request *req, double *out_terms) {
     cudaSetDevice(ctx->device);
     DevPlan dp;
     rc = create_devplan(ctx, req, req->species, req->hyd_weights, true, host_radius(req), dp,
-                        ctx->stream);
+                        ctx->stream, nullptr, /*exact_radius=*/true);
     if (rc) return rc;
     rc = run_devplan(ctx, dp, nullptr, ctx->stream);
     if (rc == PD_OK) {
+        // the result and the status word behind it, in one copy to pinned memory
+        const size_t n6 = static_cast<size_t>(6) * dp.P.nq;
+        const double *res = dp.hptr<double>(dp.L.hres);
         int32_t dev_status = 0;
-        cudaError_t e = cudaMemcpyAsync(out_terms, dp.dptr<double>(dp.L.out),
-                                        static_cast<size_t>(6) * dp.P.nq * 8,
-                                        cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(&dev_status, dp.base + dp.L.status, sizeof(int32_t),
-                                cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+        cudaError_t e = cudaMemcpyAsync(dp.hptr<double>(dp.L.hres), dp.dptr<double>(dp.L.out),
+                                        n6 * 8 + 8, cudaMemcpyDeviceToHost, ctx->stream);
+        const cudaError_t es = cudaStreamSynchronize(ctx->stream);
+        if (e == cudaSuccess) e = es;
         if (e != cudaSuccess) rc = cuda_fail(ctx, e, "pd_solve");
-        if (rc == PD_OK) rc = result_status(ctx, dp.P, dev_status, out_terms);
+        if (rc == PD_OK) {
+            std::memcpy(out_terms, res, n6 * 8);
+            std::memcpy(&dev_status, res + n6, sizeof(int32_t));
+            rc = result_status(ctx, dp.P, dev_status, out_terms);
+        }
+    } else {
+        cudaStreamSynchronize(ctx->stream);  // nothing may still read the pinned image
     }
     free_devplan(ctx, dp, ctx->stream);
-    cudaStreamSynchronize(ctx->stream);
     return rc;
 }
 
@@ -2681,6 +2713,12 @@ struct pd_stream {
     uint32_t B = 0;
     uint64_t frame_doubles = 0;       // 3·N
     cudaStream_t cs = nullptr, us = nullptr;  // compute, upload
+    // One device block (two batches of coordinates, the sum, a batch's result) from
+    // the context's pool and one pinned block (two batches and their weights):
+    // two cudaMalloc, four cudaHostAlloc and their frees were 6 to 25 of the 12 to
+    // 31 ms of a 150-frame stream of 2,003 atoms.
+    char *d_block = nullptr, *h_block = nullptr;
+    uint64_t h_cls = 0;
     double *d_xyz[2] = {nullptr, nullptr};
     double *h_xyz[2] = {nullptr, nullptr};
     double *h_w[2] = {nullptr, nullptr};
@@ -2700,14 +2738,11 @@ void stream_free(pd_ctx *ctx, pd_stream *s) {
     if (s->cs) cudaStreamSynchronize(s->cs);
     if (s->us) cudaStreamSynchronize(s->us);
     for (int b = 0; b < 2; ++b) {
-        if (s->d_xyz[b]) cudaFree(s->d_xyz[b]);
-        if (s->h_xyz[b]) cudaFreeHost(s->h_xyz[b]);
-        if (s->h_w[b]) cudaFreeHost(s->h_w[b]);
         if (s->uploaded[b]) cudaEventDestroy(s->uploaded[b]);
         if (s->computed[b]) cudaEventDestroy(s->computed[b]);
     }
-    if (s->d_acc) cudaFree(s->d_acc);
-    if (s->d_batch) cudaFree(s->d_batch);
+    if (s->d_block) cudaFreeAsync(s->d_block, s->cs);
+    if (s->h_block) ctx->pinned.put(s->h_block, s->h_cls);
     free_devplan(ctx, s->dp, s->cs ? s->cs : ctx->stream);
     if (s->cs) cudaStreamSynchronize(s->cs);
     if (s->cs) cudaStreamDestroy(s->cs);
@@ -2769,9 +2804,9 @@ extern "C" int pd_stream_open(pd_ctx *ctx, const pd_request *req, uint32_t frame
         ctx->set_error("streamed trajectories take atoms only (lattice sets need one frame)");
         return PD_EINVAL;
     }
-    r.n_frames = frames_per_batch;
+    r.n_frames = 1;  // the checks of one frame hold for every one
     r.frame_weights = nullptr;
-    dummy.assign(static_cast<size_t>(r.n_atoms) * 3 * frames_per_batch, 0.0);
+    if (r.n_atoms <= (1ull << 30)) dummy.assign(static_cast<size_t>(r.n_atoms) * 3, 0.0);
     r.xyz = dummy.data();
     std::string msg;
     int rc = pd::validate_request(&r, false, msg);
@@ -2779,6 +2814,7 @@ extern "C" int pd_stream_open(pd_ctx *ctx, const pd_request *req, uint32_t frame
         ctx->set_error(msg);
         return rc;
     }
+    r.n_frames = frames_per_batch;
     std::lock_guard<std::mutex> g(ctx->solve_mu);
     cudaSetDevice(ctx->device);
     auto *s = new pd_stream();
@@ -2798,15 +2834,21 @@ extern "C" int pd_stream_open(pd_ctx *ctx, const pd_request *req, uint32_t frame
     }
     const size_t fb = s->frame_doubles * 8 * s->B;
     const size_t nq6 = 6ull * r.nq * 8;
+    const size_t db = align_up(fb, 256), rb = align_up(nq6, 256), wb = align_up(8ull * s->B, 256);
+    e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(&s->d_block), 2 * (db + rb), ctx->pool,
+                                s->cs);
+    if (e == cudaSuccess) e = ctx->pinned.get(2 * (db + wb), &s->h_block, &s->h_cls);
     for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
-        e = cudaMalloc(reinterpret_cast<void **>(&s->d_xyz[b]), fb);
-        if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void **>(&s->h_xyz[b]), fb, 0);
-        if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void **>(&s->h_w[b]), 8ull * s->B, 0);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->uploaded[b], cudaEventDisableTiming);
+        s->d_xyz[b] = reinterpret_cast<double *>(s->d_block + b * db);
+        s->h_xyz[b] = reinterpret_cast<double *>(s->h_block + b * db);
+        s->h_w[b] = reinterpret_cast<double *>(s->h_block + 2 * db + b * wb);
+        e = cudaEventCreateWithFlags(&s->uploaded[b], cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->computed[b], cudaEventDisableTiming);
     }
-    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&s->d_acc), nq6);
-    if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&s->d_batch), nq6);
+    if (e == cudaSuccess) {
+        s->d_acc = reinterpret_cast<double *>(s->d_block + 2 * db);
+        s->d_batch = reinterpret_cast<double *>(s->d_block + 2 * db + rb);
+    }
     if (e == cudaSuccess) e = cudaMemsetAsync(s->d_acc, 0, nq6, s->cs);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->cs);
     if (e != cudaSuccess) {
@@ -2824,11 +2866,12 @@ extern "C" int pd_stream_push(pd_ctx *ctx, pd_stream *s, const double *xyz,
         ctx->set_error("the stream failed earlier");
         return PD_EDEVICE;
     }
-    for (uint64_t i = 0; i < n_frames * s->frame_doubles; ++i)
-        if (!std::isfinite(xyz[i])) {
-            ctx->set_error("non-finite coordinate at index " + std::to_string(i));
-            return PD_EINVAL;
-        }
+    if (!pd::all_finite(xyz, n_frames * s->frame_doubles)) {
+        uint64_t i = 0;
+        while (std::isfinite(xyz[i])) ++i;
+        ctx->set_error("non-finite coordinate at index " + std::to_string(i));
+        return PD_EINVAL;
+    }
     for (uint64_t f = 0; weights && f < n_frames; ++f)
         if (!std::isfinite(weights[f])) {
             ctx->set_error("non-finite frame weight");

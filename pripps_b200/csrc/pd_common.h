@@ -112,6 +112,7 @@ constexpr int PD_MAX_MOMENTS = 512;
 // and the shared memory of the kernel that sums the class pairs.
 constexpr int PD_MAX_DIR_MOMENTS = 256;
 constexpr int PD_DIR_SMEM = 200 * 1024;
+constexpr int PD_DIR_DIRS = 8;  // directions of a work unit
 
 // When a frame may run in the moment form (block = 0: never).
 struct PdMomentRule {
@@ -130,6 +131,7 @@ struct PdMomentRule {
     int64_t slot_cap;     // doubles per frame for the chunks' sums
     int64_t n_atoms;
     int32_t nq;
+    int32_t dir_only;     // the plan has no tiles: every frame takes the direction form
 };
 
 // Sizes the direction kernels share.
@@ -151,6 +153,7 @@ struct PdReduceShape {
     int32_t n_chunk;      // blocks that share a slot list
     int32_t max_moments;  // moments or nodes
     int32_t node_cap;     // nodes (direction form)
+    int32_t dir_only;     // no tiles (a frame without directions has no result: NaN)
     int64_t slots_per_frame;
 };
 

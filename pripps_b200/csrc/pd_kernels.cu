@@ -1691,7 +1691,7 @@ __global__ void __launch_bounds__(PD_PACK_THREADS)
                      m8 <= rule.amp_cap && nodes <= rule.node_cap &&
                      static_cast<int64_t>(rule.n_chunk) * rule.nv2 *
                              ((groups + rule.world - 1) / rule.world) * m8 * 32 <= rule.slot_cap &&
-                     groups >= rule.world && dir_cost < pair_cost;
+                     groups >= rule.world && (rule.dir_only || dir_cost < pair_cost);
     if (use) {
         fr.n_grp = mine;
         fr.n_amp = m8;
@@ -2294,7 +2294,8 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
         double v = 0.0;
 #pragma unroll
         for (int w = 0; w < PD_PROF_THREADS / 32; ++w) v += s_sum[w][t][ql];
-        if (err && *err) v = __longlong_as_double(0x7ff8000000000000ll);  // a point off its lattice
+        // a point off its lattice, or a frame whose form the plan has nothing for
+        if ((err && *err) || (sh.dir_only && !nodes)) v = __longlong_as_double(0x7ff8000000000000ll);
         if (ok) terms[(static_cast<int64_t>(f) * 6 + t) * sh.nq + q] = v;
     }
 }

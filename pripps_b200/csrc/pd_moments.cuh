@@ -232,7 +232,6 @@ __device__ __forceinline__ void moments_range(const float4 *__restrict__ at, int
 // shared memory, for its direction dv = n/(2·r1); same layout of the sums. With
 // room in registers (ILP) two atoms at a time: their sequences' dependency
 // chains overlap.
-constexpr int PD_DIR_DIRS = 8;                           // directions of a work unit
 constexpr int PD_DIR_LANES = PD_THREADS / PD_DIR_DIRS;   // atoms it takes at once
 
 template <int KM, bool WEIGHTED, bool ILP>

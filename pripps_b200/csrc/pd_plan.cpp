@@ -4,10 +4,12 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <numeric>
 #include <utility>
 
 #include "pd_kernels.h"
+#include "pd_tuning.h"
 
 namespace pd {
 
@@ -20,6 +22,12 @@ __attribute__((optimize("O3"))) bool all_finite(const double *x, uint64_t n) {
     for (; i < n; ++i) s[0] += 0.0 * x[i];
     for (int k = 1; k < 8; ++k) s[0] += s[k];
     return s[0] == 0.0;
+}
+
+__attribute__((optimize("O3"))) static uint32_t max_species(const uint32_t *x, uint64_t n) {
+    uint32_t m = 0;
+    for (uint64_t i = 0; i < n; ++i) m = m > x[i] ? m : x[i];
+    return m;
 }
 
 int validate_request(const pd_request *req, bool device_pointers, std::string &msg) {
@@ -105,38 +113,35 @@ int validate_request(const pd_request *req, bool device_pointers, std::string &m
     if (device_pointers) return PD_OK;
     // Host buffers: check the values the planner and the kernels rely on.
     const uint64_t n = req->n_atoms;
-    for (uint64_t i = 0; i < n; ++i) {
-        if (req->species[i] >= req->n_species) {
-            msg = "species id " + std::to_string(req->species[i]) + " at atom " +
-                  std::to_string(i) + " is >= n_species";
-            return PD_EINVAL;
-        }
+    // (whole-array scans first; the loops only name the offending entry)
+    if (max_species(req->species, n) >= req->n_species) {
+        uint64_t i = 0;
+        while (req->species[i] < req->n_species) ++i;
+        msg = "species id " + std::to_string(req->species[i]) + " at atom " + std::to_string(i) +
+              " is >= n_species";
+        return PD_EINVAL;
     }
-    for (uint64_t i = 0; i < n * 3 * nf; ++i) {
-        if (!std::isfinite(req->xyz[i])) {
-            msg = "non-finite coordinate at index " + std::to_string(i);
-            return PD_EINVAL;
-        }
+    if (!all_finite(req->xyz, n * 3 * nf)) {
+        uint64_t i = 0;
+        while (std::isfinite(req->xyz[i])) ++i;
+        msg = "non-finite coordinate at index " + std::to_string(i);
+        return PD_EINVAL;
     }
     const uint64_t nt = static_cast<uint64_t>(req->n_species) * req->nq;
-    for (uint64_t i = 0; i < nt; ++i) {
-        if (!std::isfinite(req->ff_atoms[i]) ||
-            (req->ff_excluded && !std::isfinite(req->ff_excluded[i]))) {
-            msg = "non-finite form-factor table entry";
-            return PD_EINVAL;
-        }
+    if (!all_finite(req->ff_atoms, nt) ||
+        (req->ff_excluded && !all_finite(req->ff_excluded, nt))) {
+        msg = "non-finite form-factor table entry";
+        return PD_EINVAL;
     }
     if (req->hyd_weights) {
-        for (uint64_t i = 0; i < n; ++i)
-            if (!std::isfinite(req->hyd_weights[i])) {
-                msg = "non-finite hydration weight";
-                return PD_EINVAL;
-            }
-        for (uint64_t i = 0; i < req->nq; ++i)
-            if (!std::isfinite(req->ff_water[i])) {
-                msg = "non-finite water form factor";
-                return PD_EINVAL;
-            }
+        if (!all_finite(req->hyd_weights, n)) {
+            msg = "non-finite hydration weight";
+            return PD_EINVAL;
+        }
+        if (!all_finite(req->ff_water, req->nq)) {
+            msg = "non-finite water form factor";
+            return PD_EINVAL;
+        }
     }
     if (req->frame_weights) {
         double s = 0.0;
@@ -228,27 +233,58 @@ Tuning default_tuning(int64_t n_atoms, int64_t nq, int precision, int64_t n_fram
     return t;
 }
 
+// Index of a (species, weight) key among at most max_keys distinct ones in
+// first-seen order, or -1 for one too many: a table of 256 places, probed from
+// a multiplicative hash (at most 48 keys, so a probe rarely steps on). Equality
+// of the weights as numbers: adding +0 gives both zeros one bit pattern.
+struct KeySet {
+    std::vector<std::pair<uint32_t, double>> seen;
+    int16_t at[256];
+    int max_keys;
+    explicit KeySet(int max) : max_keys(max) {
+        static_assert(PD_MAX_CLASSES < 128, "places of the key table");
+        std::fill(at, at + 256, int16_t{-1});
+        seen.reserve(max);
+    }
+    int find(uint32_t species, double w) {
+        const double z = w + 0.0;
+        uint64_t bits;
+        std::memcpy(&bits, &z, 8);
+        uint64_t h = ((bits ^ (uint64_t{species} << 32) ^ species) * 0x9E3779B97F4A7C15ull) >> 56;
+        for (;; h = (h + 1) & 255) {
+            const int k = at[h];
+            if (k < 0) break;
+            if (seen[k].first == species && seen[k].second == w) return k;
+        }
+        if (static_cast<int>(seen.size()) == max_keys) return -1;
+        at[h] = static_cast<int16_t>(seen.size());
+        seen.emplace_back(species, w);
+        return at[h];
+    }
+};
+
+int request_mode(const pd_request *req, const uint32_t *species, const double *weights) {
+    if (!req->hyd_weights || !weights) return PD_MODE_CLASS;
+    KeySet keys(PD_MAX_CLASSES);
+    for (uint64_t i = 0; i < req->n_atoms; ++i)
+        if (keys.find(species[i], weights[i]) < 0) return PD_MODE_WEIGHTED;
+    return PD_MODE_CLASS;
+}
+
 // The distinct (species, weight) keys of the atoms in ascending order and
 // each atom's index among them; false as soon as there are more than
 // max_keys. Weights are finite (validated), so equality is the map order's
-// equivalence. A linear search from the previous atom's key: atoms of one
-// residue or surface patch repeat keys, and there are at most max_keys.
+// equivalence.
 static bool weight_class_keys(int64_t n, const uint32_t *species, const double *w,
                               int max_keys, std::vector<std::pair<uint32_t, double>> &keys,
                               std::vector<int32_t> &atom_key) {
-    std::vector<std::pair<uint32_t, double>> seen;  // first-seen order
-    size_t last = 0;
+    KeySet set(max_keys);
     for (int64_t i = 0; i < n; ++i) {
-        const std::pair<uint32_t, double> k(species[i], w[i]);
-        if (seen.empty() || !(seen[last] == k)) {
-            last = std::find(seen.begin(), seen.end(), k) - seen.begin();
-            if (last == seen.size()) {
-                if (static_cast<int>(seen.size()) == max_keys) return false;
-                seen.push_back(k);
-            }
-        }
-        atom_key[i] = static_cast<int32_t>(last);
+        const int k = set.find(species[i], w[i]);
+        if (k < 0) return false;
+        atom_key[i] = k;
     }
+    const auto &seen = set.seen;
     std::vector<int32_t> order(seen.size()), rank(seen.size());
     std::iota(order.begin(), order.end(), 0);
     std::sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return seen[a] < seen[b]; });
@@ -276,9 +312,11 @@ static void species_class_keys(int64_t n, const uint32_t *species, int32_t n_spe
     for (int64_t i = 0; i < n; ++i) atom_key[i] = rank[species[i]];
 }
 
+static bool direction_only(Plan &P);
+
 int build_plan(const pd_request *req, const uint32_t *species, const double *w,
                const Tuning &tun, Plan &P, std::string &msg, bool count_pairs,
-               double radius_hint) {
+               double radius_hint, bool allow_dir_only) {
     P = Plan();
     P.radius_hint = radius_hint;
     P.n_atoms = static_cast<int64_t>(req->n_atoms);
@@ -353,14 +391,14 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
         lat_of_cls[found] = static_cast<int>(P.lat.size());
         P.lat.push_back(d);
     }
-    std::vector<std::vector<int32_t>> members(c);
-    for (int64_t i = 0; i < n; ++i) members[atom_cls[i]].push_back(static_cast<int32_t>(i));
+    std::vector<int64_t> count(c, 0);
+    for (int64_t i = 0; i < n; ++i) ++count[atom_cls[i]];
     // ---- padded layout
     P.cls_start.assign(c, 0);
     int64_t cur = 0;
     for (int k = 0; k < c; ++k) {
         P.cls_start[k] = static_cast<int32_t>(cur);
-        const int64_t nk = static_cast<int64_t>(members[k].size());
+        const int64_t nk = count[k];
         cur += (nk + PD_GRANULE - 1) / PD_GRANULE * PD_GRANULE;
     }
     cur = (cur + PD_IBLOCK - 1) / PD_IBLOCK * PD_IBLOCK;
@@ -373,17 +411,20 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
     const int ng = P.n_pad / PD_GRANULE;
     P.gvalid.assign(ng, 0);
     P.gclass.assign(ng, -1);
+    {
+        std::vector<int32_t> next(P.cls_start);
+        for (int64_t i = 0; i < n; ++i)
+            P.perm[next[atom_cls[i]]++] = static_cast<int32_t>(i);
+    }
     for (int k = 0; k < c; ++k) {
-        const int64_t nk = static_cast<int64_t>(members[k].size());
+        const int64_t nk = count[k];
         double s1 = 0, s2 = 0;
-        for (int64_t r = 0; r < nk; ++r) {
-            const int32_t src = members[k][r];
-            P.perm[P.cls_start[k] + r] = src;
-            if (P.has_hyd) {
-                s1 += w[src];
-                s2 += w[src] * w[src];
+        if (P.has_hyd)
+            for (int64_t r = 0; r < nk; ++r) {
+                const double wr = w[P.perm[P.cls_start[k] + r]];
+                s1 += wr;
+                s2 += wr * wr;
             }
-        }
         P.cls[k].n = static_cast<double>(nk);
         P.cls[k].w1 = s1;
         P.cls[k].w2 = s2;
@@ -411,9 +452,9 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
                 pd.q0[0] = na * (na - 1.0) / 2.0;
                 // Σ_{i<j} w_i and Σ_{i<j} w_j in padded order within the class.
                 double ti = 0, tj = 0, tij = 0, pre = 0;
-                const int64_t nk = static_cast<int64_t>(members[a].size());
+                const int64_t nk = P.has_hyd ? count[a] : 0;
                 for (int64_t r = 0; r < nk; ++r) {
-                    const double wr = P.has_hyd ? w[members[a][r]] : 0.0;
+                    const double wr = w[P.perm[P.cls_start[a] + r]];
                     ti += wr * static_cast<double>(nk - 1 - r);
                     tj += wr * static_cast<double>(r);
                     tij += wr * pre;
@@ -430,19 +471,13 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
     // lattice layout: class range, self pair, histogram bins, count tiles
     {
         int64_t off = 0;
-        P.lat_tiles.clear();
         for (size_t l = 0; l < P.lat.size(); ++l) {
             PdLatDev &d = P.lat[l];
             d.start = P.cls_start[d.cls];
-            d.n = static_cast<int32_t>(members[d.cls].size());
+            d.n = static_cast<int32_t>(P.cls[d.cls].n);
             d.pair = pair_index[d.cls * c + d.cls];
             d.hist_off = off;
             off += d.n_bins;
-            for (int32_t i0 = 0; i0 < d.n; i0 += PD_LAT_IBLOCK)
-                for (int32_t j0 = i0; j0 < d.n; j0 += PD_LAT_JCHUNK)
-                    if (std::min(d.n, j0 + PD_LAT_JCHUNK) - 1 > i0)
-                        P.lat_tiles.push_back(PdLatTile{static_cast<int32_t>(l), i0, j0,
-                                                        std::min(d.n, j0 + PD_LAT_JCHUNK)});
         }
         P.lat_bins = off;
     }
@@ -453,7 +488,7 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
     {
         const int64_t len = std::clamp<int64_t>(n / 6, 256, 16384);
         for (int k = 0; k < c; ++k) {
-            const int64_t nk = static_cast<int64_t>(members[k].size());
+            const int64_t nk = count[k];
             const int64_t parts = (nk + len - 1) / len;
             for (int64_t t = 0; t < parts; ++t)
                 P.chunks.push_back(PdChunk{k, P.cls_start[k] + static_cast<int32_t>(nk * t / parts),
@@ -472,9 +507,22 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
         }
     }
 
-    // ---- tiles of one frame, in creation order
     const int K = P.tun.K, TJ = P.tun.TJ;
     P.nqb = (P.nq + K - 1) / K;
+    if (allow_dir_only && radius_hint >= 0.0 && direction_only(P)) return PD_OK;
+
+    // ---- pair-count tiles of the lattice sets
+    P.lat_tiles.clear();
+    for (size_t l = 0; l < P.lat.size(); ++l) {
+        const PdLatDev &d = P.lat[l];
+        for (int32_t i0 = 0; i0 < d.n; i0 += PD_LAT_IBLOCK)
+            for (int32_t j0 = i0; j0 < d.n; j0 += PD_LAT_JCHUNK)
+                if (std::min(d.n, j0 + PD_LAT_JCHUNK) - 1 > i0)
+                    P.lat_tiles.push_back(PdLatTile{static_cast<int32_t>(l), i0, j0,
+                                                    std::min(d.n, j0 + PD_LAT_JCHUNK)});
+    }
+
+    // ---- tiles of one frame, in creation order
     struct Tile {
         int32_t i0, j0, j1, cls;
     };
@@ -492,7 +540,7 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
         }
         if (min_cls < 0) continue;
         for (int k = min_cls; k < c; ++k) {
-            const int32_t cend = P.cls_start[k] + static_cast<int32_t>(members[k].size());
+            const int32_t cend = P.cls_start[k] + static_cast<int32_t>(count[k]);
             const int32_t s0 = std::max(i0, P.cls_start[k]);
             if (cend - 1 <= i0) continue;  // no j > the block's first atom
             if (lat_of_cls[k] >= 0) {
@@ -620,20 +668,105 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
     return PD_OK;
 }
 
-double max_radius(const double *xyz, int64_t n, int64_t n_frames) {
+__attribute__((optimize("O3"))) double max_radius(const double *xyz, int64_t n, int64_t n_frames) {
     double best = 0.0;
     for (int64_t f = 0; f < n_frames; ++f) {
         const double *p = xyz + 3 * n * f;
-        double s[3] = {0, 0, 0};
-        for (int64_t i = 0; i < n; ++i)
+        // four atoms at a time in twelve sums: vector additions
+        double s[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0}, c[12], far = 0.0;
+        int64_t i = 0;
+        for (; i + 4 <= n; i += 4)
+            for (int a = 0; a < 12; ++a) s[a] += p[3 * i + a];
+        for (; i < n; ++i)
             for (int a = 0; a < 3; ++a) s[a] += p[3 * i + a];
-        for (double &v : s) v /= static_cast<double>(n);
-        for (int64_t i = 0; i < n; ++i) {
-            const double x = p[3 * i] - s[0], y = p[3 * i + 1] - s[1], z = p[3 * i + 2] - s[2];
-            best = std::max(best, x * x + y * y + z * z);
+        for (int a = 0; a < 3; ++a) {
+            c[a] = ((s[a] + s[a + 3]) + (s[a + 6] + s[a + 9])) / static_cast<double>(n);
+            c[a + 3] = c[a + 6] = c[a + 9] = c[a];
+            far = std::max(far, std::fabs(c[a]));
         }
+        double m[4] = {0, 0, 0, 0};
+        for (i = 0; i + 4 <= n; i += 4) {
+            double t[12];
+            for (int a = 0; a < 12; ++a) {
+                t[a] = p[3 * i + a] - c[a];
+                t[a] *= t[a];
+            }
+            for (int k = 0; k < 4; ++k) {
+                const double r2 = t[3 * k] + t[3 * k + 1] + t[3 * k + 2];
+                m[k] = m[k] > r2 ? m[k] : r2;
+            }
+        }
+        for (; i < n; ++i) {
+            const double x = p[3 * i] - c[0], y = p[3 * i + 1] - c[1], z = p[3 * i + 2] - c[2];
+            m[0] = std::max(m[0], x * x + y * y + z * z);
+        }
+        const double r2 = std::max(std::max(m[0], m[1]), std::max(m[2], m[3]));
+        best = std::max(best, std::sqrt(r2) * (1.0 + 1e-6) + 1e-9 * far);
     }
-    return std::sqrt(best);
+    return best;
+}
+
+// Terms of a Bessel series of argument z (as bessel_order on the device).
+static double series_order(double z, bool fp64) {
+    return fp64 ? z + 13.0 * std::cbrt(0.5 * z) + 3.0 : z + 8.0 * std::cbrt(0.5 * z) + 2.0;
+}
+
+// A plan without tiles, where the frames' exact radius (radius_hint, the largest
+// one) is known and the direction form is the cheaper one by pd_pack's own
+// comparison: planning and upload of the tiles, slots and lists were 4.7 of the
+// 10 ms of a 100,000-atom solve, 0.14 of 0.3 ms at 3,000 atoms. The sizes hold for
+// every frame: the counts of rings, ring points, moments and nodes grow with the
+// radius. False (and the tiles follow) where the tiles' plan might be refused.
+static bool direction_only(Plan &P) {
+    const double frames = P.n_frames, K = P.tun.K;
+    const double tiles = static_cast<double>(P.n_pad / PD_IBLOCK) *
+                         (P.n_cls + static_cast<double>(P.n_pad) / P.tun.TJ);
+    const double jobs = tiles * P.nqb, slots = jobs * PD_WARPS;
+    if (jobs * frames > 2147483647.0 ||
+        slots * frames >= static_cast<double>(int64_t{1} << (PD_SLOT_MAP_SHIFT - 1)))
+        return false;
+    P.jobs_per_frame = 2;  // (any: this rank has jobs of every frame)
+    P.lptr.assign(static_cast<size_t>(P.n_pairs) * P.nqb + 1, 0);
+    P.dir_only = true;
+    set_reduction(P);
+    bool use = P.amp.dir_cap > 0;
+    if (use && P.mom.block > 0) {
+        const bool fp64 = P.precision == PD_FP64;
+        const double d = std::max(2.0 * 1.03 * P.radius_hint, 1e-6);
+        const double z = P.qmax * d;  // the moments of pd_pack's pair form
+        const double m = fp64 ? series_order(z, true) : z + 9.7 * std::cbrt(0.5 * z) + 3.5;
+        const int64_t m8 = (static_cast<int64_t>(0.5 * m) + 1 + 7) & ~int64_t{7};
+        const int64_t blocks = (m8 + P.mom.block - 1) / P.mom.block;
+        if (m8 <= P.mom.max_moments && blocks <= P.nqb)
+            use = P.dir_cost < 0.5 * static_cast<double>(P.n_atoms) * P.n_atoms *
+                                   (44.0 * blocks + 1.25 * m8);
+    }
+    if (!use) {
+        P.dir_only = false;
+        return false;
+    }
+    const double row = std::max<double>(P.nq, PD_MAX_MOMENTS) + 128.0;
+    P.pair_bytes = frames * (slots * P.nv * K * 8.0 + jobs * sizeof(PdJob)) + slots * 8.0 +
+                   17.0 * frames * P.n_pairs * P.nv * row * 8.0 +
+                   static_cast<double>(P.lat_bins) * 8.0 + (1 << 20);
+    // Jobs: shares of the frame's units for the serving loop's steps (a whole
+    // plan's blocks take the units by number instead).
+    const int64_t per = std::min<int64_t>(
+        P.dir_units, std::max<int64_t>(1, (1024 + P.n_frames - 1) / P.n_frames));
+    P.jobs_per_frame = per;
+    P.job_cost = P.dir_cost / (3.0 * static_cast<double>(per));
+    if (P.precision == PD_FP64) P.job_cost *= 2.0;
+    if (P.mode == PD_MODE_WEIGHTED) P.job_cost *= 1.5;
+    P.jobs.resize(static_cast<size_t>(per) * P.n_frames);
+    for (int64_t o = 0; o < per; ++o)
+        for (int f = 0; f < P.n_frames; ++f) {
+            PdJob &jb = P.jobs[static_cast<size_t>(o) * P.n_frames + f];
+            jb = PdJob{};
+            jb.frame = f;
+            jb.ord = static_cast<int32_t>(o);
+            jb.n_ord = static_cast<int32_t>(per);
+        }
+    return true;
 }
 
 // Sizes of the direction form for frames of up to the hinted radius (pd_pack
@@ -659,9 +792,7 @@ static void set_directions(Plan &P) {
             ? P.radius_hint
             : 1.9 * std::cbrt(static_cast<double>(P.n_atoms) * 20.0 * 3.0 / (4.0 * M_PI));
     const bool fp64 = P.precision == PD_FP64;
-    auto order = [&](double z) {
-        return fp64 ? z + 13.0 * std::cbrt(0.5 * z) + 3.0 : z + 8.0 * std::cbrt(0.5 * z) + 2.0;
-    };
+    auto order = [&](double z) { return series_order(z, fp64); };
     const double z = 2.0 * radius * P.qmax;
     const double top = order(z), mo = order(1.03 * radius * P.qmax);
     if (!(top < 500.0) || !(mo < PD_MAX_DIR_MOMENTS - 8.0)) return;
@@ -672,7 +803,7 @@ static void set_directions(Plan &P) {
     const int64_t groups = (S + 31) / 32, mine = (groups + P.world - 1) / P.world;
     const int64_t m8 = (static_cast<int64_t>(mo) + 8) & ~int64_t{7};
     const double zn = 2.0 * 1.03 * radius * P.qmax;
-    const int64_t nodes = static_cast<int64_t>(0.5 * (zn + 13.0 * std::cbrt(0.5 * zn) + 3.0)) + 1;
+    const int64_t nodes = static_cast<int64_t>(0.5 * series_order(zn, true)) + 1;
     // The sums' kernel: a block's shared memory holds the coefficients and the
     // amplitudes of every class at a tile of nodes (16, or fewer while that leaves
     // SMs without a block), and the moments of as many classes as fit; up to
@@ -693,6 +824,12 @@ static void set_directions(Plan &P) {
     P.amp.node_cap = static_cast<int32_t>(nodes);
     P.amp.node_tile = static_cast<int32_t>(tile);
     P.amp.slot_cap = slots;
+    const double ablk = static_cast<double>((m8 + P.mom.block - 1) / P.mom.block);
+    P.dir_cost = static_cast<double>(S) *
+                 (static_cast<double>(P.n_atoms) * (44.0 * ablk + 1.25 * m8) +
+                  4.0 * P.n_cls * static_cast<double>(m8) * static_cast<double>(nodes));
+    P.dir_units = static_cast<int64_t>(P.amp.n_chunk) * static_cast<int64_t>(ablk) * mine *
+                  (32 / PD_DIR_DIRS);
 }
 
 void drop_directions(Plan &P) {
@@ -731,6 +868,7 @@ void set_reduction(Plan &P) {
     m.slot_cap = P.amp.slot_cap;
     m.n_atoms = P.n_atoms;
     m.nq = P.nq;
+    m.dir_only = P.dir_only ? 1 : 0;
     PdReduceShape &r = P.red;
     r = PdReduceShape{};
     r.n_pairs = P.n_pairs;
@@ -742,6 +880,7 @@ void set_reduction(Plan &P) {
     r.n_z = (std::max(P.nq, r.max_moments) + 127) / 128;
     r.max_moments = std::max(r.max_moments, P.amp.node_cap);
     r.node_cap = P.amp.node_cap;
+    r.dir_only = m.dir_only;
     r.width = std::max(P.nq, r.max_moments);
     // A block adds its share of a class pair's slot list serially: lists of
     // more than a few hundred entries are shared by up to 16 blocks (one

@@ -67,6 +67,13 @@ struct Plan {
     std::vector<int32_t> cls_ptr, cls_chunk;
     PdAmpShape amp{};
     double radius_hint = -1.0;  // largest distance from the centroid, < 0: not known
+    // Host coordinates whose exact radius makes the direction form the cheaper
+    // one: no tiles, slots or lists; the jobs only carry the direction units.
+    bool dir_only = false;
+    double dir_cost = 0.0;   // FP32 lane operations of a frame in the direction form
+    int64_t dir_units = 0;   // its work units
+    double job_cost = 0.0;   // relative cost of a job (dir_only)
+    double pair_bytes = 0.0; // at least what the tiles' plan would take (dir_only)
     uint32_t rank = 0, world = 1;
     uint64_t pairs_covered = 0; // per frame, unordered pairs over all tiles
 
@@ -103,11 +110,14 @@ int shard_plan(const Plan &full, uint32_t rank, uint32_t world, Plan &out);
 // that only pd_plan_inspect needs). radius_hint sizes the direction form's arrays: the
 // largest distance of an atom from its frame's centroid, or < 0 when the
 // coordinates are not known yet (a generous estimate from the atom count).
+// With allow_dir_only the hint is the exact radius (a little more is fine), and
+// a plan whose frames all take the direction form gets no tiles.
 int build_plan(const pd_request *req, const uint32_t *species_host, const double *weights_host,
                const Tuning &tun, Plan &plan, std::string &msg, bool count_pairs = false,
-               double radius_hint = -1.0);
+               double radius_hint = -1.0, bool allow_dir_only = false);
 
-// Largest distance of an atom from its frame's centroid (host coordinates).
+// Largest distance of an atom from its frame's centroid (host coordinates), not
+// below the same taken with the centroid summed in another order.
 double max_radius(const double *xyz, int64_t n_atoms, int64_t n_frames);
 
 // Give up the direction form's arrays (a request that only fits without them).

@@ -27,23 +27,6 @@ TuneKey tune_key(int64_t n_atoms, int64_t nq, int precision, int mode, int64_t n
                    floor_log2(std::max<int64_t>(nq, 1)));
 }
 
-int request_mode(const pd_request *req, const uint32_t *species, const double *weights) {
-    if (!req->hyd_weights || !weights) return PD_MODE_CLASS;
-    // distinct (species, weight) keys, searched from the previous atom's
-    std::vector<std::pair<uint32_t, double>> keys;
-    size_t last = 0;
-    for (uint64_t i = 0; i < req->n_atoms; ++i) {
-        const std::pair<uint32_t, double> k(species[i], weights[i]);
-        if (!keys.empty() && keys[last] == k) continue;
-        last = std::find(keys.begin(), keys.end(), k) - keys.begin();
-        if (last == keys.size()) {
-            if (static_cast<int>(keys.size()) == PD_MAX_CLASSES) return PD_MODE_WEIGHTED;
-            keys.push_back(k);
-        }
-    }
-    return PD_MODE_CLASS;
-}
-
 bool valid_tuning(int precision, int mode, const Tuning &t) {
     if (!valid_q_block(precision, t.K) || t.TJ < 32 || t.TJ % 32 != 0) return false;
     if (precision == PD_FP64) return t.NP == 1;

@@ -22,7 +22,7 @@ import numpy as np
 from . import _lib
 from .dummies import DummySet
 from .errors import ValidationError
-from .formfactor import FormFactorMap, linear_q_values, read_formfactors
+from .formfactor import FormFactorMap, linear_q_values, read_formfactors, tabulate
 from .solvent import (SolventConfig, distinct_dummy_sets, excluded_table, sasa_weights,
                       water_table)
 from .structure import Structure, structure_from_xyz
@@ -246,7 +246,7 @@ def union_request(pos: np.ndarray, species: np.ndarray, ffA: np.ndarray,
         rows_a.append(np.zeros((1, nq)))
         rows_c.append(np.zeros((1, nq)))
         wts.append(hyd.weights)
-        water = np.array([hyd.form_factors[0].eval(float(q)) for q in q_values])
+        water = tabulate(hyd.form_factors[0], q_values)
         if hyd.lattice is not None and np.all(hyd.weights == hyd.weights[0]):
             lattices.append((nxt,) + tuple(hyd.lattice))
         nxt += 1

@@ -30,7 +30,7 @@ from typing import Optional, Sequence
 import numpy as np
 
 from .errors import InternalError, ValidationError
-from .formfactor import FormFactor, FormFactorMap, SingleGaussian
+from .formfactor import FormFactor, FormFactorMap, SingleGaussian, tabulate
 
 PEPSI_DENOMINATOR = 4.0 * math.pi   # src/solvent/fraser.rs:29
 WATER_KIND_NAME = "H2O"             # src/solvent/mod.rs:43
@@ -99,10 +99,10 @@ class DummySet:
         each dummy's form factor, which is the row's value at every q."""
         q_values = np.asarray(q_values, dtype=np.float64)
         if self.weights is not None:
-            base = np.array([self.form_factors[0].eval(float(q)) for q in q_values])
+            base = tabulate(self.form_factors[0], q_values)
             uniq, idx = np.unique(self.weights, return_inverse=True)
             return idx.astype(np.int64), uniq[:, None] * base[None, :]
-        tabs = np.array([[f.eval(float(q)) for q in q_values] for f in self.form_factors])
+        tabs = np.array([tabulate(f, q_values) for f in self.form_factors])
         used, idx = np.unique(self.kinds, return_inverse=True)
         return idx.astype(np.int64), tabs[used].reshape(len(used), len(q_values))
 

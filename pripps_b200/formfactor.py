@@ -79,6 +79,9 @@ class Constant(FormFactor):
     def _eval(self, q):
         return self.c
 
+    def _eval_many(self, q):
+        return np.full_like(q, self.c)
+
 
 @dataclass
 class Polynomial(FormFactor):
@@ -97,6 +100,9 @@ class Polynomial(FormFactor):
                 p *= q
             total += c * p
         return total
+
+    def _eval_many(self, q):
+        return self._eval(q) + np.zeros_like(q)
 
 
 @dataclass
@@ -145,6 +151,15 @@ class Gaussian(FormFactor):
             total += a * math.exp(-b * s2)
         return total + self.c
 
+    def _eval_many(self, q):
+        s2 = q * q / (16.0 * math.pi * math.pi)
+        total = np.zeros_like(q)
+        if self.ab:
+            e = _exp(np.array([[-b] for _, b in self.ab]) * s2)
+            for (a, _), row in zip(self.ab, e):
+                total += a * row
+        return total + self.c
+
 
 @dataclass
 class SingleGaussian(FormFactor):
@@ -156,6 +171,31 @@ class SingleGaussian(FormFactor):
 
     def _eval(self, q):
         return self.a * math.exp(-self.b * q * q)
+
+    def _eval_many(self, q):
+        return self.a * _exp(-self.b * q * q)
+
+
+def _exp(x: np.ndarray) -> np.ndarray:
+    """math.exp of every value: numpy's own exp may differ in the last bit, and
+    tables are compared bit by bit."""
+    return np.fromiter(map(math.exp, x.ravel().tolist()), np.float64, x.size).reshape(x.shape)
+
+
+def tabulate(ff, q_values) -> np.ndarray:
+    """``ff.eval`` at every q. The built-in closed forms are evaluated on the whole
+    array, in the same order of operations (a call per value was 0.7 of the 0.9
+    ms of a 1,500-atom model); a value out of range or one that overflows is left
+    to ``eval``, which raises."""
+    q = np.asarray(q_values, dtype=np.float64)
+    if type(ff) in (Constant, Polynomial, Gaussian, SingleGaussian):
+        lo, hi = ff.qrange()
+        if ((q >= lo) & (q <= hi)).all():
+            with np.errstate(all="ignore"):
+                out = ff._eval_many(q)
+            if np.isfinite(out).all():
+                return out
+    return np.array([ff.eval(float(v)) for v in q], dtype=np.float64)
 
 
 @dataclass
@@ -230,8 +270,7 @@ class FormFactorMap:
                                  grid[2], ctx)
         out = np.empty((len(ids), len(q_values)), dtype=np.float64)
         for r, idx in enumerate(ids):
-            ff = self.entries[idx].formfactor
-            out[r] = [ff.eval(q) for q in q_values]
+            out[r] = tabulate(self.entries[idx].formfactor, q_values)
         return out
 
 

@@ -32,7 +32,7 @@ import numpy as np
 
 from .dummies import DummySet, grid_excluded_dummies, grid_hydration_dummies
 from .errors import UsageError, ValidationError
-from .formfactor import FormFactorMap
+from .formfactor import FormFactorMap, SingleGaussian, tabulate
 
 WATER_KIND_NAME = "H2O"          # src/solvent/mod.rs:43
 WATER_VOLUME = 30.0              # Å³, src/solvent/mod.rs:46
@@ -121,8 +121,8 @@ def excluded_table(cfg: ExcludedVolume, formfactors: FormFactorMap, species: np.
                     f"atom kind {kind.name} has no `displaced_volume`; required by "
                     "ExcludedVolume::Fraser")
             vol = 1.0 * kind.displaced_volume
-            out[r] = [fraser_form_factor(float(q), vol, bulk_electron_density, denom)
-                      for q in q_values]
+            out[r] = tabulate(SingleGaussian(bulk_electron_density * vol,
+                                             vol ** (2.0 / 3.0) / denom), q_values)
         return out
     if cfg.kind == "per_kind":
         for r, sid in enumerate(species):
@@ -131,7 +131,7 @@ def excluded_table(cfg: ExcludedVolume, formfactors: FormFactorMap, species: np.
                 raise ValidationError(
                     f"atom kind {formfactors.kind(int(sid)).name} has no `excluded_solvent` "
                     "form factor; required by ExcludedVolume::PerKind")
-            out[r] = [ff.eval(float(q)) for q in q_values]
+            out[r] = tabulate(ff, q_values)
         return out
     raise UsageError(f"excluded volume '{cfg.kind}' places dummies away from the atoms; "
                      "the CUDA Debye backend serves colocated dummies only")
@@ -221,7 +221,7 @@ def water_table(formfactors: FormFactorMap, q_values: np.ndarray) -> np.ndarray:
     if ff is None:
         raise ValidationError(
             f"Hydration::Sasa requires an `{WATER_KIND_NAME}` entry in the form-factor YAML")
-    return np.array([ff.eval(float(q)) for q in q_values], dtype=np.float64)
+    return tabulate(ff, q_values)
 
 
 # --------------------------------------------------------------- top level

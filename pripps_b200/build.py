@@ -50,7 +50,7 @@ def _stale(target: Path, deps) -> bool:
 def build(force: bool = False, verbose: bool = False) -> Path:
     nvcc = nvcc_path()
     BUILD.mkdir(exist_ok=True)
-    headers = list(CSRC.glob("*.h")) + list(INCLUDE.glob("*.h"))
+    headers = list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
     objs = []
     ptxas_log = []
     for src in sources():

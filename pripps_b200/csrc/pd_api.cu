@@ -70,7 +70,7 @@ struct Layout {
     uint64_t upload_bytes;
     uint64_t hres;         // host-only: pinned landing area of the [6][nq] result
     uint64_t stage_bytes;  // pinned image size (upload + result area)
-    uint64_t centroid, cent_part, frames, atoms, slots, red, chunk_sums, terms, out;
+    uint64_t centroid, cent_part, frames, atoms, slots, dir_slots, red, chunk_sums, terms, out;
     uint64_t status;  // int32 device status of the pair kernel, right after out
     // counters and maxima that every execution starts from zero (one memset)
     uint64_t ctl, counter, cent_done, pack_done, rad2, red_done, dir_done, ctl_bytes;
@@ -119,9 +119,12 @@ Layout make_layout(const Plan &P, bool host_xyz) {
     L.frames = take(F * sizeof(PdFrameDev));
     L.atoms = take(static_cast<uint64_t>(P.n_pad) * P.n_frames *
                    (P.precision == PD_FP64 ? sizeof(double4) : sizeof(float4)));
-    // one region for the tiles' slots or the direction form's chunk sums
-    L.slots = take(std::max(static_cast<uint64_t>(P.slots_per_frame) * P.nv * P.tun.K,
-                            static_cast<uint64_t>(P.amp.slot_cap)) * F * 8);
+    // the tiles' slots and the direction form's chunk sums: one region for both where
+    // the only frame takes one of them, two where a batch may hold frames of both
+    const uint64_t b_tile = static_cast<uint64_t>(P.slots_per_frame) * P.nv * P.tun.K * F * 8,
+                   b_dir = static_cast<uint64_t>(P.amp.slot_cap) * F * 8;
+    L.slots = take(F > 1 ? b_tile : std::max(b_tile, b_dir));
+    L.dir_slots = F > 1 ? take(b_dir) : L.slots;
     const PdReduceShape &sh = P.red;
     const uint64_t red_rows = F * static_cast<uint64_t>(P.n_pairs);
     L.red = take(red_rows * P.nv * sh.width * 8);
@@ -475,6 +478,7 @@ void stage_structure(DevPlan &dp) {
     rd.gvalid = dp.dptr<int32_t>(L.gvalid);
     rd.qv = dp.dptr<double>(L.qv);
     rd.slots = dp.dptr<double>(L.slots);
+    rd.dir_slots = dp.dptr<double>(L.dir_slots);
     rd.frames = dp.dptr<PdFrameDev>(L.frames);
     rd.dirs = dp.dptr<double4>(L.dirs);
     rd.chunks = dp.dptr<PdChunk>(L.chunks);
@@ -508,17 +512,29 @@ int plan_host(pd_ctx *ctx, const pd_request *req, const uint32_t *species, const
     std::string msg;
     const Tuning tun = force ? *force : tuning_for_request(ctx, req, species, weights);
     dp.host_xyz = host_xyz;
-    for (bool tiles = !exact_radius;; tiles = true) {
-        int rc = pd::build_plan(req, species, weights, tun, dp.P, msg, false, radius_hint, !tiles);
+    auto plan = [&](Plan &P, Layout &L, bool allow_dir_only) {
+        const int rc =
+            pd::build_plan(req, species, weights, tun, P, msg, false, radius_hint, allow_dir_only);
         if (rc != PD_OK) {
             ctx->set_error(msg);
             return rc;
         }
-        dp.L = make_layout(dp.P, host_xyz);
-        // without tiles only where their plan would have fitted too
-        if (!dp.P.dir_only || static_cast<double>(dp.L.total) + dp.P.pair_bytes <=
-                                  static_cast<double>(ctx->budget))
-            break;
+        // known coordinates: every frame sums directions (the plan has no tiles) or none
+        if (exact_radius && !P.dir_only) pd::drop_directions(P);
+        L = make_layout(P, host_xyz);
+        return PD_OK;
+    };
+    if (int rc = plan(dp.P, dp.L, exact_radius)) return rc;
+    // without tiles only where the pair form would have fitted too
+    if (dp.P.dir_only &&
+        static_cast<double>(dp.L.total) + dp.P.pair_bytes > static_cast<double>(ctx->budget)) {
+        Plan P;
+        Layout L;
+        if (int rc = plan(P, L, false)) return rc;
+        if (L.total > ctx->budget || dp.L.total > ctx->budget) {
+            dp.P = std::move(P);
+            dp.L = L;
+        }
     }
     if (dp.L.total > ctx->budget) {  // the pair form alone may fit
         pd::drop_directions(dp.P);
@@ -599,8 +615,15 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st) {
         ctx->launches += 1;
     }
     if (P.amp.dir_cap > 0) {
+        if (static_cast<int>(P.chunks.size()) > P.n_cls) {
+            PD_CUDA(ctx, pd::launch_class_sums(dp.dptr<double>(L.dir_slots),
+                                               dp.dptr<PdFrameDev>(L.frames), P.amp, P.n_frames,
+                                               dp.dptr<int32_t>(L.cls_ptr),
+                                               dp.dptr<int32_t>(L.cls_chunk), st));
+            ctx->launches += 1;
+        }
         PD_CUDA(ctx, pd::launch_direction_sums(
-                         dp.dptr<double>(L.slots), dp.dptr<double4>(L.dirs),
+                         dp.dptr<double>(L.dir_slots), dp.dptr<double4>(L.dirs),
                          dp.dptr<PdFrameDev>(L.frames), P.amp, P.qmax, P.n_frames,
                          dp.dptr<PdClassDev>(L.cls), dp.dptr<PdPairDev>(L.pairs), P.n_pairs,
                          dp.dptr<int32_t>(L.cls_ptr), dp.dptr<int32_t>(L.cls_chunk), P.red.width,
@@ -693,7 +716,18 @@ int run_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st,
                                      static_cast<size_t>(P.slots_per_frame) * P.n_frames * P.nv *
                                          P.tun.K * 8,
                                      st));
-    if (!P.jobs.empty()) {
+    if (P.amp.dir_cap > 0) {
+        NvtxRange nvtx("pd direction kernel");
+        const int v = pd::directions_variant(P.precision, P.amp.amp_cap);
+        const int64_t grid =
+            std::min<int64_t>(std::max<int64_t>(P.dir_units, 1) * P.n_frames,
+                              static_cast<int64_t>(ctx->sm_count) * pd::directions_blocks_per_sm(v));
+        PD_CUDA(ctx, pd::launch_directions(v, dp.dptr<PdJob>(L.jobs), dp.dptr<int>(L.njobs),
+                                           dp.dptr<PdReqDev>(L.req), dp.dptr<int>(L.counter),
+                                           P.n_frames, static_cast<int>(grid), st));
+        ctx->launches += 1;
+    }
+    if (!P.jobs.empty() && !P.dir_only) {
         NvtxRange nvtx("pd pair kernel");
         PD_CUDA(ctx, pd::launch_pairs(P.precision, P.tun.K, P.tun.NP, P.mode, dp.dptr<PdJob>(L.jobs),
                                       dp.dptr<int>(L.njobs), dp.dptr<PdReqDev>(L.req),
@@ -807,6 +841,16 @@ double tile_cost(const Plan &P, const PdJob &jb) {
     return c;
 }
 
+// The kernel a request's jobs run in: a pair-kernel shape (precision, q block, pairs
+// per thread, mode), or the direction kernel for its number of moments.
+constexpr int LANE_DIRECTIONS = -1;
+std::tuple<int, int, int, int> lane_variant(const Plan &P) {
+    if (P.dir_only)
+        return std::make_tuple(P.precision, pd::directions_variant(P.precision, P.amp.amp_cap), 0,
+                               LANE_DIRECTIONS);
+    return std::make_tuple(P.precision, P.tun.K, P.tun.NP, P.mode);
+}
+
 int lane_graph(pd_ctx *ctx, Lane &ln, int precision, int K, int NP, int mode,
                cudaGraphExec_t *out) {
     auto key = std::make_tuple(precision, K, NP, mode);
@@ -815,12 +859,14 @@ int lane_graph(pd_ctx *ctx, Lane &ln, int precision, int K, int NP, int mode,
         *out = it->second;
         return PD_OK;
     }
+    const bool dirs = mode == LANE_DIRECTIONS;
     Plan dummy;
     dummy.precision = precision;
     dummy.tun.K = K;
     dummy.tun.NP = NP;
     dummy.mode = mode;
-    const int grid = persistent_grid(ctx, dummy, 1 << 30);
+    const int grid = dirs ? ctx->sm_count * std::max(1, pd::directions_blocks_per_sm(K))
+                          : persistent_grid(ctx, dummy, 1 << 30);
     cudaGraph_t g = nullptr;
     PD_CUDA(ctx, cudaStreamBeginCapture(ln.st, cudaStreamCaptureModeThreadLocal));
     cudaMemcpyAsync(ln.d_n, ln.h_n, sizeof(int), cudaMemcpyHostToDevice, ln.st);
@@ -829,8 +875,11 @@ int lane_graph(pd_ctx *ctx, Lane &ln, int precision, int K, int NP, int mode,
     cudaMemcpyAsync(ln.d_jobs, ln.h_jobs, STEP_MAX_JOBS * sizeof(PdJob), cudaMemcpyHostToDevice,
                     ln.st);
     cudaMemsetAsync(ln.d_counter, 0, sizeof(int), ln.st);
-    pd::launch_pairs(precision, K, NP, mode, ln.d_jobs, ln.d_n, ln.d_reqs, ln.d_counter, 0, grid,
-                     ln.st);
+    if (dirs)
+        pd::launch_directions(K, ln.d_jobs, ln.d_n, ln.d_reqs, ln.d_counter, 0, grid, ln.st);
+    else
+        pd::launch_pairs(precision, K, NP, mode, ln.d_jobs, ln.d_n, ln.d_reqs, ln.d_counter, 0,
+                         grid, ln.st);
     PD_CUDA(ctx, cudaStreamEndCapture(ln.st, &g));
     cudaGraphExec_t ge = nullptr;
     cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
@@ -1051,7 +1100,7 @@ void worker_main(pd_ctx *ctx) {
                     t->express_wait = false;
                     continue;
                 }
-                const auto key = std::make_tuple(P.precision, P.tun.K, P.tun.NP, P.mode);
+                const auto key = lane_variant(P);
                 int l = -1;
                 for (int c = 0; c < STEP_LANES && l < 0; ++c)
                     if (ex_used[c] && ex_key[c] == key && ex_nj[c] + P.jobs.size() <= STEP_MAX_JOBS &&
@@ -1134,7 +1183,7 @@ void worker_main(pd_ctx *ctx) {
                     const Plan &P = t->dp.P;
                     if (t->next_job >= P.jobs.size()) continue;
                     if (lane_of[ci] < 0) {
-                        const auto key = std::make_tuple(P.precision, P.tun.K, P.tun.NP, P.mode);
+                        const auto key = lane_variant(P);
                         int l = 0;
                         while (l < n_lanes && lane_key[l] != key) ++l;
                         if (l == n_lanes) {

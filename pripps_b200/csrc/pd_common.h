@@ -113,6 +113,8 @@ constexpr int PD_MAX_MOMENTS = 512;
 constexpr int PD_MAX_DIR_MOMENTS = 256;
 constexpr int PD_DIR_SMEM = 200 * 1024;
 constexpr int PD_DIR_DIRS = 8;  // directions of a work unit
+// Moments of its first block (FP32, FP64) and of each later one.
+constexpr int PD_DIR_MBLOCK = 128, PD_DIR_MBLOCK64 = 64;
 
 // When a frame may run in the moment form (block = 0: never).
 struct PdMomentRule {
@@ -122,6 +124,7 @@ struct PdMomentRule {
     int32_t max_moments;  // beyond this the grid points are cheaper (or do not fit)
     int32_t fp64;
     // direction form (dir_cap = 0: never)
+    int32_t dir_block;    // moments per unit
     int32_t dir_cap;      // directions the frame's table holds (a multiple of 32)
     int32_t grp_cap;      // direction groups of this rank that the sums hold
     int32_t amp_cap;      // moments
@@ -140,7 +143,7 @@ struct PdAmpShape {
     int32_t dir_cap, grp_cap, amp_cap, node_cap;
     int32_t node_tile;  // nodes per block of the sums' kernel (a multiple of 4)
     int32_t sum_smem;   // its shared memory in doubles
-    int32_t rank, world, block, pad_;
+    int32_t rank, world, block, dir_block;
     int64_t slot_cap;
 };
 
@@ -164,6 +167,7 @@ struct PdReqDev {
     const int32_t *gvalid;    // [n_pad / 32] valid atoms per granule
     const double *qv;         // [nq] grid (FP64 form reads it directly)
     double *slots;            // [n_slots][nv][K]
+    double *dir_slots;        // [n_frames][slot_cap] (direction form)
     const PdFrameDev *frames; // [n_frames]
     const double4 *dirs;      // [n_frames][dir_cap] direction/(2·r1) and quadrature weight
     const PdChunk *chunks;    // [n_chunk]

@@ -804,151 +804,6 @@ __device__ __forceinline__ MomJob moment_job(int j0, int j1, int qb, int n_mblk,
     return m;
 }
 
-// Atoms a thread sums in FP32 for its direction before the CTA's sums go, in FP64,
-// into the unit's slot.
-#ifndef PD_DIR_RUN
-#define PD_DIR_RUN 512
-#endif
-
-// Atoms staged at once: two buffers of 16 KB, filled by asynchronous copies (a
-// thread's pass is shorter than a read from L2, and the pair kernels' shared
-// memory leaves little L1).
-constexpr int PD_DIR_BLOCK = 1024;
-static_assert(PD_DIR_RUN * PD_DIR_LANES % PD_DIR_BLOCK == 0, "a run is whole blocks");
-static_assert(2 * PD_DIR_BLOCK * sizeof(float4) + PD_WARPS * 128 * PD_DIR_DIRS * sizeof(float) <=
-                  2 * PD_JSTAGE_ATOMS * sizeof(float4),
-              "blocks and sums share the staging memory");
-
-__device__ __forceinline__ void direction_stage(float4 *dst, const float4 *__restrict__ at, int j0,
-                                                int j1) {
-    for (int k = threadIdx.x; k < j1 - j0; k += PD_THREADS)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst + k)),
-                     "l"(at + j0 + k)
-                     : "memory");
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
-// The sums of a warp's four atom lanes (lane / 8), reduce-scattered: afterwards
-// atom lane a holds acc[t], a·NT/4 <= t < (a + 1)·NT/4, in acc[0 .. NT/4).
-template <int NT>
-__device__ __forceinline__ void direction_scatter(float2 (&v)[NT], int lane) {
-#pragma unroll
-    for (int lev = 0; lev < 2; ++lev) {
-        const int o = 16 >> lev, h = (NT >> lev) / 2;
-        const bool up = (lane & o) != 0;
-#pragma unroll
-        for (int k = 0; k < h; ++k) {
-            const float2 lo = v[k], hi = v[k + h];
-            const float2 keep = up ? hi : lo;
-            const float2 send = up ? lo : hi;
-            v[k] = __fadd2_rn(keep, make_float2(__shfl_xor_sync(0xffffffffu, send.x, o),
-                                                __shfl_xor_sync(0xffffffffu, send.y, o)));
-        }
-    }
-}
-
-// Direction form: one work unit. A lane is one of 8 directions for every 16th atom
-// of the chunk, so 128 threads share 8·n_amp sums: few enough units fill the GPU
-// with short loops on small structures, and the slots stay small. A run's FP32 sums
-// of the 16 atom lanes meet by shuffles and in shared memory and are added to
-// the slot in warp order, in FP64.
-template <int KM, bool W, bool ILP>
-__device__ __forceinline__ void direction_unit_run(const float4 *__restrict__ at, const PdChunk &ck,
-                                                   float3 dv, const DirUnit &un, int n_amp,
-                                                   float4 *__restrict__ buf,
-                                                   double *__restrict__ out0,
-                                                   double *__restrict__ out1) {
-    constexpr int DBL = KM == 128 ? 4 : (KM == 64 ? 3 : 2);
-    constexpr int NT = KM / 2, RUN = PD_DIR_RUN * PD_DIR_LANES;
-    float *sums = reinterpret_cast<float *>(buf + 2 * PD_DIR_BLOCK);  // [v][warp][e][8]
-    const int nj = min(KM, n_amp - un.mb * KM) >> 3;
-    int b = 0;
-    direction_stage(buf, at, ck.j0, min(ck.j1, ck.j0 + PD_DIR_BLOCK));
-    for (int r0 = ck.j0; r0 < ck.j1; r0 += RUN) {
-        float2 acc[NT], accw[W ? NT : 1];
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-            acc[t] = make_float2(0.0f, 0.0f);
-            if constexpr (W) accw[t] = make_float2(0.0f, 0.0f);
-        }
-        for (int j0 = r0; j0 < min(ck.j1, r0 + RUN); j0 += PD_DIR_BLOCK, b ^= 1) {
-            const int j1 = min(ck.j1, j0 + PD_DIR_BLOCK);
-            direction_stage(buf + (b ^ 1) * PD_DIR_BLOCK, at, j1, min(ck.j1, j1 + PD_DIR_BLOCK));
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-            __syncthreads();
-            direction_range<KM, W, ILP>(buf + b * PD_DIR_BLOCK, dv,
-                                        static_cast<int>(threadIdx.x) / PD_DIR_DIRS, j1 - j0, nj,
-                                        un.mb, DBL, acc, accw);
-            __syncthreads();  // the block is read before its buffer is refilled
-        }
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const int dir = lane % PD_DIR_DIRS, a = lane / PD_DIR_DIRS;
-#pragma unroll
-        for (int v = 0; v < (W ? 2 : 1); ++v) {
-            float2 *x = acc;
-            if constexpr (W)
-                if (v) x = accw;
-            float *o = sums + (v * PD_WARPS + warp) * KM * PD_DIR_DIRS + dir;
-            if (v == 0) direction_scatter<NT>(acc, lane);
-            if constexpr (W)
-                if (v == 1) direction_scatter<NT>(accw, lane);
-#pragma unroll
-            for (int t = 0; t < NT / 4; ++t) {
-                // row e ^ a: the four atom lanes write different banks
-                const int e = 2 * (a * (NT / 4) + t);
-                o[(e ^ a) * PD_DIR_DIRS] = x[t].x;
-                o[((e + 1) ^ a) * PD_DIR_DIRS] = x[t].y;
-            }
-        }
-        __syncthreads();
-        for (int k = threadIdx.x; k < nj * 4 * PD_DIR_DIRS; k += PD_THREADS) {
-            const int d = k % PD_DIR_DIRS, i = k / PD_DIR_DIRS, al = i / (NT / 4);  // i = 4·jj + t
-#pragma unroll
-            for (int v = 0; v < (W ? 2 : 1); ++v) {
-                double x = 0.0, y = 0.0;
-#pragma unroll
-                for (int w = 0; w < PD_WARPS; ++w) {
-                    const float *c = sums + (v * PD_WARPS + w) * KM * PD_DIR_DIRS + d;
-                    x += static_cast<double>(c[((2 * i) ^ al) * PD_DIR_DIRS]);
-                    y += static_cast<double>(c[((2 * i + 1) ^ al) * PD_DIR_DIRS]);
-                }
-                direction_put(v ? out1 : out0, un.mb * KM, i >> 2, i & 3, d, x, y, r0 == ck.j0);
-            }
-        }
-        __syncthreads();  // sums are rewritten by the next run
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");  // (the last, empty block)
-}
-
-// Units of a frame.
-__device__ __forceinline__ int64_t direction_unit_count(const PdReqDev &rq, const PdFrameDev &fr) {
-    return static_cast<int64_t>(rq.amp.n_chunk) * fr.n_ablk * fr.n_grp * (32 / PD_DIR_DIRS);
-}
-
-// Work unit u of a frame (see direction_unit).
-template <int K, int MODE>
-__device__ __noinline__ void direction_unit_f32(int frame, int64_t u, const PdReqDev &rq,
-                                                const PdFrameDev &fr, float4 *__restrict__ buf) {
-    constexpr int KM = pd_moment_block(K);
-    constexpr bool W = MODE == PD_MODE_WEIGHTED;
-    const int lane = threadIdx.x & 31;
-    const float4 *__restrict__ at = rq.atoms32 + static_cast<size_t>(frame) * rq.n_pad;
-    const DirUnit un = direction_unit(u, fr);
-    const PdChunk ck = rq.chunks[un.chunk];
-    const double4 D = rq.dirs[static_cast<int64_t>(frame) * rq.amp.dir_cap +
-                              (static_cast<int64_t>(un.grp) * rq.amp.world + rq.amp.rank) * 32 +
-                              un.sub * PD_DIR_DIRS + lane % PD_DIR_DIRS];
-    const float3 dv = make_float3(static_cast<float>(D.x), static_cast<float>(D.y),
-                                  static_cast<float>(D.z));
-    double *slots = rq.slots + static_cast<int64_t>(frame) * rq.amp.slot_cap + un.sub * PD_DIR_DIRS;
-    double *out0 = slots + direction_slot(un.chunk, 0, un.grp, rq.amp.nv2, fr);
-    double *out1 = W ? slots + direction_slot(un.chunk, 1, un.grp, rq.amp.nv2, fr) : out0;
-    if (KM > 64 && fr.n_amp <= 64)  // half the accumulators: two atoms at a time
-        direction_unit_run<64, W, true>(at, ck, dv, un, fr.n_amp, buf, out0, out1);
-    else
-        direction_unit_run<KM, W, KM <= 64 && !W>(at, ck, dv, un, fr.n_amp, buf, out0, out1);
-}
-
 // Weighted-mode flush of one accumulator array: the warp sums of acc and of
 // w_i·acc, added to part[k] and part[stride + k].
 template <int K>
@@ -989,6 +844,14 @@ __device__ __forceinline__ void merge_tile_slots(const double *__restrict__ part
     }
 }
 
+// Whether any frame of a request sums pairs: without one the pair kernel of a
+// plan is left at once, its job list unread (uniform; the frames are read side by side).
+__device__ __forceinline__ bool plan_sums_pairs(const PdReqDev &rq, int n_frames) {
+    int any = 0;
+    for (int f = threadIdx.x; f < n_frames; f += PD_THREADS) any |= rq.frames[f].n_grp == 0;
+    return __syncthreads_or(any) != 0;
+}
+
 template <int K, int MODE, int NP>
 __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
     pd_pairs_fp32(const PdJob *__restrict__ jobs, const int *__restrict__ n_jobs_ptr,
@@ -1027,37 +890,7 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
     __syncthreads();
     uint32_t phase = 0;  // bit b: parity of buffer b's next completion
     double *part = s_part + warp * NV * K;
-    // The whole plan of one request: the CTAs take its direction frames' units by
-    // number, without the job list (an idle job costs a chain of four dependent
-    // loads), and the list runs only if some frame sums pairs. The next number
-    // is fetched while a unit is computed.
-    if (plan_frames > 0) {
-        const PdReqDev rq = reqs[0];
-        bool pairs = false;
-        int64_t base = 0;  // units of the frames before f
-        if (threadIdx.x == 0) s_job = atomicAdd(&counter[1], 1);
-        __syncthreads();
-        int64_t cur = s_job;
-        for (int f = 0; f < plan_frames; ++f) {
-            const PdFrameDev fr = rq.frames[f];
-            if (fr.n_grp == 0) {
-                pairs = true;
-                continue;
-            }
-            const int64_t n_units = direction_unit_count(rq, fr);
-            while (cur < base + n_units) {
-                __syncthreads();  // s_job is read
-                if (threadIdx.x == 0) s_job = atomicAdd(&counter[1], 1);
-                const int64_t u = cur - base;
-                direction_unit_f32<K, MODE>(f, u, rq, fr, pd_dyn_atoms);
-                __syncthreads();
-                cur = s_job;
-            }
-            base += n_units;
-        }
-        if (!pairs) return;
-        __syncthreads();
-    }
+    if (plan_frames > 0 && !plan_sums_pairs(reqs[0], plan_frames)) return;
     for (;;) {
         if (threadIdx.x == 0) s_job = atomicAdd(counter, 1);
         __syncthreads();
@@ -1067,11 +900,7 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
         const PdReqDev rq = reqs[jb.req];
         const int kq0 = jb.qb * K;
         const PdFrameDev fr = rq.frames[jb.frame];
-        if (fr.n_grp > 0) {
-            // (the whole plan's units are done already)
-            const int64_t n_units = plan_frames ? 0 : direction_unit_count(rq, fr);
-            for (int64_t u = jb.ord; u < n_units; u += jb.n_ord)
-                direction_unit_f32<K, MODE>(jb.frame, u, rq, fr, pd_dyn_atoms);
+        if (fr.n_grp > 0) {  // direction form (pd_directions_*)
             __syncthreads();  // every thread has read s_job
             continue;
         }
@@ -1323,63 +1152,6 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
 }
 
 // ---------------------------------------------------------------- K2 (FP64)
-// direction_unit_f32 in FP64 (one run per unit; the atom lanes of a warp meet by
-// shuffles, the warps in shared memory, part[v][warp][e][8]).
-template <int K, int MODE>
-__device__ __noinline__ void direction_unit_f64(int frame, int64_t u, const PdReqDev &rq,
-                                                const PdFrameDev &fr, double *__restrict__ part) {
-    constexpr int DBL = K == 64 ? 3 : (K == 32 ? 2 : 1);
-    constexpr bool W = MODE == PD_MODE_WEIGHTED;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const double4 *__restrict__ at = rq.atoms64 + static_cast<size_t>(frame) * rq.n_pad;
-    const DirUnit un = direction_unit(u, fr);
-    const PdChunk ck = rq.chunks[un.chunk];
-    const double4 D = rq.dirs[static_cast<int64_t>(frame) * rq.amp.dir_cap +
-                              (static_cast<int64_t>(un.grp) * rq.amp.world + rq.amp.rank) * 32 +
-                              un.sub * PD_DIR_DIRS + lane % PD_DIR_DIRS];
-    const int nj = min(K, fr.n_amp - un.mb * K) >> 3;
-    double acc[K], accw[W ? K : 1];
-#pragma unroll
-    for (int e = 0; e < K; ++e) {
-        acc[e] = 0.0;
-        if constexpr (W) accw[e] = 0.0;
-    }
-    direction_range_f64<K, W>(at, D, ck.j0 + static_cast<int>(threadIdx.x) / PD_DIR_DIRS, ck.j1, nj,
-                              un.mb, DBL, acc, accw);
-#pragma unroll
-    for (int e = 0; e < K; ++e) {
-        if (e >= 8 * nj) break;
-        double a = acc[e];
-        a += __shfl_xor_sync(0xffffffffu, a, 8);
-        a += __shfl_xor_sync(0xffffffffu, a, 16);
-        if (lane < PD_DIR_DIRS) part[(warp * K + e) * PD_DIR_DIRS + lane] = a;
-        if constexpr (W) {
-            double b = accw[e];
-            b += __shfl_xor_sync(0xffffffffu, b, 8);
-            b += __shfl_xor_sync(0xffffffffu, b, 16);
-            if (lane < PD_DIR_DIRS) part[((PD_WARPS + warp) * K + e) * PD_DIR_DIRS + lane] = b;
-        }
-    }
-    __syncthreads();
-    double *slots = rq.slots + static_cast<int64_t>(frame) * rq.amp.slot_cap + un.sub * PD_DIR_DIRS;
-    for (int k = threadIdx.x; k < nj * 4 * PD_DIR_DIRS; k += PD_THREADS) {
-        const int dir = k % PD_DIR_DIRS, i = k / PD_DIR_DIRS;
-#pragma unroll
-        for (int v = 0; v < (W ? 2 : 1); ++v) {
-            double x = 0.0, y = 0.0;
-#pragma unroll
-            for (int w = 0; w < PD_WARPS; ++w) {
-                const double *c = part + ((v * PD_WARPS + w) * K + 2 * i) * PD_DIR_DIRS + dir;
-                x += c[0];
-                y += c[PD_DIR_DIRS];
-            }
-            direction_put(slots + direction_slot(un.chunk, v, un.grp, rq.amp.nv2, fr), un.mb * K,
-                          i >> 2, i & 3, dir, x, y, true);
-        }
-    }
-    __syncthreads();  // part is rewritten by the next unit
-}
-
 template <int K, int MODE>
 __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(const PdJob *__restrict__ jobs,
                                                             const int *__restrict__ n_jobs_ptr,
@@ -1391,42 +1163,11 @@ __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(con
     __shared__ int s_job;
     __shared__ double s_q[K];
     __shared__ double s_part[PD_WARPS * NV * K];
-    __shared__ double s_dir[NACC * PD_WARPS * K * PD_DIR_DIRS];  // direction form
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int n_jobs = *n_jobs_ptr;
     double *part = s_part + warp * NV * K;
-    // The whole plan of one request: the CTAs take its direction frames' units by
-    // number, without the job list (an idle job costs a chain of four dependent
-    // loads), and the list runs only if some frame sums pairs. The next number
-    // is fetched while a unit is computed.
-    if (plan_frames > 0) {
-        const PdReqDev rq = reqs[0];
-        bool pairs = false;
-        int64_t base = 0;  // units of the frames before f
-        if (threadIdx.x == 0) s_job = atomicAdd(&counter[1], 1);
-        __syncthreads();
-        int64_t cur = s_job;
-        for (int f = 0; f < plan_frames; ++f) {
-            const PdFrameDev fr = rq.frames[f];
-            if (fr.n_grp == 0) {
-                pairs = true;
-                continue;
-            }
-            const int64_t n_units = direction_unit_count(rq, fr);
-            while (cur < base + n_units) {
-                __syncthreads();  // s_job is read
-                if (threadIdx.x == 0) s_job = atomicAdd(&counter[1], 1);
-                const int64_t u = cur - base;
-                direction_unit_f64<K, MODE>(f, u, rq, fr, s_dir);
-                __syncthreads();
-                cur = s_job;
-            }
-            base += n_units;
-        }
-        if (!pairs) return;
-        __syncthreads();
-    }
+    if (plan_frames > 0 && !plan_sums_pairs(reqs[0], plan_frames)) return;
     for (;;) {
         if (threadIdx.x == 0) s_job = atomicAdd(counter, 1);
         __syncthreads();
@@ -1435,10 +1176,7 @@ __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(con
         const PdJob jb = jobs[jid];
         const PdReqDev rq = reqs[jb.req];
         const PdFrameDev fr = rq.frames[jb.frame];
-        if (fr.n_grp > 0) {
-            const int64_t n_units = plan_frames ? 0 : direction_unit_count(rq, fr);
-            for (int64_t u = jb.ord; u < n_units; u += jb.n_ord)
-                direction_unit_f64<K, MODE>(jb.frame, u, rq, fr, s_dir);
+        if (fr.n_grp > 0) {  // direction form (pd_directions_*)
             __syncthreads();  // every thread has read s_job
             continue;
         }
@@ -1578,6 +1316,12 @@ __global__ void __launch_bounds__(PD_CENT_THREADS)
 // 300 atoms, directions above.
 constexpr int PD_PACK_THREADS = 256;
 
+// Nodes and weights of the 2h-point Gauss–Legendre rules, upper half
+// (x > 0, ascending), h = 1 … PD_GL_MAX: rule h at h·(h − 1)/2. The weights of
+// a half add up to 1. Filled once per device (prepare_direction_rules).
+constexpr int PD_GL_MAX = 128;
+__device__ double2 pd_gl_rules[PD_GL_MAX * (PD_GL_MAX + 1) / 2];
+
 __device__ __forceinline__ int ring_points(double z_sin, bool fp64) {
     return max(4, static_cast<int>(direction_order(z_sin, fp64)) + 1);
 }
@@ -1681,10 +1425,11 @@ __global__ void __launch_bounds__(PD_PACK_THREADS)
     const int mine = rule.rank < groups ? (groups - rule.rank + rule.world - 1) / rule.world : 0;
     const double mo = direction_order(fr.r1 * rule.qmax, fp64);
     const int m8 = mo < 1e6 ? ((static_cast<int>(mo) + 8) & ~7) : 1000000;
-    const int ablk = (m8 + rule.block - 1) / max(rule.block, 1);
+    const int ablk = (m8 + rule.dir_block - 1) / rule.dir_block;
     const int nodes = moments_needed(2.0 * fr.r1 * rule.qmax, true);
     const double dir_cost =
-        static_cast<double>(S) * (static_cast<double>(rule.n_atoms) * (44.0 * ablk + 1.25 * m8) +
+        static_cast<double>(S) * (static_cast<double>(rule.n_atoms) * rule.nv2 *
+                                      (44.0 * ablk - 30.0 + 1.25 * m8) +
                                   4.0 * rule.n_cls * m8 * nodes);
     const bool use = S > 0 && rule.block > 0 && groups * 32 <= rule.dir_cap && mine > 0 &&
                      (groups + rule.world - 1) / rule.world <= rule.grp_cap &&
@@ -1898,6 +1643,22 @@ __device__ double direction_coefficients(double y, int n_mom, double *__restrict
     return 1.0 / fma(2.0, even, cur);
 }
 
+// The coefficients of the first block's product sums from those of its moments (n <
+// lim, a multiple of 8): m_8j+t = 2·P_{j,t} − m_8j−t, so a coefficient passes on
+// with the other sign from n = 8j + t to 8j − t, a chain of 8(j − 1) + (8 − t) next:
+// seven chains, one for a thread (t: the chain's element of the last eight).
+__device__ void direction_fold(double *__restrict__ g, int lim, int t, int stride) {
+    double prev = 0.0;
+#pragma unroll 4
+    for (int j = lim / 8 - 1; j >= 0; --j) {
+        double &c = g[(8 * j + t) * stride];
+        const double v = c - prev;
+        c = j > 0 ? 2.0 * v : v;
+        prev = v;
+        t = 8 - t;
+    }
+}
+
 // Node k of n on the q range [0, qmax]: q = qmax·cos((2k+1)π/4n).
 __device__ __forceinline__ double direction_node(int k, int n, double qmax) {
     return qmax * cospi((2 * k + 1) / (4.0 * n));
@@ -1933,6 +1694,9 @@ __global__ void __launch_bounds__(PD_DSUM_THREADS)
         if (lane < nn)
             s_scale[lane] = direction_coefficients(
                 direction_node(tile * NT + lane, fr.n_node, qmax) * fr.r1, M, s_g + lane, NT);
+        __syncwarp();
+        for (int k = lane; k < 7 * nn; k += 32)
+            direction_fold(s_g + k % nn, min(M, sh.dir_block), 1 + k / nn, NT);
         s_w[lane] = dirs[static_cast<int64_t>(f) * sh.dir_cap +
                          (static_cast<int64_t>(grp) * sh.world + sh.rank) * 32 + lane].w;
     }
@@ -1948,14 +1712,11 @@ __global__ void __launch_bounds__(PD_DSUM_THREADS)
             const int c = (c0 + cb) / NV2, v = (c0 + cb) % NV2;
             const int rows = min(16, M - r0);  // 16 or 8
             double m[16];
+            // the class's sums, left at its first chunk
+            const double *src =
+                sl + direction_slot(cls_chunk[cls_ptr[c]], v, grp, NV2, fr) + r0 * 32 + lane;
 #pragma unroll
-            for (int u = 0; u < 16; ++u) m[u] = 0.0;
-            for (int e = cls_ptr[c]; e < cls_ptr[c + 1]; ++e) {
-                const double *src =
-                    sl + direction_slot(cls_chunk[e], v, grp, NV2, fr) + r0 * 32 + lane;
-#pragma unroll
-                for (int u = 0; u < 16; ++u) m[u] += u < rows ? __ldg(src + u * 32) : 0.0;
-            }
+            for (int u = 0; u < 16; ++u) m[u] = u < rows ? __ldg(src + u * 32) : 0.0;
             if (r0 == 0) m[0] = v ? cls[c].w1 : cls[c].n;
             double *dst = s_m + (cb * M + r0) * 32 + lane;
 #pragma unroll
@@ -3207,6 +2968,8 @@ cudaError_t prepare_pair_kernels() {
                              {64, 1, 4}};
     for (const auto &sh : shapes)
         if (pairs_blocks_per_sm(0, sh[0], sh[2], sh[1]) <= 0) return cudaErrorInvalidValue;
+    for (const int v : {0, 64, 128})
+        if (directions_blocks_per_sm(v) <= 0) return cudaErrorInvalidValue;
     return cudaSuccess;
 }
 

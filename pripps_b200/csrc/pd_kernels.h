@@ -24,6 +24,14 @@ cudaError_t prepare_pair_kernels();
 cudaError_t launch_pairs(int precision, int K, int NP, int mode, const PdJob *jobs,
                          const int *n_jobs, const PdReqDev *reqs, int *counter, int plan_frames,
                          int grid, cudaStream_t st);
+// The direction form's first stage, for the frames that take it; the other arguments
+// are those of launch_pairs (plan_frames > 0 uses the second counter). A variant holds
+// up to its number of moments (directions_variant of the most a frame may have).
+int directions_variant(int precision, int32_t n_amp);
+int directions_blocks_per_sm(int variant);
+cudaError_t launch_directions(int variant, const PdJob *jobs, const int *n_jobs,
+                              const PdReqDev *reqs, int *counter, int plan_frames, int grid,
+                              cudaStream_t st);
 // Blocks per frame of the centroid kernel (3 partial sums each).
 int32_t centroid_blocks(int64_t n_atoms);
 // `done` (one counter per frame) must be zero; `status`, if given, is cleared.
@@ -39,6 +47,10 @@ cudaError_t launch_pack(const double *xyz, const double *weights, const int32_t 
 // The quadrature rules of the direction form on the current device (before any
 // launch_pack there, and before a stream capture).
 cudaError_t prepare_direction_rules();
+// Adds the chunk sums of each class up (needed where a class has more than one).
+cudaError_t launch_class_sums(double *slots, const PdFrameDev *frames, const PdAmpShape &sh,
+                              int n_frames, const int32_t *cls_ptr, const int32_t *cls_chunk,
+                              cudaStream_t st);
 // Direction form: class-pair sums at the nodes, from the chunks' moments, into
 // red (does nothing for frames in the other forms). part holds grp_cap·pairs·nv·
 // node_cap doubles per frame, done one zeroed counter per node tile and frame.

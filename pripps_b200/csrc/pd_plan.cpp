@@ -313,6 +313,7 @@ static void species_class_keys(int64_t n, const uint32_t *species, int32_t n_spe
 }
 
 static bool direction_only(Plan &P);
+static void set_chunks(Plan &P);
 
 int build_plan(const pd_request *req, const uint32_t *species, const double *w,
                const Tuning &tun, Plan &P, std::string &msg, bool count_pairs,
@@ -482,31 +483,7 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
         P.lat_bins = off;
     }
 
-    // ---- atom chunks of the direction form: at most 1/6 of the atoms each (a few
-    // direction groups then fill the GPU already; shorter chunks mean more sums
-    // to hold and to add up), longest first
-    {
-        const int64_t len = std::clamp<int64_t>(n / 6, 256, 16384);
-        for (int k = 0; k < c; ++k) {
-            const int64_t nk = count[k];
-            const int64_t parts = (nk + len - 1) / len;
-            for (int64_t t = 0; t < parts; ++t)
-                P.chunks.push_back(PdChunk{k, P.cls_start[k] + static_cast<int32_t>(nk * t / parts),
-                                           P.cls_start[k] +
-                                               static_cast<int32_t>(nk * (t + 1) / parts),
-                                           0});
-        }
-        std::stable_sort(P.chunks.begin(), P.chunks.end(), [](const PdChunk &x, const PdChunk &y) {
-            return x.j1 - x.j0 > y.j1 - y.j0;
-        });
-        P.cls_ptr.assign(c + 1, 0);
-        for (int k = 0; k < c; ++k) {
-            for (size_t t = 0; t < P.chunks.size(); ++t)
-                if (P.chunks[t].cls == k) P.cls_chunk.push_back(static_cast<int32_t>(t));
-            P.cls_ptr[k + 1] = static_cast<int32_t>(P.cls_chunk.size());
-        }
-    }
-
+    set_chunks(P);
     const int K = P.tun.K, TJ = P.tun.TJ;
     P.nqb = (P.nq + K - 1) / K;
     if (allow_dir_only && radius_hint >= 0.0 && direction_only(P)) return PD_OK;
@@ -711,6 +688,40 @@ static double series_order(double z, bool fp64) {
     return fp64 ? z + 13.0 * std::cbrt(0.5 * z) + 3.0 : z + 8.0 * std::cbrt(0.5 * z) + 2.0;
 }
 
+// Atom chunks of the direction form, longest first. A longer chunk means fewer sums
+// to hold and to add up, a shorter one more units to share: 2.5 units per block
+// that the GPU holds (four per SM), at least 1,024 atoms and at most 16,384, with the
+// directions of a globule of the request's atom count (its coordinates would be
+// better, but then a solve's rounding would depend on when they are known). Measured,
+// whole execution in µs with chunks of 512 / 1,024 / 2,048 / 4,096 / 16,384 atoms: 3,000
+// atoms 77 / 75 / 83 / 83 / 83, 10,000 atoms 101 / 102 / 101 / 112 / 144, 20,000 atoms 503 /
+// 457 / 443 / 441 / 468, 100,000 atoms 5,165 / 4,599 / 4,346 / 4,229 / 4,155.
+static void set_chunks(Plan &P) {
+    const double n = static_cast<double>(P.n_atoms);
+    const double z = 2.0 * P.qmax * std::cbrt(n * 17.0 * 3.0 / (4.0 * M_PI));
+    const double top = series_order(z, P.precision == PD_FP64);
+    const double want = 0.4 * n * P.n_frames * (0.2 * top * top / PD_DIR_DIRS) / 592.0;
+    const int64_t len = want < 1024.0 ? 1024 : (want < 16384.0 ? static_cast<int64_t>(want) : 16384);
+    P.chunks.clear();
+    P.cls_chunk.clear();
+    for (int k = 0; k < P.n_cls; ++k) {
+        const int64_t nk = static_cast<int64_t>(P.cls[k].n), parts = (nk + len - 1) / len;
+        for (int64_t t = 0; t < parts; ++t)
+            P.chunks.push_back(PdChunk{k, P.cls_start[k] + static_cast<int32_t>(nk * t / parts),
+                                       P.cls_start[k] + static_cast<int32_t>(nk * (t + 1) / parts),
+                                       0});
+    }
+    std::stable_sort(P.chunks.begin(), P.chunks.end(), [](const PdChunk &x, const PdChunk &y) {
+        return x.j1 - x.j0 > y.j1 - y.j0;
+    });
+    P.cls_ptr.assign(P.n_cls + 1, 0);
+    for (int k = 0; k < P.n_cls; ++k) {
+        for (size_t t = 0; t < P.chunks.size(); ++t)
+            if (P.chunks[t].cls == k) P.cls_chunk.push_back(static_cast<int32_t>(t));
+        P.cls_ptr[k + 1] = static_cast<int32_t>(P.cls_chunk.size());
+    }
+}
+
 // A plan without tiles, where the frames' exact radius (radius_hint, the largest
 // one) is known and the direction form is the cheaper one by pd_pack's own
 // comparison: planning and upload of the tiles, slots and lists were 4.7 of the
@@ -756,7 +767,6 @@ static bool direction_only(Plan &P) {
     P.jobs_per_frame = per;
     P.job_cost = P.dir_cost / (3.0 * static_cast<double>(per));
     if (P.precision == PD_FP64) P.job_cost *= 2.0;
-    if (P.mode == PD_MODE_WEIGHTED) P.job_cost *= 1.5;
     P.jobs.resize(static_cast<size_t>(per) * P.n_frames);
     for (int64_t o = 0; o < per; ++o)
         for (int f = 0; f < P.n_frames; ++f) {
@@ -775,6 +785,7 @@ static void set_directions(Plan &P) {
     P.amp = PdAmpShape{};
     P.amp.nq = P.nq;
     P.amp.block = P.mom.block;
+    P.amp.dir_block = P.precision == PD_FP64 ? PD_DIR_MBLOCK64 : PD_DIR_MBLOCK;
     P.amp.rank = static_cast<int32_t>(P.rank);
     P.amp.world = static_cast<int32_t>(P.world);
     P.amp.n_cls = P.n_cls;
@@ -824,12 +835,12 @@ static void set_directions(Plan &P) {
     P.amp.node_cap = static_cast<int32_t>(nodes);
     P.amp.node_tile = static_cast<int32_t>(tile);
     P.amp.slot_cap = slots;
-    const double ablk = static_cast<double>((m8 + P.mom.block - 1) / P.mom.block);
+    const double ablk = static_cast<double>((m8 + P.amp.dir_block - 1) / P.amp.dir_block);
     P.dir_cost = static_cast<double>(S) *
-                 (static_cast<double>(P.n_atoms) * (44.0 * ablk + 1.25 * m8) +
+                 (static_cast<double>(P.n_atoms) * P.amp.nv2 * (44.0 * ablk - 30.0 + 1.25 * m8) +
                   4.0 * P.n_cls * static_cast<double>(m8) * static_cast<double>(nodes));
-    P.dir_units = static_cast<int64_t>(P.amp.n_chunk) * static_cast<int64_t>(ablk) * mine *
-                  (32 / PD_DIR_DIRS);
+    P.dir_units = static_cast<int64_t>(P.amp.n_chunk) * P.amp.nv2 *
+                  static_cast<int64_t>(ablk) * mine * (32 / PD_DIR_DIRS);
 }
 
 void drop_directions(Plan &P) {
@@ -856,6 +867,7 @@ void set_reduction(Plan &P) {
                            per_q * P.nq + 8 * P.nqb}) & ~int64_t{7});
     if (m.max_moments < 8) m.block = 0;
     set_directions(P);
+    m.dir_block = P.amp.dir_block;
     m.dir_cap = P.amp.dir_cap;
     m.grp_cap = P.amp.grp_cap;
     m.amp_cap = P.amp.amp_cap;

@@ -18,8 +18,8 @@ import pytest
 
 from conftest import term_errors
 from oracle import oracle as O
-from pripps_b200 import _lib
-from pripps_b200.debye import DebyeRequest, solve
+from pripps_b200 import _lib, workloads
+from pripps_b200.debye import DebyeRequest, TrajectoryStream, solve
 
 pytestmark = pytest.mark.gpu
 TOL = {"fp64": 1e-10, "fp32": 1e-5}
@@ -102,7 +102,7 @@ def test_moment_extreme_distances(gpu_ctx, precision, name):
 
 
 # The direction form (amplitudes over a quadrature of the sphere) runs where
-# there are more atoms than directions: sizes around the chunk length (256), a
+# there are more atoms than directions: sizes around the chunk length (1,024), a
 # chunk of one atom, several chunks of a class; z = 2·radius·qmax of a few rings,
 # of 33/64/65 directions' worth of moments, and past one moment block; 49 grid
 # points that hit an interpolation node (qmin = qmax·cos(π/4M) is not on the grid:
@@ -120,6 +120,26 @@ def test_direction_form(gpu_ctx, precision, mode, n, qmax, nq, qmin):
     req = _request(xyz, nq, qmin, qmax, precision, mode, n)
     req.species[:] = rng.choice(3, size=n, p=[0.6, 0.4 - 1.0 / n, 1.0 / n])
     _check(req, gpu_ctx, precision)
+
+
+# A direction unit is compiled for every 8 (from 64 moments on 16) moments up to
+# 128 (FP64: 64), later blocks hold the rest: each of them, with the two grid points
+# that leave large moment counts to this form (a grid point direct: 1,500 atoms'
+# pairs); radius and order as in the form's own rule.
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("mode", ["vacuum", "weighted"])
+@pytest.mark.parametrize("moments", [8, 16, 24, 32, 40, 48, 56, 64, 72, 80, 96, 104, 112, 120, 128,
+                                     136, 168, 240])
+def test_direction_moment_counts(gpu_ctx, precision, mode, moments):
+    a, b = (13.0, 3.0) if precision == "fp64" else (8.0, 2.0)
+    z = np.linspace(0.0, 300.0, 30001)
+    z = z[np.searchsorted(z + a * np.cbrt(0.5 * z) + b, max(moments - 4.0, b + 0.1))]
+    rng = np.random.default_rng(moments)
+    v = rng.normal(size=(1500, 3))
+    xyz = v / np.linalg.norm(v, axis=1)[:, None] * rng.random((1500, 1)) ** (1 / 3)
+    xyz -= xyz.mean(axis=0)
+    xyz *= 10.0 / np.linalg.norm(xyz, axis=1).max()
+    _check(_request(xyz, 2, 0.0, z / 10.3, precision, mode, moments), gpu_ctx, precision)
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
@@ -152,3 +172,28 @@ def test_direction_form_shards_add_up(precision):
         assert np.all(term_errors(total, whole) < 1e-12)
     finally:
         ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_frames_of_both_forms_share_a_batch(gpu_ctx, precision):
+    """A batch whose frames take different forms (a globule sums directions, the
+    same points blown up eight times need more directions than there are pairs):
+    every frame keeps its own sums. The frames of the batch are solved one by
+    one for comparison; FP64 rounding, and the FP32 sums' grouping."""
+    w = workloads.small_globule(800, 5, nq=45, solvent=False, precision=precision)
+    rng = np.random.default_rng(8)
+    frames = w.request.xyz[None] + rng.normal(0, 0.4, (12, 800, 3))
+    frames[::3] *= 8.0
+    weights = rng.exponential(1.0, 12)
+    r = w.request
+
+    def req(xyz, fw):
+        return DebyeRequest(xyz, r.species, r.ff_atoms, None, None, None, r.qmin, r.qmax, r.nq,
+                            fw, precision)
+    want = sum(f * solve(req(x, None), gpu_ctx) for f, x in zip(weights, frames)) / weights.sum()
+    s = TrajectoryStream(req(r.xyz, None), 12, gpu_ctx)
+    s.push(frames, weights)
+    tol = 1e-12 if precision == "fp64" else 1e-5
+    assert np.all(term_errors(s.finish(), want) < tol)
+    assert np.all(term_errors(solve(req(frames, weights), gpu_ctx), want) < tol)

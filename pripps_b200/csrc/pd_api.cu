@@ -599,7 +599,8 @@ int create_devplan(pd_ctx *ctx, const pd_request *req, const uint32_t *species,
 
 // Everything after the pair kernel: slot reduction, six-profile combine and
 // the frame mean; leaves the [6][nq] result at L.out (or out_dev).
-int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st) {
+int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st,
+                   bool after = false) {
     NvtxRange nvtx("pd reduce + combine");
     const Plan &P = dp.P;
     const Layout &L = dp.L;
@@ -611,25 +612,20 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st) {
                                        P.nv, P.n_frames, P.precision == PD_FP32_FP64RED ? 1 : 0,
                                        add_exact, dp.dptr<double>(L.chunk_sums),
                                        dp.dptr<unsigned int>(L.red_done), dp.dptr<double>(L.red),
-                                       st));
+                                       st, after));
         ctx->launches += 1;
+        after = true;
     }
     if (P.amp.dir_cap > 0) {
-        if (static_cast<int>(P.chunks.size()) > P.n_cls) {
-            PD_CUDA(ctx, pd::launch_class_sums(dp.dptr<double>(L.dir_slots),
-                                               dp.dptr<PdFrameDev>(L.frames), P.amp, P.n_frames,
-                                               dp.dptr<int32_t>(L.cls_ptr),
-                                               dp.dptr<int32_t>(L.cls_chunk), st));
-            ctx->launches += 1;
-        }
         PD_CUDA(ctx, pd::launch_direction_sums(
                          dp.dptr<double>(L.dir_slots), dp.dptr<double4>(L.dirs),
                          dp.dptr<PdFrameDev>(L.frames), P.amp, P.qmax, P.n_frames,
                          dp.dptr<PdClassDev>(L.cls), dp.dptr<PdPairDev>(L.pairs), P.n_pairs,
                          dp.dptr<int32_t>(L.cls_ptr), dp.dptr<int32_t>(L.cls_chunk), P.red.width,
                          add_exact, dp.dptr<double>(L.dir_part),
-                         dp.dptr<unsigned int>(L.dir_done), dp.dptr<double>(L.red), st));
+                         dp.dptr<unsigned int>(L.dir_done), dp.dptr<double>(L.red), st, after));
         ctx->launches += 1;
+        after = true;
     }
     if (!P.lat.empty() && !P.dir_only) {
         PD_CUDA(ctx, pd::launch_lattice_sums(
@@ -638,6 +634,7 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st) {
                          dp.dptr<double>(L.qv), P.nq, add_exact, dp.dptr<int>(L.lat_err),
                          dp.dptr<PdFrameDev>(L.frames), dp.dptr<double>(L.lat_sums), st));
         ctx->launches += 1;
+        after = false;  // (the lattice kernels are outside the chain)
     }
     double *dst = out_dev ? out_dev : dp.dptr<double>(L.out);
     double *terms = P.n_frames > 1 ? dp.dptr<double>(L.terms) : dst;
@@ -648,11 +645,11 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st) {
                                      dp.dptr<double>(L.ffA), P.has_exc ? dp.dptr<double>(L.ffC) : nullptr,
                                      P.has_hyd ? dp.dptr<double>(L.ffW) : nullptr, add_exact,
                                      P.qmax, P.lat.empty() ? nullptr : dp.dptr<int>(L.lat_err),
-                                     terms, st));
+                                     terms, st, after));
     ctx->launches += 1;
     if (P.n_frames > 1) {
         PD_CUDA(ctx, pd::launch_frame_mean(dp.dptr<double>(L.terms), dp.dptr<double>(L.fw),
-                                           P.n_frames, P.nq, dst, st, !dp.frame_sum));
+                                           P.n_frames, P.nq, dst, st, !dp.frame_sum, true));
         ctx->launches += 1;
     }
     return PD_OK;
@@ -664,22 +661,20 @@ int pack_devplan(pd_ctx *ctx, DevPlan &dp, cudaStream_t st) {
     const Plan &P = dp.P;
     const Layout &L = dp.L;
     PD_CUDA(ctx, cudaMemsetAsync(dp.base + L.ctl, 0, L.ctl_bytes, st));
-    // a streamed trajectory keeps the status of all its batches
-    PD_CUDA(ctx, pd::launch_centroid(dp.xyz_dev, P.n_atoms, P.n_frames,
-                                     dp.dptr<double>(L.cent_part),
-                                     dp.dptr<unsigned int>(L.cent_done),
-                                     dp.dptr<double>(L.centroid),
-                                     dp.frame_sum ? nullptr : dp.dptr<int32_t>(L.status), st));
-    PD_CUDA(ctx, pd::launch_pack(dp.xyz_dev, P.has_hyd ? dp.dptr<double>(L.hw) : nullptr,
-                                 dp.dptr<int32_t>(L.perm), dp.dptr<double>(L.centroid), P.n_atoms,
-                                 P.n_pad, P.n_frames,
-                                 P.precision == PD_FP64 ? nullptr : dp.dptr<float4>(L.atoms),
-                                 P.precision == PD_FP64 ? dp.dptr<double4>(L.atoms) : nullptr,
-                                 P.mom, dp.dptr<unsigned long long>(L.rad2),
-                                 dp.dptr<unsigned int>(L.pack_done),
-                                 dp.dptr<PdFrameDev>(L.frames), dp.dptr<double4>(L.dirs),
-                                 dp.dptr<double2>(L.nodes), st));
-    ctx->launches += 2;
+    int launches = 0;
+    PD_CUDA(ctx, pd::launch_pack(
+                     dp.xyz_dev, P.has_hyd ? dp.dptr<double>(L.hw) : nullptr,
+                     dp.dptr<int32_t>(L.perm), P.n_atoms, P.n_pad, P.n_frames,
+                     dp.dptr<double>(L.cent_part), dp.dptr<unsigned int>(L.cent_done),
+                     dp.dptr<double>(L.centroid),
+                     // a streamed trajectory keeps the status of all its batches
+                     dp.frame_sum ? nullptr : dp.dptr<int32_t>(L.status),
+                     P.precision == PD_FP64 ? nullptr : dp.dptr<float4>(L.atoms),
+                     P.precision == PD_FP64 ? dp.dptr<double4>(L.atoms) : nullptr, P.mom,
+                     dp.dptr<unsigned long long>(L.rad2), dp.dptr<unsigned int>(L.pack_done),
+                     dp.dptr<PdFrameDev>(L.frames), dp.dptr<double4>(L.dirs),
+                     dp.dptr<double2>(L.nodes), st, &launches));
+    ctx->launches += launches;
     if (!P.lat.empty()) {
         PD_CUDA(ctx, pd::launch_lattice(dp.xyz_dev, dp.dptr<int32_t>(L.perm),
                                         dp.dptr<PdLatDev>(L.lat), P.lat.data(),
@@ -710,12 +705,15 @@ int run_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st,
     const Layout &L = dp.L;
     int rc = pack_devplan(ctx, dp, st);
     if (rc) return rc;
+    bool after = P.lat.empty() && !ev;  // the next kernel follows one of the chain directly
     if (ev) cudaEventRecord(ev->first, st);
-    if (dp.world > 1)  // a frame's slot may be written by another rank's tile only
+    if (dp.world > 1) {  // a frame's slot may be written by another rank's tile only
+        after = false;
         PD_CUDA(ctx, cudaMemsetAsync(dp.dptr<double>(L.slots), 0,
                                      static_cast<size_t>(P.slots_per_frame) * P.n_frames * P.nv *
                                          P.tun.K * 8,
                                      st));
+    }
     if (P.amp.dir_cap > 0) {
         NvtxRange nvtx("pd direction kernel");
         const int v = pd::directions_variant(P.precision, P.amp.amp_cap);
@@ -724,8 +722,9 @@ int run_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st,
                               static_cast<int64_t>(ctx->sm_count) * pd::directions_blocks_per_sm(v));
         PD_CUDA(ctx, pd::launch_directions(v, dp.dptr<PdJob>(L.jobs), dp.dptr<int>(L.njobs),
                                            dp.dptr<PdReqDev>(L.req), dp.dptr<int>(L.counter),
-                                           P.n_frames, static_cast<int>(grid), st));
+                                           P.n_frames, static_cast<int>(grid), st, after));
         ctx->launches += 1;
+        after = true;
     }
     if (!P.jobs.empty() && !P.dir_only) {
         NvtxRange nvtx("pd pair kernel");
@@ -733,11 +732,15 @@ int run_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st,
                                       dp.dptr<int>(L.njobs), dp.dptr<PdReqDev>(L.req),
                                       dp.dptr<int>(L.counter), P.n_frames,
                                       persistent_grid(ctx, P, static_cast<int64_t>(P.jobs.size())),
-                                      st));
+                                      st, after));
         ctx->launches += 1;
+        after = true;
     }
-    if (ev) cudaEventRecord(ev->second, st);
-    return finish_devplan(ctx, dp, out_dev, st);
+    if (ev) {
+        cudaEventRecord(ev->second, st);
+        after = false;
+    }
+    return finish_devplan(ctx, dp, out_dev, st, after);
 }
 
 }  // namespace

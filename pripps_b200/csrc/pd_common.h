@@ -112,6 +112,8 @@ constexpr int PD_MAX_MOMENTS = 512;
 // and the shared memory of the kernel that sums the class pairs.
 constexpr int PD_MAX_DIR_MOMENTS = 256;
 constexpr int PD_DIR_SMEM = 200 * 1024;
+// Lane operations that the pair form is charged beyond its pairs (frame_constants).
+constexpr double PD_PAIRS_LATENCY = 1e7;
 constexpr int PD_DIR_DIRS = 8;  // directions of a work unit
 // Moments of its first block (FP32, FP64) and of each later one.
 constexpr int PD_DIR_MBLOCK = 128, PD_DIR_MBLOCK64 = 64;

@@ -4,6 +4,7 @@
 #include <algorithm>
 
 #include "pd_kernels.h"
+#include "pd_launch.cuh"
 #include "pd_moments.cuh"
 
 namespace pd {
@@ -397,6 +398,7 @@ __global__ void __launch_bounds__(PD_THREADS, MAXM <= 64 ? 4 : 3)
     pd_directions_fp32(const PdJob *__restrict__ jobs, const int *__restrict__ n_jobs_ptr,
                        const PdReqDev *__restrict__ reqs, int *__restrict__ counter,
                        int plan_frames) {
+    chain_enter();
     extern __shared__ __align__(128) float4 s_buf[];
     dir_units<float4, MAXM>(jobs, n_jobs_ptr, reqs, counter, plan_frames, s_buf);
 }
@@ -405,40 +407,10 @@ __global__ void __launch_bounds__(PD_THREADS, 2)
     pd_directions_fp64(const PdJob *__restrict__ jobs, const int *__restrict__ n_jobs_ptr,
                        const PdReqDev *__restrict__ reqs, int *__restrict__ counter,
                        int plan_frames) {
+    chain_enter();
     extern __shared__ __align__(128) float4 s_buf[];
     dir_units<double4, PD_DIR_MBLOCK64>(jobs, n_jobs_ptr, reqs, counter, plan_frames,
                                         reinterpret_cast<double4 *>(s_buf));
-}
-
-// The sums of a class's chunks, added to the first one's in chunk order, so that the
-// class pairs' kernel, which reads them once per tile of nodes, finds one array per
-// class (left to that kernel, 10,000 atoms in chunks of 2,048 and 512 atoms took it 27
-// and 60 µs). Block: a (class, v) of a group.
-__global__ void __launch_bounds__(256)
-    pd_class_sums(double *__restrict__ slots, const PdFrameDev *__restrict__ frames, PdAmpShape sh,
-                  const int32_t *__restrict__ cls_ptr, const int32_t *__restrict__ cls_chunk) {
-    const int f = blockIdx.z, cv = blockIdx.y, grp = blockIdx.x;
-    const int n_grp = frames[f].n_grp, n_amp = frames[f].n_amp;
-    const int c = cv / sh.nv2, v = cv % sh.nv2;
-    const int e0 = cls_ptr[c], n = cls_ptr[c + 1] - e0;
-    if (grp >= n_grp || n <= 1) return;
-    double *base = slots + static_cast<int64_t>(f) * sh.slot_cap +
-                   (static_cast<int64_t>(v) * n_grp + grp) * n_amp * 32;
-    const int64_t step = static_cast<int64_t>(sh.nv2) * n_grp * n_amp * 32;  // of a chunk
-    const int32_t *list = cls_chunk + e0;
-    for (int k = threadIdx.x; k < n_amp * 32; k += 512) {
-        const bool two = k + 256 < n_amp * 32;
-        double *dst = base + list[0] * step + k;
-        double s0 = dst[0], s1 = two ? dst[256] : 0.0;
-#pragma unroll 4
-        for (int e = 1; e < n; ++e) {
-            const double *src = base + list[e] * step + k;
-            s0 += __ldg(src);
-            if (two) s1 += __ldg(src + 256);
-        }
-        dst[0] = s0;
-        if (two) dst[256] = s1;
-    }
 }
 
 namespace {
@@ -466,28 +438,15 @@ int directions_blocks_per_sm(int variant) {
 
 cudaError_t launch_directions(int variant, const PdJob *jobs, const int *n_jobs,
                               const PdReqDev *reqs, int *counter, int plan_frames, int grid,
-                              cudaStream_t st) {
+                              cudaStream_t st, bool after) {
     if (variant == 0)
-        pd_directions_fp64<<<grid, PD_THREADS, DIR_SMEM64, st>>>(jobs, n_jobs, reqs, counter, plan_frames);
-    else if (variant == 64)
-        pd_directions_fp32<64><<<grid, PD_THREADS, dir_smem_bytes<64>(), st>>>(
-            jobs, n_jobs, reqs, counter, plan_frames);
-    else
-        pd_directions_fp32<128><<<grid, PD_THREADS, dir_smem_bytes<128>(), st>>>(
-            jobs, n_jobs, reqs, counter, plan_frames);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_class_sums(double *slots, const PdFrameDev *frames, const PdAmpShape &sh,
-                              int n_frames, const int32_t *cls_ptr, const int32_t *cls_chunk,
-                              cudaStream_t st) {
-    const int ncv = sh.n_cls * sh.nv2;
-    for (int f = 0; f < n_frames; f += 65535) {  // (the grid's z limit)
-        const int nf = std::min(n_frames - f, 65535);
-        pd_class_sums<<<dim3(sh.grp_cap, ncv, nf), 256, 0, st>>>(
-            slots + static_cast<int64_t>(f) * sh.slot_cap, frames + f, sh, cls_ptr, cls_chunk);
-    }
-    return cudaGetLastError();
+        return chain_launch(after, pd_directions_fp64, grid, PD_THREADS, DIR_SMEM64, st, jobs,
+                            n_jobs, reqs, counter, plan_frames);
+    if (variant == 64)
+        return chain_launch(after, pd_directions_fp32<64>, grid, PD_THREADS, dir_smem_bytes<64>(),
+                            st, jobs, n_jobs, reqs, counter, plan_frames);
+    return chain_launch(after, pd_directions_fp32<128>, grid, PD_THREADS, dir_smem_bytes<128>(), st,
+                        jobs, n_jobs, reqs, counter, plan_frames);
 }
 
 }  // namespace pd

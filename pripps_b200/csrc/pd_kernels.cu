@@ -1,5 +1,10 @@
 // Device kernels of the Debye backend (sm_100a).
 //
+// A frame takes one of three forms, by the rule in frame_constants: class
+// amplitudes over directions (pd_directions.cu, pd_direction_sums here), moments of
+// the pairs (pd_moments.cuh, in the pair kernels), or, where the moments outnumber
+// what they replace, the grid points one by one:
+//
 // K1 (pd_pairs_fp32): for each tile (i-block × j-range × q-block) every thread
 // owns one i atom and walks the j atoms of the range NP at a time. For a pair
 // at distance r it needs sin(q_k r) for the K consecutive grid points
@@ -26,6 +31,7 @@
 //
 // K2 (pd_pairs_fp64): the same tiling with sin(q_k r) from the FP64 sin() for
 // every pair and q, and FP64 accumulation throughout.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -38,6 +44,7 @@
 
 #include "pd_common.h"
 #include "pd_kernels.h"
+#include "pd_launch.cuh"
 #include "pd_moments.cuh"
 #include "pripps_debye.h"
 
@@ -856,6 +863,7 @@ template <int K, int MODE, int NP>
 __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
     pd_pairs_fp32(const PdJob *__restrict__ jobs, const int *__restrict__ n_jobs_ptr,
                   const PdReqDev *__restrict__ reqs, int *__restrict__ counter, int plan_frames) {
+    chain_enter();
     constexpr int NACC = (MODE == PD_MODE_WEIGHTED) ? 2 : 1;
     constexpr int NV = (MODE == PD_MODE_WEIGHTED) ? 4 : 1;  // FP64 values per q in a slot
     constexpr bool PACKED = (MODE == PD_MODE_CLASS);
@@ -1158,6 +1166,7 @@ __global__ void __launch_bounds__(PD_THREADS, K <= 16 ? 4 : 2) pd_pairs_fp64(con
                                                             const PdReqDev *__restrict__ reqs,
                                                             int *__restrict__ counter,
                                                             int plan_frames) {
+    chain_enter();
     constexpr int NACC = (MODE == PD_MODE_WEIGHTED) ? 2 : 1;
     constexpr int NV = (MODE == PD_MODE_WEIGHTED) ? 4 : 1;
     __shared__ int s_job;
@@ -1262,6 +1271,7 @@ __global__ void __launch_bounds__(PD_CENT_THREADS)
     pd_centroid(const double *__restrict__ xyz, int64_t n_atoms, int32_t n_blk,
                 double *__restrict__ part, unsigned int *__restrict__ done,
                 double *__restrict__ centroid, int32_t *__restrict__ status) {
+    chain_enter();
     __shared__ double red[3][PD_CENT_THREADS];
     __shared__ bool s_last;
     const int f = blockIdx.x / n_blk, b = blockIdx.x % n_blk;
@@ -1309,11 +1319,14 @@ __global__ void __launch_bounds__(PD_CENT_THREADS)
 // frame's last block turns it into the frame's constants (PdFrameDev): which form
 // its pairs are summed in, the expansion's size and the direction table.
 //
-// The rule counts FP32 lane operations. A pair, or an atom in one direction, costs
-// about 44 for its sequences (in each moment block) and 1.25 per moment; a
-// direction also n_cls·M terms per node in FP64. Measured on both
-// sides of the line (FP32, nq 200, R 16·(N/1000)^{1/3}): pairs are the faster form below about
-// 300 atoms, directions above.
+// The rule counts FP32 lane operations: a pair costs about 44 for its sequences (in
+// each moment block) and 1.25 per moment, an atom in one direction 14 (44 more for each
+// later block) and 1.25 per moment, a direction also n_cls·M terms per node in FP64;
+// PD_PAIRS_LATENCY stands for the pair form's longer chain of short kernels.
+// Whole solves on both sides (vacuum; pairs / directions, µs): FP32, q_max 0.5, 200 /
+// 300 / 600 / 1,200 atoms 68/65, 80/66, 83/70, 90/84, q_max 1.0 71/75, 84/72, 89/82,
+// 97/89; FP64 68/65, 69/65, 83/79, 103/86 and 82/79, 84/80, 93/86, 110/111. Elongated 2.5 : 1,
+// q_max 1.0, 300 / 500 / 800 atoms: FP32 73/79, 82/92, 101/122, FP64 79/97, 87/111, 114/153.
 constexpr int PD_PACK_THREADS = 256;
 
 // Nodes and weights of the 2h-point Gauss–Legendre rules, upper half
@@ -1326,6 +1339,113 @@ __device__ __forceinline__ int ring_points(double z_sin, bool fp64) {
     return max(4, static_cast<int>(direction_order(z_sin, fp64)) + 1);
 }
 
+// A frame's constants (PdFrameDev) from its radius: which form its pairs are summed
+// in, the expansion's size, and the direction table, whose entries the n_part blocks
+// share. T threads, all of each block.
+template <int T>
+__device__ __forceinline__ void frame_constants(double radius, const PdMomentRule &rule, int f,
+                                                int part, int n_part,
+                                                PdFrameDev *__restrict__ frames,
+                                                double4 *__restrict__ dirs,
+                                                double2 *__restrict__ node_tab) {
+    static_assert(T >= PD_GL_MAX, "a thread per ring");
+    __shared__ int s_off[PD_GL_MAX + 1];  // first direction of each ring
+    const bool fp64 = rule.fp64 != 0;
+    PdFrameDev fr{};
+    fr.radius = radius;
+    // d follows the FP32 value of 1/d² that the pairs are scaled with: rounding
+    // 1/d² alone would stretch every distance by the same 1 + 3e-8
+    fr.d = fmax(2.0 * PD_MOM_STRETCH * radius, 1e-6);
+    fr.inv_d2 = static_cast<double>(static_cast<float>(1.0 / (fr.d * fr.d)));
+    fr.d = 1.0 / sqrt(fr.inv_d2);
+    fr.r1 = fmax(PD_MOM_STRETCH * radius, 1e-6);
+    double pair_cost = 1e300;
+    if (rule.block > 0) {
+        const int m8 = (moments_needed(rule.qmax * fr.d, fp64) + 7) & ~7;
+        const int blocks = (m8 + rule.block - 1) / rule.block;
+        if (m8 <= rule.max_moments && blocks <= rule.nqb) {
+            fr.n_mom = m8;
+            fr.n_mblk = blocks;
+            fr.n_parts = rule.nqb / blocks;
+            pair_cost = 0.5 * static_cast<double>(rule.n_atoms) * rule.n_atoms *
+                        (44.0 * blocks + 1.25 * m8);
+        }
+    }
+    // ---- directions: 2h Gauss rings (upper half: h), enough points on each
+    if (rule.dir_cap == 0) {
+        if (part == 0 && threadIdx.x == 0) frames[f] = fr;
+        return;
+    }
+    const double z = 2.0 * radius * rule.qmax;
+    const double order = direction_order(z, fp64);
+    const int h = order < 4.0 * PD_GL_MAX - 4.0 ? static_cast<int>(order * 0.25) + 1 : 0;
+    const double2 *gl = pd_gl_rules + h * (h - 1) / 2;
+    if (threadIdx.x < h) {
+        const double x = gl[threadIdx.x].x;
+        s_off[threadIdx.x + 1] = ring_points(z * sqrt(1.0 - x * x), fp64);
+    }
+    __syncthreads();
+    for (int o = 1; o < h; o <<= 1) {  // inclusive scan of s_off[1 .. h]
+        const int k = threadIdx.x + 1;
+        const int v = (k <= h && k > o) ? s_off[k - o] : 0;
+        __syncthreads();
+        if (k <= h) s_off[k] += v;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) s_off[0] = 0;
+    __syncthreads();
+    const int S = h > 0 ? s_off[h] : 0;
+    const int groups = (S + 31) / 32;
+    const int mine = rule.rank < groups ? (groups - rule.rank + rule.world - 1) / rule.world : 0;
+    const double mo = direction_order(fr.r1 * rule.qmax, fp64);
+    const int m8 = mo < 1e6 ? ((static_cast<int>(mo) + 8) & ~7) : 1000000;
+    const int ablk = (m8 + rule.dir_block - 1) / rule.dir_block;
+    const int nodes = moments_needed(2.0 * fr.r1 * rule.qmax, true);
+    const double dir_cost =
+        static_cast<double>(S) * (static_cast<double>(rule.n_atoms) * rule.nv2 *
+                                      (44.0 * ablk - 30.0 + 1.25 * m8) +
+                                  4.0 * rule.n_cls * m8 * nodes);
+    const bool use = S > 0 && rule.block > 0 && groups * 32 <= rule.dir_cap && mine > 0 &&
+                     (groups + rule.world - 1) / rule.world <= rule.grp_cap &&
+                     m8 <= rule.amp_cap && nodes <= rule.node_cap &&
+                     static_cast<int64_t>(rule.n_chunk) * rule.nv2 *
+                             ((groups + rule.world - 1) / rule.world) * m8 * 32 <= rule.slot_cap &&
+                     groups >= rule.world && (rule.dir_only || dir_cost < pair_cost + PD_PAIRS_LATENCY);
+    if (use) {
+        fr.n_grp = mine;
+        fr.n_amp = m8;
+        fr.n_ablk = ablk;
+        fr.n_node = nodes;
+        // Chebyshev nodes of the q range: y_k and the barycentric weight
+        for (int k = part * T + threadIdx.x; k < nodes; k += n_part * T) {
+            double sn, cs;
+            sincospi((2 * k + 1) / (2.0 * nodes), &sn, &cs);
+            node_tab[static_cast<int64_t>(f) * rule.node_cap + k] =
+                make_double2(cs, (k & 1) ? -sn : sn);
+        }
+        const double sc = 0.5 / fr.r1;
+        double4 *o = dirs + static_cast<int64_t>(f) * rule.dir_cap;
+        for (int s = part * T + threadIdx.x; s < groups * 32; s += n_part * T) {
+            double4 d = make_double4(0.0, 0.0, 0.0, 0.0);
+            if (s < S) {
+                int lo = 0, hi = h;  // ring with s_off[lo] <= s < s_off[lo + 1]
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (s_off[mid] <= s) lo = mid; else hi = mid;
+                }
+                const double2 nw = gl[lo];
+                const int n = s_off[lo + 1] - s_off[lo];
+                const double st = sqrt(1.0 - nw.x * nw.x) * sc;
+                double sn, cs;
+                sincospi(2.0 * (s - s_off[lo]) / n, &sn, &cs);
+                d = make_double4(st * cs, st * sn, nw.x * sc, nw.y / n);
+            }
+            o[s] = d;
+        }
+    }
+    if (part == 0 && threadIdx.x == 0) frames[f] = fr;
+}
+
 __global__ void __launch_bounds__(PD_PACK_THREADS)
     pd_pack(const double *__restrict__ xyz, const double *__restrict__ weights,
             const int32_t *__restrict__ perm, const double *__restrict__ centroid,
@@ -1333,10 +1453,10 @@ __global__ void __launch_bounds__(PD_PACK_THREADS)
             double4 *__restrict__ out64, PdMomentRule rule, unsigned long long *__restrict__ rad2,
             unsigned int *__restrict__ done, PdFrameDev *__restrict__ frames,
             double4 *__restrict__ dirs, double2 *__restrict__ node_tab) {
+    chain_enter();
     __shared__ double s_max[PD_PACK_THREADS / 32];
     __shared__ bool s_last;
     __shared__ double s_radius;
-    __shared__ int s_off[PD_GL_MAX + 1];  // first direction of each ring
     const int f = blockIdx.x / n_blk, b = blockIdx.x % n_blk;
     const int p = b * PD_PACK_THREADS + threadIdx.x;
     double r2 = 0.0;
@@ -1375,101 +1495,93 @@ __global__ void __launch_bounds__(PD_PACK_THREADS)
     __syncthreads();
     if (!s_last) return;
 
-    const double radius = s_radius;
-    const bool fp64 = rule.fp64 != 0;
-    PdFrameDev fr{};
-    fr.radius = radius;
-    // d follows the FP32 value of 1/d² that the pairs are scaled with: rounding
-    // 1/d² alone would stretch every distance by the same 1 + 3e-8
-    fr.d = fmax(2.0 * PD_MOM_STRETCH * radius, 1e-6);
-    fr.inv_d2 = static_cast<double>(static_cast<float>(1.0 / (fr.d * fr.d)));
-    fr.d = 1.0 / sqrt(fr.inv_d2);
-    fr.r1 = fmax(PD_MOM_STRETCH * radius, 1e-6);
-    double pair_cost = 1e300;
-    if (rule.block > 0) {
-        const int m8 = (moments_needed(rule.qmax * fr.d, fp64) + 7) & ~7;
-        const int blocks = (m8 + rule.block - 1) / rule.block;
-        if (m8 <= rule.max_moments && blocks <= rule.nqb) {
-            fr.n_mom = m8;
-            fr.n_mblk = blocks;
-            fr.n_parts = rule.nqb / blocks;
-            pair_cost = 0.5 * static_cast<double>(rule.n_atoms) * rule.n_atoms *
-                        (44.0 * blocks + 1.25 * m8);
-        }
-    }
-    // ---- directions: 2h Gauss rings (upper half: h), enough points on each
-    if (rule.dir_cap == 0) {
-        if (threadIdx.x == 0) frames[f] = fr;
-        return;
-    }
-    const double z = 2.0 * radius * rule.qmax;
-    const double order = direction_order(z, fp64);
-    const int h = order < 4.0 * PD_GL_MAX - 4.0 ? static_cast<int>(order * 0.25) + 1 : 0;
-    const double2 *gl = pd_gl_rules + h * (h - 1) / 2;
-    if (threadIdx.x < h) {
-        const double x = gl[threadIdx.x].x;
-        s_off[threadIdx.x + 1] = ring_points(z * sqrt(1.0 - x * x), fp64);
+    frame_constants<PD_PACK_THREADS>(s_radius, rule, f, 0, 1, frames, dirs, node_tab);
+}
+
+// Centroid, pack and constants of a frame in one kernel: a cluster of PD_FRAME_CTAS
+// blocks per frame, whose partial sums and maxima meet in distributed shared memory. For
+// frames of up to PD_FRAME_MAX padded atoms, where the two kernels are latency (8
+// SMs read the frame here): 300 atoms 15.7 -> 7.5 µs, 3,000 atoms 18.3 -> 12.0 µs;
+// whole executions at the line, 16,000 atoms (one kernel) 116 µs, 17,000 (two) 126 µs.
+constexpr int PD_FRAME_CTAS = 8, PD_FRAME_THREADS = 512;
+constexpr int32_t PD_FRAME_MAX = 16384;
+
+__global__ void __cluster_dims__(PD_FRAME_CTAS, 1, 1) __launch_bounds__(PD_FRAME_THREADS)
+    pd_pack_frames(const double *__restrict__ xyz, const double *__restrict__ weights,
+                   const int32_t *__restrict__ perm, int32_t n_atoms, int32_t n_pad,
+                   float4 *__restrict__ out32, double4 *__restrict__ out64, PdMomentRule rule,
+                   PdFrameDev *__restrict__ frames, double4 *__restrict__ dirs,
+                   double2 *__restrict__ node_tab, int32_t *__restrict__ status) {
+    chain_enter();
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ double s_red[PD_FRAME_THREADS / 32][3];
+    __shared__ double s_mine[4];  // this block's sums and maximum, read by the cluster
+    constexpr int STEP = PD_FRAME_CTAS * PD_FRAME_THREADS;
+    const int f = blockIdx.x / PD_FRAME_CTAS, rank = blockIdx.x % PD_FRAME_CTAS;
+    const int first = rank * PD_FRAME_THREADS + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double *p = xyz + static_cast<size_t>(f) * n_atoms * 3;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && status) *status = 0;
+    double sum[3] = {0.0, 0.0, 0.0};
+#pragma unroll 4
+    for (int i = first; i < n_atoms; i += STEP)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) sum[a] += p[3 * static_cast<size_t>(i) + a];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        sum[a] = warp_sum(sum[a]);
+        if (lane == 0) s_red[warp][a] = sum[a];
     }
     __syncthreads();
-    for (int o = 1; o < h; o <<= 1) {  // inclusive scan of s_off[1 .. h]
-        const int k = threadIdx.x + 1;
-        const int v = (k <= h && k > o) ? s_off[k - o] : 0;
-        __syncthreads();
-        if (k <= h) s_off[k] += v;
-        __syncthreads();
+    if (threadIdx.x < 3) {
+        double s = 0.0;
+        for (int w = 0; w < PD_FRAME_THREADS / 32; ++w) s += s_red[w][threadIdx.x];
+        s_mine[threadIdx.x] = s;
     }
-    if (threadIdx.x == 0) s_off[0] = 0;
+    cluster.sync();
+    double c[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int b = 0; b < PD_FRAME_CTAS; ++b) {
+        const double *o = cluster.map_shared_rank(s_mine, b);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) c[a] += o[a];
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) c[a] /= static_cast<double>(n_atoms);
+    double r2 = 0.0;
+#pragma unroll 2
+    for (int k = first; k < n_pad; k += STEP) {
+        const int src = perm[k];
+        double x = 0, y = 0, z = 0, w = 0;
+        if (src >= 0) {
+            const double *s = p + static_cast<size_t>(src) * 3;
+            x = s[0] - c[0];
+            y = s[1] - c[1];
+            z = s[2] - c[2];
+            w = weights ? weights[src] : 0.0;
+            r2 = fmax(r2, x * x + y * y + z * z);
+        }
+        const size_t t = static_cast<size_t>(f) * n_pad + k;
+        if (out32) out32[t] = make_float4(static_cast<float>(x), static_cast<float>(y),
+                                          static_cast<float>(z), static_cast<float>(w));
+        if (out64) out64[t] = make_double4(x, y, z, w);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) r2 = fmax(r2, __shfl_xor_sync(0xffffffffu, r2, o));
+    if (lane == 0) s_red[warp][0] = r2;
     __syncthreads();
-    const int S = h > 0 ? s_off[h] : 0;
-    const int groups = (S + 31) / 32;
-    const int mine = rule.rank < groups ? (groups - rule.rank + rule.world - 1) / rule.world : 0;
-    const double mo = direction_order(fr.r1 * rule.qmax, fp64);
-    const int m8 = mo < 1e6 ? ((static_cast<int>(mo) + 8) & ~7) : 1000000;
-    const int ablk = (m8 + rule.dir_block - 1) / rule.dir_block;
-    const int nodes = moments_needed(2.0 * fr.r1 * rule.qmax, true);
-    const double dir_cost =
-        static_cast<double>(S) * (static_cast<double>(rule.n_atoms) * rule.nv2 *
-                                      (44.0 * ablk - 30.0 + 1.25 * m8) +
-                                  4.0 * rule.n_cls * m8 * nodes);
-    const bool use = S > 0 && rule.block > 0 && groups * 32 <= rule.dir_cap && mine > 0 &&
-                     (groups + rule.world - 1) / rule.world <= rule.grp_cap &&
-                     m8 <= rule.amp_cap && nodes <= rule.node_cap &&
-                     static_cast<int64_t>(rule.n_chunk) * rule.nv2 *
-                             ((groups + rule.world - 1) / rule.world) * m8 * 32 <= rule.slot_cap &&
-                     groups >= rule.world && (rule.dir_only || dir_cost < pair_cost);
-    if (use) {
-        fr.n_grp = mine;
-        fr.n_amp = m8;
-        fr.n_ablk = ablk;
-        fr.n_node = nodes;
-        // Chebyshev nodes of the q range: y_k and the barycentric weight
-        for (int k = threadIdx.x; k < nodes; k += PD_PACK_THREADS) {
-            double sn, cs;
-            sincospi((2 * k + 1) / (2.0 * nodes), &sn, &cs);
-            node_tab[static_cast<int64_t>(f) * rule.node_cap + k] =
-                make_double2(cs, (k & 1) ? -sn : sn);
-        }
-        const double sc = 0.5 / fr.r1;
-        double4 *o = dirs + static_cast<int64_t>(f) * rule.dir_cap;
-        for (int s = threadIdx.x; s < groups * 32; s += PD_PACK_THREADS) {
-            double4 d = make_double4(0.0, 0.0, 0.0, 0.0);
-            if (s < S) {
-                int lo = 0, hi = h;  // ring with s_off[lo] <= s < s_off[lo + 1]
-                while (hi - lo > 1) {
-                    const int mid = (lo + hi) >> 1;
-                    if (s_off[mid] <= s) lo = mid; else hi = mid;
-                }
-                const double2 nw = gl[lo];
-                const int n = s_off[lo + 1] - s_off[lo];
-                const double st = sqrt(1.0 - nw.x * nw.x) * sc;
-                double sn, cs;
-                sincospi(2.0 * (s - s_off[lo]) / n, &sn, &cs);
-                d = make_double4(st * cs, st * sn, nw.x * sc, nw.y / n);
-            }
-            o[s] = d;
-        }
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < PD_FRAME_THREADS / 32; ++w) r2 = fmax(r2, s_red[w][0]);
+        s_mine[3] = r2;
     }
-    if (threadIdx.x == 0) frames[f] = fr;
+    cluster.sync();
+    r2 = 0.0;
+#pragma unroll
+    for (int b = 0; b < PD_FRAME_CTAS; ++b) r2 = fmax(r2, cluster.map_shared_rank(s_mine, b)[3]);
+    cluster.sync();  // the blocks' shared memory is read
+    frame_constants<PD_FRAME_THREADS>(sqrt(r2), rule, f, rank, PD_FRAME_CTAS, frames, dirs,
+                                      node_tab);
 }
 
 // ------------------------------------------------------------ reductions
@@ -1519,6 +1631,7 @@ __global__ void __launch_bounds__(PD_RED_THREADS)
                     PdReduceShape sh, int32_t residual_form, int32_t add_exact,
                     double *__restrict__ chunk_sums, unsigned int *__restrict__ done,
                     double *__restrict__ red) {
+    chain_enter();
     __shared__ double s_run[PD_RED_GROUPS][NV][128];
     __shared__ bool s_last;
     const int z = blockIdx.x % sh.n_z;
@@ -1617,8 +1730,12 @@ __global__ void __launch_bounds__(PD_RED_THREADS)
 // moment the exact atom count or weight sum — then Σ w·Re(E_a E_b*) over the directions
 // of every class pair. The frame's last block of these nodes adds the groups in
 // group order and takes the i = j terms out of the self sums.
+//
+// Bound: latency — a chain of loads, a Bessel recurrence, two short FP64
+// contractions and the last block's sum. 512 threads: 256 took 20.0 µs per frame
+// more at 20,000 atoms (whole execution 425 against 403 µs), the same at 3,000.
 constexpr int PD_DNODE_T = 16;
-constexpr int PD_DSUM_THREADS = 256;
+constexpr int PD_DSUM_THREADS = 512;
 constexpr int PD_DSUM_WARPS = PD_DSUM_THREADS / 32;
 
 // (2 − δ_n0)·J_n(y)·(sign of i^n) for n < n_mom, unnormalised, into g[n·stride];
@@ -1670,9 +1787,10 @@ __global__ void __launch_bounds__(PD_DSUM_THREADS)
                       const PdFrameDev *__restrict__ frames, PdAmpShape sh, double qmax,
                       const PdClassDev *__restrict__ cls, const PdPairDev *__restrict__ pairs,
                       int32_t n_pairs, const int32_t *__restrict__ cls_ptr,
-                      const int32_t *__restrict__ cls_chunk, int32_t width, int32_t add_exact,
-                      double *__restrict__ part, unsigned int *__restrict__ done,
+                      const int32_t *__restrict__ cls_chunk, int32_t width,
+                      int32_t add_exact, double *__restrict__ part, unsigned int *__restrict__ done,
                       double *__restrict__ red) {
+    chain_enter();
     extern __shared__ double s_dyn[];
     __shared__ double s_scale[PD_DNODE_T], s_w[32];
     __shared__ bool s_last;
@@ -1704,24 +1822,28 @@ __global__ void __launch_bounds__(PD_DSUM_THREADS)
     for (int c0 = 0; c0 < ncv; c0 += batch) {  // as many classes at once as fit
         const int nb = min(batch, ncv - c0);
         if (c0) __syncthreads();  // the previous classes' moments are read
-        // (class, 16 moments) per warp and step: the rows of 32 directions of one
-        // chunk are 16 independent loads
-        const int n16 = (M + 15) / 16;
-        for (int k = warp; k < nb * n16 && warp < LOADERS; k += LOADERS) {
-            const int cb = k / n16, r0 = (k - cb * n16) * 16;
+        // (class, 8 moments) per warp and step: rows of 32 directions, those of four
+        // chunks in flight
+        const int n8 = M / 8;
+        for (int k = warp; k < nb * n8 && warp < LOADERS; k += LOADERS) {
+            const int cb = k / n8, r0 = (k - cb * n8) * 8;
             const int c = (c0 + cb) / NV2, v = (c0 + cb) % NV2;
-            const int rows = min(16, M - r0);  // 16 or 8
-            double m[16];
-            // the class's sums, left at its first chunk
-            const double *src =
-                sl + direction_slot(cls_chunk[cls_ptr[c]], v, grp, NV2, fr) + r0 * 32 + lane;
+            const int e0 = cls_ptr[c], n = cls_ptr[c + 1] - e0;
+            const double *src = sl + direction_slot(0, v, grp, NV2, fr) + r0 * 32 + lane;
+            const int64_t step = static_cast<int64_t>(NV2) * fr.n_grp * M * 32;  // of a chunk
+            double m[8];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) m[u] = u < rows ? __ldg(src + u * 32) : 0.0;
+            for (int u = 0; u < 8; ++u) m[u] = 0.0;
+#pragma unroll 4
+            for (int e = 0; e < n; ++e) {
+                const double *row = src + cls_chunk[e0 + e] * step;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) m[u] += __ldg(row + u * 32);
+            }
             if (r0 == 0) m[0] = v ? cls[c].w1 : cls[c].n;
             double *dst = s_m + (cb * M + r0) * 32 + lane;
 #pragma unroll
-            for (int u = 0; u < 16; ++u)
-                if (u < rows) dst[u * 32] = m[u];
+            for (int u = 0; u < 8; ++u) dst[u * 32] = m[u];
         }
         __syncthreads();
         // (class, four nodes) per warp and step
@@ -1865,6 +1987,7 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
                 const double *__restrict__ ffA, const double *__restrict__ ffC,
                 const double *__restrict__ ffW, int32_t add_diag, double qmax,
                 const int *__restrict__ err, double *__restrict__ terms) {
+    chain_enter();
     extern __shared__ double s_dyn[];
     __shared__ double s_c0[PD_PROF_Q], s_scale[PD_PROF_Q];
     __shared__ double s_sum[PD_PROF_THREADS / 32][6][PD_PROF_Q];
@@ -2174,6 +2297,7 @@ __global__ void __launch_bounds__(256) pd_lattice_sums(const unsigned long long 
 __global__ void pd_frame_mean(const double *__restrict__ terms, const double *__restrict__ fw,
                               int32_t n_frames, int32_t nq, int32_t normalize,
                               double *__restrict__ out) {
+    chain_enter();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 6 * nq) return;
     double s = 0.0, wsum = 0.0;
@@ -2190,6 +2314,7 @@ __global__ void pd_frame_mean(const double *__restrict__ terms, const double *__
 // Batches are added in submission order.
 __global__ void pd_stream_accumulate(const double *__restrict__ batch, double scale, int32_t n,
                                      double *__restrict__ acc) {
+    chain_enter();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) acc[t] += scale * batch[t];
 }
@@ -2883,18 +3008,19 @@ static cudaError_t fp32_smem_attr() {
 }
 template <int K, int MODE, int NP>
 static cudaError_t launch_fp32_t(const PdJob *jobs, const int *n_jobs, const PdReqDev *reqs,
-                                 int *counter, int plan_frames, int grid, cudaStream_t st) {
+                                 int *counter, int plan_frames, int grid, cudaStream_t st,
+                                 bool after) {
     cudaError_t e = fp32_smem_attr<K, MODE, NP>();
     if (e != cudaSuccess) return e;
-    pd_pairs_fp32<K, MODE, NP><<<grid, PD_THREADS, PD_FP32_DYN_SMEM, st>>>(
-        jobs, n_jobs, reqs, counter, plan_frames);
-    return cudaGetLastError();
+    return chain_launch(after, pd_pairs_fp32<K, MODE, NP>, grid, PD_THREADS, PD_FP32_DYN_SMEM, st,
+                        jobs, n_jobs, reqs, counter, plan_frames);
 }
 template <int K, int MODE>
 static cudaError_t launch_fp64_t(const PdJob *jobs, const int *n_jobs, const PdReqDev *reqs,
-                                 int *counter, int plan_frames, int grid, cudaStream_t st) {
-    pd_pairs_fp64<K, MODE><<<grid, PD_THREADS, 0, st>>>(jobs, n_jobs, reqs, counter, plan_frames);
-    return cudaGetLastError();
+                                 int *counter, int plan_frames, int grid, cudaStream_t st,
+                                 bool after) {
+    return chain_launch(after, pd_pairs_fp64<K, MODE>, grid, PD_THREADS, 0, st, jobs, n_jobs, reqs,
+                        counter, plan_frames);
 }
 template <int K, int MODE, int NP>
 static int occupancy_fp32() {
@@ -2928,13 +3054,13 @@ bool valid_q_block(int precision, int K) {
 
 #define PD_F32(K, M, NP)                                                                 \
     if (K_ == K && mode == M && NP_ == NP)                                               \
-        return launch_fp32_t<K, M, NP>(jobs, n_jobs, reqs, counter, plan_frames, grid, st);
+        return launch_fp32_t<K, M, NP>(jobs, n_jobs, reqs, counter, plan_frames, grid, st, after);
 #define PD_F64(K, M) \
-    if (K_ == K && mode == M) return launch_fp64_t<K, M>(jobs, n_jobs, reqs, counter, plan_frames, grid, st);
+    if (K_ == K && mode == M) return launch_fp64_t<K, M>(jobs, n_jobs, reqs, counter, plan_frames, grid, st, after);
 
 cudaError_t launch_pairs(int precision, int K_, int NP_, int mode, const PdJob *jobs,
                          const int *n_jobs, const PdReqDev *reqs, int *counter, int plan_frames,
-                         int grid, cudaStream_t st) {
+                         int grid, cudaStream_t st, bool after) {
     if (precision == 1) {
         PD_F64(16, 0) PD_F64(16, 1) PD_F64(32, 0) PD_F64(32, 1) PD_F64(64, 0)
         return cudaErrorInvalidValue;
@@ -2978,26 +3104,30 @@ int32_t centroid_blocks(int64_t n_atoms) {
         std::min<int64_t>(std::max<int64_t>((n_atoms + PD_CENT_RUN - 1) / PD_CENT_RUN, 1), 256));
 }
 
-cudaError_t launch_centroid(const double *xyz, int64_t n_atoms, int n_frames, double *part,
-                            unsigned int *done, double *centroid, int32_t *status,
-                            cudaStream_t st) {
-    const int32_t nb = centroid_blocks(n_atoms);
-    pd_centroid<<<static_cast<unsigned>(n_frames) * nb, PD_CENT_THREADS, 0, st>>>(
-        xyz, n_atoms, nb, part, done, centroid, status);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_pack(const double *xyz, const double *weights, const int32_t *perm,
-                        const double *centroid, int64_t n_atoms, int32_t n_pad, int32_t n_frames,
-                        float4 *out32, double4 *out64, const PdMomentRule &rule,
-                        unsigned long long *rad2, unsigned int *done, PdFrameDev *frames,
-                        double4 *dirs, double2 *node_tab, cudaStream_t st) {
+                        int64_t n_atoms, int32_t n_pad, int32_t n_frames, double *part,
+                        unsigned int *cent_done, double *centroid, int32_t *status, float4 *out32,
+                        double4 *out64, const PdMomentRule &rule, unsigned long long *rad2,
+                        unsigned int *done, PdFrameDev *frames, double4 *dirs, double2 *node_tab,
+                        cudaStream_t st, int *launches) {
+    if (n_pad <= PD_FRAME_MAX && n_frames <= 0x7fffffff / PD_FRAME_CTAS) {
+        *launches = 1;
+        return chain_launch(false, pd_pack_frames, static_cast<unsigned>(n_frames) * PD_FRAME_CTAS,
+                            PD_FRAME_THREADS, 0, st, xyz, weights, perm,
+                            static_cast<int32_t>(n_atoms), n_pad, out32, out64, rule, frames, dirs,
+                            node_tab, status);
+    }
+    *launches = 2;
+    const int32_t nc = centroid_blocks(n_atoms);
     const int64_t nb = (static_cast<int64_t>(n_pad) + PD_PACK_THREADS - 1) / PD_PACK_THREADS;
     if (nb * n_frames > 0x7fffffffLL) return cudaErrorInvalidValue;
-    pd_pack<<<static_cast<unsigned>(nb * n_frames), PD_PACK_THREADS, 0, st>>>(
-        xyz, weights, perm, centroid, n_atoms, n_pad, static_cast<int32_t>(nb), out32, out64, rule,
-        rad2, done, frames, dirs, node_tab);
-    return cudaGetLastError();
+    const cudaError_t e =
+        chain_launch(false, pd_centroid, static_cast<unsigned>(n_frames) * nc, PD_CENT_THREADS, 0,
+                     st, xyz, n_atoms, nc, part, cent_done, centroid, status);
+    if (e != cudaSuccess) return e;
+    return chain_launch(true, pd_pack, static_cast<unsigned>(nb * n_frames), PD_PACK_THREADS, 0, st,
+                        xyz, weights, perm, centroid, n_atoms, n_pad, static_cast<int32_t>(nb),
+                        out32, out64, rule, rad2, done, frames, dirs, node_tab);
 }
 
 // Gauss–Legendre rules: Newton's method on P_2h from Tricomi's estimate, in
@@ -3059,8 +3189,9 @@ cudaError_t launch_direction_sums(const double *slots, const double4 *dirs,
                                   const PdFrameDev *frames, const PdAmpShape &sh, double qmax,
                                   int32_t n_frames, const PdClassDev *cls, const PdPairDev *pairs,
                                   int32_t n_pairs, const int32_t *cls_ptr,
-                                  const int32_t *cls_chunk, int32_t width, int add_exact,
-                                  double *part, unsigned int *done, double *red, cudaStream_t st) {
+                                  const int32_t *cls_chunk, int32_t width,
+                                  int add_exact, double *part, unsigned int *done, double *red,
+                                  cudaStream_t st, bool after) {
     const size_t smem = static_cast<size_t>(sh.sum_smem) * sizeof(double);
     auto kern = sh.nv2 == 2 ? pd_direction_sums<2> : pd_direction_sums<1>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3072,12 +3203,12 @@ cudaError_t launch_direction_sums(const double *slots, const double4 *dirs,
     for (int32_t f0 = 0; f0 < n_frames; f0 += 65535) {  // grid.y limit
         const dim3 grid(static_cast<unsigned>(n_nt * sh.grp_cap),
                         static_cast<unsigned>(std::min(n_frames - f0, 65535)));
-        kern<<<grid, PD_DSUM_THREADS, smem, st>>>(
-            slots + f0 * sh.slot_cap, dirs + static_cast<int64_t>(f0) * sh.dir_cap, frames + f0, sh,
+        e = chain_launch(
+            after, kern, grid, PD_DSUM_THREADS, smem, st, slots + f0 * sh.slot_cap, dirs + static_cast<int64_t>(f0) * sh.dir_cap, frames + f0, sh,
             qmax, cls, pairs, n_pairs, cls_ptr, cls_chunk, width, add_exact,
             part + f0 * static_cast<int64_t>(sh.grp_cap) * n_pairs * nv * sh.node_cap,
             done + f0 * n_nt, red + f0 * static_cast<int64_t>(n_pairs) * nv * width);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
@@ -3086,19 +3217,13 @@ cudaError_t launch_reduce(const double *slots, const int64_t *lptr, const int64_
                           const PdPairDev *pairs, const double *qv, const PdFrameDev *frames,
                           const PdReduceShape &sh, int32_t nv, int32_t n_frames, int residual_form,
                           int add_exact, double *chunk_sums, unsigned int *done, double *red,
-                          cudaStream_t st) {
+                          cudaStream_t st, bool after) {
     const int64_t blocks = static_cast<int64_t>(n_frames) * sh.n_pairs * sh.n_z;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
     const dim3 grid(static_cast<unsigned>(blocks), static_cast<unsigned>(sh.n_chunk));
-    if (nv == 4)
-        pd_reduce_pairs<4><<<grid, PD_RED_THREADS, 0, st>>>(slots, lptr, lidx, pairs, qv, frames,
-                                                            sh, residual_form, add_exact,
-                                                            chunk_sums, done, red);
-    else
-        pd_reduce_pairs<1><<<grid, PD_RED_THREADS, 0, st>>>(slots, lptr, lidx, pairs, qv, frames,
-                                                            sh, residual_form, add_exact,
-                                                            chunk_sums, done, red);
-    return cudaGetLastError();
+    return chain_launch(after, nv == 4 ? pd_reduce_pairs<4> : pd_reduce_pairs<1>, grid,
+                        PD_RED_THREADS, 0, st, slots, lptr, lidx, pairs, qv, frames, sh,
+                        residual_form, add_exact, chunk_sums, done, red);
 }
 
 cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdClassDev *cls,
@@ -3106,7 +3231,7 @@ cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdC
                             int32_t nv, int32_t n_frames, const double *qv,
                             const PdFrameDev *frames, const double2 *node_tab, const double *ffA,
                             const double *ffC, const double *ffW, int add_diag, double qmax, const int *err,
-                            double *terms, cudaStream_t st) {
+                            double *terms, cudaStream_t st, bool after) {
     const int64_t blocks =
         static_cast<int64_t>(n_frames) * ((sh.nq + PD_PROF_Q - 1) / PD_PROF_Q);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
@@ -3120,10 +3245,9 @@ cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdC
             kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
         if (e != cudaSuccess) return e;
     }
-    kern<<<static_cast<unsigned>(blocks), PD_PROF_THREADS, smem, st>>>(
-        red, lat_sums, cls, pairs, n_cls, sh, qv, frames, node_tab, ffA, ffC, ffW, add_diag, qmax,
-        err, terms);
-    return cudaGetLastError();
+    return chain_launch(after, kern, static_cast<unsigned>(blocks), PD_PROF_THREADS, smem, st, red,
+                        lat_sums, cls, pairs, n_cls, sh, qv, frames, node_tab, ffA, ffC, ffW,
+                        add_diag, qmax, err, terms);
 }
 
 cudaError_t launch_lattice(const double *xyz, const int32_t *perm, const PdLatDev *lat_dev,
@@ -3173,10 +3297,10 @@ cudaError_t launch_lattice_sums(const unsigned long long *hist, const PdLatDev *
 }
 
 cudaError_t launch_frame_mean(const double *terms, const double *fw, int32_t n_frames, int32_t nq,
-                              double *out, cudaStream_t st, bool normalize) {
+                              double *out, cudaStream_t st, bool normalize, bool after) {
     const int grid = (6 * nq + 127) / 128;
-    pd_frame_mean<<<grid, 128, 0, st>>>(terms, fw, n_frames, nq, normalize ? 1 : 0, out);
-    return cudaGetLastError();
+    return chain_launch(after, pd_frame_mean, grid, 128, 0, st, terms, fw, n_frames, nq,
+                        normalize ? 1 : 0, out);
 }
 
 cudaError_t launch_stream_accumulate(const double *batch, double scale, int32_t n, double *acc,

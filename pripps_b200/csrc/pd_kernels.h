@@ -17,13 +17,16 @@ int pairs_blocks_per_sm(int precision, int K, int NP, int mode);
 // stream capture included — has to.
 cudaError_t prepare_pair_kernels();
 
+// `after` of a launcher: the operation before it on the stream is one of these kernels
+// (chain_launch in pd_launch.cuh).
+//
 // n_jobs points to the tile count in device memory (read once per CTA).
 // plan_frames > 0: the jobs are those of one request (reqs[0]) with that many
 // frames, all of them (counter: two zeroed ints); 0: any jobs of any requests
 // (one).
 cudaError_t launch_pairs(int precision, int K, int NP, int mode, const PdJob *jobs,
                          const int *n_jobs, const PdReqDev *reqs, int *counter, int plan_frames,
-                         int grid, cudaStream_t st);
+                         int grid, cudaStream_t st, bool after = false);
 // The direction form's first stage, for the frames that take it; the other arguments
 // are those of launch_pairs (plan_frames > 0 uses the second counter). A variant holds
 // up to its number of moments (directions_variant of the most a frame may have).
@@ -31,26 +34,21 @@ int directions_variant(int precision, int32_t n_amp);
 int directions_blocks_per_sm(int variant);
 cudaError_t launch_directions(int variant, const PdJob *jobs, const int *n_jobs,
                               const PdReqDev *reqs, int *counter, int plan_frames, int grid,
-                              cudaStream_t st);
+                              cudaStream_t st, bool after = false);
 // Blocks per frame of the centroid kernel (3 partial sums each).
 int32_t centroid_blocks(int64_t n_atoms);
-// `done` (one counter per frame) must be zero; `status`, if given, is cleared.
-cudaError_t launch_centroid(const double *xyz, int64_t n_atoms, int n_frames, double *part,
-                            unsigned int *done, double *centroid, int32_t *status,
-                            cudaStream_t st);
-// rad2 and done (one per frame) must be zero; writes the frames' constants.
+// Centres the frames, packs their atoms in the classes' order and sets the frames'
+// constants; clears `status` if given. cent_done, done and rad2 (one per frame) must
+// be zero. `launches`: how many kernels it took.
 cudaError_t launch_pack(const double *xyz, const double *weights, const int32_t *perm,
-                        const double *centroid, int64_t n_atoms, int32_t n_pad, int32_t n_frames,
-                        float4 *out32, double4 *out64, const PdMomentRule &rule,
-                        unsigned long long *rad2, unsigned int *done, PdFrameDev *frames,
-                        double4 *dirs, double2 *node_tab, cudaStream_t st);
+                        int64_t n_atoms, int32_t n_pad, int32_t n_frames, double *part,
+                        unsigned int *cent_done, double *centroid, int32_t *status, float4 *out32,
+                        double4 *out64, const PdMomentRule &rule, unsigned long long *rad2,
+                        unsigned int *done, PdFrameDev *frames, double4 *dirs, double2 *node_tab,
+                        cudaStream_t st, int *launches);
 // The quadrature rules of the direction form on the current device (before any
 // launch_pack there, and before a stream capture).
 cudaError_t prepare_direction_rules();
-// Adds the chunk sums of each class up (needed where a class has more than one).
-cudaError_t launch_class_sums(double *slots, const PdFrameDev *frames, const PdAmpShape &sh,
-                              int n_frames, const int32_t *cls_ptr, const int32_t *cls_chunk,
-                              cudaStream_t st);
 // Direction form: class-pair sums at the nodes, from the chunks' moments, into
 // red (does nothing for frames in the other forms). part holds grp_cap·pairs·nv·
 // node_cap doubles per frame, done one zeroed counter per node tile and frame.
@@ -58,21 +56,21 @@ cudaError_t launch_direction_sums(const double *slots, const double4 *dirs,
                                   const PdFrameDev *frames, const PdAmpShape &sh, double qmax,
                                   int32_t n_frames, const PdClassDev *cls, const PdPairDev *pairs,
                                   int32_t n_pairs, const int32_t *cls_ptr,
-                                  const int32_t *cls_chunk, int32_t width, int add_exact,
-                                  double *part, unsigned int *done, double *red, cudaStream_t st);
+                                  const int32_t *cls_chunk, int32_t width,
+                                  int add_exact, double *part, unsigned int *done, double *red, cudaStream_t st, bool after = false);
 // Slot sums (red: [frame][pair][nv][width]); with n_chunk > 1, chunk_sums holds
 // 128·nv·n_chunk doubles and done one zeroed counter per (frame, pair, n_z).
 cudaError_t launch_reduce(const double *slots, const int64_t *lptr, const int64_t *lidx,
                           const PdPairDev *pairs, const double *qv, const PdFrameDev *frames,
                           const PdReduceShape &sh, int32_t nv, int32_t n_frames, int residual_form,
                           int add_exact, double *chunk_sums, unsigned int *done, double *red,
-                          cudaStream_t st);
+                          cudaStream_t st, bool after = false);
 cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdClassDev *cls,
                             const PdPairDev *pairs, int32_t n_cls, const PdReduceShape &sh,
                             int32_t nv, int32_t n_frames, const double *qv,
                             const PdFrameDev *frames, const double2 *node_tab, const double *ffA,
                             const double *ffC, const double *ffW, int add_diag, double qmax, const int *err,
-                            double *terms, cudaStream_t st);
+                            double *terms, cudaStream_t st, bool after = false);
 // Lattice sets: integer coordinates of their points and the exact pair count
 // per squared offset (after pack), then their self pair sums, sums[lattice][q].
 cudaError_t launch_lattice(const double *xyz, const int32_t *perm, const PdLatDev *lat_dev,
@@ -83,7 +81,7 @@ cudaError_t launch_lattice_sums(const unsigned long long *hist, const PdLatDev *
                                 const double *qv, int32_t nq, int add_exact, const int *err,
                                 const PdFrameDev *frames, double *sums, cudaStream_t st);
 cudaError_t launch_frame_mean(const double *terms, const double *fw, int32_t n_frames, int32_t nq,
-                              double *out, cudaStream_t st, bool normalize = true);
+                              double *out, cudaStream_t st, bool normalize = true, bool after = false);
 // Direct transform: (Re A, Im A, |A|², Σ_m |F_m|²) per q-vector for points
 // in molecules of mol_size (n_points a multiple of it). part holds
 // direct_chunks(n_points, mol_size, n_vec) × n_vec × 5 doubles; the launch

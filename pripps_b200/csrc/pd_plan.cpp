@@ -193,7 +193,10 @@ Tuning default_tuning(int64_t n_atoms, int64_t nq, int precision, int64_t n_fram
         // K = 64 holds the moments of q_max·d up to 85 in one block
         t.K = nq > 32 ? 64 : 32;
         t.NP = 1;
-        t.TJ = std::clamp(next_pow2(n_atoms / 16), 256, 4096);
+        // a CTA's pass over a j range is serial: short ranges fill the GPU on small
+        // structures (whole solves of 300 and 600 atoms: 91 and 110 µs at 256 j
+        // atoms, 70 and 82 µs at 64, 85 and 85 µs at 32)
+        t.TJ = std::clamp(next_pow2(n_atoms / 16), 64, 4096);
         return t;
     }
     // Measured on B200 (class mode): K = 128 with 4 pairs per thread (three
@@ -750,7 +753,8 @@ static bool direction_only(Plan &P) {
         const int64_t blocks = (m8 + P.mom.block - 1) / P.mom.block;
         if (m8 <= P.mom.max_moments && blocks <= P.nqb)
             use = P.dir_cost < 0.5 * static_cast<double>(P.n_atoms) * P.n_atoms *
-                                   (44.0 * blocks + 1.25 * m8);
+                                       (44.0 * blocks + 1.25 * m8) +
+                                   PD_PAIRS_LATENCY;
     }
     if (!use) {
         P.dir_only = false;
@@ -793,9 +797,10 @@ static void set_directions(Plan &P) {
     P.amp.n_chunk = static_cast<int32_t>(P.chunks.size());
     // Below 150 atoms the pairs are always fewer than the directions. The jobs
     // carry the work units, so every rank needs jobs of every frame. The test
-    // hook needs the pair tiles.
+    // hook (of the FP32 form) needs the pair tiles.
     if (P.n_atoms < 150 || P.jobs_per_frame < 2 * static_cast<int64_t>(P.world) ||
-        (P.world > 1 && P.n_frames > 1) || P.mom.block == 0 || P.test_expire)
+        (P.world > 1 && P.n_frames > 1) || P.mom.block == 0 ||
+        (P.test_expire && P.precision != PD_FP64))
         return;
     // unknown coordinates: 20 cubic Angstrom per atom, elongated up to about 2.5 : 1
     const double radius =

@@ -1,5 +1,5 @@
-"""Debye pair·q throughput on B200: FP32-recurrence kernel vs plain FP64, with
-the reference's CPU Debye (its FP64 restatement) timed beside it.
+"""Debye pair·q throughput on B200: FP32 form vs FP64 form, with the reference's
+CPU Debye (its FP64 restatement) timed beside it.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
                     [--workload ellipsoid_solvent_100k] [--precision fp32]
@@ -36,19 +36,6 @@ sys.path.insert(0, str(ROOT))
 
 METRIC = "Debye pair·q evals/s (FP32 recurrence, FP64 reduction)"
 UNIT = "pair·q/s"
-# FP32 flops of one pair·q in the inner loop. Class mode: the d-step (FFMA,
-# 2) and the v-step (FADD, 1) of the recurrence, and the accumulation — an add
-# of terms whose weight 1/r the recurrence state already carries (FADD, 1) when
-# Δq·(largest pair distance) <= π/4, else an FFMA with the weight (2).
-# Weighted mode (a weight per atom): the same step and a second accumulator
-# of the terms times w_j (FFMA, 2); with the general step both accumulations
-# are FFMAs with the weight.
-FLOPS_PER_PAIRQ = {"class": 4, "class_general_step": 5, "weighted": 6,
-                   "weighted_general_step": 7}
-# FP32 pipe slots (lane operations) of one pair·q: three with one
-# accumulator, four with two.
-SLOTS_PER_PAIRQ = {"class": 3, "class_general_step": 3, "weighted": 4,
-                   "weighted_general_step": 4}
 PROFILES = ("atoms", "excluded", "hydration", "atom_excluded", "atom_hydration",
             "excluded_hydration")
 
@@ -408,26 +395,19 @@ def run_ours(args, ws, rank, local):
         secondary = run_secondary(ctx, args, local)
 
     if rank == 0:
-        mode = kernel_mode(req)
-        flops = FLOPS_PER_PAIRQ[mode]
-        slots = SLOTS_PER_PAIRQ[mode]
+        # of one rank: the ranks share the directions (or the pairs' tiles)
+        work = executed_work(req)
         launch_ms = pair_ms.value / max(n_pair.value, 1)
-        # Pairs of a lattice set with itself are counted, not summed by the
-        # pair kernel (see pd_lattice): the roofline counts the kernel's pairs.
-        lat_pairs = 0
-        for lat in (req.lattices or []):
-            m = int(np.count_nonzero(req.species == lat[0]))
-            lat_pairs += m * (m - 1) // 2
-        kernel_pair_q = (w.pairs - lat_pairs) * req.nq * req.n_frames
-        achieved = flops * kernel_pair_q / (launch_ms * 1e-3) / 1e12
+        seconds = launch_ms * 1e-3
+        achieved = work["flop"] / ws / seconds / 1e12
+        slots = work["lane_ops"] / ws / seconds / 1e12
         peak = peak_ffma.value
         theoretical = 2 * 128 * 148 * (clk["sm_max_mhz"] or 1965.0) * 1e-6
-        # The fixed accounting constants of an angle-addition recurrence with
-        # one accumulator (vacuum, 8 FLOP) or four (six colocated profiles,
-        # 14 FLOP) per pair·q; this kernel executes `flops` per pair·q.
+        # A recurrence with one accumulator (vacuum, 8 FLOP) or four (six
+        # colocated profiles, 14 FLOP) would execute this per pair·q.
         solvent = req.ff_excluded is not None or req.hyd_weights is not None
         fixed = 14 if solvent else 8
-        fixed_achieved = fixed * kernel_pair_q / (launch_ms * 1e-3) / 1e12
+        fixed_achieved = fixed * w.pair_q / ws / seconds / 1e12
         cpu = None
         if not args.no_cpu and ws == 1:  # the host-core baseline is an N = 1 figure
             rate, pq, dt, sample, used = cpu_sample(w, args.cpu_atoms, args.cpu_q)
@@ -447,20 +427,15 @@ def run_ours(args, ws, rank, local):
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak,
                          "traffic": load_traffic(w.name),
-                         "kernel": "pd_pairs_fp32", "flops_per_pair_q": flops,
+                         "kernel": "pd_directions_fp32" if work["form"] == "directions"
+                                   else "pd_pairs_fp32",
+                         "executed": work,
                          "fp32_pipe": {
-                             "lane_ops_per_pair_q": slots,
-                             "achieved_tops": slots * kernel_pair_q / (launch_ms * 1e-3) / 1e12,
-                             "peak_tops": peak / 2.0,
-                             "frac": slots * kernel_pair_q / (launch_ms * 1e-3) / 1e12 /
-                                     (peak / 2.0),
-                             "note": "the kernel is bound by FP32 pipe slots: each pair·q "
-                                     f"takes {slots} FP32 lane operations ({mode} mode) "
-                                     f"for {flops} FLOP; an FADD fills a slot for 1 FLOP, "
-                                     "so the FLOP fraction tops out at "
-                                     f"{flops}/{2 * slots} of the FFMA peak and the slot "
-                                     "fraction at 1"},
-                         "kernel_pair_q_per_launch": kernel_pair_q,
+                             "achieved_tops": slots, "peak_tops": peak / 2.0,
+                             "frac": slots / (peak / 2.0),
+                             "note": "the kernel is bound by FP32 pipe slots (lane operations); "
+                                     "an operation that is no multiply-add fills a slot for 1 "
+                                     "FLOP"},
                          "kernel_ms_per_launch": launch_ms,
                          "peak_source": "measured FFMA probe (pd_measure_fp32_peak), best of "
                                         "3 in this run",
@@ -471,11 +446,10 @@ def run_ours(args, ws, rank, local):
                              "flops_per_pair_q": fixed, "achieved": fixed_achieved,
                              "frac_of_measured": fixed_achieved / peak,
                              "note": "recurrence-equivalent FLOP rate: a kernel doing the "
-                                     "textbook angle-addition step plus one accumulator per "
-                                     "profile term would need this rate; this kernel executes "
-                                     f"{flops} FLOP per pair·q (species-class factoring, "
-                                     "Reinsch form, weights carried in the recurrence), so "
-                                     "the figure exceeds the FP32 peak"}},
+                                     "textbook angle-addition step for every pair and grid "
+                                     "point would need this rate; the class amplitudes over "
+                                     "directions do N·S·M terms instead of N²/2·nq, so the "
+                                     "figure exceeds the FP32 peak"}},
             "fp64_kernel": fp64,
             "parity": parity,
             "cpu_baseline": cpu,
@@ -496,21 +470,43 @@ def run_ours(args, ws, rank, local):
         torch.distributed.destroy_process_group()
 
 
-def kernel_mode(req):
-    """The pair kernel's mode for a request, as the planner picks it: class
-    mode while at most 48 (species, hydration weight) keys exist, else
-    weighted; "_general_step" where Δq·2·(largest distance from the
-    centroid) > 0.78."""
-    mode = "class"
+def executed_work(req):
+    """What a solve of the FP32 form executes for its pairs, as the planner and
+    pd_pack choose it: the form, and its FP32 lane operations and FLOP.
+
+    Directions: S directions × N atoms (twice with a weight per atom), 14 lane
+    operations (26 FLOP) to start an atom's cosines and 10 (20 FLOP) for each
+    eight of its M moments, 44 more for each later block of 128. Pairs: 44 and
+    1.25 per moment (2.5 FLOP) for each of the N(N−1)/2 pairs."""
+    weighted = False
     if req.hyd_weights is not None:
-        keys = set(zip(req.species.tolist(), req.hyd_weights.tolist()))
-        mode = "weighted" if len(keys) > 48 else "class"
-    xyz = req.xyz.reshape(-1, req.n_atoms, 3)
-    radius = max(float(np.sqrt(((f - f.mean(axis=0)) ** 2).sum(axis=1)).max()) for f in xyz)
-    dq = (req.qmax - req.qmin) / max(req.nq - 1, 1)
-    if dq * 2.0 * radius > 0.78:
-        mode += "_general_step"
-    return mode
+        weighted = len(set(zip(req.species.tolist(), req.hyd_weights.tolist()))) > 48
+    n = req.n_atoms
+    ops = flop = 0.0
+    forms, sizes = set(), None
+    for f in req.xyz.reshape(-1, n, 3):
+        radius = float(np.sqrt(((f - f.mean(axis=0)) ** 2).sum(axis=1)).max())
+        z = 2.0 * radius * req.qmax
+        top = z + 8.0 * np.cbrt(0.5 * z) + 2.0
+        h = int(top / 4.0) + 1
+        x = np.polynomial.legendre.leggauss(2 * h)[0][h:]
+        ring = z * np.sqrt(1.0 - x * x)
+        S = int(np.maximum(4, (ring + 8.0 * np.cbrt(0.5 * ring) + 2.0).astype(int) + 1).sum())
+        z1 = 1.03 * radius * req.qmax
+        M = (int(z1 + 8.0 * np.cbrt(0.5 * z1) + 2.0) + 8) // 8 * 8
+        zp = 2.0 * z1
+        Mp = (int(0.5 * (zp + 9.7 * np.cbrt(0.5 * zp) + 3.5)) + 8) // 8 * 8
+        blocks = (M + 127) // 128
+        d = S * n * (2 if weighted else 1)
+        d_ops, d_flop = d * (44 * blocks - 30 + 1.25 * M), d * (60 * blocks - 34 + 2.5 * M)
+        p_ops, p_flop = 0.5 * n * n * (44 + 1.25 * Mp), 0.5 * n * n * (60 + 2.5 * Mp)
+        direct = d_ops < p_ops + 1e7 and n >= 150
+        forms.add("directions" if direct else "pairs")
+        sizes = {"directions": S, "moments": M} if direct else {"moments": Mp}
+        ops += d_ops if direct else p_ops
+        flop += d_flop if direct else p_flop
+    return {"form": "+".join(sorted(forms)), "weighted": weighted, "lane_ops": ops, "flop": flop,
+            **sizes}
 
 
 def timed_workload(ctx, w, local, min_seconds=2.0):
@@ -603,7 +599,7 @@ def run_secondary(ctx, args, local):
         if name != args.workload:
             w = workloads.WORKLOADS[name](args.precision)
             out[name] = timed_workload(ctx, w, local)
-            out[name]["kernel_mode"] = kernel_mode(w.request)
+            out[name]["executed"] = executed_work(w.request)
     out["serving_burst_400"] = serving_burst(ctx, local, 400, args.precision)
     return out
 

@@ -68,8 +68,8 @@ extern "C" {
 #define PD_FLAG_TEST_EXPIRED_WAIT 0x80000000u
 
 /* ---- precision forms ---- */
-#define PD_FP32_FP64RED 0 /* FP32 recurrence sinc, FP32 per-tile sums, FP64 reduction */
-#define PD_FP64 1         /* plain FP64 sinc and accumulation throughout */
+#define PD_FP32_FP64RED 0 /* FP32 terms and short sums, FP64 reduction */
+#define PD_FP64 1         /* FP64 terms and accumulation throughout */
 
 /* ---- output layout ---- */
 #define PD_NUM_TERMS 6 /* rows of the [6][nq] output, see above */
@@ -343,7 +343,7 @@ int pd_combine(const double *terms, uint64_t nq, double volume_scale,
 const char *pd_last_error(pd_ctx *ctx);
 
 /* Kernel shapes. Every solve, plan, stream and request of the loop picks
- * its shape — the q-block length K of the recurrence (FP32: 32, 64, 96, 128,
+ * its shape — the q-block length K of the pair kernels (FP32: 32, 64, 96, 128,
  * 160, 192; FP64: 16, 32, and 64 in class mode), the atom-chunk length of a tile (multiple of 32)
  * and the pairs each thread advances together (FP32: 1, 2 or 4) — from the
  * context's tuning table by the request's bucket: (precision, accumulation
@@ -394,7 +394,9 @@ int pd_plan_inspect(pd_ctx *ctx, const pd_request *req, uint64_t *n_classes,
                     uint64_t *n_padded, uint64_t *n_tiles, uint64_t *pairs_covered);
 
 /* Host-only: device bytes one solve of `req` holds with the tuning the
- * context would pick (ctx may be NULL: default tuning). host_coordinates != 0
+ * context would pick (ctx may be NULL: default tuning), in the form that sums
+ * pairs: a request that needs more than the budget allows is refused. (A solve
+ * that sums directions instead holds its own arrays, where those fit too.) host_coordinates != 0
  * counts the device copy of the coordinates that pd_solve and pd_submit make;
  * 0 is the layout of a plan execution or of pd_solve_noalloc, whose
  * coordinates are the caller's device memory. No reference counterpart. */
@@ -443,7 +445,7 @@ uint64_t pd_launch_count(pd_ctx *ctx);
  *    the tuning table picks for the request's bucket as well as on N and
  *    nq. As a guide, at nq = 1,000 an FP32 solve with solvent and one
  *    hydration weight per element fits up to roughly 130,000 atoms (the
- *    100,000-atom ellipsoid needs 49 MB) and 200,000 atoms are refused;
+ *    100,000-atom ellipsoid needs 53 MB) and 200,000 atoms are refused;
  *    with a hydration weight per atom (four partial sums per grid point)
  *    up to about 20,000 atoms fit, and larger requests may not.
  *  - The array occupies PD_NOALLOC_SCRATCH_BYTES of memory on every GPU that

@@ -1339,6 +1339,30 @@ __device__ __forceinline__ int ring_points(double z_sin, bool fp64) {
     return max(4, static_cast<int>(direction_order(z_sin, fp64)) + 1);
 }
 
+// The direction of length sqrt(len2) in FP32: of the eight roundings of its components
+// the one whose length is nearest. Each to nearest would stretch all distances along
+// the direction by up to 6e-8 — and a ring's directions share their z —, which the
+// moments, expanded for the exact length, cannot tell from another structure; a
+// turn by as much is harmless. (10,000-atom sphere against FP64: 2-norm error 5.4e-9 ->
+// 7.6e-10, largest error of a profile point 6.8e-7 -> 1.5e-7.)
+__device__ __forceinline__ double4 round_direction(double4 d, double len2) {
+    const double lo[3] = {__double2float_rd(d.x), __double2float_rd(d.y), __double2float_rd(d.z)};
+    const double hi[3] = {__double2float_ru(d.x), __double2float_ru(d.y), __double2float_ru(d.z)};
+    double best = 1e300;
+    double4 r = d;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const double x = (k & 1) ? hi[0] : lo[0], y = (k & 2) ? hi[1] : lo[1],
+                     z = (k & 4) ? hi[2] : lo[2];
+        const double e = fabs(fma(x, x, fma(y, y, fma(z, z, -len2))));
+        if (e < best) {
+            best = e;
+            r = make_double4(x, y, z, d.w);
+        }
+    }
+    return r;
+}
+
 // A frame's constants (PdFrameDev) from its radius: which form its pairs are summed
 // in, the expansion's size, and the direction table, whose entries the n_part blocks
 // share. T threads, all of each block.
@@ -1439,6 +1463,7 @@ __device__ __forceinline__ void frame_constants(double radius, const PdMomentRul
                 double sn, cs;
                 sincospi(2.0 * (s - s_off[lo]) / n, &sn, &cs);
                 d = make_double4(st * cs, st * sn, nw.x * sc, nw.y / n);
+                if (!fp64) d = round_direction(d, sc * sc);
             }
             o[s] = d;
         }

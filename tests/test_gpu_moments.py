@@ -197,3 +197,36 @@ def test_frames_of_both_forms_share_a_batch(gpu_ctx, precision):
     tol = 1e-12 if precision == "fp64" else 1e-5
     assert np.all(term_errors(s.finish(), want) < tol)
     assert np.all(term_errors(solve(req(frames, weights), gpu_ctx), want) < tol)
+
+
+@pytest.mark.parametrize("n", [120, 900, 17000])
+def test_plan_execution_replays_from_a_graph(gpu_ctx, n):
+    """A plan's chained kernels (pairs; directions; the separate centroid and pack
+    kernels above 16,384 atoms) captured into a CUDA graph: every replay gives the
+    direct execution's result for the coordinates of that moment, bit for bit."""
+    import torch
+
+    from pripps_b200.shard import ShardedPlan
+    w = workloads.small_globule(min(n, 2000), 6, nq=50, precision="fp32").request
+    if n > 2000:
+        rng = np.random.default_rng(n)
+        xyz = rng.uniform(-25.0, 25.0, (n, 3))
+        w = _request(xyz, 50, 0.0, 0.3, "fp32", "vacuum", n)
+    plan = ShardedPlan(w, gpu_ctx, 0, 1)
+    try:
+        xyz = torch.tensor(w.xyz, device="cuda")
+        want = plan.execute(xyz).clone()
+        moved = xyz * 1.03
+        want2 = plan.execute(moved).clone()
+        buf, s = xyz.clone(), torch.cuda.Stream()
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            out = plan.execute(buf)
+        for src, ref in ((xyz, want), (moved, want2), (xyz, want)):
+            buf.copy_(src)
+            g.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(out, ref)
+    finally:
+        plan.close()

@@ -433,7 +433,8 @@ def run_ours(args, ws, rank, local):
             "gpu_launches": int(launches),
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak,
-                         "traffic": load_traffic(w.name),
+                         # (measured for the pair kernels only)
+                         "traffic": load_traffic(w.name) if work["form"] == "pairs" else None,
                          "kernel": "pd_directions_fp32" if work["form"] == "directions"
                                    else "pd_pairs_fp32",
                          "executed": work,

@@ -810,7 +810,8 @@ static void set_directions(Plan &P) {
     const bool fp64 = P.precision == PD_FP64;
     auto order = [&](double z) { return series_order(z, fp64); };
     const double z = 2.0 * radius * P.qmax;
-    const double top = order(z), mo = order(1.03 * radius * P.qmax);
+    const double r1 = std::max(1.03 * radius, 1e-6);  // (as pd_pack bounds it)
+    const double top = order(z), mo = order(r1 * P.qmax);
     if (!(top < 500.0) || !(mo < PD_MAX_DIR_MOMENTS - 8.0)) return;
     const int h = static_cast<int>(top * 0.25) + 1;
     int64_t S = 0;
@@ -818,7 +819,7 @@ static void set_directions(Plan &P) {
         S += std::max(4, static_cast<int>(order(z * std::sin(M_PI * (i + 0.75) / (2 * h + 0.5)))) + 2);
     const int64_t groups = (S + 31) / 32, mine = (groups + P.world - 1) / P.world;
     const int64_t m8 = (static_cast<int64_t>(mo) + 8) & ~int64_t{7};
-    const double zn = 2.0 * 1.03 * radius * P.qmax;
+    const double zn = 2.0 * r1 * P.qmax;
     const int64_t nodes = static_cast<int64_t>(0.5 * series_order(zn, true)) + 1;
     // The sums' kernel: a block's shared memory holds the coefficients and the
     // amplitudes of every class at a tile of nodes (16, or fewer while that leaves

@@ -230,3 +230,11 @@ def test_plan_execution_replays_from_a_graph(gpu_ctx, n):
             assert torch.equal(out, ref)
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_coincident_points_at_large_q(gpu_ctx, precision):
+    """A radius of zero: the expansion's own radius is bounded from below, on the
+    host that sizes the tables as on the device that fills them."""
+    xyz = np.full((300, 3), 1.5)
+    _check(_request(xyz, 4, 0.0, 5e4, precision, "vacuum", 2), gpu_ctx, precision)

@@ -1995,15 +1995,25 @@ __device__ double moment_coefficients(double z, int n_mom, double *__restrict__ 
 // Σ sinc(q r) (read, formed from the moments, or interpolated from the nodes),
 // times the class factors, all in FP64. 32 groups of eight threads (one per
 // grid point) share the class pairs, and where there are fewer pairs than
-// groups also the moments; their partial profiles are added in a fixed order. The class
-// factors and the rows of as many pairs as fit are staged in shared memory
-// with all loads in flight.
+// groups also the moments; their partial profiles are added in a fixed order. The rows
+// of as many pairs as fit are staged in shared memory with all loads in flight,
+// and so are the class factors (STAGED) unless there are too many classes for
+// that: the species are not bounded, only (species, weight) classes are. Then
+// they are read where they are used (from L2; profile_smem draws the line).
 constexpr int PD_PROF_Q = 8;
 constexpr int PD_PROF_THREADS = 256;
 constexpr int PD_PROF_GROUPS = PD_PROF_THREADS / PD_PROF_Q;
 constexpr int PD_PROF_ROWS = 2048;  // doubles of pair rows staged at once
+constexpr size_t PD_PROF_SMEM = 64 * 1024;
 
-template <int NV>
+// Its shared memory: pair rows, class factors and the coefficients of the most
+// moments a frame may have (up to 16, 9 for 48 classes, and 32 KB).
+static size_t profile_smem(const PdReduceShape &sh, int32_t n_cls_staged) {
+    return (PD_PROF_ROWS + static_cast<size_t>(n_cls_staged) * 3 * PD_PROF_Q +
+            static_cast<size_t>(sh.max_moments) * PD_PROF_Q) * sizeof(double);
+}
+
+template <int NV, bool STAGED>
 __global__ void __launch_bounds__(PD_PROF_THREADS)
     pd_profiles(const double *__restrict__ red, const double *__restrict__ lat_sums,
                 const PdClassDev *__restrict__ cls, const PdPairDev *__restrict__ pairs,
@@ -2018,7 +2028,7 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
     __shared__ double s_sum[PD_PROF_THREADS / 32][6][PD_PROF_Q];
     double *s_row = s_dyn;                                 // [pair][nv][M]
     double *s_fac = s_row + PD_PROF_ROWS;                  // [class][A, C, B][PD_PROF_Q]
-    double *s_coef = s_fac + n_cls * 3 * PD_PROF_Q;        // [M][PD_PROF_Q]
+    double *s_coef = s_fac + (STAGED ? n_cls * 3 * PD_PROF_Q : 0);  // [M][PD_PROF_Q]
     const int n_qt = (sh.nq + PD_PROF_Q - 1) / PD_PROF_Q;
     const int f = blockIdx.x / n_qt;
     const int ql = threadIdx.x % PD_PROF_Q, g = threadIdx.x / PD_PROF_Q;
@@ -2038,9 +2048,8 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
         }
     };
     stage_rows(0, fit);
-    for (int k = threadIdx.x; k < n_cls * 3 * PD_PROF_Q; k += PD_PROF_THREADS) {
-        const int c = k / (3 * PD_PROF_Q), w = k / PD_PROF_Q % 3;
-        const int qq = q - ql + k % PD_PROF_Q;
+    // factor w (atom, excluded, hydration) of class c at grid point qq
+    auto factor = [&](int c, int w, int qq) {
         double v = 0.0;
         if (qq < sh.nq) {
             const int64_t at = static_cast<int64_t>(cls[c].species) * sh.nq + qq;
@@ -2048,8 +2057,15 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
             if (w == 1 && ffC) v = ffC[at];
             if (w == 2 && ffW) v = weighted ? ffW[qq] : cls[c].w * ffW[qq];
         }
-        s_fac[k] = v;
-    }
+        return v;
+    };
+    if constexpr (STAGED)
+        for (int k = threadIdx.x; k < n_cls * 3 * PD_PROF_Q; k += PD_PROF_THREADS)
+            s_fac[k] = factor(k / (3 * PD_PROF_Q), k / PD_PROF_Q % 3, q - ql + k % PD_PROF_Q);
+    auto own_factor = [&](int c, int w) {
+        if constexpr (STAGED) return s_fac[(c * 3 + w) * PD_PROF_Q + ql];
+        return factor(c, w, q);
+    };
     const double qval = ok ? qv[q] : 0.0;
     if (nodes) {
         // interpolation from the Chebyshev nodes y_k = cos((2k+1)π/2M) of
@@ -2113,8 +2129,7 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
     if (add_diag) {  // i = j terms
         for (int c = g; c < n_cls; c += PD_PROF_GROUPS) {
             const PdClassDev cl = cls[c];
-            const double *fc = s_fac + c * 3 * PD_PROF_Q + ql;
-            const double fa = fc[0], ca = fc[PD_PROF_Q], b = fc[2 * PD_PROF_Q];
+            const double fa = own_factor(c, 0), ca = own_factor(c, 1), b = own_factor(c, 2);
             AA += cl.n * fa * fa;
             CC += cl.n * ca * ca;
             AC += cl.n * fa * ca;
@@ -2168,10 +2183,9 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
                                    (add_diag ? pr.q0[v] : 0.0) - 0.5 * (r[v * M + 6] - r[v * M + 7]),
                                    s[v]);
             }
-            const double *fa_ = s_fac + pr.a * 3 * PD_PROF_Q + ql,
-                         *fb_ = s_fac + pr.b * 3 * PD_PROF_Q + ql;
-            const double fa = fa_[0], fb = fb_[0], ca = fa_[PD_PROF_Q], cb = fb_[PD_PROF_Q];
-            const double ba = fa_[2 * PD_PROF_Q], bb = fb_[2 * PD_PROF_Q];
+            const double fa = own_factor(pr.a, 0), fb = own_factor(pr.b, 0);
+            const double ca = own_factor(pr.a, 1), cb = own_factor(pr.b, 1);
+            const double ba = own_factor(pr.a, 2), bb = own_factor(pr.b, 2);
             AA += 2.0 * fa * fb * s[0];
             CC += 2.0 * ca * cb * s[0];
             AC += (fa * cb + ca * fb) * s[0];
@@ -3260,14 +3274,14 @@ cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdC
     const int64_t blocks =
         static_cast<int64_t>(n_frames) * ((sh.nq + PD_PROF_Q - 1) / PD_PROF_Q);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-    // pair rows, class factors, and the coefficients of the most moments a frame
-    // may have: at most 16 + 9 + 32 KB
-    const size_t smem = (PD_PROF_ROWS + static_cast<size_t>(n_cls) * 3 * PD_PROF_Q +
-                         static_cast<size_t>(sh.max_moments) * PD_PROF_Q) * sizeof(double);
-    auto kern = nv == 4 ? pd_profiles<4> : pd_profiles<1>;
+    size_t smem = profile_smem(sh, n_cls);
+    const bool staged = smem <= PD_PROF_SMEM;
+    if (!staged) smem = profile_smem(sh, 0);
+    auto kern = nv == 4 ? (staged ? pd_profiles<4, true> : pd_profiles<4, false>)
+                        : (staged ? pd_profiles<1, true> : pd_profiles<1, false>);
     if (smem > 44 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(
-            kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+            kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(PD_PROF_SMEM));
         if (e != cudaSuccess) return e;
     }
     return chain_launch(after, kern, static_cast<unsigned>(blocks), PD_PROF_THREADS, smem, st, red,

@@ -718,11 +718,12 @@ static void set_chunks(Plan &P) {
         return x.j1 - x.j0 > y.j1 - y.j0;
     });
     P.cls_ptr.assign(P.n_cls + 1, 0);
-    for (int k = 0; k < P.n_cls; ++k) {
-        for (size_t t = 0; t < P.chunks.size(); ++t)
-            if (P.chunks[t].cls == k) P.cls_chunk.push_back(static_cast<int32_t>(t));
-        P.cls_ptr[k + 1] = static_cast<int32_t>(P.cls_chunk.size());
-    }
+    for (const PdChunk &ck : P.chunks) ++P.cls_ptr[ck.cls + 1];
+    std::partial_sum(P.cls_ptr.begin(), P.cls_ptr.end(), P.cls_ptr.begin());
+    P.cls_chunk.resize(P.chunks.size());
+    std::vector<int32_t> next(P.cls_ptr.begin(), P.cls_ptr.end() - 1);
+    for (size_t t = 0; t < P.chunks.size(); ++t)
+        P.cls_chunk[next[P.chunks[t].cls]++] = static_cast<int32_t>(t);
 }
 
 // A plan without tiles, where the frames' exact radius (radius_hint, the largest

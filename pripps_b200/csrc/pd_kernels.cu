@@ -738,11 +738,11 @@ __device__ __forceinline__ void pairs_range_x2w(const float4 *__restrict__ at, i
 #define PD_JFLUSH 512
 #endif
 // The same for the moments: their low orders are sums of nearly equal terms at
-// every grid point, so the rounding of long runs shows at the deep minima of a
-// profile (10,000 atoms, 512 pairs: 3.0e-5 of the minimum; 128 pairs: 9.5e-6, for
-// 3 % of the pair kernel's time).
+// every grid point, so the rounding of long runs shows in the profile (largest error
+// of a point against FP64, 8,000 atoms, q_max·d = 247: 1.1e-6 with 128 pairs, 4e-7 with
+// 32; the grid points 2e-7). The shorter runs and their flushes cost 5 to 12 %.
 #ifndef PD_MOM_FLUSH
-#define PD_MOM_FLUSH 128
+#define PD_MOM_FLUSH 32
 #endif
 // j atoms per bulk copy into shared memory (two buffers of PD_JSTAGE float4,
 // 64 KB of dynamic shared memory per CTA); a multiple of PD_JFLUSH. One CTA
@@ -796,6 +796,43 @@ __device__ __forceinline__ void flush_class(float2 (&acc)[NT], double *__restric
     }
 }
 
+// The same for moments: the lanes' sums meet in FP32 up to four of them, the rest in
+// FP64 (low moments are sums of equal terms: all five levels in FP32 cost as much
+// accuracy as runs four times as long).
+template <int NT>
+__device__ __forceinline__ void flush_moments(float2 (&acc)[NT], double *__restrict__ part,
+                                              int lane, bool first) {
+#pragma unroll
+    for (int lev = 0; lev < 2; ++lev) {  // reduce-scatter, as warp_reduce_scatter
+        const int o = 16 >> lev, h = (NT >> lev) / 2;
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const float2 keep = up ? acc[k + h] : acc[k], send = up ? acc[k] : acc[k + h];
+            acc[k] = __fadd2_rn(keep, make_float2(__shfl_xor_sync(0xffffffffu, send.x, o),
+                                                  __shfl_xor_sync(0xffffffffu, send.y, o)));
+        }
+    }
+    double v[NT / 2];
+#pragma unroll
+    for (int k = 0; k < NT / 2; ++k) v[k] = static_cast<double>((k & 1) ? acc[k / 2].y : acc[k / 2].x);
+#pragma unroll
+    for (int lev = 0; lev < 3; ++lev) {
+        const int o = 4 >> lev, h = (NT >> lev) / 4;
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int k = 0; k < h; ++k) {
+            const double keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < NT / 16; ++m) {  // values [l·NT/16, (l + 1)·NT/16) in lane l
+        double &d = part[lane * (NT / 16) + m];
+        d = (first ? 0.0 : d) + v[m];
+    }
+}
+
 // The j range and moment block of a moment-form job (see PdFrameDev): part
 // qb / n_mblk of the tile's range, cut at multiples of 32 atoms from its start.
 struct MomJob {
@@ -813,7 +850,7 @@ __device__ __forceinline__ MomJob moment_job(int j0, int j1, int qb, int n_mblk,
 
 // Weighted-mode flush of one accumulator array: the warp sums of acc and of
 // w_i·acc, added to part[k] and part[stride + k].
-template <int K>
+template <int K, bool MOMENTS>
 __device__ __forceinline__ void flush_weighted(float2 (&acc)[K / 2], float wi,
                                                double *__restrict__ part, int stride, int lane,
                                                bool first) {
@@ -821,8 +858,13 @@ __device__ __forceinline__ void flush_weighted(float2 (&acc)[K / 2], float wi,
     float2 tw[K / 2];
 #pragma unroll
     for (int t = 0; t < K / 2; ++t) tw[t] = __fmul2_rn(wi2, acc[t]);
-    flush_class<K / 2>(acc, part, lane, first);
-    flush_class<K / 2>(tw, part + stride, lane, first);
+    if constexpr (MOMENTS) {
+        flush_moments<K / 2>(acc, part, lane, first);
+        flush_moments<K / 2>(tw, part + stride, lane, first);
+    } else {
+        flush_class<K / 2>(acc, part, lane, first);
+        flush_class<K / 2>(tw, part + stride, lane, first);
+    }
 }
 
 // End of a tile: the warps' FP64 partial sums (part[w·nvk + e], e < nvk) of
@@ -1004,7 +1046,7 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
                             float2 none[1];
                             moments_range<KM, false>(chunk, jss, pi, i, ivalid, js, je, inv_d2, nj,
                                                      mblk, DBL, acc0, none);
-                            flush_class<KM / 2>(acc0, part, lane, first);
+                            flush_moments<KM / 2>(acc0, part, lane, first);
                         } else {
                             float2 acc1[KM / 2];
 #pragma unroll
@@ -1012,8 +1054,8 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
                             moments_range<KM, true>(chunk, jss, pi, i, ivalid, js, je, inv_d2, nj,
                                                     mblk, DBL, acc0, acc1);
                             const float wi = ivalid ? pi.w : 0.0f;
-                            flush_weighted<KM>(acc0, wi, part, K, lane, first);
-                            flush_weighted<KM>(acc1, wi, part + 2 * K, K, lane, first);
+                            flush_weighted<KM, true>(acc0, wi, part, K, lane, first);
+                            flush_weighted<KM, true>(acc1, wi, part + 2 * K, K, lane, first);
                         }
                     } else if constexpr (PACKED) {
                         const float2 *q2 = reinterpret_cast<const float2 *>(s_qres);
@@ -1081,8 +1123,8 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
                         // the four warp sums of each grid point: Σ acc0,
                         // Σ w_i·acc0, Σ acc1, Σ w_i·acc1
                         const float wi = ivalid ? pi.w : 0.0f;
-                        flush_weighted<K>(acc0, wi, part, K, lane, first);
-                        flush_weighted<K>(acc1, wi, part + 2 * K, K, lane, first);
+                        flush_weighted<K, false>(acc0, wi, part, K, lane, first);
+                        flush_weighted<K, false>(acc1, wi, part + 2 * K, K, lane, first);
                     } else {
                         const float wi = ivalid ? pi.w : 0.0f;
                         float acc[NACC][K];
@@ -1319,9 +1361,10 @@ __global__ void __launch_bounds__(PD_CENT_THREADS)
 // frame's last block turns it into the frame's constants (PdFrameDev): which form
 // its pairs are summed in, the expansion's size and the direction table.
 //
-// The rule counts FP32 lane operations: a pair costs about 44 for its sequences (in
-// each moment block) and 1.25 per moment, an atom in one direction 14 (44 more for each
-// later block) and 1.25 per moment, a direction also n_cls·M terms per node in FP64;
+// The rule counts FP32 lane operations: a pair costs about 44 for its sequences and 12
+// for its share of the flushes (in each moment block) and 1.5 per moment, an atom in
+// one direction 14 (44 more for each later block) and 1.25 per moment, a direction
+// also n_cls·M terms per node in FP64;
 // PD_PAIRS_LATENCY stands for the pair form's longer chain of short kernels.
 // Whole solves on both sides (vacuum; pairs / directions, µs): FP32, q_max 0.5, 200 /
 // 300 / 600 / 1,200 atoms 68/65, 80/66, 83/70, 90/84, q_max 1.0 71/75, 84/72, 89/82,
@@ -1392,7 +1435,7 @@ __device__ __forceinline__ void frame_constants(double radius, const PdMomentRul
             fr.n_mblk = blocks;
             fr.n_parts = rule.nqb / blocks;
             pair_cost = 0.5 * static_cast<double>(rule.n_atoms) * rule.n_atoms *
-                        (44.0 * blocks + 1.25 * m8);
+                        (56.0 * blocks + 1.5 * m8);
         }
     }
     // ---- directions: 2h Gauss rings (upper half: h), enough points on each
@@ -2112,11 +2155,9 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
         // hi = 8j + 4 + t
         for (int j = g; j < M / 8; j += PD_PROF_GROUPS) {
             double c[8];
-            // the tiles' sums carry the signs + + − − of their group within the block
-            const double sg = (j % (sh.block / 8)) & 2 ? -0.5 : 0.5;
 #pragma unroll
             for (int n = 0; n < 8; ++n)
-                c[n] = sg * s_scale[ql] * s_coef[(8 * j + n) * PD_PROF_Q + ql];
+                c[n] = 0.5 * s_scale[ql] * s_coef[(8 * j + n) * PD_PROF_Q + ql];
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 s_coef[(8 * j + 2 * t) * PD_PROF_Q + ql] = c[3 - t] + c[4 + t];

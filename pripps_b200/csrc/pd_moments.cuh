@@ -23,10 +23,18 @@
 //
 // the four b of a pair are computed once, and the pair (cos cφ, sin cφ) is turned
 // by 8φ from j to j + 1. One packed FFMA2 per (j, t) then accumulates two
-// moments: 8 lane operations per 8 moments, plus 4 for the turn, against 3 per
+// moments: 8 lane operations per 8 moments, plus 4 for the turn (12 in all), against 3 per
 // grid point in the direct form. The sines and cosines are kept divided by
 // sin(φ/2) and cos(φ/2) in the long sequence (X, Y) and multiplied by them in
 // the short one, which removes both square roots.
+//
+// The turn has full relative accuracy too: it is the sine, not the cosine, that is
+// doubled (sin²2θ = 4 sin²θ cos²θ), and the steps are Reinsch differences in
+// 4·sin²4φ = 2 − 2cos 8φ. In a long structure the close pairs have a small 8φ; a
+// cosine of it rounded near 1 is a phase error of one sign for all of them
+// (cos 8φ by three doublings of cos φ and a plain three-term recurrence: rods of
+// 5,000 atoms, q_max·d = 258, and 6,000 atoms, 930: largest relative error of I(q)
+// 1.3e-5 and 3.8e-5, root mean square 6e-6 and 1e-5).
 //
 // Direction form. The sum over all pairs is an average over directions,
 //
@@ -72,54 +80,39 @@ __device__ __forceinline__ double direction_order(double z, bool fp64) {
     return fp64 ? bessel_order(z, 13.0, 3.0) : bessel_order(z, 8.0, 2.0);
 }
 
-// A pair's sequences. U_j = (cos(cφ)/cos(φ/2), sin(cφ)/sin(φ/2)) at c = 8j + 3.5
-// follows the three-term recurrence U_{j+1} = 2cos(8φ)·U_j − U_{j−1}. It is kept
-// as W_j = s_j·U_j with the signs s = + + − − + + − − …, which turns every step into one
-// multiply-add, W_{j+1} = ±2cos(8φ)·W_j + W_{j−1} (+ for even j): no negation, no
-// half swapped, the older of the two registers overwritten. V_t = (2cos((t+½)φ)cos(φ/2),
-// −2sin((t+½)φ)sin(φ/2)), so that U.x·V.x = m_{c+b} + m_{c−b}, U.y·V.y =
-// m_{c+b} − m_{c−b}.
+// A pair's sequences. U_j = (cos(cφ)/cos(φ/2), sin(cφ)/sin(φ/2)) at c = 8j + 3.5 steps by
+// U_{j+1} = U_j + D_j, D_{j+1} = D_j − 4sin²4φ·U_{j+1}.
+// V_t = (2cos((t+½)φ)cos(φ/2), −2sin((t+½)φ)sin(φ/2)), so that U.x·V.x = m_{c+b} + m_{c−b},
+// U.y·V.y = m_{c+b} − m_{c−b}.
 struct MomPair {
-    float2 w0, w1;  // W at the first two j of the block
-    float cc;       // 2cos(8φ)
+    float2 u, d;  // U at the first j of the block, and the step to the next
+    float m4;     // −4sin²4φ
     float2 v[4];
 };
 
-// U at the first c of a later moment block: turned by the angle of `rep` blocks,
-// 8·2^dbl·φ each. (xx, yy) → turned, from sin(nφ) = u_n sin φ and cos(nφ) = c_n at n = 8.
-__device__ __forceinline__ void mom_later_block(float c8, float u8, float nq, float ts, float te,
-                                                int rep, int dbl, float &X, float &Y) {
-    for (int k = 0; k < dbl; ++k) {
-        const float uu = u8 * u8;
-        u8 = 2.0f * c8 * u8;
-        c8 = fmaf(c8, c8, nq * uu);
-    }
-    const float T1 = ts * u8, T2 = te * u8;
-    for (int k = 0; k < rep; ++k) {
-        const float x = fmaf(X, c8, -(Y * T1));
-        Y = fmaf(Y, c8, X * T2);
-        X = x;
-    }
+// X, Y turned by an angle of θ = 2·half: t = sin²(half), T1 = sin θ·tan(φ/2) and
+// T2 = sin θ/tan(φ/2): what it adds.
+__device__ __forceinline__ float2 mom_turn(float X, float Y, float t, float T1, float T2) {
+    const float m = -2.0f * t;
+    return make_float2(fmaf(X, m, -(Y * T1)), fmaf(Y, m, X * T2));
 }
 
 // Scalar operations throughout: they cost the FP32 pipe the same lane slots as
 // packed ones over two pairs would, and write the halves of the packed operands in place
 // (packed over two pairs, the transposition was 90 register moves per pair:
 // 20,000 atoms, 72 moments: 2.05 ms, FMA pipe 41 % and ALU pipe 48 % busy).
-// s2 = sin²(φ/2).
+// s2 = sin²(φ/2). U is that of the first c of the block: turned by the angle of `rep`
+// blocks, 8·2^dbl·φ each.
 __device__ __forceinline__ void mom_seed(float s2, int rep, int dbl, bool valid, MomPair &P) {
     const float e = 1.0f - s2;             // cos²(φ/2)
     const float na = -4.0f * s2;           // −α
-    const float nq = na * e;               // −sin²φ
     const float d1 = -2.0f * s2;
     const float C1 = 1.0f + d1;            // cos φ
-    // cos(nφ), u_n = sin(nφ)/sin φ for n = 2, 4, 8
-    const float c1q = C1 * C1;
-    const float c2 = c1q + nq;
-    const float c4 = fmaf(c2, c2, 4.0f * nq * c1q);
-    const float w4 = 4.0f * (C1 * c2);
-    const float c8 = fmaf(c4, c4, nq * w4 * w4);
-    const float u8 = 2.0f * (w4 * c4);
+    // sin²(nφ), cos(nφ) and u_n = sin(nφ)/sin φ, n = 1, 2, 4, (8)
+    const float t1 = -na * e;
+    const float t2 = 4.0f * t1 * (C1 * C1), c2 = fmaf(-2.0f, t1, 1.0f);
+    const float t4 = 4.0f * t2 * (c2 * c2), c4 = fmaf(-2.0f, t2, 1.0f);
+    const float u8 = 8.0f * (C1 * c2) * c4;
     // cos tφ by Reinsch differences d_{t+1} = d_t − α cos tφ
     const float d2 = fmaf(na, C1, d1), C2 = C1 + d2;
     const float d3 = fmaf(na, C2, d2), C3 = C2 + d3;
@@ -128,24 +121,37 @@ __device__ __forceinline__ void mom_seed(float s2, int rep, int dbl, bool valid,
     P.v[1] = make_float2(C1 + C2, d2);
     P.v[2] = make_float2(C2 + C3, d3);
     P.v[3] = make_float2(C3 + (C3 + d4), d4);
-    // c = 3.5: cos(3.5φ)/cos(φ/2) and sin(3.5φ)/sin(φ/2)
-    const float c13 = C1 + C3;
-    float X = fmaf(2.0f, c13 - C2, -1.0f), Y = fmaf(2.0f, c13 + C2, 1.0f);
+    // c = 3.5: cos(3.5φ)/cos(φ/2) and sin(3.5φ)/sin(φ/2), from the differences
+    float X = fmaf(2.0f, d1 + d3, 1.0f);
+    float Y = fmaf(2.0f, fmaf(3.0f, d1, fmaf(2.0f, d2, d3)), 7.0f);
     const float ts = s2 + s2, te = e + e;
-    if (rep > 0) mom_later_block(c8, u8, nq, ts, te, rep, dbl, X, Y);
+    if (rep > 0) {
+        float t = t4, c = c4, u = u8;  // sin²θ, cos θ, sin 2θ/sin φ at θ = 4φ
+        for (int k = 0; k < dbl; ++k) {
+            const float cn = fmaf(-2.0f, t, 1.0f);
+            t = 4.0f * t * (c * c);
+            c = cn;
+            u = 2.0f * c * u;
+        }
+        for (int k = 0; k < rep; ++k) {
+            const float2 step = mom_turn(X, Y, t, ts * u, te * u);
+            X += step.x;
+            Y += step.y;
+        }
+    }
     X = valid ? X : 0.0f;
     Y = valid ? Y : 0.0f;
-    P.w0 = make_float2(X, Y);
-    P.w1 = make_float2(fmaf(X, c8, -(Y * (ts * u8))), fmaf(Y, c8, X * (te * u8)));
-    P.cc = c8 + c8;
+    P.u = make_float2(X, Y);
+    P.d = mom_turn(X, Y, t4, ts * u8, te * u8);
+    P.m4 = -4.0f * t4;
 }
 
 template <int KM, bool WEIGHTED>
 __device__ __forceinline__ void mom_accumulate(const MomPair &P, float w, int nj,
                                                float2 (&acc)[KM / 2],
                                                float2 (&accw)[WEIGHTED ? KM / 2 : 1]) {
-    const float2 cp = make_float2(P.cc, P.cc), cn = make_float2(-P.cc, -P.cc);
-    float2 W[2] = {P.w0, P.w1};
+    const float2 m4 = make_float2(P.m4, P.m4);
+    float2 U = P.u, D = P.d;
     float2 WV[WEIGHTED ? 4 : 1];
     if constexpr (WEIGHTED)
 #pragma unroll
@@ -155,38 +161,18 @@ __device__ __forceinline__ void mom_accumulate(const MomPair &P, float w, int nj
         if (jj >= nj) break;
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-            acc[4 * jj + t] = __ffma2_rn(W[jj & 1], P.v[t], acc[4 * jj + t]);
-            if constexpr (WEIGHTED)
-                accw[4 * jj + t] = __ffma2_rn(W[jj & 1], WV[t], accw[4 * jj + t]);
+            acc[4 * jj + t] = __ffma2_rn(U, P.v[t], acc[4 * jj + t]);
+            if constexpr (WEIGHTED) accw[4 * jj + t] = __ffma2_rn(U, WV[t], accw[4 * jj + t]);
         }
-        // W_{jj+2} = ±2cos(8φ)·W_{jj+1} + W_jj
-        if (jj + 2 < KM / 8)
-            W[jj & 1] = __ffma2_rn((jj & 1) ? cp : cn, W[(jj & 1) ^ 1], W[jj & 1]);
-    }
-}
-
-// The same for two terms at once, all KM moments.
-template <int KM>
-__device__ __forceinline__ void mom_accumulate2(const MomPair &A, const MomPair &C,
-                                                float2 (&acc)[KM / 2]) {
-    const float2 ap = make_float2(A.cc, A.cc), an = make_float2(-A.cc, -A.cc);
-    const float2 bp = make_float2(C.cc, C.cc), bn = make_float2(-C.cc, -C.cc);
-    float2 U[2] = {A.w0, A.w1}, W[2] = {C.w0, C.w1};
-#pragma unroll
-    for (int jj = 0; jj < KM / 8; ++jj) {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) acc[4 * jj + t] = __ffma2_rn(U[jj & 1], A.v[t], acc[4 * jj + t]);
-#pragma unroll
-        for (int t = 0; t < 4; ++t) acc[4 * jj + t] = __ffma2_rn(W[jj & 1], C.v[t], acc[4 * jj + t]);
-        if (jj + 2 < KM / 8) {
-            U[jj & 1] = __ffma2_rn((jj & 1) ? ap : an, U[(jj & 1) ^ 1], U[jj & 1]);
-            W[jj & 1] = __ffma2_rn((jj & 1) ? bp : bn, W[(jj & 1) ^ 1], W[jj & 1]);
+        if (jj + 1 < KM / 8) {
+            if (jj > 0) D = __ffma2_rn(m4, U, D);
+            U = __fadd2_rn(U, D);
         }
     }
 }
 
 // Moments of the pairs (i, j), j0 <= j < j1, j > i, of one thread's i into
-// acc[4·jj + t] = s_jj·(Σ U.x·V.x, Σ U.y·V.y), for the first nj groups of eight of
+// acc[4·jj + t] = (Σ U.x·V.x, Σ U.y·V.y), for the first nj groups of eight of
 // the block. `at` holds the atoms [jbase, ...) in shared memory. Weighted mode
 // (WEIGHTED): the sums weighted by the j atom's w in accw as well.
 template <int KM, bool WEIGHTED>
@@ -215,7 +201,17 @@ constexpr int PD_DIR_LANES = PD_THREADS / PD_DIR_DIRS;   // atoms a unit takes a
 // 112 moments: 5.2 -> 4.05 ms). Rounding of x costs 6e-8·r1 of a position, whatever
 // the form; only pairs, whose distances may be short, need sin²(φ/2). w multiplies
 // the atom's terms.
-__device__ __forceinline__ void dir_seed(float3 dv, float4 p, float w, MomPair &P) {
+//
+// P_{j,t} steps with j by the three-term recurrence P_{j+1} = 2T_8·P_j − P_{j−1}, kept as
+// W_j = s_j·P_j with the signs s = + + − − + + − − …, which turns every step into one
+// multiply-add, W_{j+1} = ±2T_8·W_j + W_{j−1} (+ for even j): no negation, no half
+// swapped, the older of the two registers overwritten.
+struct DirSeed {
+    float2 w0, w1;  // W_0, W_1
+    float cc;       // 2T_8
+    float2 v[4];    // T_0 … T_7
+};
+__device__ __forceinline__ void dir_seed(float3 dv, float4 p, float w, DirSeed &P) {
     const float x2 = fmaf(dv.x, p.x, fmaf(dv.y, p.y, dv.z * p.z)) * 4.0f;  // 2x (dv is n/(2·r1))
     const float x = 0.5f * x2;
     const float T2 = fmaf(x2, x, -1.0f), T3 = fmaf(x2, T2, -x), T4 = fmaf(x2, T3, -T2);
@@ -231,6 +227,31 @@ __device__ __forceinline__ void dir_seed(float3 dv, float4 p, float w, MomPair &
     P.cc = T8 + T8;
 }
 
+// N atoms' terms at once, all KM sums: with two, their chains overlap.
+template <int KM, int N>
+__device__ __forceinline__ void dir_accumulate(const DirSeed (&P)[N], float2 (&acc)[KM / 2]) {
+    float2 W[N][2];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+        W[n][0] = P[n].w0;
+        W[n][1] = P[n].w1;
+    }
+#pragma unroll
+    for (int jj = 0; jj < KM / 8; ++jj) {
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                acc[4 * jj + t] = __ffma2_rn(W[n][jj & 1], P[n].v[t], acc[4 * jj + t]);
+        if (jj + 2 < KM / 8)
+#pragma unroll
+            for (int n = 0; n < N; ++n) {
+                const float c = (jj & 1) ? P[n].cc : -P[n].cc;
+                W[n][jj & 1] = __ffma2_rn(make_float2(c, c), W[n][(jj & 1) ^ 1], W[n][jj & 1]);
+            }
+    }
+}
+
 // A thread's atoms j0, j0 + PD_DIR_LANES, … < j1 of a block staged in shared memory,
 // for its direction dv = n/(2·r1), weighted by w or not. With room in registers
 // (ILP) two atoms at a time: their sequences' dependency chains overlap.
@@ -242,17 +263,16 @@ __device__ __forceinline__ void direction_range(const float4 *__restrict__ at, f
     if constexpr (ILP)
         for (; j + PD_DIR_LANES < j1; j += 2 * PD_DIR_LANES) {
             const float4 pa = at[j], pb = at[j + PD_DIR_LANES];
-            MomPair A, C;
-            dir_seed(dv, pa, weighted ? pa.w : 1.0f, A);
-            dir_seed(dv, pb, weighted ? pb.w : 1.0f, C);
-            mom_accumulate2<KM>(A, C, acc);
+            DirSeed S[2];
+            dir_seed(dv, pa, weighted ? pa.w : 1.0f, S[0]);
+            dir_seed(dv, pb, weighted ? pb.w : 1.0f, S[1]);
+            dir_accumulate<KM, 2>(S, acc);
         }
     for (; j < j1; j += PD_DIR_LANES) {
         const float4 pa = at[j];
-        MomPair A;
-        dir_seed(dv, pa, weighted ? pa.w : 1.0f, A);
-        float2 none[1];
-        mom_accumulate<KM, false>(A, 0.0f, KM / 8, acc, none);
+        DirSeed S[1];
+        dir_seed(dv, pa, weighted ? pa.w : 1.0f, S[0]);
+        dir_accumulate<KM, 1>(S, acc);
     }
 }
 
@@ -270,27 +290,25 @@ __device__ __forceinline__ void direction_range_later(const float4 *__restrict__
         MomPair A;
         mom_seed(s2, rep, DBL, true, A);
         const float w = weighted ? p.w : 1.0f;
-        A.w0 = __fmul2_rn(make_float2(w, w), A.w0);
-        A.w1 = __fmul2_rn(make_float2(w, w), A.w1);
+        A.u = __fmul2_rn(make_float2(w, w), A.u);
+        A.d = __fmul2_rn(make_float2(w, w), A.d);
         float2 none[1];
         mom_accumulate<KM, false>(A, 0.0f, nj, acc, none);
     }
 }
 
 // FP64 form: the same sequences in double for one s2 = sin²(φ/2);
-// acc[8·jj + 2t + {0, 1}] = s_jj·(Σ U.x·V.x, Σ U.y·V.y) (and weighted by w in accw).
+// acc[8·jj + 2t + {0, 1}] = (Σ U.x·V.x, Σ U.y·V.y) (and weighted by w in accw).
 template <int KM, bool WEIGHTED>
 __device__ __forceinline__ void mom_accumulate_f64(double s2, double scale, double w, int nj,
                                                    int rep, int dbl, double (&acc)[KM],
                                                    double (&accw)[WEIGHTED ? KM : 1]) {
-    const double e = 1.0 - s2, na = -4.0 * s2, nq = na * e;
+    const double e = 1.0 - s2, na = -4.0 * s2;
     const double C1 = fma(-2.0, s2, 1.0);
-    const double c1q = C1 * C1;
-    const double c2 = c1q + nq;
-    const double c4 = fma(c2, c2, 4.0 * nq * c1q);
-    const double w4 = 4.0 * C1 * c2;
-    double c8 = fma(c4, c4, nq * w4 * w4);
-    double u8 = 2.0 * w4 * c4;
+    const double t1 = -na * e;
+    const double t2 = 4.0 * t1 * (C1 * C1), c2 = fma(-2.0, t1, 1.0);
+    const double t4 = 4.0 * t2 * (c2 * c2), c4 = fma(-2.0, t2, 1.0);
+    const double u8 = 8.0 * (C1 * c2) * c4;
     double vx[4], vy[4];
     vy[0] = -2.0 * s2;
     vx[0] = 1.0 + C1;
@@ -302,50 +320,50 @@ __device__ __forceinline__ void mom_accumulate_f64(double s2, double scale, doub
     vx[2] = C2 + C3;
     vy[3] = fma(na, C3, vy[2]);
     vx[3] = C3 + (C3 + vy[3]);
-    const double c13 = C1 + C3;
-    double X = fma(2.0, c13 - C2, -1.0), Y = fma(2.0, c13 + C2, 1.0);
+    double X = fma(2.0, vy[0] + vy[2], 1.0);
+    double Y = fma(2.0, fma(3.0, vy[0], fma(2.0, vy[1], vy[2])), 7.0);
     const double ts = 2.0 * s2, te = 2.0 * e;
-    const double t1 = ts * u8, t2 = te * u8, cc = c8;
     if (rep > 0) {
+        double t = t4, c = c4, u = u8;
         for (int k = 0; k < dbl; ++k) {
-            const double uu = u8 * u8;
-            u8 = 2.0 * c8 * u8;
-            c8 = fma(c8, c8, nq * uu);
+            const double cn = fma(-2.0, t, 1.0);
+            t = 4.0 * t * (c * c);
+            c = cn;
+            u = 2.0 * c * u;
         }
-        const double T1 = ts * u8, T2 = te * u8;
+        const double m = -2.0 * t, T1 = ts * u, T2 = te * u;
         for (int k = 0; k < rep; ++k) {
-            const double x = fma(X, c8, -(Y * T1));
-            Y = fma(Y, c8, X * T2);
-            X = x;
+            const double x = fma(X, m, -(Y * T1));
+            Y += fma(Y, m, X * T2);
+            X += x;
         }
     }
-    double WX[2], WY[2];
-    WX[0] = scale * X;
-    WY[0] = scale * Y;
-    WX[1] = fma(WX[0], cc, -(WY[0] * t1));
-    WY[1] = fma(WY[0], cc, WX[0] * t2);
-    const double c2x = 2.0 * cc;
+    double UX = scale * X, UY = scale * Y;
+    double DX = fma(UX, -2.0 * t4, -(UY * (ts * u8))), DY = fma(UY, -2.0 * t4, UX * (te * u8));
+    const double m4 = -4.0 * t4;
 #pragma unroll
     for (int jj = 0; jj < KM / 8; ++jj) {
         if (jj >= nj) break;
-        const double wx = WX[jj & 1], wy = WY[jj & 1];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
             if constexpr (WEIGHTED) {
-                const double px = wx * vx[t], py = wy * vy[t];
+                const double px = UX * vx[t], py = UY * vy[t];
                 acc[8 * jj + 2 * t] += px;
                 acc[8 * jj + 2 * t + 1] += py;
                 accw[8 * jj + 2 * t] = fma(w, px, accw[8 * jj + 2 * t]);
                 accw[8 * jj + 2 * t + 1] = fma(w, py, accw[8 * jj + 2 * t + 1]);
             } else {
-                acc[8 * jj + 2 * t] = fma(wx, vx[t], acc[8 * jj + 2 * t]);
-                acc[8 * jj + 2 * t + 1] = fma(wy, vy[t], acc[8 * jj + 2 * t + 1]);
+                acc[8 * jj + 2 * t] = fma(UX, vx[t], acc[8 * jj + 2 * t]);
+                acc[8 * jj + 2 * t + 1] = fma(UY, vy[t], acc[8 * jj + 2 * t + 1]);
             }
         }
-        if (jj + 2 < KM / 8) {
-            const double sc = (jj & 1) ? c2x : -c2x;
-            WX[jj & 1] = fma(sc, WX[(jj & 1) ^ 1], wx);
-            WY[jj & 1] = fma(sc, WY[(jj & 1) ^ 1], wy);
+        if (jj + 1 < KM / 8) {
+            if (jj > 0) {
+                DX = fma(m4, UX, DX);
+                DY = fma(m4, UY, DY);
+            }
+            UX += DX;
+            UY += DY;
         }
     }
 }
@@ -384,7 +402,7 @@ __device__ __forceinline__ void dir_accumulate_f64(DirSeed64 &S, int jj, double 
     const double u = S.u[jj & 1];
 #pragma unroll
     for (int t = 0; t < 8; ++t) acc[8 * jj + t] = fma(u, S.T[t], acc[8 * jj + t]);
-    // signs + + − − as in the pairs' sequences
+    // signs + + − − as in dir_accumulate
     if (jj + 2 < KM / 8) S.u[jj & 1] = fma((jj & 1) ? S.c : -S.c, S.u[(jj & 1) ^ 1], u);
 }
 template <int KM, bool ILP>
@@ -442,15 +460,14 @@ __device__ __forceinline__ void direction_put(double *__restrict__ out, int jj, 
     o[0] = (first ? 0.0 : o[0]) + s * x;
     o[32] = (first ? 0.0 : o[32]) + s * y;
 }
-// of a later one from moment n0 on, x = s_jj·Σ U.x·V.x and y of group jj, element t: the
-// moments of cos(nφ) are s_jj·(x ± y)/2.
+// of a later one from moment n0 on, x = Σ U.x·V.x and y of group jj, element t: the
+// moments of cos(nφ) are (x ± y)/2.
 __device__ __forceinline__ void direction_put_later(double *__restrict__ out, int n0, int jj, int t,
                                                     int dir, double x, double y, bool first) {
-    const double h = (jj & 2) ? -0.5 : 0.5;
     double *hi = out + static_cast<int64_t>(n0 + 8 * jj + 4 + t) * 32 + dir;
     double *lo = out + static_cast<int64_t>(n0 + 8 * jj + 3 - t) * 32 + dir;
-    *hi = (first ? 0.0 : *hi) + h * (x + y);
-    *lo = (first ? 0.0 : *lo) + h * (x - y);
+    *hi = (first ? 0.0 : *hi) + 0.5 * (x + y);
+    *lo = (first ? 0.0 : *lo) + 0.5 * (x - y);
 }
 
 }  // namespace pd

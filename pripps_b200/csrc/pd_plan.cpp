@@ -754,7 +754,7 @@ static bool direction_only(Plan &P) {
         const int64_t blocks = (m8 + P.mom.block - 1) / P.mom.block;
         if (m8 <= P.mom.max_moments && blocks <= P.nqb)
             use = P.dir_cost < 0.5 * static_cast<double>(P.n_atoms) * P.n_atoms *
-                                       (44.0 * blocks + 1.25 * m8) +
+                                       (56.0 * blocks + 1.5 * m8) +
                                    PD_PAIRS_LATENCY;
     }
     if (!use) {
@@ -864,8 +864,8 @@ void set_reduction(Plan &P) {
     m.nqb = P.nqb;
     m.fp64 = P.precision == PD_FP64 ? 1 : 0;
     m.block = pd_moment_block(P.tun.K);
-    // FP32 lane operations per pair: 1.5 per moment and about 42 for the
-    // sequences, against 3 per grid point and 55 for each q-block's seeds (weighted
+    // FP32 lane operations per pair: 1.5 per moment and about 56 for the
+    // sequences and flushes, against 3 per grid point and 55 for each q-block's seeds (weighted
     // mode: 2.5 against 4); so up to two moments per grid point are cheaper.
     // FP64: a grid point costs a double sin, some 25 moments' worth.
     const int64_t per_q = m.fp64 ? 16 : 2;

@@ -180,6 +180,13 @@ int pd_plan_info(const pd_plan *plan, uint32_t *q_block, uint32_t *j_chunk,
                  uint32_t *pairs_per_thread, uint64_t *n_tiles, uint64_t *device_bytes,
                  uint64_t *upload_bytes);
 
+/* Diagnostic: how each frame of the plan's latest execution summed its pairs,
+ * form[n_frames] and moments[n_frames]: form 0, the grid points one by one
+ * (moments 0); 1, moments of the pairs; 2, class amplitudes over directions
+ * (moments along each). Waits for the device; PD_EINVAL before the first execution.
+ * No reference counterpart. */
+int pd_plan_forms(pd_ctx *ctx, pd_plan *plan, uint32_t *form, uint32_t *moments);
+
 /* Multi-GPU: restrict a plan to rank's share of the tiles (every world-th
  * tile in cost order). Each execution then yields partial profiles whose sum
  * over the ranks is the full [6][nq] result — rank 0 also carries the i = j

@@ -105,6 +105,7 @@ SIGNATURES = {
     "pd_plan_execute": (C.c_int, [_P, _P, C.c_void_p, C.c_void_p, C.c_void_p]),
     "pd_plan_execute_host": (C.c_int, [_P, _P, _D, _D]),
     "pd_plan_info": (C.c_int, [_P, _U32P, _U32P, _U32P, _U64P, _U64P, _U64P]),
+    "pd_plan_forms": (C.c_int, [_P, _P, _U32P, _U32P]),
     "pd_plan_set_profiling": (C.c_int, [_P, _P, C.c_int]),
     "pd_plan_pair_kernel_ms": (C.c_int, [_P, _P, _D, _U64P]),
     "pd_plan_destroy": (None, [_P, _P]),

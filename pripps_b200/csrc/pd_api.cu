@@ -1659,6 +1659,25 @@ int pd_plan_info(const pd_plan *plan, uint32_t *q_block, uint32_t *j_chunk, uint
     return PD_OK;
 }
 
+int pd_plan_forms(pd_ctx *ctx, pd_plan *plan, uint32_t *form, uint32_t *moments) {
+    if (!ctx || !plan || !form || !moments) return PD_EINVAL;
+    std::lock_guard<std::mutex> g(ctx->solve_mu);
+    cudaSetDevice(ctx->device);
+    if (!plan->dp.xyz_dev) {
+        ctx->set_error("pd_plan_forms: the plan has not been executed");
+        return PD_EINVAL;
+    }
+    std::vector<PdFrameDev> fr(static_cast<size_t>(plan->dp.P.n_frames));
+    PD_CUDA(ctx, cudaDeviceSynchronize());  // (executions may be on caller streams)
+    PD_CUDA(ctx, cudaMemcpy(fr.data(), plan->dp.base + plan->dp.L.frames,
+                            fr.size() * sizeof(PdFrameDev), cudaMemcpyDeviceToHost));
+    for (size_t f = 0; f < fr.size(); ++f) {
+        form[f] = fr[f].n_grp > 0 ? 2 : (fr[f].n_mom > 0 ? 1 : 0);
+        moments[f] = static_cast<uint32_t>(fr[f].n_grp > 0 ? fr[f].n_amp : fr[f].n_mom);
+    }
+    return PD_OK;
+}
+
 int pd_plan_set_shard(pd_ctx *ctx, pd_plan *plan, uint32_t rank, uint32_t world) {
     if (!ctx || !plan || world == 0 || rank >= world) return PD_EINVAL;
     std::lock_guard<std::mutex> g(ctx->solve_mu);

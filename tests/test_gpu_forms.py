@@ -1,0 +1,124 @@
+"""Which form a frame's pairs are summed in (pd_plan_forms): the other tests hold
+every form to the same tolerances, so only this one sees a rule that quietly
+falls back to another form."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import term_errors
+from oracle import oracle as O
+from pripps_b200 import _lib, synth
+from pripps_b200.debye import DebyeRequest
+
+pytestmark = pytest.mark.gpu
+GRID, MOMENTS, DIRECTIONS = 0, 1, 2
+TOL = {"fp64": 1e-10, "fp32": 1e-5}
+
+
+def _ball(n, radius, seed=1):
+    rng = np.random.default_rng(seed)
+    v = rng.normal(size=(n, 3))
+    xyz = v / np.linalg.norm(v, axis=1)[:, None] * rng.random((n, 1)) ** (1 / 3)
+    xyz -= xyz.mean(axis=0)
+    return xyz * (radius / np.linalg.norm(xyz, axis=1).max())
+
+
+def _globule(n, seed=1):
+    r = synth.sphere_radius_for(n)
+    return synth.rsa_points(n, (r, r, r), np.random.default_rng(seed))
+
+
+def _rod(n, length, seed=1):
+    rng = np.random.default_rng(seed)
+    xy = rng.uniform(-1, 1, (4 * n, 2))
+    xy = xy[(xy ** 2).sum(axis=1) < 1][:n] * 10.0
+    return np.column_stack([xy, rng.uniform(-length / 2, length / 2, n)])
+
+
+def _request(xyz, qmax, nq, precision, mode="vacuum", seed=2):
+    rng = np.random.default_rng(seed)
+    n = xyz.shape[-2]
+    sp = rng.integers(0, 3, n)
+    ff = rng.uniform(1, 8, (3, nq))
+    if mode == "vacuum":
+        return DebyeRequest(xyz, sp, ff, None, None, None, 0.0, qmax, nq, None, precision)
+    return DebyeRequest(xyz, sp, ff, rng.uniform(0.2, 3, (3, nq)), rng.uniform(0, 2, n),
+                        rng.uniform(5, 10, nq), 0.0, qmax, nq, None, precision)
+
+
+def _run(ctx, req, shard=None):
+    """Profiles of a plan's execution, and each frame's (form, moments)."""
+    lib = _lib.lib()
+    r, p = req.c_struct(), C.c_void_p()
+    nf = req.xyz.shape[0] if req.xyz.ndim == 3 else 1
+    form, mom = (C.c_uint32 * nf)(), (C.c_uint32 * nf)()
+    out = np.empty((6, req.nq))
+    _lib.check(lib.pd_plan_create(ctx.handle, C.byref(r), C.byref(p)), ctx.handle)
+    try:
+        assert lib.pd_plan_forms(ctx.handle, p, form, mom) == _lib.PD_EINVAL
+        if shard:
+            _lib.check(lib.pd_plan_set_shard(ctx.handle, p, *shard), ctx.handle)
+        xyz = np.ascontiguousarray(req.xyz, dtype=np.float64)
+        _lib.check(lib.pd_plan_execute_host(ctx.handle, p, _lib.dptr(xyz), _lib.dptr(out)),
+                   ctx.handle)
+        _lib.check(lib.pd_plan_forms(ctx.handle, p, form, mom), ctx.handle)
+    finally:
+        lib.pd_plan_destroy(ctx.handle, p)
+    return out, list(form), list(mom)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("mode", ["vacuum", "weighted"])
+def test_globules_sum_directions(gpu_ctx, precision, mode):
+    for n, qmax, nq in ((700, 0.3, 60), (3000, 0.5, 200), (9000, 0.8, 120)):
+        _, form, mom = _run(gpu_ctx, _request(_globule(n), qmax, nq, precision, mode))
+        assert form == [DIRECTIONS] and mom[0] >= 8, (n, form, mom)
+
+
+def test_extended_structures_sum_pair_moments(gpu_ctx):
+    for xyz, qmax, nq in ((_rod(3000, 500.0), 0.5, 300), (_rod(2000, 900.0), 1.0, 600)):
+        for mode in ("vacuum", "weighted"):
+            _, form, _ = _run(gpu_ctx, _request(xyz, qmax, nq, "fp32", mode))
+            assert form[0] in (MOMENTS, GRID if mode == "weighted" else MOMENTS), form
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_every_rank_of_a_shard_sums_directions(gpu_ctx, precision):
+    req = _request(_globule(2500), 0.7, 150, precision)
+    whole, form, _ = _run(gpu_ctx, req)
+    assert form == [DIRECTIONS]
+    total = np.zeros_like(whole)
+    for rank in range(3):
+        out, form, _ = _run(gpu_ctx, req, (rank, 3))
+        assert form == [DIRECTIONS], (rank, form)
+        total += out
+    assert np.all(term_errors(total, whole) < 1e-12)
+
+
+CASES = ([("fp32", m, 4000, 400) for m in (16, 24, 32, 40, 48, 56)] +
+         [("fp32", m, 6000, 400) for m in (64, 72, 80)] +
+         [("fp32", m, 12000, 400) for m in (96, 104, 112)] +
+         [("fp32", m, 18000, 400) for m in (120, 128)] +
+         [("fp32", 136, 20000, 600), ("fp32", 168, 30000, 800)])
+
+
+# The direction kernels are compiled for every 8 (from 64 moments on 16) moments up to
+# 128 (FP64: 64), later blocks hold the rest: structures with so many atoms and grid
+# points that the directions are the cheaper form at the given moment count.
+@pytest.mark.parametrize("precision,moments,n,nq", CASES)
+def test_direction_kernels_of_every_moment_count(gpu_ctx, precision, moments, n, nq):
+    """The moment count asked for is the one that ran; the last grid point and, for
+    small structures, the middle one against the oracle."""
+    xyz = _ball(n, 10.0, moments)
+    lo, hi = 0.0, 40.0  # the largest q_max whose moments do not exceed the count
+    while hi - lo > 0.1:
+        q = 0.5 * (lo + hi)
+        _, form, mom = _run(gpu_ctx, _request(xyz, q, nq, precision))
+        lo, hi = (q, hi) if mom[0] <= moments and form == [DIRECTIONS] else (lo, q)
+    req = _request(xyz, lo, nq, precision)
+    got, form, mom = _run(gpu_ctx, req)
+    assert form == [DIRECTIONS] and mom == [moments], (form, mom)
+    qi = np.array([nq // 2, nq - 1] if n < 10000 else [nq - 1])
+    err = term_errors(got[:, qi], O.terms_for_request(req, q_index=qi, precise=True))
+    assert np.all(err < TOL[precision]), err

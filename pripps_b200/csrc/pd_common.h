@@ -114,6 +114,9 @@ constexpr int PD_MAX_DIR_MOMENTS = 256;
 constexpr int PD_DIR_SMEM = 200 * 1024;
 // Lane operations that the pair form is charged beyond its pairs (frame_constants).
 constexpr double PD_PAIRS_LATENCY = 1e7;
+// The same where the grid points are summed one by one: a thread's pass over its j
+// atoms is a longer chain (800 atoms, 1 to 16 points: 111 us, directions 75 us).
+constexpr double PD_GRID_LATENCY = 4e7;
 constexpr int PD_DIR_DIRS = 8;  // directions of a work unit
 // Moments of its first block (FP32, FP64) and of each later one.
 constexpr int PD_DIR_MBLOCK = 128, PD_DIR_MBLOCK64 = 64;
@@ -123,8 +126,11 @@ struct PdMomentRule {
     double qmax;          // last grid point
     int32_t block;        // moments per job, pd_moment_block(K)
     int32_t nqb;          // jobs per tile
-    int32_t max_moments;  // beyond this the grid points are cheaper (or do not fit)
+    int32_t max_moments;  // more do not fit
     int32_t fp64;
+    // Cost of a pair: all grid points, the moment form per moment and per block (the
+    // cheaper one sums the pairs), and the grid points in the directions' unit.
+    double grid_cost, mom_cost, mom_block_cost, grid_dir_cost;
     // direction form (dir_cap = 0: never)
     int32_t dir_block;    // moments per unit
     int32_t dir_cap;      // directions the frame's table holds (a multiple of 32)

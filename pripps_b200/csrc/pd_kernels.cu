@@ -867,6 +867,39 @@ __device__ __forceinline__ void flush_weighted(float2 (&acc)[K / 2], float wi,
     }
 }
 
+// Moment form: a stage's j atoms [jss, jse) of a job that starts at tj0, in runs of
+// PD_MOM_FLUSH. Not inlined: its accumulators would cost the grid points' steps
+// registers (weighted mode, K = 64: 448 bytes of spills against 164).
+template <int K, int MODE>
+__device__ __noinline__ void moments_stage(const float4 *__restrict__ chunk, int jss, int jse,
+                                           int tj0, float4 pi, int i, bool ivalid, float inv_d2,
+                                           int nj, int mblk, double *__restrict__ part, int lane) {
+    constexpr int KM = pd_moment_block(K);
+    constexpr int DBL = KM == 128 ? 4 : (KM == 64 ? 3 : 2);
+    for (int js = jss; js < jse; js += PD_MOM_FLUSH) {
+        const int je = min(jse, js + PD_MOM_FLUSH);
+        const bool first = js == tj0;
+        float2 acc0[KM / 2];
+#pragma unroll
+        for (int t = 0; t < KM / 2; ++t) acc0[t] = make_float2(0.0f, 0.0f);
+        if constexpr (MODE == PD_MODE_CLASS) {
+            float2 none[1];
+            moments_range<KM, false>(chunk, jss, pi, i, ivalid, js, je, inv_d2, nj, mblk, DBL, acc0,
+                                     none);
+            flush_moments<KM / 2>(acc0, part, lane, first);
+        } else {
+            float2 acc1[KM / 2];
+#pragma unroll
+            for (int t = 0; t < KM / 2; ++t) acc1[t] = make_float2(0.0f, 0.0f);
+            moments_range<KM, true>(chunk, jss, pi, i, ivalid, js, je, inv_d2, nj, mblk, DBL, acc0,
+                                    acc1);
+            const float wi = ivalid ? pi.w : 0.0f;
+            flush_weighted<KM, true>(acc0, wi, part, K, lane, first);
+            flush_weighted<KM, true>(acc1, wi, part + 2 * K, K, lane, first);
+        }
+    }
+}
+
 // End of a tile: the warps' FP64 partial sums (part[w·nvk + e], e < nvk) of
 // one class are added in warp order and written to that class's slot; a CTA
 // whose copy wait expired writes NaN instead, and an empty tile zeros.
@@ -1030,34 +1063,16 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
             // below: no branch around the steps.
             const float4 *chunk = s_atoms[b];
             {
-                const int run = moments ? PD_MOM_FLUSH : PD_JFLUSH;
-                for (int js = jss; js < jse; js += run) {
-                    const int je = min(jse, js + run);
+                if (moments) {
+                    constexpr int KM = pd_moment_block(K);
+                    moments_stage<K, MODE>(chunk, jss, jse, tj0, pi, i, ivalid,
+                                           static_cast<float>(fr.inv_d2),
+                                           min(KM, fr.n_mom - mblk * KM) >> 3, mblk, part, lane);
+                }
+                for (int js = moments ? jse : jss; js < jse; js += PD_JFLUSH) {
+                    const int je = min(jse, js + PD_JFLUSH);
                     const bool first = js == tj0;
-                    if (moments) {
-                        constexpr int KM = pd_moment_block(K);
-                        constexpr int DBL = KM == 128 ? 4 : (KM == 64 ? 3 : 2);
-                        const int nj = min(KM, fr.n_mom - mblk * KM) >> 3;
-                        const float inv_d2 = static_cast<float>(fr.inv_d2);
-                        float2 acc0[KM / 2];
-#pragma unroll
-                        for (int t = 0; t < KM / 2; ++t) acc0[t] = make_float2(0.0f, 0.0f);
-                        if constexpr (MODE == PD_MODE_CLASS) {
-                            float2 none[1];
-                            moments_range<KM, false>(chunk, jss, pi, i, ivalid, js, je, inv_d2, nj,
-                                                     mblk, DBL, acc0, none);
-                            flush_moments<KM / 2>(acc0, part, lane, first);
-                        } else {
-                            float2 acc1[KM / 2];
-#pragma unroll
-                            for (int t = 0; t < KM / 2; ++t) acc1[t] = make_float2(0.0f, 0.0f);
-                            moments_range<KM, true>(chunk, jss, pi, i, ivalid, js, je, inv_d2, nj,
-                                                    mblk, DBL, acc0, acc1);
-                            const float wi = ivalid ? pi.w : 0.0f;
-                            flush_weighted<KM, true>(acc0, wi, part, K, lane, first);
-                            flush_weighted<KM, true>(acc1, wi, part + 2 * K, K, lane, first);
-                        }
-                    } else if constexpr (PACKED) {
+                    if constexpr (PACKED) {
                         const float2 *q2 = reinterpret_cast<const float2 *>(s_qres);
                         // 16-point chunks of this block that lie on the grid.
                         // The small-q residual blocks (the first of a grid)
@@ -1426,18 +1441,20 @@ __device__ __forceinline__ void frame_constants(double radius, const PdMomentRul
     fr.inv_d2 = static_cast<double>(static_cast<float>(1.0 / (fr.d * fr.d)));
     fr.d = 1.0 / sqrt(fr.inv_d2);
     fr.r1 = fmax(PD_MOM_STRETCH * radius, 1e-6);
-    double pair_cost = 1e300;
+    double pair_cost = rule.grid_dir_cost;
     if (rule.block > 0) {
         const int m8 = (moments_needed(rule.qmax * fr.d, fp64) + 7) & ~7;
         const int blocks = (m8 + rule.block - 1) / rule.block;
-        if (m8 <= rule.max_moments && blocks <= rule.nqb) {
+        if (m8 <= rule.max_moments && blocks <= rule.nqb &&
+            rule.mom_cost * m8 + rule.mom_block_cost * blocks < rule.grid_cost) {
             fr.n_mom = m8;
             fr.n_mblk = blocks;
             fr.n_parts = rule.nqb / blocks;
-            pair_cost = 0.5 * static_cast<double>(rule.n_atoms) * rule.n_atoms *
-                        (56.0 * blocks + 1.5 * m8);
+            pair_cost = 56.0 * blocks + 1.5 * m8;
         }
     }
+    pair_cost *= 0.5 * static_cast<double>(rule.n_atoms) * rule.n_atoms;
+    pair_cost += fr.n_mom > 0 ? PD_PAIRS_LATENCY : PD_GRID_LATENCY;
     // ---- directions: 2h Gauss rings (upper half: h), enough points on each
     if (rule.dir_cap == 0) {
         if (part == 0 && threadIdx.x == 0) frames[f] = fr;
@@ -1477,7 +1494,7 @@ __device__ __forceinline__ void frame_constants(double radius, const PdMomentRul
                      m8 <= rule.amp_cap && nodes <= rule.node_cap &&
                      static_cast<int64_t>(rule.n_chunk) * rule.nv2 *
                              ((groups + rule.world - 1) / rule.world) * m8 * 32 <= rule.slot_cap &&
-                     groups >= rule.world && (rule.dir_only || dir_cost < pair_cost + PD_PAIRS_LATENCY);
+                     groups >= rule.world && (rule.dir_only || dir_cost < pair_cost);
     if (use) {
         fr.n_grp = mine;
         fr.n_amp = m8;

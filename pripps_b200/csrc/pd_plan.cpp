@@ -744,19 +744,24 @@ static bool direction_only(Plan &P) {
     P.lptr.assign(static_cast<size_t>(P.n_pairs) * P.nqb + 1, 0);
     P.dir_only = true;
     set_reduction(P);
-    bool use = P.amp.dir_cap > 0;
-    if (use && P.mom.block > 0) {
+    double pair_cost = P.mom.grid_dir_cost;
+    bool moments = false;
+    if (P.mom.block > 0) {
         const bool fp64 = P.precision == PD_FP64;
         const double d = std::max(2.0 * 1.03 * P.radius_hint, 1e-6);
         const double z = P.qmax * d;  // the moments of pd_pack's pair form
         const double m = fp64 ? series_order(z, true) : z + 9.7 * std::cbrt(0.5 * z) + 3.5;
-        const int64_t m8 = (static_cast<int64_t>(0.5 * m) + 1 + 7) & ~int64_t{7};
-        const int64_t blocks = (m8 + P.mom.block - 1) / P.mom.block;
-        if (m8 <= P.mom.max_moments && blocks <= P.nqb)
-            use = P.dir_cost < 0.5 * static_cast<double>(P.n_atoms) * P.n_atoms *
-                                       (56.0 * blocks + 1.5 * m8) +
-                                   PD_PAIRS_LATENCY;
+        const double m8 = m < 1e6 ? static_cast<double>((static_cast<int64_t>(0.5 * m) + 8) & ~int64_t{7}) : 1e6;
+        const double blocks = std::ceil(m8 / P.mom.block);
+        if (m8 <= P.mom.max_moments && blocks <= P.nqb &&
+            P.mom.mom_cost * m8 + P.mom.mom_block_cost * blocks < P.mom.grid_cost) {
+            moments = true;
+            pair_cost = 56.0 * blocks + 1.5 * m8;
+        }
     }
+    pair_cost *= 0.5 * static_cast<double>(P.n_atoms) * P.n_atoms;
+    pair_cost += moments ? PD_PAIRS_LATENCY : PD_GRID_LATENCY;
+    const bool use = P.amp.dir_cap > 0 && P.dir_cost < pair_cost;
     if (!use) {
         P.dir_only = false;
         return false;
@@ -864,14 +869,30 @@ void set_reduction(Plan &P) {
     m.nqb = P.nqb;
     m.fp64 = P.precision == PD_FP64 ? 1 : 0;
     m.block = pd_moment_block(P.tun.K);
-    // FP32 lane operations per pair: 1.5 per moment and about 56 for the
-    // sequences and flushes, against 3 per grid point and 55 for each q-block's seeds (weighted
-    // mode: 2.5 against 4); so up to two moments per grid point are cheaper.
-    // FP64: a grid point costs a double sin, some 25 moments' worth.
-    const int64_t per_q = m.fp64 ? 16 : 2;
     m.max_moments = static_cast<int32_t>(
-        std::min<int64_t>({PD_MAX_MOMENTS, static_cast<int64_t>(P.nqb) * m.block,
-                           per_q * P.nq + 8 * P.nqb}) & ~int64_t{7});
+        std::min<int64_t>(PD_MAX_MOMENTS, static_cast<int64_t>(P.nqb) * m.block) & ~int64_t{7});
+    // As measured, whole solves of 3,000 to 20,000 atoms, FP32, in units of 83 % of the
+    // FFMA peak: 3 lane operations per grid point (in 16s) and 55 for each q-block's
+    // seeds, against 1.25 per moment and 140 for a block of 128 (sequences and flush);
+    // weighted mode (two sums per value) 4 and 55 against 2.1 and 200 for a block of 64.
+    // Grid points / moments: a rod of 5,000 atoms, 160 moments, 150 points 511 / 414 us,
+    // 300 points 819 / 414, weighted 708 / 757 and 1,040 / 757; 20,000 atoms, 208 moments,
+    // 150 points 5.5 / 4.4 ms, weighted 7.8 / 10.0 and, 300 points, 12.3 / 10.0. The
+    // directions' own operations run at 57 % of the peak (FP64: 29 %), hence the
+    // factor 0.7. FP64: a grid point costs a double sin, 110 operations, for whole
+    // q-blocks.
+    const double points = static_cast<double>((P.nq + 15) & ~15);
+    if (m.fp64) {
+        m.grid_cost = 110.0 * P.nqb * P.tun.K;
+        m.mom_cost = 6.0;
+        m.grid_dir_cost = 0.29 * m.grid_cost;
+    } else {
+        const bool weighted = P.mode == PD_MODE_WEIGHTED;
+        m.grid_cost = (weighted ? 4.0 : 3.0) * points + 55.0 * P.nqb;
+        m.mom_cost = weighted ? 2.1 : 1.25;
+        m.mom_block_cost = weighted ? 72.0 + 2.0 * m.block : 60.0 + 0.625 * m.block;
+        m.grid_dir_cost = 0.7 * m.grid_cost;
+    }
     if (m.max_moments < 8) m.block = 0;
     set_directions(P);
     m.dir_block = P.amp.dir_block;

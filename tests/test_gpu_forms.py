@@ -122,3 +122,29 @@ def test_direction_kernels_of_every_moment_count(gpu_ctx, precision, moments, n,
     qi = np.array([nq // 2, nq - 1] if n < 10000 else [nq - 1])
     err = term_errors(got[:, qi], O.terms_for_request(req, q_index=qi, precise=True))
     assert np.all(err < TOL[precision]), err
+
+
+def test_cheaper_form_for_few_grid_points(gpu_ctx):
+    """A few grid points up to a large q cost less one by one than the directions (or
+    pair moments) that the range needs, and more of them do not."""
+    for precision in ("fp32", "fp64"):
+        for xyz, qmax in ((_ball(4000, 25.0), 4.0), (_rod(3000, 500.0), 0.5)):
+            for mode in ("vacuum", "weighted"):
+                req = _request(xyz, qmax, 4, precision, mode)
+                got, form, _ = _run(gpu_ctx, req)
+                assert form == [GRID], (precision, mode, form)
+                err = term_errors(got, O.terms_for_request(req, precise=True))
+                assert np.all(err < TOL[precision]), err
+                _, form, _ = _run(gpu_ctx, _request(xyz, qmax, 600, precision, mode))
+                assert form != [GRID] or precision == "fp64", (precision, mode, form)
+    # weighted mode: two sums per value make the moments' sequences and flushes weigh more
+    _, form, mom = _run(gpu_ctx, _request(_rod(3000, 900.0), 1.0, 500, "fp32", "weighted"))
+    assert form == [GRID], (form, mom)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_frames_of_a_batch_take_their_own_form(gpu_ctx, precision):
+    xyz = _globule(800)
+    frames = np.stack([xyz, 8.0 * xyz, xyz + 1.0])
+    _, form, _ = _run(gpu_ctx, _request(frames, 0.6, 45, precision))
+    assert form[0] == form[2] == DIRECTIONS and form[1] != DIRECTIONS, form

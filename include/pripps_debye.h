@@ -351,7 +351,7 @@ const char *pd_last_error(pd_ctx *ctx);
 
 /* Kernel shapes. Every solve, plan, stream and request of the loop picks
  * its shape — the q-block length K of the pair kernels (FP32: 32, 64, 96, 128,
- * 160, 192; FP64: 16, 32, and 64 in class mode), the atom-chunk length of a tile (multiple of 32)
+ * 160, 192; FP64: 16, 32), the atom-chunk length of a tile (multiple of 32)
  * and the pairs each thread advances together (FP32: 1, 2 or 4) — from the
  * context's tuning table by the request's bucket: (precision, accumulation
  * mode (class or weighted), one frame or several, floor(log2 n_atoms),

@@ -1942,7 +1942,7 @@ std::vector<Tuning> tune_candidates(const pd_request *req, int mode) {
     const int64_t n = static_cast<int64_t>(req->n_atoms), nq = static_cast<int64_t>(req->nq);
     std::vector<std::pair<int, int>> shapes;
     if (precision == PD_FP64)
-        shapes = {{16, 1}, {32, 1}, {64, 1}};  // 64: class mode only (valid_tuning)
+        shapes = {{16, 1}, {32, 1}};
     else if (mode == PD_MODE_WEIGHTED)
         shapes = {{32, 2}, {64, 2}, {64, 4}};
     else if (nq <= 32)

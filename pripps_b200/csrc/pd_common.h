@@ -103,7 +103,7 @@ struct PdChunk {
 // Moments per job of a kernel shape with q-block K: at most K (they share its
 // slots) and what the accumulators of the shape's register budget hold.
 constexpr int pd_moment_block(int K) {
-    return K >= 128 ? 128 : (K >= 64 ? 64 : (K >= 32 ? 32 : 16));
+    return K >= 128 ? 128 : (K >= 64 ? 64 : 32);
 }
 // The moment form is bounded to this many moments (q_max·d up to about 900).
 constexpr int PD_MAX_MOMENTS = 512;
@@ -121,7 +121,7 @@ constexpr int PD_DIR_DIRS = 8;  // directions of a work unit
 // Moments of its first block (FP32, FP64) and of each later one.
 constexpr int PD_DIR_MBLOCK = 128, PD_DIR_MBLOCK64 = 64;
 
-// When a frame may run in the moment form (block = 0: never).
+// When a frame may run in the moment form (block = 0, the FP64 form: never).
 struct PdMomentRule {
     double qmax;          // last grid point
     int32_t block;        // moments per job, pd_moment_block(K)

@@ -1,5 +1,5 @@
-// Moment form of the pair sum (device code shared by the FP32 and FP64 pair
-// kernels).
+// Moment form of the pair sum (FP32 pair kernels) and the direction form (FP32 and
+// FP64).
 //
 // For one pair at distance r <= 2·radius < d, with sin(φ/2) = r/d and z = q·d,
 //
@@ -297,12 +297,13 @@ __device__ __forceinline__ void direction_range_later(const float4 *__restrict__
     }
 }
 
-// FP64 form: the same sequences in double for one s2 = sin²(φ/2);
-// acc[8·jj + 2t + {0, 1}] = (Σ U.x·V.x, Σ U.y·V.y) (and weighted by w in accw).
-template <int KM, bool WEIGHTED>
-__device__ __forceinline__ void mom_accumulate_f64(double s2, double scale, double w, int nj,
-                                                   int rep, int dbl, double (&acc)[KM],
-                                                   double (&accw)[WEIGHTED ? KM : 1]) {
+// The same sequences in double for one s2 = sin²(φ/2) (a direction's later blocks; pairs
+// in FP64 are summed at the grid points: their moments, sums of N² terms that cancel
+// in a profile point, cost it up to three digits of its sixteen).
+// acc[8·jj + 2t + {0, 1}] = scale·(Σ U.x·V.x, Σ U.y·V.y).
+template <int KM>
+__device__ __forceinline__ void mom_accumulate_f64(double s2, double scale, int nj, int rep,
+                                                   int dbl, double (&acc)[KM]) {
     const double e = 1.0 - s2, na = -4.0 * s2;
     const double C1 = fma(-2.0, s2, 1.0);
     const double t1 = -na * e;
@@ -346,16 +347,8 @@ __device__ __forceinline__ void mom_accumulate_f64(double s2, double scale, doub
         if (jj >= nj) break;
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-            if constexpr (WEIGHTED) {
-                const double px = UX * vx[t], py = UY * vy[t];
-                acc[8 * jj + 2 * t] += px;
-                acc[8 * jj + 2 * t + 1] += py;
-                accw[8 * jj + 2 * t] = fma(w, px, accw[8 * jj + 2 * t]);
-                accw[8 * jj + 2 * t + 1] = fma(w, py, accw[8 * jj + 2 * t + 1]);
-            } else {
-                acc[8 * jj + 2 * t] = fma(UX, vx[t], acc[8 * jj + 2 * t]);
-                acc[8 * jj + 2 * t + 1] = fma(UY, vy[t], acc[8 * jj + 2 * t + 1]);
-            }
+            acc[8 * jj + 2 * t] = fma(UX, vx[t], acc[8 * jj + 2 * t]);
+            acc[8 * jj + 2 * t + 1] = fma(UY, vy[t], acc[8 * jj + 2 * t + 1]);
         }
         if (jj + 1 < KM / 8) {
             if (jj > 0) {
@@ -365,19 +358,6 @@ __device__ __forceinline__ void mom_accumulate_f64(double s2, double scale, doub
             UX += DX;
             UY += DY;
         }
-    }
-}
-
-template <int KM, bool WEIGHTED>
-__device__ __forceinline__ void moments_range_f64(const double4 *__restrict__ at, double4 pi, int i,
-                                                  bool ivalid, int j0, int j1, double inv_d2,
-                                                  int nj, int rep, int dbl, double (&acc)[KM],
-                                                  double (&accw)[WEIGHTED ? KM : 1]) {
-    for (int j = j0; j < j1; ++j) {
-        const double4 pj = at[j];
-        const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
-        mom_accumulate_f64<KM, WEIGHTED>((dx * dx + dy * dy + dz * dz) * inv_d2,
-                                         ivalid && j > i ? 1.0 : 0.0, pj.w, nj, rep, dbl, acc, accw);
     }
 }
 
@@ -440,8 +420,7 @@ __device__ __forceinline__ void direction_range_later_f64(const double4 *__restr
     for (int j = j0; j < j1; j += PD_DIR_LANES) {
         const double4 p = at[j];
         const double s2 = fma(-dv.x, p.x, fma(-dv.y, p.y, fma(-dv.z, p.z, 0.5)));
-        double none[1];
-        mom_accumulate_f64<KM, false>(s2, weighted ? p.w : 1.0, 0.0, nj, rep, DBL, acc, none);
+        mom_accumulate_f64<KM>(s2, weighted ? p.w : 1.0, nj, rep, DBL, acc);
     }
 }
 

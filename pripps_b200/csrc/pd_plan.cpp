@@ -175,7 +175,6 @@ Tuning fit_tuning(int precision, int mode, Tuning t) {
     // pair per pass.
     if (precision == PD_FP64) {
         t.NP = 1;
-        if (mode == PD_MODE_WEIGHTED && t.K > 32) t.K = 32;
     } else if (!valid_shape(precision, mode, t.K, t.NP)) {
         if (mode == PD_MODE_WEIGHTED) {
             t.K = t.K > 32 ? 64 : 32;
@@ -190,13 +189,9 @@ Tuning fit_tuning(int precision, int mode, Tuning t) {
 Tuning default_tuning(int64_t n_atoms, int64_t nq, int precision, int64_t n_frames) {
     Tuning t;
     if (precision == PD_FP64) {
-        // K = 64 holds the moments of q_max·d up to 85 in one block
-        t.K = nq > 32 ? 64 : 32;
+        t.K = 32;
         t.NP = 1;
-        // a CTA's pass over a j range is serial: short ranges fill the GPU on small
-        // structures (whole solves of 300 and 600 atoms: 91 and 110 µs at 256 j
-        // atoms, 70 and 82 µs at 64, 85 and 85 µs at 32)
-        t.TJ = std::clamp(next_pow2(n_atoms / 16), 64, 4096);
+        t.TJ = std::clamp(next_pow2(n_atoms / 16), 256, 4096);
         return t;
     }
     // Measured on B200 (class mode): K = 128 with 4 pairs per thread (three
@@ -747,10 +742,9 @@ static bool direction_only(Plan &P) {
     double pair_cost = P.mom.grid_dir_cost;
     bool moments = false;
     if (P.mom.block > 0) {
-        const bool fp64 = P.precision == PD_FP64;
         const double d = std::max(2.0 * 1.03 * P.radius_hint, 1e-6);
         const double z = P.qmax * d;  // the moments of pd_pack's pair form
-        const double m = fp64 ? series_order(z, true) : z + 9.7 * std::cbrt(0.5 * z) + 3.5;
+        const double m = z + 9.7 * std::cbrt(0.5 * z) + 3.5;
         const double m8 = m < 1e6 ? static_cast<double>((static_cast<int64_t>(0.5 * m) + 8) & ~int64_t{7}) : 1e6;
         const double blocks = std::ceil(m8 / P.mom.block);
         if (m8 <= P.mom.max_moments && blocks <= P.nqb &&
@@ -805,7 +799,7 @@ static void set_directions(Plan &P) {
     // carry the work units, so every rank needs jobs of every frame. The test
     // hook (of the FP32 form) needs the pair tiles.
     if (P.n_atoms < 150 || P.jobs_per_frame < 2 * static_cast<int64_t>(P.world) ||
-        (P.world > 1 && P.n_frames > 1) || P.mom.block == 0 ||
+        (P.world > 1 && P.n_frames > 1) ||
         (P.test_expire && P.precision != PD_FP64))
         return;
     // unknown coordinates: 20 cubic Angstrom per atom, elongated up to about 2.5 : 1
@@ -868,7 +862,7 @@ void set_reduction(Plan &P) {
     m.qmax = P.qmax;
     m.nqb = P.nqb;
     m.fp64 = P.precision == PD_FP64 ? 1 : 0;
-    m.block = pd_moment_block(P.tun.K);
+    m.block = m.fp64 ? 0 : pd_moment_block(P.tun.K);
     m.max_moments = static_cast<int32_t>(
         std::min<int64_t>(PD_MAX_MOMENTS, static_cast<int64_t>(P.nqb) * m.block) & ~int64_t{7});
     // As measured, whole solves of 3,000 to 20,000 atoms, FP32, in units of 83 % of the
@@ -883,9 +877,7 @@ void set_reduction(Plan &P) {
     // q-blocks.
     const double points = static_cast<double>((P.nq + 15) & ~15);
     if (m.fp64) {
-        m.grid_cost = 110.0 * P.nqb * P.tun.K;
-        m.mom_cost = 6.0;
-        m.grid_dir_cost = 0.29 * m.grid_cost;
+        m.grid_dir_cost = 0.29 * 110.0 * P.nqb * P.tun.K;
     } else {
         const bool weighted = P.mode == PD_MODE_WEIGHTED;
         m.grid_cost = (weighted ? 4.0 : 3.0) * points + 55.0 * P.nqb;
@@ -893,7 +885,6 @@ void set_reduction(Plan &P) {
         m.mom_block_cost = weighted ? 72.0 + 2.0 * m.block : 60.0 + 0.625 * m.block;
         m.grid_dir_cost = 0.7 * m.grid_cost;
     }
-    if (m.max_moments < 8) m.block = 0;
     set_directions(P);
     m.dir_block = P.amp.dir_block;
     m.dir_cap = P.amp.dir_cap;

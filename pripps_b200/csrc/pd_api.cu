@@ -770,6 +770,8 @@ struct PdTicket {
     size_t next_job = 0;              // first tile not yet issued
     bool express_wait = false;        // small: waits for a free express lane
     bool small = false;               // by its pair·q count: goes before larger ones
+    double linger = 0, hold_max = 0;  // how long a larger one waits for small ones (s)
+    double held = 0;                  // how long it has
     bool finish_issued = false;       // reduction (or, if cancelled, the drain) enqueued
     bool drained_only = false;        // cancelled after admission: no reduction was run
     uint32_t used_streams = 0;        // lane streams that ran some of its tiles
@@ -823,15 +825,19 @@ constexpr double EXPRESS_COST = PD_EXPRESS_COST;
 #define PD_EXPRESS_MAX_WAIT 0.25
 #endif
 constexpr double EXPRESS_MAX_WAIT = PD_EXPRESS_MAX_WAIT;
-// Larger requests leave the GPU to a burst of small ones: while a small request
-// is queued, and for this long (s) after one was submitted, the steps issue
-// nothing of a larger request that was admitted less than EXPRESS_MAX_WAIT
-// ago. (A 25,000-atom request takes under a millisecond, less than it takes a
-// client to submit a burst; without this it would run between its members.)
-#ifndef PD_SMALL_GRACE
-#define PD_SMALL_GRACE 0.5e-3
-#endif
-constexpr double SMALL_GRACE = PD_SMALL_GRACE;
+// Larger requests leave the GPU to a burst of small ones. A 25,000-atom request is done in
+// 0.7 ms, less than a client takes to submit the burst around it, so its tiles are
+// held: while a small request is queued or running and SMALL_GRACE longer; and, where
+// small requests were submitted within the last MIXED_TRAFFIC, for a while after its
+// own submission. Both are measured in the time that its pairs take at the grid points
+// (GRID_RATE pair·q per second), so that it is never done later than that form was:
+// at most 0.15 of it (and LINGER_MAX) for small ones to arrive, and the whole of it.
+// (Eighty small requests behind two of 25,000 atoms: the burst takes 4.4 ms to submit and
+// solve, the first small one comes 0.4 ms after the large ones. 10,000 and 30,000 atoms
+// beside a steady flow of small requests: 4.2 and 23.6 ms with the grid points, 3.3 and
+// 21 ms now; the latter alone 24 and 1.4 ms.)
+constexpr double SMALL_GRACE = 0.25e-3, LINGER_MAX = 1e-3, MIXED_TRAFFIC = 60.0;
+constexpr double GRID_RATE = 9e12;
 constexpr int EXPRESS = STEP_BUFS;  // row of the express lanes
 static_assert((STEP_BUFS + 1) * STEP_LANES <= 32, "lane bits of PdTicket::used_streams");
 
@@ -984,9 +990,11 @@ void worker_main(pd_ctx *ctx) {
     bool admit_recorded = false;
     int cur = 0;
     size_t rr = 0;
+    double small_seen = -1e9;  // when a small request was last queued or running
+    double last_step = 0;
     for (;;) {
         std::vector<std::shared_ptr<PdTicket>> head;  // planned front of the queue
-        bool hold_large = false;
+        bool mixed = false, small_queued = false;
         {
             std::unique_lock<std::mutex> lk(ctx->qmu);
             bool waiting_device = false;
@@ -1009,8 +1017,8 @@ void worker_main(pd_ctx *ctx) {
                     ++it;
                 }
             }
-            hold_large = now_s() - ctx->last_small < SMALL_GRACE;
-            for (uint64_t id : ctx->pending) hold_large |= ctx->tickets[id]->small;
+            mixed = now_s() - ctx->last_small < MIXED_TRAFFIC;
+            for (uint64_t id : ctx->pending) small_queued |= ctx->tickets[id]->small;
             for (uint64_t id : ctx->pending) {
                 auto t = ctx->tickets[id];
                 if (t->plan_state == 0) break;  // FIFO: wait for its planning
@@ -1162,11 +1170,24 @@ void worker_main(pd_ctx *ctx) {
         // requests (rotating start), each request's tiles into the lane of
         // its kernel variant; up to STEP_LANES variants per step.
         std::vector<std::shared_ptr<PdTicket>> cand;
-        for (auto &t : active) hold_large |= t->small && t->express_wait;
         const double t_step = now_s();
+        for (auto &t : active) small_queued |= t->small && t->status == 1;
+        if (small_queued) small_seen = t_step;
+        // (a pass counts for at most 1 ms: one that built a graph or waited for pinned
+        // memory gave no small request a turn)
+        const double pass = std::min(t_step - last_step, 1e-3);
+        last_step = t_step;
+        auto held = [&](PdTicket &t) {
+            if (t.small || t.held >= t.hold_max ||
+                !(t_step - small_seen < SMALL_GRACE ||
+                  (mixed && t_step - t.t_submit < t.linger)))
+                return false;
+            t.held += pass;
+            return true;
+        };
         for (auto &t : active)
             if (!t->canceled && !t->express_wait && t->next_job < t->dp.P.jobs.size() &&
-                (t->small || !hold_large || t_step - t->t_admit > EXPRESS_MAX_WAIT))
+                !held(*t))
                 cand.push_back(t);
         Lane *step = lanes[cur];
         std::tuple<int, int, int, int> lane_key[STEP_LANES];
@@ -1797,9 +1818,12 @@ int pd_submit(pd_ctx *ctx, const pd_request *req, uint64_t *ticket) {
     t->req.ff_water = req->hyd_weights ? t->ffW.data() : nullptr;
     t->req.frame_weights = req->frame_weights ? t->fw.data() : nullptr;
     t->t_submit = now_s();
-    t->small = 0.5 * static_cast<double>(n) * static_cast<double>(n) * static_cast<double>(nq) *
-                   static_cast<double>(nf) * (req->precision == PD_FP64 ? 24.0 : 1.0) <=
-               EXPRESS_COST;
+    const double work = 0.5 * static_cast<double>(n) * static_cast<double>(n) *
+                        static_cast<double>(nq) * static_cast<double>(nf) *
+                        (req->precision == PD_FP64 ? 24.0 : 1.0);
+    t->small = work <= EXPRESS_COST;
+    t->linger = std::min(LINGER_MAX, 0.15 * work / GRID_RATE);
+    t->hold_max = work / GRID_RATE;
     {
         std::lock_guard<std::mutex> lk(ctx->qmu);
         if (t->small) ctx->last_small = t->t_submit;

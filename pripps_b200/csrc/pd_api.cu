@@ -144,7 +144,7 @@ Layout make_layout(const Plan &P, bool host_xyz) {
     L.dir_done = take(F * n_nt * 4);
     L.ctl_bytes = o - L.ctl;
     L.dirs = take(F * P.amp.dir_cap * sizeof(double4));
-    L.nodes = take(F * P.amp.node_cap * sizeof(double2));
+    L.nodes = take(P.precision == PD_FP64 ? 0 : F * P.amp.node_cap * sizeof(double2));
     L.dir_part = take(F * P.amp.grp_cap * static_cast<uint64_t>(P.n_pairs) * P.nv *
                       P.amp.node_cap * 8);
     L.lat_sums = take(P.lat.size() * nq * 8);
@@ -619,7 +619,8 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st,
     if (P.amp.dir_cap > 0) {
         PD_CUDA(ctx, pd::launch_direction_sums(
                          dp.dptr<double>(L.dir_slots), dp.dptr<double4>(L.dirs),
-                         dp.dptr<PdFrameDev>(L.frames), P.amp, P.qmax, P.n_frames,
+                         dp.dptr<PdFrameDev>(L.frames), P.amp, P.qmax,
+                         P.precision == PD_FP64 ? dp.dptr<double>(L.qv) : nullptr, P.n_frames,
                          dp.dptr<PdClassDev>(L.cls), dp.dptr<PdPairDev>(L.pairs), P.n_pairs,
                          dp.dptr<int32_t>(L.cls_ptr), dp.dptr<int32_t>(L.cls_chunk), P.red.width,
                          add_exact, dp.dptr<double>(L.dir_part),

@@ -89,9 +89,9 @@ struct PdFrameDev {
     int32_t n_parts;
     int32_t n_grp;   // this rank's groups of 32 directions; 0: no direction form
     int32_t n_amp;   // moments of the direction form, a multiple of 8
-    int32_t n_ablk;  // their blocks
-    int32_t n_node;  // Chebyshev nodes of the q range (direction form)
-    int32_t pad_;
+    int32_t n_node;  // values of q that the class-pair sums are formed at (direction form):
+                     // Chebyshev nodes of the q range, or (FP64) the grid points
+    int32_t pad_[2];
 };
 static_assert(sizeof(PdFrameDev) == 64, "PdFrameDev layout");
 
@@ -114,9 +114,6 @@ constexpr int PD_MAX_DIR_MOMENTS = 256;
 constexpr int PD_DIR_SMEM = 200 * 1024;
 // Lane operations that the pair form is charged beyond its pairs (frame_constants).
 constexpr double PD_PAIRS_LATENCY = 1e7;
-// The same where the grid points are summed one by one: a thread's pass over its j
-// atoms is a longer chain (800 atoms, 1 to 16 points: 111 us, directions 75 us).
-constexpr double PD_GRID_LATENCY = 4e7;
 constexpr int PD_DIR_DIRS = 8;  // directions of a work unit
 // Moments of its first block (FP32, FP64) and of each later one.
 constexpr int PD_DIR_MBLOCK = 128, PD_DIR_MBLOCK64 = 64;
@@ -131,12 +128,16 @@ struct PdMomentRule {
     // Cost of a pair: all grid points, the moment form per moment and per block (the
     // cheaper one sums the pairs), and the grid points in the directions' unit.
     double grid_cost, mom_cost, mom_block_cost, grid_dir_cost;
+    // What the grid points are charged beyond that, as PD_PAIRS_LATENCY: a thread's pass
+    // over its j atoms is a chain (FP32, 800 atoms, 1 to 16 points: 111 us, directions
+    // 75; FP64, 100 atoms: 2 us for each, 230 us, directions 62).
+    double grid_latency;
     // direction form (dir_cap = 0: never)
     int32_t dir_block;    // moments per unit
     int32_t dir_cap;      // directions the frame's table holds (a multiple of 32)
     int32_t grp_cap;      // direction groups of this rank that the sums hold
     int32_t amp_cap;      // moments
-    int32_t node_cap;     // Chebyshev nodes
+    int32_t node_cap;     // Chebyshev nodes, or (FP64) the grid points
     int32_t n_chunk, n_cls, nv2;  // nv2: 1, or 2 with sums weighted by w (weighted mode)
     int32_t rank, world;
     int64_t slot_cap;     // doubles per frame for the chunks' sums
@@ -163,8 +164,9 @@ struct PdReduceShape {
     int32_t n_z;          // 128-value blocks per row
     int32_t n_chunk;      // blocks that share a slot list
     int32_t max_moments;  // moments or nodes
-    int32_t node_cap;     // nodes (direction form)
+    int32_t node_cap;     // nodes or grid points (direction form)
     int32_t dir_only;     // no tiles (a frame without directions has no result: NaN)
+    int32_t fp64;         // directions are summed at the grid points, not at nodes
     int64_t slots_per_frame;
 };
 

@@ -1446,7 +1446,7 @@ __device__ __forceinline__ void frame_constants(double radius, const PdMomentRul
         }
     }
     pair_cost *= 0.5 * static_cast<double>(rule.n_atoms) * rule.n_atoms;
-    pair_cost += fr.n_mom > 0 ? PD_PAIRS_LATENCY : PD_GRID_LATENCY;
+    pair_cost += fr.n_mom > 0 ? PD_PAIRS_LATENCY : rule.grid_latency;
     // ---- directions: 2h Gauss rings (upper half: h), enough points on each
     if (rule.dir_cap == 0) {
         if (part == 0 && threadIdx.x == 0) frames[f] = fr;
@@ -1476,7 +1476,7 @@ __device__ __forceinline__ void frame_constants(double radius, const PdMomentRul
     const double mo = direction_order(fr.r1 * rule.qmax, fp64);
     const int m8 = mo < 1e6 ? ((static_cast<int>(mo) + 8) & ~7) : 1000000;
     const int ablk = (m8 + rule.dir_block - 1) / rule.dir_block;
-    const int nodes = moments_needed(2.0 * fr.r1 * rule.qmax, true);
+    const int nodes = fp64 ? rule.nq : moments_needed(2.0 * fr.r1 * rule.qmax, true);
     const double dir_cost =
         static_cast<double>(S) * (static_cast<double>(rule.n_atoms) * rule.nv2 *
                                       (44.0 * ablk - 30.0 + 1.25 * m8) +
@@ -1490,10 +1490,9 @@ __device__ __forceinline__ void frame_constants(double radius, const PdMomentRul
     if (use) {
         fr.n_grp = mine;
         fr.n_amp = m8;
-        fr.n_ablk = ablk;
         fr.n_node = nodes;
         // Chebyshev nodes of the q range: y_k and the barycentric weight
-        for (int k = part * T + threadIdx.x; k < nodes; k += n_part * T) {
+        for (int k = part * T + threadIdx.x; k < nodes && !fp64; k += n_part * T) {
             double sn, cs;
             sincospi((2 * k + 1) / (2.0 * nodes), &sn, &cs);
             node_tab[static_cast<int64_t>(f) * rule.node_cap + k] =
@@ -1795,13 +1794,18 @@ __global__ void __launch_bounds__(PD_RED_THREADS)
     for (int v = 0; v < NV; ++v) o[static_cast<int64_t>(v) * sh.width] = s[v];
 }
 
-// Direction form: class-pair sums at Chebyshev nodes of the q range.
+// Direction form: class-pair sums at Chebyshev nodes of the q range, or at the grid
+// points.
 //
 // S_ab(q) = Σ sinc(q r) is an even entire function of q whose expansion in
 // T_2k(q/q_max) ends, like the moments, at k ≈ q_max·d/2 + …: its values at that many
 // nodes q_k = q_max·cos((2k+1)π/4M) give every grid point by interpolation (pd_profiles), so
 // the amplitudes are formed at 30 to 120 nodes instead of 200 to 1,000 grid
-// points. A block takes 32 directions and PD_DNODE_T nodes (fewer where many
+// points. The interpolation mixes values from N² to N: it keeps 1e-16 of N², which at
+// a deep minimum is up to 1e-11 of the point, far below the FP32 moments' rounding.
+// The FP64 form takes the grid points themselves (qv; largest error of a point, 30,000
+// atoms to q = 2: 8.7e-12 -> 4e-15; 6,001 atoms, 301 points: 8e-15 -> 5e-15 for 234 ->
+// 296 us). A block takes 32 directions and PD_DNODE_T nodes (fewer where many
 // classes share its memory): E_c = Σ_n g_n(q_k r1)·m_n, g_n = i^n (2 − δ_n0) J_n, of every class in
 // FP64 — the sums of the class's chunks added in chunk order, the zeroth
 // moment the exact atom count or weight sum — then Σ w·Re(E_a E_b*) over the directions
@@ -1823,7 +1827,7 @@ __device__ double direction_coefficients(double y, int n_mom, double *__restrict
         return 1.0;
     }
     const double ty = 2.0 / y;
-    const int top = static_cast<int>(bessel_order(y, 14.0, 8.0)) | 1;
+    const int top = static_cast<int>(bessel_order(y, 16.0, 10.0)) | 1;
     for (int n = top + 1; n < n_mom; ++n) g[n * stride] = 0.0;
     double hi = 0.0, cur = 1e-200, even = 0.0;
     for (int n = top; n > 0; --n) {  // cur = J_n
@@ -1862,6 +1866,7 @@ template <int NV2>
 __global__ void __launch_bounds__(PD_DSUM_THREADS)
     pd_direction_sums(const double *__restrict__ slots, const double4 *__restrict__ dirs,
                       const PdFrameDev *__restrict__ frames, PdAmpShape sh, double qmax,
+                      const double *__restrict__ qv,
                       const PdClassDev *__restrict__ cls, const PdPairDev *__restrict__ pairs,
                       int32_t n_pairs, const int32_t *__restrict__ cls_ptr,
                       const int32_t *__restrict__ cls_chunk, int32_t width,
@@ -1886,9 +1891,11 @@ __global__ void __launch_bounds__(PD_DSUM_THREADS)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int LOADERS = PD_DSUM_WARPS - 1;
     if (warp == LOADERS) {  // one warp: the coefficients, while the others load
-        if (lane < nn)
-            s_scale[lane] = direction_coefficients(
-                direction_node(tile * NT + lane, fr.n_node, qmax) * fr.r1, M, s_g + lane, NT);
+        if (lane < nn) {
+            const int k = tile * NT + lane;
+            const double q = qv ? qv[k] : direction_node(k, fr.n_node, qmax);
+            s_scale[lane] = direction_coefficients(q * fr.r1, M, s_g + lane, NT);
+        }
         __syncwarp();
         for (int k = lane; k < 7 * nn; k += 32)
             direction_fold(s_g + k % nn, min(M, sh.dir_block), 1 + k / nn, NT);
@@ -2088,8 +2095,9 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
     const bool ok = q < sh.nq;
     constexpr bool weighted = NV == 4;
     const PdFrameDev fr = frames[f];
-    const bool nodes = fr.n_grp > 0;
-    const int M = nodes ? fr.n_node : fr.n_mom;
+    // M values per class-pair row: nodes, or moments of the pairs; 0: grid points
+    const bool dirs = fr.n_grp > 0, nodes = dirs && !sh.fp64;
+    const int M = nodes ? fr.n_node : (dirs ? 0 : fr.n_mom);
     const double *rows = red + static_cast<int64_t>(f) * sh.n_pairs * NV * sh.width;
     // the rows of pairs [p0, p0 + n): n·NV rows of M
     const int fit = M > 0 ? min(sh.n_pairs, PD_PROF_ROWS / (NV * M)) : 0;
@@ -2205,17 +2213,17 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
             double s[NV];
 #pragma unroll
             for (int v = 0; v < NV; ++v) s[v] = 0.0;
-            if (!nodes && pr.lat >= 0) {  // from the lattice set's pair counts (class mode, one frame)
+            if (!dirs && pr.lat >= 0) {  // from the lattice set's pair counts (class mode, one frame)
                 if (sub == 0 && ok) s[0] = lat_sums[static_cast<int64_t>(pr.lat) * sh.nq + q];
+            } else if (!(qval > 0.0)) {  // exact pair sums
+                if (sub == 0 && add_diag)
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) s[v] = pr.q0[v];
             } else if (M == 0) {
                 if (sub == 0 && ok)
 #pragma unroll
                     for (int v = 0; v < NV; ++v)
                         s[v] = rows[static_cast<int64_t>(p * NV + v) * sh.width + q];
-            } else if (!(qval > 0.0)) {  // exact pair sums
-                if (sub == 0 && add_diag)
-#pragma unroll
-                    for (int v = 0; v < NV; ++v) s[v] = pr.q0[v];
             } else {
                 const double *r = s_row + pl * NV * M;
 #pragma unroll 4
@@ -2268,7 +2276,7 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
 #pragma unroll
         for (int w = 0; w < PD_PROF_THREADS / 32; ++w) v += s_sum[w][t][ql];
         // a point off its lattice, or a frame whose form the plan has nothing for
-        if ((err && *err) || (sh.dir_only && !nodes)) v = __longlong_as_double(0x7ff8000000000000ll);
+        if ((err && *err) || (sh.dir_only && !dirs)) v = __longlong_as_double(0x7ff8000000000000ll);
         if (ok) terms[(static_cast<int64_t>(f) * 6 + t) * sh.nq + q] = v;
     }
 }
@@ -3275,7 +3283,7 @@ cudaError_t prepare_direction_rules() {
 
 cudaError_t launch_direction_sums(const double *slots, const double4 *dirs,
                                   const PdFrameDev *frames, const PdAmpShape &sh, double qmax,
-                                  int32_t n_frames, const PdClassDev *cls, const PdPairDev *pairs,
+                                  const double *qv, int32_t n_frames, const PdClassDev *cls, const PdPairDev *pairs,
                                   int32_t n_pairs, const int32_t *cls_ptr,
                                   const int32_t *cls_chunk, int32_t width,
                                   int add_exact, double *part, unsigned int *done, double *red,
@@ -3293,7 +3301,7 @@ cudaError_t launch_direction_sums(const double *slots, const double4 *dirs,
                         static_cast<unsigned>(std::min(n_frames - f0, 65535)));
         e = chain_launch(
             after, kern, grid, PD_DSUM_THREADS, smem, st, slots + f0 * sh.slot_cap, dirs + static_cast<int64_t>(f0) * sh.dir_cap, frames + f0, sh,
-            qmax, cls, pairs, n_pairs, cls_ptr, cls_chunk, width, add_exact,
+            qmax, qv, cls, pairs, n_pairs, cls_ptr, cls_chunk, width, add_exact,
             part + f0 * static_cast<int64_t>(sh.grp_cap) * n_pairs * nv * sh.node_cap,
             done + f0 * n_nt, red + f0 * static_cast<int64_t>(n_pairs) * nv * width);
         if (e != cudaSuccess) return e;

@@ -49,12 +49,13 @@ cudaError_t launch_pack(const double *xyz, const double *weights, const int32_t 
 // The quadrature rules of the direction form on the current device (before any
 // launch_pack there, and before a stream capture).
 cudaError_t prepare_direction_rules();
-// Direction form: class-pair sums at the nodes, from the chunks' moments, into
-// red (does nothing for frames in the other forms). part holds grp_cap·pairs·nv·
+// Direction form: class-pair sums at the nodes, or at the grid points qv if given, from
+// the chunks' moments, into red (does nothing for frames in the other forms). part holds grp_cap·pairs·nv·
 // node_cap doubles per frame, done one zeroed counter per node tile and frame.
 cudaError_t launch_direction_sums(const double *slots, const double4 *dirs,
                                   const PdFrameDev *frames, const PdAmpShape &sh, double qmax,
-                                  int32_t n_frames, const PdClassDev *cls, const PdPairDev *pairs,
+                                  const double *qv, int32_t n_frames, const PdClassDev *cls,
+                                  const PdPairDev *pairs,
                                   int32_t n_pairs, const int32_t *cls_ptr,
                                   const int32_t *cls_chunk, int32_t width,
                                   int add_exact, double *part, unsigned int *done, double *red, cudaStream_t st, bool after = false);

@@ -75,9 +75,9 @@ __device__ __forceinline__ int moments_needed(double z, bool fp64) {
 constexpr double PD_MOM_STRETCH = 1.03;
 
 // Direction form: orders kept of the rule and of the expansion; the tails are
-// below 1e-9 (FP32 form) and 1e-14 (FP64 form) of one pair's or atom's term.
+// below 1e-9 (FP32 form) and 1e-17 (FP64 form) of one pair's or atom's term.
 __device__ __forceinline__ double direction_order(double z, bool fp64) {
-    return fp64 ? bessel_order(z, 13.0, 3.0) : bessel_order(z, 8.0, 2.0);
+    return fp64 ? bessel_order(z, 15.0, 5.0) : bessel_order(z, 8.0, 2.0);
 }
 
 // A pair's sequences. U_j = (cos(cφ)/cos(φ/2), sin(cφ)/sin(φ/2)) at c = 8j + 3.5 steps by

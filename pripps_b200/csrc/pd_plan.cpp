@@ -681,10 +681,12 @@ __attribute__((optimize("O3"))) double max_radius(const double *xyz, int64_t n, 
     return best;
 }
 
-// Terms of a Bessel series of argument z (as bessel_order on the device).
+// Terms of a Bessel series of argument z, as direction_order on the device, and of
+// the interpolation nodes.
 static double series_order(double z, bool fp64) {
-    return fp64 ? z + 13.0 * std::cbrt(0.5 * z) + 3.0 : z + 8.0 * std::cbrt(0.5 * z) + 2.0;
+    return fp64 ? z + 15.0 * std::cbrt(0.5 * z) + 5.0 : z + 8.0 * std::cbrt(0.5 * z) + 2.0;
 }
+static double node_order(double z) { return z + 13.0 * std::cbrt(0.5 * z) + 3.0; }
 
 // Atom chunks of the direction form, longest first. A longer chunk means fewer sums
 // to hold and to add up, a shorter one more units to share: 2.5 units per block
@@ -754,7 +756,7 @@ static bool direction_only(Plan &P) {
         }
     }
     pair_cost *= 0.5 * static_cast<double>(P.n_atoms) * P.n_atoms;
-    pair_cost += moments ? PD_PAIRS_LATENCY : PD_GRID_LATENCY;
+    pair_cost += moments ? PD_PAIRS_LATENCY : P.mom.grid_latency;
     const bool use = P.amp.dir_cap > 0 && P.dir_cost < pair_cost;
     if (!use) {
         P.dir_only = false;
@@ -795,12 +797,15 @@ static void set_directions(Plan &P) {
     P.amp.n_cls = P.n_cls;
     P.amp.nv2 = P.mode == PD_MODE_WEIGHTED ? 2 : 1;
     P.amp.n_chunk = static_cast<int32_t>(P.chunks.size());
-    // Below 150 atoms the pairs are always fewer than the directions. The jobs
-    // carry the work units, so every rank needs jobs of every frame. The test
-    // hook (of the FP32 form) needs the pair tiles.
-    if (P.n_atoms < 150 || P.jobs_per_frame < 2 * static_cast<int64_t>(P.world) ||
-        (P.world > 1 && P.n_frames > 1) ||
-        (P.test_expire && P.precision != PD_FP64))
+    // Below 150 atoms the moments of the pairs are cheaper than the directions. In FP64 a
+    // grid point costs a double sin and a chain of them per atom (whole solves, 100
+    // points, pairs / directions: 8 atoms 71 / 59 us, 16 atoms 88 / 59, 100 atoms 233 /
+    // 59): only a handful of atoms stay pairs, whose sums have no quadrature. The jobs
+    // carry the work units, so every rank needs jobs of every frame. The test hook (of
+    // the FP32 form) needs the pair tiles.
+    const int64_t fewest = P.precision == PD_FP64 ? 12 : 150;
+    if (P.n_atoms < fewest || P.jobs_per_frame < 2 * static_cast<int64_t>(P.world) ||
+        (P.world > 1 && P.n_frames > 1) || (P.test_expire && P.precision != PD_FP64))
         return;
     // unknown coordinates: 20 cubic Angstrom per atom, elongated up to about 2.5 : 1
     const double radius =
@@ -820,7 +825,7 @@ static void set_directions(Plan &P) {
     const int64_t groups = (S + 31) / 32, mine = (groups + P.world - 1) / P.world;
     const int64_t m8 = (static_cast<int64_t>(mo) + 8) & ~int64_t{7};
     const double zn = 2.0 * r1 * P.qmax;
-    const int64_t nodes = static_cast<int64_t>(0.5 * series_order(zn, true)) + 1;
+    const int64_t nodes = fp64 ? P.nq : static_cast<int64_t>(0.5 * node_order(zn)) + 1;
     // The sums' kernel: a block's shared memory holds the coefficients and the
     // amplitudes of every class at a tile of nodes (16, or fewer while that leaves
     // SMs without a block), and the moments of as many classes as fit; up to
@@ -834,7 +839,8 @@ static void set_directions(Plan &P) {
     P.amp.sum_smem = static_cast<int32_t>(std::max(
         least, std::min<int64_t>(110 * 1024 / 8, m8 * tile + ncv * (tile * 64 + m8 * 32))));
     const int64_t slots = P.amp.n_chunk * P.amp.nv2 * mine * m8 * 32;
-    if (slots * 8 * P.n_frames > (int64_t{4} << 30)) return;
+    const int64_t parts = mine * P.n_pairs * P.nv * nodes;
+    if (std::max(slots, parts) * 8 * P.n_frames > (int64_t{4} << 30)) return;
     P.amp.dir_cap = static_cast<int32_t>(groups * 32);
     P.amp.grp_cap = static_cast<int32_t>(mine);
     P.amp.amp_cap = static_cast<int32_t>(std::min<int64_t>(m8, PD_MAX_DIR_MOMENTS));
@@ -878,12 +884,14 @@ void set_reduction(Plan &P) {
     const double points = static_cast<double>((P.nq + 15) & ~15);
     if (m.fp64) {
         m.grid_dir_cost = 0.29 * 110.0 * P.nqb * P.tun.K;
+        m.grid_latency = 8e6 * static_cast<double>(std::min<int64_t>(P.n_atoms, 256));
     } else {
         const bool weighted = P.mode == PD_MODE_WEIGHTED;
         m.grid_cost = (weighted ? 4.0 : 3.0) * points + 55.0 * P.nqb;
         m.mom_cost = weighted ? 2.1 : 1.25;
         m.mom_block_cost = weighted ? 72.0 + 2.0 * m.block : 60.0 + 0.625 * m.block;
         m.grid_dir_cost = 0.7 * m.grid_cost;
+        m.grid_latency = 4e7;
     }
     set_directions(P);
     m.dir_block = P.amp.dir_block;
@@ -909,9 +917,10 @@ void set_reduction(Plan &P) {
     r.block = m.block;
     r.max_moments = m.block ? m.max_moments : 0;
     r.n_z = (std::max(P.nq, r.max_moments) + 127) / 128;
-    r.max_moments = std::max(r.max_moments, P.amp.node_cap);
+    if (!m.fp64) r.max_moments = std::max(r.max_moments, P.amp.node_cap);
     r.node_cap = P.amp.node_cap;
     r.dir_only = m.dir_only;
+    r.fp64 = m.fp64;
     r.width = std::max(P.nq, r.max_moments);
     // A block adds its share of a class pair's slot list serially: lists of
     // more than a few hundred entries are shared by up to 16 blocks (one

@@ -100,7 +100,9 @@ CASES = ([("fp32", m, 4000, 400) for m in (16, 24, 32, 40, 48, 56)] +
          [("fp32", m, 6000, 400) for m in (64, 72, 80)] +
          [("fp32", m, 12000, 400) for m in (96, 104, 112)] +
          [("fp32", m, 18000, 400) for m in (120, 128)] +
-         [("fp32", 136, 20000, 600), ("fp32", 168, 30000, 800)])
+         [("fp32", 136, 20000, 600), ("fp32", 168, 30000, 800)] +
+         [("fp64", m, 1500, 400) for m in (24, 32, 40, 48, 56, 64, 72, 128)] +
+         [("fp64", m, 3000, 800) for m in (136, 176, 208)])
 
 
 # The direction kernels are compiled for every 8 (from 64 moments on 16) moments up to
@@ -145,6 +147,7 @@ def test_cheaper_form_for_few_grid_points(gpu_ctx):
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_frames_of_a_batch_take_their_own_form(gpu_ctx, precision):
     xyz = _globule(800)
-    frames = np.stack([xyz, 8.0 * xyz, xyz + 1.0])
+    far = 8.0 if precision == "fp32" else 12.0  # (a grid point costs a double sin)
+    frames = np.stack([xyz, far * xyz, xyz + 1.0])
     _, form, _ = _run(gpu_ctx, _request(frames, 0.6, 45, precision))
     assert form[0] == form[2] == DIRECTIONS and form[1] != DIRECTIONS, form

@@ -6,7 +6,10 @@ profiles, whose terms are products of doubles, are themselves 1e-14 off): a pair
 term is rounded to 2e-16 with random signs, a thread's run of up to 4,096 of them to
 about ten times that; twice their sum is allowed. (Sums over moments of the pairs of
 size N², or an interpolation between points of very different size, lose a digit or
-more.)
+more.) Directions: 1e-14; an amplitude is a sum over N atoms, rounded to 1e-16·√N and
+a few times that, of the size of √N where the profile is deep; that share of it
+averages over the directions, and the rule's weights and the Bessel coefficients add
+1e-15; a factor of three is to spare.
 """
 import numpy as np
 import pytest
@@ -15,7 +18,7 @@ from conftest import term_errors
 from pripps_b200.debye import DebyeRequest, solve
 
 pytestmark = pytest.mark.gpu
-TOL = 5e-15
+TOL, TOL_DIRECTIONS = 5e-15, 1e-14
 
 
 def _long_double(req, qi):
@@ -38,7 +41,7 @@ def _long_double(req, qi):
     return out
 
 
-def _check(xyz, qmax, nq, mode, ctx):
+def _check(xyz, qmax, nq, mode, ctx, tol=TOL):
     rng = np.random.default_rng(len(xyz))
     n = len(xyz)
     sp = rng.integers(0, 3, n)
@@ -52,7 +55,7 @@ def _check(xyz, qmax, nq, mode, ctx):
     got = solve(req, ctx)
     qi = np.unique(np.linspace(0, nq - 1, 10).astype(int))
     err = term_errors(got[:, qi], _long_double(req, qi))
-    assert np.all(err < TOL), err
+    assert np.all(err < tol), err
 
 
 def _rod(n, length):
@@ -67,3 +70,19 @@ def _rod(n, length):
                                               (100, 60.0, 0.8, 200)])
 def test_pairs(gpu_ctx, mode, n, length, qmax, nq):
     _check(_rod(n, length), qmax, nq, mode, gpu_ctx)
+
+
+@pytest.mark.parametrize("mode", ["vacuum", "class", "weighted"])
+@pytest.mark.parametrize("n,radius,ratio,qmax,nq", [(12, 4.0, 1.0, 0.5, 17), (60, 7.0, 1.0, 1.0, 100),
+                                                    (700, 14.0, 1.0, 0.5, 97),
+                                                    (1500, 18.0, 1.0, 0.6, 200),
+                                                    (1200, 17.0, 2.5, 1.0, 64),
+                                                    (1400, 12.0, 1.0, 4.0, 80)])
+def test_directions(gpu_ctx, mode, n, radius, ratio, qmax, nq):
+    """Balls and an ellipsoid of uniform density: their profiles have minima of 1e-3 to
+    1e-4 of the value at q = 0 (the last: several moment blocks)."""
+    rng = np.random.default_rng(n)
+    v = rng.normal(size=(n, 3))
+    xyz = radius * v / np.linalg.norm(v, axis=1)[:, None] * rng.random((n, 1)) ** (1 / 3)
+    _check(xyz * np.array([ratio, ratio ** -0.5, ratio ** -0.5]), qmax, nq, mode, gpu_ctx,
+           TOL_DIRECTIONS)

@@ -628,12 +628,12 @@ int finish_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st,
         ctx->launches += 1;
         after = true;
     }
-    if (!P.lat.empty() && !P.dir_only) {
+    if (!P.lat.empty()) {
         PD_CUDA(ctx, pd::launch_lattice_sums(
                          reinterpret_cast<const unsigned long long *>(dp.dptr<char>(L.hist)),
                          dp.dptr<PdLatDev>(L.lat), static_cast<int>(P.lat.size()),
                          dp.dptr<double>(L.qv), P.nq, add_exact, dp.dptr<int>(L.lat_err),
-                         dp.dptr<PdFrameDev>(L.frames), dp.dptr<double>(L.lat_sums), st));
+                         dp.dptr<double>(L.lat_sums), st));
         ctx->launches += 1;
         after = false;  // (the lattice kernels are outside the chain)
     }
@@ -684,8 +684,7 @@ int pack_devplan(pd_ctx *ctx, DevPlan &dp, cudaStream_t st) {
                                         static_cast<int64_t>(P.lat_tiles.size()),
                                         dp.dptr<int4>(L.lat_idx),
                                         reinterpret_cast<unsigned long long *>(dp.dptr<char>(L.hist)),
-                                        P.lat_bins, dp.dptr<int>(L.lat_err),
-                                        dp.dptr<PdFrameDev>(L.frames), st));
+                                        P.lat_bins, dp.dptr<int>(L.lat_err), st));
         ctx->launches += P.lat_tiles.empty() ? 1 : 2;
     }
     return PD_OK;

@@ -142,6 +142,7 @@ struct PdMomentRule {
     int32_t rank, world;
     int64_t slot_cap;     // doubles per frame for the chunks' sums
     int64_t n_atoms;
+    double n_tile_pairs;  // pairs of a frame that the tiles sum (not a lattice set's own)
     int32_t nq;
     int32_t dir_only;     // the plan has no tiles: every frame takes the direction form
 };

@@ -1445,7 +1445,7 @@ __device__ __forceinline__ void frame_constants(double radius, const PdMomentRul
             pair_cost = 56.0 * blocks + 1.5 * m8;
         }
     }
-    pair_cost *= 0.5 * static_cast<double>(rule.n_atoms) * rule.n_atoms;
+    pair_cost *= rule.n_tile_pairs;
     pair_cost += fr.n_mom > 0 ? PD_PAIRS_LATENCY : rule.grid_latency;
     // ---- directions: 2h Gauss rings (upper half: h), enough points on each
     if (rule.dir_cap == 0) {
@@ -2213,7 +2213,7 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
             double s[NV];
 #pragma unroll
             for (int v = 0; v < NV; ++v) s[v] = 0.0;
-            if (!dirs && pr.lat >= 0) {  // from the lattice set's pair counts (class mode, one frame)
+            if (pr.lat >= 0) {  // from the lattice set's pair counts (class mode, one frame)
                 if (sub == 0 && ok) s[0] = lat_sums[static_cast<int64_t>(pr.lat) * sh.nq + q];
             } else if (!(qval > 0.0)) {  // exact pair sums
                 if (sub == 0 && add_diag)
@@ -2319,10 +2319,8 @@ __global__ void __launch_bounds__(128) pd_lattice_hist(const PdLatTile *__restri
                                                        const PdLatDev *__restrict__ lat,
                                                        const int4 *__restrict__ idx,
                                                        unsigned long long *__restrict__ hist,
-                                                       const PdFrameDev *__restrict__ frames,
                                                        int shared_bins) {
     extern __shared__ unsigned int s_hist[];
-    if (frames[0].n_grp > 0) return;  // direction form: no pairs are counted
     const PdLatTile t = tiles[blockIdx.x];
     const PdLatDev d = lat[t.lat];
     const bool use_shared = shared_bins > 0;
@@ -2354,17 +2352,16 @@ __global__ void __launch_bounds__(128) pd_lattice_hist(const PdLatTile *__restri
 // Σ_{i<j} sinc(q r_ij) = Σ_n count(n)·sinc(q·spacing·√n), FP64, one CTA per
 // (q, lattice); each thread adds the bins n ≡ thread (mod 256) in ascending
 // order and a fixed tree adds the threads, so the sum is deterministic. The
-// values are sums[lattice][q] (the pair tiles skip those pairs). Only the rank
+// values are sums[lattice][q] (the pair tiles skip those pairs; where directions are
+// summed, whose FP32 terms these counts are exact beside, their own sum goes unused). Only the rank
 // that adds the exact terms writes a sum; the others write 0. *err set: NaN.
 __global__ void __launch_bounds__(256) pd_lattice_sums(const unsigned long long *__restrict__ hist,
                                                        const PdLatDev *__restrict__ lat,
                                                        const double *__restrict__ qv, int32_t nq,
                                                        int32_t add_exact,
                                                        const int *__restrict__ err,
-                                                       const PdFrameDev *__restrict__ frames,
                                                        double *__restrict__ sums) {
     __shared__ double s_part[256];
-    if (frames[0].n_grp > 0) return;  // direction form
     const int q = blockIdx.x;
     const PdLatDev d = lat[blockIdx.y];
     const double qval = qv[q];
@@ -3349,7 +3346,7 @@ cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdC
 cudaError_t launch_lattice(const double *xyz, const int32_t *perm, const PdLatDev *lat_dev,
                            const PdLatDev *lat_host, int n_lat, const PdLatTile *tiles,
                            int64_t n_tiles, int4 *idx, unsigned long long *hist, int64_t n_bins,
-                           int *err, const PdFrameDev *frames, cudaStream_t st) {
+                           int *err, cudaStream_t st) {
     if (n_lat == 0) return cudaSuccess;
     cudaError_t e = cudaMemsetAsync(hist, 0, static_cast<size_t>(n_bins) * 8, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, sizeof(int), st);
@@ -3379,16 +3376,15 @@ cudaError_t launch_lattice(const double *xyz, const int32_t *perm, const PdLatDe
         }
     }
     pd_lattice_hist<<<static_cast<unsigned>(n_tiles), 128, smem, st>>>(tiles, lat_dev, idx, hist,
-                                                                        frames, shared_bins);
+                                                                        shared_bins);
     return cudaGetLastError();
 }
 
 cudaError_t launch_lattice_sums(const unsigned long long *hist, const PdLatDev *lat, int n_lat,
                                 const double *qv, int32_t nq, int add_exact, const int *err,
-                                const PdFrameDev *frames, double *sums, cudaStream_t st) {
+                                double *sums, cudaStream_t st) {
     if (n_lat == 0) return cudaSuccess;
-    pd_lattice_sums<<<dim3(nq, n_lat), 256, 0, st>>>(hist, lat, qv, nq, add_exact, err, frames,
-                                                       sums);
+    pd_lattice_sums<<<dim3(nq, n_lat), 256, 0, st>>>(hist, lat, qv, nq, add_exact, err, sums);
     return cudaGetLastError();
 }
 

@@ -77,10 +77,10 @@ cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdC
 cudaError_t launch_lattice(const double *xyz, const int32_t *perm, const PdLatDev *lat_dev,
                            const PdLatDev *lat_host, int n_lat, const PdLatTile *tiles,
                            int64_t n_tiles, int4 *idx, unsigned long long *hist, int64_t n_bins,
-                           int *err, const PdFrameDev *frames, cudaStream_t st);
+                           int *err, cudaStream_t st);
 cudaError_t launch_lattice_sums(const unsigned long long *hist, const PdLatDev *lat, int n_lat,
                                 const double *qv, int32_t nq, int add_exact, const int *err,
-                                const PdFrameDev *frames, double *sums, cudaStream_t st);
+                                double *sums, cudaStream_t st);
 cudaError_t launch_frame_mean(const double *terms, const double *fw, int32_t n_frames, int32_t nq,
                               double *out, cudaStream_t st, bool normalize = true, bool after = false);
 // Direct transform: (Re A, Im A, |A|², Σ_m |F_m|²) per q-vector for points

@@ -191,8 +191,10 @@ int pd_plan_forms(pd_ctx *ctx, pd_plan *plan, uint32_t *form, uint32_t *moments)
  * tile in cost order). Each execution then yields partial profiles whose sum
  * over the ranks is the full [6][nq] result — rank 0 also carries the i = j
  * terms and the exact q = 0 sums — so the caller adds them across devices
- * (one all-reduce of 6·nq doubles). world = 1 restores the whole plan. No
- * reference counterpart (the reference is single-process). */
+ * (one all-reduce of 6·nq doubles). Ranks create their contexts with the same
+ * memory budget: a plan sums directions on every rank or, where their arrays do
+ * not fit, pairs on every rank. world = 1 restores the whole plan. No reference
+ * counterpart (the reference is single-process). */
 int pd_plan_set_shard(pd_ctx *ctx, pd_plan *plan, uint32_t rank, uint32_t world);
 
 /* Host-only view of a request's tiles in rank's share: five int32 per tile

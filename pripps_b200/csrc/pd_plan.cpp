@@ -809,7 +809,8 @@ static void set_directions(Plan &P) {
     // carry the work units, so every rank needs jobs of every frame. The test hook (of
     // the FP32 form) needs the pair tiles.
     const int64_t fewest = P.precision == PD_FP64 ? 12 : 150;
-    if (P.n_atoms < fewest || P.jobs_per_frame < 2 * static_cast<int64_t>(P.world) ||
+    if (P.no_directions || P.n_atoms < fewest ||
+        P.jobs_per_frame < 2 * static_cast<int64_t>(P.world) ||
         (P.world > 1 && P.n_frames > 1) || (P.test_expire && P.precision != PD_FP64))
         return;
     // unknown coordinates: 20 cubic Angstrom per atom, elongated up to about 2.5 : 1
@@ -861,10 +862,8 @@ static void set_directions(Plan &P) {
 }
 
 void drop_directions(Plan &P) {
-    P.amp.dir_cap = P.amp.grp_cap = P.amp.amp_cap = P.amp.node_cap = 0;
-    P.amp.slot_cap = 0;
-    P.mom.dir_cap = P.mom.grp_cap = P.mom.amp_cap = P.mom.node_cap = 0;
-    P.mom.slot_cap = 0;
+    P.no_directions = true;
+    set_reduction(P);
 }
 
 void set_reduction(Plan &P) {

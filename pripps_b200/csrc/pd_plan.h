@@ -70,6 +70,7 @@ struct Plan {
     // Host coordinates whose exact radius makes the direction form the cheaper
     // one: no tiles, slots or lists; the jobs only carry the direction units.
     bool dir_only = false;
+    bool no_directions = false;  // given up (drop_directions); a shard's share inherits it
     double dir_cost = 0.0;   // FP32 lane operations of a frame in the direction form
     int64_t dir_units = 0;   // its work units
     double job_cost = 0.0;   // relative cost of a job (dir_only)
@@ -120,7 +121,8 @@ int build_plan(const pd_request *req, const uint32_t *species_host, const double
 // below the same taken with the centroid summed in another order.
 double max_radius(const double *xyz, int64_t n_atoms, int64_t n_frames);
 
-// Give up the direction form's arrays (a request that only fits without them).
+// Give up the direction form (a request that only fits without its arrays), also in
+// every shard of the plan: the ranks' partial sums are of one form.
 void drop_directions(Plan &P);
 
 }  // namespace pd

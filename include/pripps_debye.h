@@ -402,13 +402,14 @@ int pd_tuning_check(const char *path, uint64_t *n_entries);
 int pd_plan_inspect(pd_ctx *ctx, const pd_request *req, uint64_t *n_classes,
                     uint64_t *n_padded, uint64_t *n_tiles, uint64_t *pairs_covered);
 
-/* Host-only: device bytes one solve of `req` holds with the tuning the
- * context would pick (ctx may be NULL: default tuning), in the form that sums
- * pairs: a request that needs more than the budget allows is refused. (A solve
- * that sums directions instead holds its own arrays, where those fit too.) host_coordinates != 0
- * counts the device copy of the coordinates that pd_solve and pd_submit make;
- * 0 is the layout of a plan execution or of pd_solve_noalloc, whose
- * coordinates are the caller's device memory. No reference counterpart. */
+/* Host-only: the least device bytes one solve of `req` can run in with the
+ * tuning the context would pick (ctx may be NULL: default tuning): a request that
+ * needs more than the budget allows is refused. Where there is room a solve
+ * holds more (the arrays of the direction form, shared sums).
+ * host_coordinates != 0 counts the device copy of the coordinates that
+ * pd_solve and pd_submit make; 0 is the layout of a plan execution or of
+ * pd_solve_noalloc, whose coordinates are the caller's device memory. No
+ * reference counterpart. */
 int pd_request_device_bytes(pd_ctx *ctx, const pd_request *req, int host_coordinates,
                             uint64_t *device_bytes);
 
@@ -454,7 +455,7 @@ uint64_t pd_launch_count(pd_ctx *ctx);
  *    the tuning table picks for the request's bucket as well as on N and
  *    nq. As a guide, at nq = 1,000 an FP32 solve with solvent and one
  *    hydration weight per element fits up to roughly 130,000 atoms (the
- *    100,000-atom ellipsoid needs 53 MB) and 200,000 atoms are refused;
+ *    100,000-atom ellipsoid needs 48 MB) and 200,000 atoms are refused;
  *    with a hydration weight per atom (four partial sums per grid point)
  *    up to about 20,000 atoms fit, and larger requests may not.
  *  - The array occupies PD_NOALLOC_SCRATCH_BYTES of memory on every GPU that

@@ -88,6 +88,7 @@ Layout make_layout(const Plan &P, bool host_xyz) {
         o = align_up(o + std::max<uint64_t>(bytes, 1), 256);
         return at;
     };
+    auto some = [&](uint64_t bytes) { return bytes ? take(bytes) : o; };  // may be empty
     const uint64_t nq = P.nq, S = P.n_species;
     L.qv = take(nq * 8);
     L.ffA = take(S * nq * 8);
@@ -107,51 +108,69 @@ Layout make_layout(const Plan &P, bool host_xyz) {
     L.xyz = take(host_xyz ? static_cast<uint64_t>(P.n_atoms) * 3 * P.n_frames * 8 : 0);
     L.lat = take(P.lat.size() * sizeof(PdLatDev));
     L.lat_tiles = take(P.lat_tiles.size() * sizeof(PdLatTile));
-    L.chunks = take(P.chunks.size() * sizeof(PdChunk));
-    L.cls_ptr = take(P.cls_ptr.size() * 4);
-    L.cls_chunk = take(P.cls_chunk.size() * 4);
+    const bool dirs = P.amp.dir_cap > 0;
+    L.chunks = some(dirs ? P.chunks.size() * sizeof(PdChunk) : 0);
+    L.cls_ptr = some(dirs ? P.cls_ptr.size() * 4 : 0);
+    L.cls_chunk = some(dirs ? P.cls_chunk.size() * 4 : 0);
     L.upload_bytes = o;
     L.hres = o;
     L.stage_bytes = align_up(o + 6 * nq * 8 + 8, 256);  // result and status land here
     const uint64_t F = static_cast<uint64_t>(P.n_frames);
-    L.centroid = take(F * 3 * 8);
-    L.cent_part = take(F * pd::centroid_blocks(P.n_atoms) * 3 * 8);
     L.frames = take(F * sizeof(PdFrameDev));
     L.atoms = take(static_cast<uint64_t>(P.n_pad) * P.n_frames *
                    (P.precision == PD_FP64 ? sizeof(double4) : sizeof(float4)));
-    // the tiles' slots and the direction form's chunk sums: one region for both where
-    // the only frame takes one of them, two where a batch may hold frames of both
-    const uint64_t b_tile = static_cast<uint64_t>(P.slots_per_frame) * P.nv * P.tun.K * F * 8,
+    // One region for what is dead before the next is written: the centroids' parts (pack),
+    // the tiles' slots, a batch's profiles before their mean; and the direction form's
+    // chunk sums where the only frame takes one of the two forms (a batch may hold
+    // frames of both).
+    const uint64_t b_cent = F * 3 * 8 * (1 + pd::centroid_blocks(P.n_atoms)),
+                   b_tile = static_cast<uint64_t>(P.slots_per_frame) * P.nv * P.tun.K * F * 8,
+                   b_terms = F > 1 ? F * 6 * nq * 8 : 0,
                    b_dir = static_cast<uint64_t>(P.amp.slot_cap) * F * 8;
-    L.slots = take(F > 1 ? b_tile : std::max(b_tile, b_dir));
-    L.dir_slots = F > 1 ? take(b_dir) : L.slots;
+    L.slots = take(std::max({b_cent, b_tile, b_terms, F > 1 ? 0 : b_dir}));
+    L.dir_slots = F > 1 ? some(b_dir) : L.slots;
+    L.centroid = L.terms = L.slots;
+    L.cent_part = L.slots + F * 3 * 8;
     const PdReduceShape &sh = P.red;
     const uint64_t red_rows = F * static_cast<uint64_t>(P.n_pairs);
     L.red = take(red_rows * P.nv * sh.width * 8);
     L.chunk_sums =
-        take(sh.n_chunk > 1 ? red_rows * sh.n_z * sh.n_chunk * P.nv * 128 * 8 : 0);
-    L.terms = take(static_cast<uint64_t>(P.n_frames) * 6 * nq * 8);
+        some(sh.n_chunk > 1 ? red_rows * sh.n_z * sh.n_chunk * P.nv * 128 * 8 : 0);
     L.out = take(6 * nq * 8 + 8);
     L.status = L.out + 6 * nq * 8;
-    L.ctl = o;
-    L.rad2 = take(F * 8);
-    L.counter = take(2 * sizeof(int));  // next job, next direction unit
-    L.cent_done = take(F * 4);
-    L.pack_done = take(F * 4);
-    L.red_done = take(sh.n_chunk > 1 ? red_rows * sh.n_z * 4 : 0);
-    const uint64_t n_nt =
-        P.amp.dir_cap ? (P.amp.node_cap + P.amp.node_tile - 1) / P.amp.node_tile : 0;
-    L.dir_done = take(F * n_nt * 4);
-    L.ctl_bytes = o - L.ctl;
-    L.dirs = take(F * P.amp.dir_cap * sizeof(double4));
-    L.nodes = take(P.precision == PD_FP64 ? 0 : F * P.amp.node_cap * sizeof(double2));
-    L.dir_part = take(F * P.amp.grp_cap * static_cast<uint64_t>(P.n_pairs) * P.nv *
+    const uint64_t n_nt = dirs ? (P.amp.node_cap + P.amp.node_tile - 1) / P.amp.node_tile : 0;
+    L.ctl = L.rad2 = o;
+    L.counter = L.rad2 + F * 8;  // next job, next direction unit
+    L.cent_done = L.counter + 8;
+    L.pack_done = L.cent_done + F * 4;
+    L.red_done = L.pack_done + F * 4;
+    L.dir_done = L.red_done + (sh.n_chunk > 1 ? red_rows * sh.n_z * 4 : 0);
+    L.ctl_bytes = L.dir_done + F * n_nt * 4 - L.ctl;
+    take(L.ctl_bytes);
+    L.dirs = some(F * P.amp.dir_cap * sizeof(double4));
+    L.nodes = some(P.precision == PD_FP64 ? 0 : F * P.amp.node_cap * sizeof(double2));
+    L.dir_part = some(F * P.amp.grp_cap * static_cast<uint64_t>(P.n_pairs) * P.nv *
                       P.amp.node_cap * 8);
-    L.lat_sums = take(P.lat.size() * nq * 8);
+    L.lat_sums = some(P.lat.size() * nq * 8);
     L.lat_idx = take(P.lat.empty() ? 0 : static_cast<uint64_t>(P.n_pad) * sizeof(int4));
     L.hist = take(static_cast<uint64_t>(P.lat_bins) * 8);
     L.lat_err = take(sizeof(int));
     L.total = o;
+    return L;
+}
+
+// The layout of a plan with tiles that fits `bytes`, or the smallest one: with the
+// directions, as pairs alone, compact.
+Layout fit_layout(Plan &P, bool host_xyz, uint64_t bytes) {
+    Layout L = make_layout(P, host_xyz);
+    if (L.total > bytes && !P.dir_only) {
+        pd::drop_directions(P);
+        L = make_layout(P, host_xyz);
+    }
+    if (L.total > bytes && !P.dir_only) {
+        pd::make_compact(P);
+        L = make_layout(P, host_xyz);
+    }
     return L;
 }
 
@@ -467,9 +486,11 @@ void stage_structure(DevPlan &dp) {
         std::memcpy(dp.hptr<char>(L.lat_tiles), P.lat_tiles.data(),
                     P.lat_tiles.size() * sizeof(PdLatTile));
     }
-    std::memcpy(dp.hptr<char>(L.chunks), P.chunks.data(), P.chunks.size() * sizeof(PdChunk));
-    std::memcpy(dp.hptr<char>(L.cls_ptr), P.cls_ptr.data(), P.cls_ptr.size() * 4);
-    std::memcpy(dp.hptr<char>(L.cls_chunk), P.cls_chunk.data(), P.cls_chunk.size() * 4);
+    if (P.amp.dir_cap > 0) {
+        std::memcpy(dp.hptr<char>(L.chunks), P.chunks.data(), P.chunks.size() * sizeof(PdChunk));
+        std::memcpy(dp.hptr<char>(L.cls_ptr), P.cls_ptr.data(), P.cls_ptr.size() * 4);
+        std::memcpy(dp.hptr<char>(L.cls_chunk), P.cls_chunk.data(), P.cls_chunk.size() * 4);
+    }
     PdReqDev rd{};
     if (P.precision == PD_FP64)
         rd.atoms64 = dp.dptr<double4>(L.atoms);
@@ -504,10 +525,11 @@ double host_radius(const pd_request *req) {
 
 constexpr int kBudgetWait = -100;  // internal: does not fit the budget right now
 
-// Host planning only: tiles, lists and the device layout.
+// Host planning only: tiles, lists and the device layout, for `avail` bytes of device
+// memory if it can be (a request that needs more than the budget is refused).
 int plan_host(pd_ctx *ctx, const pd_request *req, const uint32_t *species, const double *weights,
-              bool host_xyz, double radius_hint, DevPlan &dp, const Tuning *force = nullptr,
-              bool exact_radius = false) {
+              bool host_xyz, double radius_hint, uint64_t avail, DevPlan &dp,
+              const Tuning *force = nullptr, bool exact_radius = false) {
     NvtxRange nvtx("pd plan (host)");
     std::string msg;
     const Tuning tun = force ? *force : tuning_for_request(ctx, req, species, weights);
@@ -521,24 +543,20 @@ int plan_host(pd_ctx *ctx, const pd_request *req, const uint32_t *species, const
         }
         // known coordinates: every frame sums directions (the plan has no tiles) or none
         if (exact_radius && !P.dir_only) pd::drop_directions(P);
-        L = make_layout(P, host_xyz);
+        L = fit_layout(P, host_xyz, avail);
         return PD_OK;
     };
     if (int rc = plan(dp.P, dp.L, exact_radius)) return rc;
     // without tiles only where the pair form would have fitted too
     if (dp.P.dir_only &&
-        static_cast<double>(dp.L.total) + dp.P.pair_bytes > static_cast<double>(ctx->budget)) {
+        static_cast<double>(dp.L.total) + dp.P.pair_bytes > static_cast<double>(avail)) {
         Plan P;
         Layout L;
         if (int rc = plan(P, L, false)) return rc;
-        if (L.total > ctx->budget || dp.L.total > ctx->budget) {
+        if (L.total > avail || dp.L.total > avail) {
             dp.P = std::move(P);
             dp.L = L;
         }
-    }
-    if (dp.L.total > ctx->budget) {  // the pair form alone may fit
-        pd::drop_directions(dp.P);
-        dp.L = make_layout(dp.P, host_xyz);
     }
     if (dp.L.total > ctx->budget) {
         ctx->set_error("request needs " + std::to_string(dp.L.total) +
@@ -591,8 +609,9 @@ int plan_device(pd_ctx *ctx, const pd_request *req, DevPlan &dp, cudaStream_t st
 int create_devplan(pd_ctx *ctx, const pd_request *req, const uint32_t *species,
                    const double *weights, bool host_xyz, double radius_hint, DevPlan &dp,
                    cudaStream_t st, const Tuning *force = nullptr, bool exact_radius = false) {
-    int rc = plan_host(ctx, req, species, weights, host_xyz, radius_hint, dp, force,
-                       exact_radius);
+    const uint64_t used = std::min(ctx->in_use.load(), ctx->budget);
+    int rc = plan_host(ctx, req, species, weights, host_xyz, radius_hint, ctx->budget - used, dp,
+                       force, exact_radius);
     if (rc) return rc;
     return plan_device(ctx, req, dp, st, false);
 }
@@ -922,7 +941,8 @@ void planner_main(pd_ctx *ctx) {
         std::string m;
         if (!t->canceled) {
             rc = plan_host(ctx, &t->req, t->req.species, t->req.hyd_weights, true,
-                           host_radius(&t->req), t->dp, nullptr, /*exact_radius=*/true);
+                           host_radius(&t->req), ctx->budget, t->dp, nullptr,
+                           /*exact_radius=*/true);
             if (rc != PD_OK) {
                 std::lock_guard<std::mutex> g(ctx->mu);
                 m = ctx->errors[std::this_thread::get_id()];
@@ -2271,8 +2291,7 @@ int pd_request_device_bytes(pd_ctx *ctx, const pd_request *req, int host_coordin
         if (ctx) ctx->set_error(msg);
         return rc;
     }
-    pd::drop_directions(P);
-    *device_bytes = make_layout(P, host_coordinates != 0).total;
+    *device_bytes = fit_layout(P, host_coordinates != 0, 0).total;
     return PD_OK;
 }
 
@@ -3169,11 +3188,7 @@ extern "C" int pd_solve_noalloc(const pd_request *req, const double *xyz_dev,
     Tuning tun = tuning_for_request(nullptr, &r, r.species, r.hyd_weights);
     rc = pd::build_plan(&r, r.species, r.hyd_weights, tun, dp.P, msg);
     if (rc) return noalloc_fail(rc, "pd_solve_noalloc: " + msg);
-    dp.L = make_layout(dp.P, false);
-    if (dp.L.total > PD_NOALLOC_SCRATCH_BYTES) {  // the pair form alone may fit
-        pd::drop_directions(dp.P);
-        dp.L = make_layout(dp.P, false);
-    }
+    dp.L = fit_layout(dp.P, false, PD_NOALLOC_SCRATCH_BYTES);
     if (dp.L.total > PD_NOALLOC_SCRATCH_BYTES)
         return noalloc_fail(PD_EBUDGET,
                             "pd_solve_noalloc: the request needs " + std::to_string(dp.L.total) +

@@ -45,17 +45,16 @@ struct PdJob {
     int32_t req;    // request index within the launch
     int32_t frame;  // frame of the request
     int32_t i0;     // first padded i index (multiple of PD_IBLOCK)
-    int32_t j0, j1; // padded j range [j0, j1): real atoms of one class
+    int32_t j0, j1; // padded j range [j0, j1): real atoms of one class; of a plan without
+                    // tiles: the job's ordinal in its frame, and the frame's jobs
     int32_t qb;     // q-block index
     // bits 0..47: first output slot of this tile; bits 48..55: the slot of
     // each warp relative to it, 2 bits per warp (warp w at bits 48 + 2w).
     // Warps of one class share a slot; slot numbers follow the first warp
     // of each class, so warp 0 always has relative slot 0.
     int64_t slot;
-    int32_t ord;    // ordinal among the frame's jobs (direction form)
-    int32_t n_ord;  // jobs of the frame
 };
-static_assert(sizeof(PdJob) == 40, "PdJob layout");
+static_assert(sizeof(PdJob) == 32, "PdJob layout");
 constexpr int PD_SLOT_MAP_SHIFT = 48;
 constexpr int64_t PD_SLOT_MASK = (int64_t{1} << PD_SLOT_MAP_SHIFT) - 1;
 
@@ -196,7 +195,7 @@ struct PdReqDev {
 // Per-class constants for the combine kernel.
 struct PdClassDev {
     int32_t species;
-    int32_t pad;
+    int32_t lat;   // lattice set whose pair counts give the class's self pair sum, or -1
     double n;   // atoms in the class
     double w;   // hydration weight (class mode)
     double w1;  // Σ w_i over the class (weighted mode)
@@ -207,8 +206,6 @@ struct PdClassDev {
 // (sinc = 1 for every pair): count, Σ w_i, Σ w_j, Σ w_i w_j.
 struct PdPairDev {
     int32_t a, b;
-    int32_t lat;   // lattice set whose pair counts give this self pair sum, or -1
-    int32_t pad;
     double q0[4];
 };
 

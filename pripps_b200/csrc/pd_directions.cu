@@ -278,7 +278,7 @@ __device__ __forceinline__ int dir_unit(const DirUnit &un, const DirUnit &next,
 
 // Persistent blocks. plan_frames > 0: the units of every frame of one request
 // (reqs[0]) are taken by number (counter[1]); 0: the jobs of any requests, each a
-// share of its frame's units (every n_ord-th from ord on). Frames in the other forms
+// share of its frame's units (every j1-th from j0 on). Frames in the other forms
 // are passed over. Thread 0 draws the numbers and describes the next unit while the
 // block sums the current one; a plan's frames (512 at a time) and chunks are kept in
 // shared memory for that.
@@ -386,11 +386,11 @@ __device__ __forceinline__ void dir_units(const PdJob *__restrict__ jobs,
             n_units = n_grp == 0 ? 0
                                  : dir_unit_count(rq.amp.n_chunk, rq.amp.nv2,
                                                   (n_amp + MBLOCK - 1) / MBLOCK, n_grp);
-            u = jb.ord;
+            u = jb.j0;
         }
         const PdReqDev &rq = reqs[jb.req];
         dir_unit_set<Atom>(d, rq, rq.chunks, jb.frame, n_grp, n_amp, u);
-        u += jb.n_ord;
+        u += jb.j1;
         return true;
     });
 }

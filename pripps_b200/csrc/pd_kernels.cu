@@ -2213,8 +2213,9 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
             double s[NV];
 #pragma unroll
             for (int v = 0; v < NV; ++v) s[v] = 0.0;
-            if (pr.lat >= 0) {  // from the lattice set's pair counts (class mode, one frame)
-                if (sub == 0 && ok) s[0] = lat_sums[static_cast<int64_t>(pr.lat) * sh.nq + q];
+            const int lat = pr.a == pr.b ? cls[pr.a].lat : -1;
+            if (lat >= 0) {  // from the lattice set's pair counts (class mode, one frame)
+                if (sub == 0 && ok) s[0] = lat_sums[static_cast<int64_t>(lat) * sh.nq + q];
             } else if (!(qval > 0.0)) {  // exact pair sums
                 if (sub == 0 && add_diag)
 #pragma unroll

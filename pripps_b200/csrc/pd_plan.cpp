@@ -424,6 +424,7 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
                 s1 += wr;
                 s2 += wr * wr;
             }
+        P.cls[k].lat = lat_of_cls[k];
         P.cls[k].n = static_cast<double>(nk);
         P.cls[k].w1 = s1;
         P.cls[k].w2 = s2;
@@ -440,7 +441,6 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
             PdPairDev pd{};
             pd.a = a;
             pd.b = b;
-            pd.lat = a == b ? lat_of_cls[a] : -1;
             const double na = P.cls[a].n, nb = P.cls[b].n;
             if (a != b) {
                 pd.q0[0] = na * nb;
@@ -637,8 +637,6 @@ int build_plan(const pd_request *req, const uint32_t *species, const double *w,
             for (int f = 0; f < P.n_frames; ++f) {
                 PdJob jb = frame_jobs[o * P.nqb + qb];
                 jb.frame = f;
-                jb.ord = static_cast<int32_t>(P.jobs.size() / P.n_frames);
-                jb.n_ord = static_cast<int32_t>(P.jobs_per_frame);
                 jb.slot += static_cast<int64_t>(f) * P.slots_per_frame;
                 P.jobs.push_back(jb);
             }
@@ -784,8 +782,8 @@ static bool direction_only(Plan &P) {
             PdJob &jb = P.jobs[static_cast<size_t>(o) * P.n_frames + f];
             jb = PdJob{};
             jb.frame = f;
-            jb.ord = static_cast<int32_t>(o);
-            jb.n_ord = static_cast<int32_t>(per);
+            jb.j0 = static_cast<int32_t>(o);
+            jb.j1 = static_cast<int32_t>(per);
         }
     return true;
 }
@@ -866,6 +864,11 @@ void drop_directions(Plan &P) {
     set_reduction(P);
 }
 
+void make_compact(Plan &P) {
+    P.no_directions = P.compact = true;
+    set_reduction(P);
+}
+
 void set_reduction(Plan &P) {
     PdMomentRule &m = P.mom;
     m = PdMomentRule{};
@@ -874,7 +877,9 @@ void set_reduction(Plan &P) {
     m.fp64 = P.precision == PD_FP64 ? 1 : 0;
     m.block = m.fp64 ? 0 : pd_moment_block(P.tun.K);
     m.max_moments = static_cast<int32_t>(
-        std::min<int64_t>(PD_MAX_MOMENTS, static_cast<int64_t>(P.nqb) * m.block) & ~int64_t{7});
+        std::min<int64_t>({PD_MAX_MOMENTS, static_cast<int64_t>(P.nqb) * m.block,
+                           P.compact ? P.nq : PD_MAX_MOMENTS}) & ~int64_t{7});
+    if (m.max_moments < 8) m.block = 0;
     // As measured, whole solves of 3,000 to 20,000 atoms, FP32, in units of 83 % of the
     // FFMA peak: 3 lane operations per grid point (in 16s) and 55 for each q-block's
     // seeds, against 1.25 per moment and 140 for a block of 128 (sequences and flush);
@@ -936,7 +941,7 @@ void set_reduction(Plan &P) {
     for (int p = 0; p < P.n_pairs; ++p)
         longest = std::max(longest, P.lptr[static_cast<size_t>(p + 1) * P.nqb] -
                                         P.lptr[static_cast<size_t>(p) * P.nqb]);
-    r.n_chunk = P.n_frames > 1 ? 1
+    r.n_chunk = P.n_frames > 1 || P.compact ? 1
                                : static_cast<int32_t>(
                                      std::min<int64_t>(std::max<int64_t>(longest / 256, 1), 16));
     r.slots_per_frame = P.slots_per_frame;
@@ -985,10 +990,6 @@ int shard_plan(const Plan &full, uint32_t rank, uint32_t world, Plan &out) {
         }
         out.lptr[e + 1] = static_cast<int64_t>(out.lidx.size());
     }
-    // ordinals among the rank's own jobs of each frame
-    std::vector<int32_t> count(static_cast<size_t>(out.n_frames), 0);
-    for (PdJob &jb : out.jobs) jb.ord = count[static_cast<size_t>(jb.frame)]++;
-    for (PdJob &jb : out.jobs) jb.n_ord = count[static_cast<size_t>(jb.frame)];
     set_reduction(out);
     return PD_OK;
 }

@@ -71,6 +71,7 @@ struct Plan {
     // one: no tiles, slots or lists; the jobs only carry the direction units.
     bool dir_only = false;
     bool no_directions = false;  // given up (drop_directions); a shard's share inherits it
+    bool compact = false;        // the least memory (make_compact)
     double dir_cost = 0.0;   // FP32 lane operations of a frame in the direction form
     int64_t dir_units = 0;   // its work units
     double job_cost = 0.0;   // relative cost of a job (dir_only)
@@ -124,5 +125,9 @@ double max_radius(const double *xyz, int64_t n_atoms, int64_t n_frames);
 // Give up the direction form (a request that only fits without its arrays), also in
 // every shard of the plan: the ranks' partial sums are of one form.
 void drop_directions(Plan &P);
+
+// The least device memory that the request can run in: pairs, no more moments than
+// grid points, every slot list summed by one block.
+void make_compact(Plan &P);
 
 }  // namespace pd

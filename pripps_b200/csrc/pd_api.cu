@@ -2433,49 +2433,61 @@ struct LineSet {
     std::vector<uint32_t> slot;     // per given vector: j·n_line + line
 };
 
+// A vector's place: the line (its primitive direction, or the fixed indices) above the
+// position on it, 11 bits each; the next position of a line is the next key.
 struct LineKey {
-    int32_t d[3];  // the line: direction (primitive), or the fixed indices
-    int32_t p;     // position on it
-    uint32_t i;    // vector
+    uint64_t key;
+    uint32_t i;  // vector
 };
+constexpr int32_t LINE_BIAS = 512;  // |indices| are at most this
 
-// Sort keys of the vectors for one kind of line: axis < 0: multiples of a
-// primitive direction; else along that axis.
-void line_keys(const int32_t *hkl, uint64_t nv, int axis, std::vector<LineKey> &keys) {
-    keys.resize(nv);
-    for (uint64_t i = 0; i < nv; ++i) {
-        LineKey &k = keys[i];
-        k.i = static_cast<uint32_t>(i);
-        const int32_t *n = hkl + 3 * i;
-        if (axis < 0) {
-            int32_t g = std::gcd(std::gcd(std::abs(n[0]), std::abs(n[1])), std::abs(n[2]));
-            if (g == 0) g = 1;
-            for (int a = 0; a < 3; ++a) k.d[a] = n[a] / g;
-            k.p = g;
-        } else {
-            for (int a = 0; a < 3; ++a) k.d[a] = a == axis ? 0 : n[a];
-            k.p = n[axis];
-        }
-    }
-    std::sort(keys.begin(), keys.end(), [](const LineKey &x, const LineKey &y) {
-        if (x.d[0] != y.d[0]) return x.d[0] < y.d[0];
-        if (x.d[1] != y.d[1]) return x.d[1] < y.d[1];
-        if (x.d[2] != y.d[2]) return x.d[2] < y.d[2];
-        if (x.p != y.p) return x.p < y.p;
-        return x.i < y.i;
-    });
+uint64_t line_pack(int32_t x, int32_t y, int32_t z, int32_t p) {
+    const auto f = [](int32_t v) { return static_cast<uint64_t>(v + LINE_BIAS); };
+    return f(x) << 33 | f(y) << 22 | f(z) << 11 | f(p);
 }
 
-// Whether b continues the segment of a at the next position.
-bool line_next(const LineKey &a, const LineKey &b) {
-    return a.d[0] == b.d[0] && a.d[1] == b.d[1] && a.d[2] == b.d[2] && b.p == a.p + 1;
+// Key of a vector for one kind of line: axis < 0: multiples of a primitive
+// direction; else along that axis.
+uint64_t line_key(const int32_t *n, int axis) {
+    if (axis < 0) {
+        int32_t g = std::gcd(std::gcd(std::abs(n[0]), std::abs(n[1])), std::abs(n[2]));
+        if (g == 0) g = 1;
+        return line_pack(n[0] / g, n[1] / g, n[2] / g, g);
+    }
+    return line_pack(axis == 0 ? 0 : n[0], axis == 1 ? 0 : n[1], axis == 2 ? 0 : n[2], n[axis]);
+}
+
+// Keys of all vectors in ascending (key, vector) order.
+void line_keys(const int32_t *hkl, uint64_t nv, int axis, std::vector<LineKey> &keys) {
+    keys.resize(nv);
+    for (uint64_t i = 0; i < nv; ++i)
+        keys[i] = LineKey{line_key(hkl + 3 * i, axis), static_cast<uint32_t>(i)};
+    if (nv < 1024) {
+        std::sort(keys.begin(), keys.end(), [](const LineKey &x, const LineKey &y) {
+            return x.key != y.key ? x.key < y.key : x.i < y.i;
+        });
+        return;
+    }
+    std::vector<LineKey> other(nv);
+    for (int shift = 0; shift < 44; shift += 11) {  // stable counting sorts, low bits first
+        uint32_t at[2048] = {0};
+        for (const LineKey &k : keys) ++at[k.key >> shift & 2047];
+        uint32_t sum = 0;
+        for (uint32_t &c : at) {
+            const uint32_t n = c;
+            c = sum;
+            sum += n;
+        }
+        for (const LineKey &k : keys) other[at[k.key >> shift & 2047]++] = k;
+        keys.swap(other);
+    }
 }
 
 uint64_t line_segments(const std::vector<LineKey> &k) {
     uint64_t n = 0;
     int len = 0;
     for (size_t i = 0; i < k.size(); ++i) {
-        if (i == 0 || len == LINE_J || !line_next(k[i - 1], k[i])) {
+        if (i == 0 || len == LINE_J || k[i].key != k[i - 1].key + 1) {
             ++n;
             len = 0;
         }
@@ -2484,13 +2496,60 @@ uint64_t line_segments(const std::vector<LineKey> &k) {
     return n;
 }
 
+// Which kinds of line may have four vectors per segment: vectors whose predecessor on
+// the line is not in the list start a run, and runs may be a quarter of them. A sample of
+// the vectors is looked up in a hashed bitmap of all (16 bits each, so 6 % are found by
+// chance: the sorted keys decide). Scattered vectors cost 5 ns each this way; sorting
+// them by all four kinds first cost 590, four times what the table kernel's own order
+// costs (100,000 vectors: 59 ms).
+void line_kinds(const int32_t *hkl, uint64_t nv, bool (&maybe)[4]) {
+    uint64_t bits = 1024;
+    int shift = 64 - 10;
+    while (bits < 16 * nv) {
+        bits <<= 1;
+        --shift;
+    }
+    std::vector<uint64_t> map(bits / 64, 0);
+    const auto hash = [shift](uint64_t key) { return key * 0x9E3779B97F4A7C15ull >> shift; };
+    for (uint64_t i = 0; i < nv; ++i) {
+        const uint64_t h = hash(line_pack(hkl[3 * i], hkl[3 * i + 1], hkl[3 * i + 2], 0));
+        map[h >> 6] |= uint64_t{1} << (h & 63);
+    }
+    const uint64_t sample = std::min<uint64_t>(nv, 320);
+    uint64_t starts[4] = {0, 0, 0, 0};
+    for (uint64_t k = 0; k < sample; ++k) {
+        const uint64_t i = sample == nv ? k : k * 0x9E3779B97F4A7C15ull % nv;
+        const int32_t *n = hkl + 3 * i;
+        int32_t g = std::gcd(std::gcd(std::abs(n[0]), std::abs(n[1])), std::abs(n[2]));
+        if (g == 0) g = 1;
+        for (int kind = 0; kind < 4; ++kind) {  // axes 0 to 2, primitive direction
+            int32_t v[3] = {n[0], n[1], n[2]};
+            bool has = kind < 3 || g > 1;
+            if (kind < 3)
+                has = --v[kind] >= -LINE_BIAS;
+            else
+                for (int a = 0; a < 3; ++a) v[a] -= n[a] / g;
+            if (has) {
+                const uint64_t h = hash(line_pack(v[0], v[1], v[2], 0));
+                has = map[h >> 6] >> (h & 63) & 1;
+            }
+            starts[kind] += !has;
+        }
+    }
+    for (int kind = 0; kind < 4; ++kind)
+        maybe[kind] = static_cast<double>(starts[kind]) <= 0.30 * static_cast<double>(sample) + 1.0;
+}
+
 // False when the vectors lie on no lines worth the segments (fewer than four
 // vectors per segment: the table kernel reads less than the padded lines compute).
 bool find_lines(const int32_t *hkl, uint64_t nv, LineSet &out) {
+    bool maybe[4];
+    line_kinds(hkl, nv, maybe);
     std::vector<LineKey> keys, best;
     uint64_t fewest = ~uint64_t{0};
     int best_axis = -1;
     for (int axis : {-1, 2, 1, 0}) {
+        if (!maybe[axis < 0 ? 3 : axis]) continue;
         line_keys(hkl, nv, axis, keys);
         const uint64_t n = line_segments(keys);
         if (n < fewest) {
@@ -2500,6 +2559,7 @@ bool find_lines(const int32_t *hkl, uint64_t nv, LineSet &out) {
         }
         if (fewest * 10 <= nv) break;  // ten of 16 lanes: good enough to stop looking
     }
+    if (best.empty()) return false;
     if (fewest * 4 > nv || fewest > (uint64_t{1} << 26)) return false;
     std::vector<std::array<int32_t, 6>> raw;  // start, step
     out.slot.assign(nv, 0);
@@ -2507,11 +2567,13 @@ bool find_lines(const int32_t *hkl, uint64_t nv, LineSet &out) {
     int len = 0;
     for (size_t i = 0; i < best.size(); ++i) {
         const LineKey &k = best[i];
-        if (i == 0 || len == LINE_J || !line_next(best[i - 1], k)) {
+        if (i == 0 || len == LINE_J || k.key != best[i - 1].key + 1) {
             const int32_t *n = hkl + 3 * static_cast<size_t>(k.i);
             std::array<int32_t, 6> r{n[0], n[1], n[2], 0, 0, 0};
             for (int a = 0; a < 3; ++a)
-                r[3 + a] = best_axis < 0 ? k.d[a] : (a == best_axis ? 1 : 0);
+                r[3 + a] = best_axis < 0
+                               ? static_cast<int32_t>(k.key >> (33 - 11 * a) & 2047) - LINE_BIAS
+                               : (a == best_axis ? 1 : 0);
             raw.push_back(r);
             len = 0;
         }
@@ -2647,6 +2709,7 @@ int direct_run_lines(pd_ctx *ctx, const pd_direct_request *req, const LineSet &l
 // row costs more than the sincos it saves, and the vectors go to the sincos
 // kernel as q = 2π·hkl/L.
 constexpr int64_t kDirectTableMaxIndex = 512;
+static_assert(kDirectTableMaxIndex == LINE_BIAS, "line keys hold every index of the tables");
 
 }  // namespace
 

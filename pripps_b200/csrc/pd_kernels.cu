@@ -2822,22 +2822,27 @@ __global__ void __launch_bounds__(PD_DLINE_THREADS, 3)
     for (int j = 0; j < 2 * J; ++j) o[static_cast<int64_t>(j) * n_line] = s_f[j * T + tid];
 }
 
-// The points of each molecule (a block each) in stable order of their kinds: every
-// thread counts the kinds of a contiguous run, the counts are scanned kind by kind,
-// and the runs are scattered in order.
+// The points of each molecule in stable order of their kinds, within pieces of up to
+// PD_DSORT_PIECE points (a block each; a slice of the line kernel meets a kind once per
+// piece): every thread counts the kinds of a contiguous run, the counts are scanned kind
+// by kind, and the runs are scattered in order. One piece of a whole molecule would
+// leave a large one to a single SM (1,000,000 points, whole call: 9.2 -> 5.1 ms).
+constexpr int64_t PD_DSORT_PIECE = 4096;
 constexpr int PD_DSORT_THREADS = 256;
 
 __global__ void __launch_bounds__(PD_DSORT_THREADS)
     pd_direct_sort(const double *__restrict__ xyz, const uint32_t *__restrict__ kind,
-                   const double *__restrict__ weight, int64_t mol_size, int32_t n_kinds,
-                   double *__restrict__ xyz_out, uint32_t *__restrict__ kind_out,
-                   double *__restrict__ weight_out) {
+                   const double *__restrict__ weight, int64_t mol_size, int32_t n_piece,
+                   int32_t n_kinds, double *__restrict__ xyz_out,
+                   uint32_t *__restrict__ kind_out, double *__restrict__ weight_out) {
     constexpr int T = PD_DSORT_THREADS;
     extern __shared__ uint32_t s_cnt[];  // [kind][thread]
     __shared__ uint32_t s_scan[T];
-    const int64_t m0 = static_cast<int64_t>(blockIdx.x) * mol_size;
+    const int64_t mol = blockIdx.x / n_piece, part = blockIdx.x % n_piece;
+    const int64_t m0 = mol * mol_size + mol_size * part / n_piece;
+    const int64_t size = mol * mol_size + mol_size * (part + 1) / n_piece - m0;
     const int t = threadIdx.x;
-    const int64_t i0 = m0 + mol_size * t / T, i1 = m0 + mol_size * (t + 1) / T;
+    const int64_t i0 = m0 + size * t / T, i1 = m0 + size * (t + 1) / T;
     for (int k = 0; k < n_kinds; ++k) s_cnt[k * T + t] = 0;
     for (int64_t i = i0; i < i1; ++i) ++s_cnt[kind[i] * T + t];
     __syncthreads();
@@ -3519,9 +3524,12 @@ cudaError_t launch_direct_sort(const double *xyz, const uint32_t *kind, const do
                                double *xyz_out, uint32_t *kind_out, double *weight_out,
                                cudaStream_t st) {
     const size_t smem = static_cast<size_t>(n_kinds) * PD_DSORT_THREADS * sizeof(uint32_t);
-    if (smem > 46 * 1024 || n_points / mol_size > 0x7fffffffLL) return cudaErrorInvalidValue;
-    pd_direct_sort<<<static_cast<unsigned>(n_points / mol_size), PD_DSORT_THREADS, smem, st>>>(
-        xyz, kind, weight, mol_size, n_kinds, xyz_out, kind_out, weight_out);
+    const int64_t pieces = (mol_size + PD_DSORT_PIECE - 1) / PD_DSORT_PIECE;
+    const int64_t blocks = n_points / mol_size * pieces;
+    if (smem > 46 * 1024 || blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+    pd_direct_sort<<<static_cast<unsigned>(blocks), PD_DSORT_THREADS, smem, st>>>(
+        xyz, kind, weight, mol_size, static_cast<int32_t>(pieces), n_kinds, xyz_out, kind_out,
+        weight_out);
     return cudaGetLastError();
 }
 

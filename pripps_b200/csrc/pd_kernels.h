@@ -103,13 +103,13 @@ cudaError_t launch_direct_table(const double *xyz, const uint32_t *kind, const d
                                 cudaStream_t st);
 int64_t direct_blocks(int64_t n_points, int64_t mol_size, int64_t n_vec);
 // Direct transform at lattice vectors on lines of PD_DLINE_J (16) consecutive ones
-// (see pd_direct_lines): points sorted by kind within each molecule, ff
+// (see pd_direct_lines): points grouped by kind within each molecule, ff
 // [n_kinds][16][n_line], index the distinct indices of the three axes; part holds
 // 32·n_line doubles per chunk, out 4 per vector (j·n_line + line).
 int direct_line_points(int32_t n_entries);
 void direct_line_layout(int64_t n_points, int64_t mol_size, int32_t n_line, int64_t *chunk,
                         int64_t *spm);
-// Points of each molecule sorted by kind (n_kinds <= 44).
+// Points of each molecule sorted by kind, in pieces of a few thousand (n_kinds <= 44).
 cudaError_t launch_direct_sort(const double *xyz, const uint32_t *kind, const double *weight,
                                int64_t n_points, int64_t mol_size, int32_t n_kinds,
                                double *xyz_out, uint32_t *kind_out, double *weight_out,

@@ -64,3 +64,40 @@ def test_scattered_vectors_cost_no_search(gpu_ctx):
             t.append(time.perf_counter() - t0)
         return min(t)
     assert best(2) < 1.5 * best(4)
+
+
+@pytest.mark.parametrize("n_mol,mol,nk", [(1, 4095, 3), (1, 4096, 2), (1, 4097, 4), (2, 9001, 5),
+                                          (1, 30000, 32), (3, 128, 1)])
+def test_molecules_sorted_in_pieces(gpu_ctx, n_mol, mol, nk):
+    """The points are grouped by kind in pieces of 4,096 and the line kernel's slices
+    cut across them: every point counts once, with its own weight."""
+    rng = np.random.default_rng(mol)
+    n, hkl = n_mol * mol, miller_indices(20)
+    xyz, kind, w = rng.uniform(-60, 60, (n, 3)), rng.integers(0, nk, n), rng.uniform(0, 2, n)
+    ff = rng.uniform(-2, 8, (nk, len(hkl)))
+    for weight in (None, w):
+        before = _lib.lib().pd_launch_count(gpu_ctx.handle)
+        got = amplitudes(xyz, kind, ff, None, n_mol, weight, gpu_ctx, hkl=hkl, box=BOX)
+        assert _lib.lib().pd_launch_count(gpu_ctx.handle) - before == 3
+        ref = amplitudes(xyz, kind, ff, 2 * np.pi * hkl / BOX, n_mol, weight, gpu_ctx)
+        scale = np.sum(np.abs(ff[kind]) * (1.0 if weight is None else w[:, None]), axis=0)
+        assert np.all(np.abs(got[:, :2] - ref[:, :2]) <= 1e-12 * scale[:, None])
+        assert np.all(np.abs(got[:, 2:] - ref[:, 2:]) <= 2e-12 * scale[:, None] ** 2)
+
+
+def test_one_large_molecule_is_no_slower_than_many(gpu_ctx):
+    """A million points as one molecule against 64 molecules: the same points and vectors,
+    and the points of one molecule are not left to one SM."""
+    rng = np.random.default_rng(6)
+    hkl, n = miller_indices(100), 1_000_000
+    xyz, kind = rng.uniform(-60, 60, (n, 3)), rng.integers(0, 3, n)
+    ff = rng.uniform(1, 8, (3, len(hkl)))
+
+    def best(n_mol):
+        t = []
+        for _ in range(5):
+            t0 = time.perf_counter()
+            amplitudes(xyz, kind, ff, None, n_mol, None, gpu_ctx, hkl=hkl, box=BOX)
+            t.append(time.perf_counter() - t0)
+        return min(t)
+    assert best(1) < 1.25 * best(64)

@@ -2615,6 +2615,8 @@ constexpr int64_t LINE_MIN_MOLECULE = 128;
 
 constexpr uint64_t LINE_MAX_KINDS = 32;  // the device sort's counters
 
+constexpr int kNoLineMemory = -101;  // internal: the table kernel needs less
+
 // One blocking solve by the line kernel. The inputs go through a pinned image, the
 // coordinates in pieces that are uploaded while the next one is copied and
 // checked; the points are sorted by kind within their molecule on the device.
@@ -2648,7 +2650,8 @@ int direct_run_lines(pd_ctx *ctx, const pd_direct_request *req, const LineSet &l
         e = cudaMallocFromPoolAsync(reinterpret_cast<void **>(&base), total, ctx->pool, st);
     if (e != cudaSuccess) {
         if (img) ctx->pinned.put(img, cls);
-        return cuda_fail(ctx, e, "pd_direct_lattice: allocation");
+        (void)cudaGetLastError();
+        return kNoLineMemory;
     }
     bool finite = true;
     constexpr uint64_t PIECE = 3 * 16384;
@@ -2755,8 +2758,11 @@ extern "C" int pd_direct_lattice(pd_ctx *ctx, const pd_direct_request *req, cons
         const double chunks = static_cast<double>(req->n_points / static_cast<uint64_t>(mol)) * spm;
         const double vb = std::ceil(static_cast<double>(ls.lines.size()) / 32.0);
         if (chunks * static_cast<double>(ls.lines.size()) * LINE_J * 16.0 <= 8.0 * (1ull << 30) &&
-            chunks * vb < 2.0e9)
-            return direct_run_lines(ctx, req, ls, box, out);
+            chunks * vb < 2.0e9) {
+            // its pinned image and the sorted copies may not fit where the points alone do
+            const int rc = direct_run_lines(ctx, req, ls, box, out);
+            if (rc != kNoLineMemory) return rc;
+        }
     }
     if (!pd::all_finite(req->xyz, 3 * req->n_points)) {
         ctx->set_error("non-finite coordinate");

@@ -43,6 +43,8 @@ class Server:
         return out
 
     def cancel(self, ticket: int) -> None:
+        """Drop a request. A result that has not been taken is dropped with it, also a
+        finished one: ``wait`` then raises PD_ECANCELED."""
         _lib.check(_lib.lib().pd_cancel(self.ctx.handle, ticket), self.ctx.handle)
 
     def times(self, ticket: int) -> Tuple[float, float, float]:

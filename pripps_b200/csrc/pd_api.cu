@@ -541,8 +541,9 @@ int plan_host(pd_ctx *ctx, const pd_request *req, const uint32_t *species, const
             ctx->set_error(msg);
             return rc;
         }
-        // known coordinates: every frame sums directions (the plan has no tiles) or none
-        if (exact_radius && !P.dir_only) pd::drop_directions(P);
+        // known coordinates: every frame sums directions (the plan has no tiles) or none; a
+        // given shape is the pair kernels' and there to be timed
+        if (force || (exact_radius && !P.dir_only)) pd::drop_directions(P);
         L = fit_layout(P, host_xyz, avail);
         return PD_OK;
     };
@@ -2019,8 +2020,10 @@ std::vector<Tuning> tune_candidates(const pd_request *req, int mode) {
     return out;
 }
 
-// Times every candidate shape on the caller's request and keeps the fastest
-// for the request's bucket. Each timed execution starts with L2 flushed (a
+// Times every candidate shape on the caller's request, its pairs summed as pairs
+// whatever form a solve of it would take (the shape is the pair kernels': with the
+// directions on, all of them would tie), and keeps the fastest for the request's
+// bucket. Each timed execution starts with L2 flushed (a
 // 256 MiB write), as a stream of independent requests would meet it.
 int autotune_request(pd_ctx *ctx, const pd_request *req, Tuning *best_out, double *best_ms) {
     NvtxRange nvtx("pd autotune");

@@ -484,8 +484,10 @@ def executed_work(req):
 
     Directions: S directions × N atoms (twice with a weight per atom), 14 lane
     operations (26 FLOP) to start an atom's cosines and 10 (20 FLOP) for each
-    eight of its M moments, 44 more for each later block of 128. Pairs: 44 and
-    1.25 per moment (2.5 FLOP) for each of the N(N−1)/2 pairs."""
+    eight of its M moments, 44 more for each later block of 128. Pairs: 56 (60
+    FLOP) for each block of 128 moments and 1.5 (2.75) per moment for each of the
+    N(N−1)/2 pairs. (The third form, grid points one by one, is for grids of fewer
+    points than these workloads have.)"""
     weighted = False
     if req.hyd_weights is not None:
         weighted = len(set(zip(req.species.tolist(), req.hyd_weights.tolist()))) > 48
@@ -507,7 +509,8 @@ def executed_work(req):
         blocks = (M + 127) // 128
         d = S * n * (2 if weighted else 1)
         d_ops, d_flop = d * (44 * blocks - 30 + 1.25 * M), d * (60 * blocks - 34 + 2.5 * M)
-        p_ops, p_flop = 0.5 * n * n * (44 + 1.25 * Mp), 0.5 * n * n * (60 + 2.5 * Mp)
+        pb = (Mp + 127) // 128
+        p_ops, p_flop = 0.5 * n * n * (56 * pb + 1.5 * Mp), 0.5 * n * n * (60 * pb + 2.75 * Mp)
         direct = d_ops < p_ops + 1e7 and n >= 150
         forms.add("directions" if direct else "pairs")
         sizes = {"directions": S, "moments": M} if direct else {"moments": Mp}

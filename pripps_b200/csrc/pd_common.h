@@ -152,7 +152,7 @@ struct PdAmpShape {
     int32_t dir_cap, grp_cap, amp_cap, node_cap;
     int32_t node_tile;  // nodes per block of the sums' kernel (a multiple of 4)
     int32_t sum_smem;   // its shared memory in doubles
-    int32_t rank, world, block, dir_block;
+    int32_t rank, world, dir_block;
     int64_t slot_cap;
 };
 

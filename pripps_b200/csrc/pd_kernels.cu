@@ -2678,8 +2678,8 @@ __global__ void __launch_bounds__(PD_DTAB_THREADS, 2)
 // a segment of PD_DLINE_J vectors of one line and needs, per point, only the
 // phases of its start and step — two products of table entries — instead of three
 // table reads and two complex products per vector (pd_direct_table: the reads
-// bound it, 0.50 ms for 128,000 points × 1,300 vectors; this kernel: see
-// launch_direct_lines). With E = e^{iφ} at the segment's index 4 (and 12) and
+// bound it, 0.50 ms for 128,000 points × 1,300 vectors; this kernel: 0.123 ms).
+// With E = e^{iφ} at the segment's index 4 (and 12) and
 // V_k = e^{ikδ·r}, the vectors ±k around it share four products,
 //   Re = x·c ∓ y·s, Im = y·c ± x·s,
 // accumulated separately: 4.6 FP64 operations per (vector, point). The points of
@@ -3155,7 +3155,8 @@ bool valid_q_block(int precision, int K) {
     if (K_ == K && mode == M && NP_ == NP)                                               \
         return launch_fp32_t<K, M, NP>(jobs, n_jobs, reqs, counter, plan_frames, grid, st, after);
 #define PD_F64(K, M) \
-    if (K_ == K && mode == M) return launch_fp64_t<K, M>(jobs, n_jobs, reqs, counter, plan_frames, grid, st, after);
+    if (K_ == K && mode == M) \
+        return launch_fp64_t<K, M>(jobs, n_jobs, reqs, counter, plan_frames, grid, st, after);
 
 cudaError_t launch_pairs(int precision, int K_, int NP_, int mode, const PdJob *jobs,
                          const int *n_jobs, const PdReqDev *reqs, int *counter, int plan_frames,
@@ -3286,7 +3287,8 @@ cudaError_t prepare_direction_rules() {
 
 cudaError_t launch_direction_sums(const double *slots, const double4 *dirs,
                                   const PdFrameDev *frames, const PdAmpShape &sh, double qmax,
-                                  const double *qv, int32_t n_frames, const PdClassDev *cls, const PdPairDev *pairs,
+                                  const double *qv, int32_t n_frames, const PdClassDev *cls,
+                                  const PdPairDev *pairs,
                                   int32_t n_pairs, const int32_t *cls_ptr,
                                   const int32_t *cls_chunk, int32_t width,
                                   int add_exact, double *part, unsigned int *done, double *red,
@@ -3303,7 +3305,8 @@ cudaError_t launch_direction_sums(const double *slots, const double4 *dirs,
         const dim3 grid(static_cast<unsigned>(n_nt * sh.grp_cap),
                         static_cast<unsigned>(std::min(n_frames - f0, 65535)));
         e = chain_launch(
-            after, kern, grid, PD_DSUM_THREADS, smem, st, slots + f0 * sh.slot_cap, dirs + static_cast<int64_t>(f0) * sh.dir_cap, frames + f0, sh,
+            after, kern, grid, PD_DSUM_THREADS, smem, st, slots + f0 * sh.slot_cap,
+            dirs + static_cast<int64_t>(f0) * sh.dir_cap, frames + f0, sh,
             qmax, qv, cls, pairs, n_pairs, cls_ptr, cls_chunk, width, add_exact,
             part + f0 * static_cast<int64_t>(sh.grp_cap) * n_pairs * nv * sh.node_cap,
             done + f0 * n_nt, red + f0 * static_cast<int64_t>(n_pairs) * nv * width);
@@ -3506,9 +3509,8 @@ int direct_line_points(int32_t n_entries) {
                                                           (n_entries * sizeof(double2))));
 }
 
-// Slices of a molecule for the line kernel: up to 4 blocks per SM (what its
-// shared memory allows) in one round where the box allows that, slices of 128 to
-// 2,048 points.
+// Slices of a molecule for the line kernel: up to 4 blocks per SM (three are resident
+// at its registers) where the box allows that, slices of 128 to 2,048 points.
 void direct_line_layout(int64_t n_points, int64_t mol_size, int32_t n_line, int64_t *chunk,
                         int64_t *spm) {
     const int64_t vblocks = (n_line + PD_DLINE_THREADS - 1) / PD_DLINE_THREADS;

@@ -58,7 +58,8 @@ cudaError_t launch_direction_sums(const double *slots, const double4 *dirs,
                                   const PdPairDev *pairs,
                                   int32_t n_pairs, const int32_t *cls_ptr,
                                   const int32_t *cls_chunk, int32_t width,
-                                  int add_exact, double *part, unsigned int *done, double *red, cudaStream_t st, bool after = false);
+                                  int add_exact, double *part, unsigned int *done, double *red,
+                                  cudaStream_t st, bool after = false);
 // Slot sums (red: [frame][pair][nv][width]); with n_chunk > 1, chunk_sums holds
 // 128·nv·n_chunk doubles and done one zeroed counter per (frame, pair, n_z).
 cudaError_t launch_reduce(const double *slots, const int64_t *lptr, const int64_t *lidx,

@@ -170,9 +170,9 @@ static int next_pow2(int64_t v) {
 
 Tuning fit_tuning(int precision, int mode, Tuning t) {
     // Two accumulators per q (weighted mode) allow q blocks up to 64 (there
-    // four pairs per thread measured fastest: 814 ms on the 100,000-atom solve
-    // with per-atom hydration weights against 835 ms with two); FP64 runs one
-    // pair per pass.
+    // four pairs per thread measured fastest: at the grid points, 814 ms on 100,000
+    // atoms with per-atom hydration weights against 835 ms with two); FP64 runs
+    // one pair per pass.
     if (precision == PD_FP64) {
         t.NP = 1;
     } else if (!valid_shape(precision, mode, t.K, t.NP)) {
@@ -194,12 +194,13 @@ Tuning default_tuning(int64_t n_atoms, int64_t nq, int precision, int64_t n_fram
         t.TJ = std::clamp(next_pow2(n_atoms / 16), 256, 4096);
         return t;
     }
-    // Measured on B200 (class mode): K = 128 with 4 pairs per thread (three
-    // CTAs per SM, seeds computed at the top of each pass) is the fastest
-    // shape from ~4k atoms up — 546.7 ms on the 100,000-atom solve against
-    // 561.5 ms with 2 pairs — and K = 64 with 4 pairs below; a j chunk of about N/8 atoms balances
-    // tile count against per-tile overhead. The last q-block of a grid runs
-    // only the 16-point chunks that lie on it, so a long block wastes at most
+    // Measured on B200 with the grid points summed one by one (class mode; structures
+    // of these sizes that are not long sum directions, which have no such shape): K = 128
+    // with 4 pairs per thread (three CTAs per SM, seeds computed at the top of each
+    // pass) is the fastest shape from ~4k atoms up — 100,000 atoms 546.7 ms against
+    // 561.5 ms with 2 pairs — and K = 64 with 4 pairs below; a j chunk of about N/8
+    // atoms balances tile count against per-tile overhead. The last q-block of a grid
+    // runs only the 16-point chunks that lie on it, so a long block wastes at most
     // 15 grid points per request. (These are the shapes of buckets the tuning
     // table does not name.)
     if (n_atoms < 4000) {
@@ -215,7 +216,7 @@ Tuning default_tuning(int64_t n_atoms, int64_t nq, int precision, int64_t n_fram
     }
     // j chunk: about N/8 atoms, halved while a solve would have fewer than
     // ~6 tiles per resident CTA of a B200 (148 SMs × 3): the longest-first
-    // tile order then ends with short tiles on every SM. Measured step times
+    // tile order then ends with short tiles on every SM. Measured at the grid points
     // (pair kernel + slot reduction): 10,000 atoms, nq 500: 3.82 / 3.51 /
     // 3.54 / 3.74 ms at 2,048 / 1,024 / 512 / 256; 20,000 atoms, nq 512:
     // 13.24 / 12.78 / 12.89 ms at 4,096 / 2,048 / 1,024; 100,000 atoms, nq
@@ -692,8 +693,9 @@ static double series_order(double z, bool fp64) {
 static double node_order(double z) { return z + 13.0 * std::cbrt(0.5 * z) + 3.0; }
 
 // Atom chunks of the direction form, longest first. A longer chunk means fewer sums
-// to hold and to add up, a shorter one more units to share: 2.5 units per block
-// that the GPU holds (four per SM), at least 1,024 atoms and at most 16,384, with the
+// to hold and to add up, a shorter one more units to share: 2.5 units for each of 592
+// blocks (four per SM, what the kernel for up to 64 moments holds; the one for more holds
+// three and the FP64 one two), at least 1,024 atoms and at most 16,384, with the
 // directions of a globule of the request's atom count (its coordinates would be
 // better, but then a solve's rounding would depend on when they are known). Measured,
 // whole execution in µs with chunks of 512 / 1,024 / 2,048 / 4,096 / 16,384 atoms: 3,000
@@ -750,7 +752,8 @@ static bool direction_only(Plan &P) {
         const double d = std::max(2.0 * 1.03 * P.radius_hint, 1e-6);
         const double z = P.qmax * d;  // the moments of pd_pack's pair form
         const double m = z + 9.7 * std::cbrt(0.5 * z) + 3.5;
-        const double m8 = m < 1e6 ? static_cast<double>((static_cast<int64_t>(0.5 * m) + 8) & ~int64_t{7}) : 1e6;
+        const double m8 =
+            m < 1e6 ? static_cast<double>((static_cast<int64_t>(0.5 * m) + 8) & ~int64_t{7}) : 1e6;
         const double blocks = std::ceil(m8 / P.mom.block);
         if (m8 <= P.mom.max_moments && blocks <= P.nqb &&
             P.mom.mom_cost * m8 + P.mom.mom_block_cost * blocks < P.mom.grid_cost) {
@@ -793,7 +796,6 @@ static bool direction_only(Plan &P) {
 static void set_directions(Plan &P) {
     P.amp = PdAmpShape{};
     P.amp.nq = P.nq;
-    P.amp.block = P.mom.block;
     P.amp.dir_block = P.precision == PD_FP64 ? PD_DIR_MBLOCK64 : PD_DIR_MBLOCK;
     P.amp.rank = static_cast<int32_t>(P.rank);
     P.amp.world = static_cast<int32_t>(P.world);

@@ -1372,11 +1372,14 @@ __global__ void __launch_bounds__(PD_CENT_THREADS)
 // for its share of the flushes (in each moment block) and 1.5 per moment, an atom in
 // one direction 14 (44 more for each later block) and 1.25 per moment, a direction
 // also n_cls·M terms per node in FP64;
-// PD_PAIRS_LATENCY stands for the pair form's longer chain of short kernels.
-// Whole solves on both sides (vacuum; pairs / directions, µs): FP32, q_max 0.5, 200 /
-// 300 / 600 / 1,200 atoms 68/65, 80/66, 83/70, 90/84, q_max 1.0 71/75, 84/72, 89/82,
-// 97/89; FP64 68/65, 69/65, 83/79, 103/86 and 82/79, 84/80, 93/86, 110/111. Elongated 2.5 : 1,
-// q_max 1.0, 300 / 500 / 800 atoms: FP32 73/79, 82/92, 101/122, FP64 79/97, 87/111, 114/153.
+// PD_PAIRS_LATENCY stands for the pair form's longer chain of short kernels, the rule's
+// grid_latency for the chain of a thread's atoms at the grid points. The costs of the
+// pairs at the grid points and as moments, which decide between those two, are the
+// plan's (set_reduction). Whole solves on both sides (vacuum, µs): FP32, moments of the
+// pairs / directions, q_max 0.5, 200 / 300 / 600 / 1,200 atoms 68/65, 80/66, 83/70, 90/84,
+// q_max 1.0 71/75, 84/72, 89/82, 97/89, elongated 2.5 : 1, q_max 1.0, 300 / 500 / 800 atoms
+// 73/79, 82/92, 101/122; FP64, grid points / directions, 100 points, 100 / 300 / 600 atoms
+// 233/59, 559/74, 983/75.
 constexpr int PD_PACK_THREADS = 256;
 
 // Nodes and weights of the 2h-point Gauss–Legendre rules, upper half

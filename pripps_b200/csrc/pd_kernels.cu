@@ -2065,13 +2065,20 @@ __device__ double moment_coefficients(double z, int n_mom, double *__restrict__ 
 constexpr int PD_PROF_Q = 8;
 constexpr int PD_PROF_THREADS = 256;
 constexpr int PD_PROF_GROUPS = PD_PROF_THREADS / PD_PROF_Q;
-constexpr int PD_PROF_ROWS = 2048;  // doubles of pair rows staged at once
-constexpr size_t PD_PROF_SMEM = 64 * 1024;
+// Doubles of pair rows staged at once. A step waits for its copies and two barriers, so
+// where the pairs take more than a few steps the steps are longer: 7,260 class pairs of
+// 5,346 atoms at 393 points take 3.0 ms in steps of 16,384 and 4.6 in steps of 2,048 (5.8
+// with loads through registers), 465 pairs of weighted atoms at 544 points 0.23 and 0.30
+// (0.43), 435 pairs of 32 frames, 2,048 on both sides, 0.52 (0.59). The middle size
+// leaves room for three blocks on an SM; above that many blocks others run while one
+// waits, and the short steps win by 2-4 % of a whole solve.
+constexpr int PD_PROF_ROWS = 2048, PD_PROF_ROWS_MANY = 6144, PD_PROF_ROWS_MOST = 16384;
+constexpr size_t PD_PROF_SMEM = 64 * 1024;  // with the class factors, at PD_PROF_ROWS
 
 // Its shared memory: pair rows, class factors and the coefficients of the most
 // moments a frame may have (up to 16, 9 for 48 classes, and 32 KB).
-static size_t profile_smem(const PdReduceShape &sh, int32_t n_cls_staged) {
-    return (PD_PROF_ROWS + static_cast<size_t>(n_cls_staged) * 3 * PD_PROF_Q +
+static size_t profile_smem(const PdReduceShape &sh, int rows, int32_t n_cls_staged) {
+    return (rows + static_cast<size_t>(n_cls_staged) * 3 * PD_PROF_Q +
             static_cast<size_t>(sh.max_moments) * PD_PROF_Q) * sizeof(double);
 }
 
@@ -2082,14 +2089,14 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
                 int32_t n_cls, PdReduceShape sh, const double *__restrict__ qv,
                 const PdFrameDev *__restrict__ frames, const double2 *__restrict__ node_tab,
                 const double *__restrict__ ffA, const double *__restrict__ ffC,
-                const double *__restrict__ ffW, int32_t add_diag, double qmax,
+                const double *__restrict__ ffW, int32_t add_diag, double qmax, int32_t n_rows,
                 const int *__restrict__ err, double *__restrict__ terms) {
     chain_enter();
     extern __shared__ double s_dyn[];
     __shared__ double s_c0[PD_PROF_Q], s_scale[PD_PROF_Q];
     __shared__ double s_sum[PD_PROF_THREADS / 32][6][PD_PROF_Q];
     double *s_row = s_dyn;                                 // [pair][nv][M]
-    double *s_fac = s_row + PD_PROF_ROWS;                  // [class][A, C, B][PD_PROF_Q]
+    double *s_fac = s_row + n_rows;                        // [class][A, C, B][PD_PROF_Q]
     double *s_coef = s_fac + (STAGED ? n_cls * 3 * PD_PROF_Q : 0);  // [M][PD_PROF_Q]
     const int n_qt = (sh.nq + PD_PROF_Q - 1) / PD_PROF_Q;
     const int f = blockIdx.x / n_qt;
@@ -2103,14 +2110,23 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
     const int M = nodes ? fr.n_node : (dirs ? 0 : fr.n_mom);
     const double *rows = red + static_cast<int64_t>(f) * sh.n_pairs * NV * sh.width;
     // the rows of pairs [p0, p0 + n): n·NV rows of M
-    const int fit = M > 0 ? min(sh.n_pairs, PD_PROF_ROWS / (NV * M)) : 0;
+    const int fit = M > 0 ? min(sh.n_pairs, n_rows / (NV * M)) : 0;
     auto stage_rows = [&](int p0, int n) {
+        const int dr = PD_PROF_THREADS / M, dm = PD_PROF_THREADS - dr * M;
+        int r = threadIdx.x / M, m = threadIdx.x - r * M;
+        const double *from = rows + static_cast<int64_t>(p0) * NV * sh.width;
+        const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(s_row));
         for (int k = threadIdx.x; k < n * NV * M; k += PD_PROF_THREADS) {
-            const int r = k / M;
-            s_row[k] = __ldg(rows + static_cast<int64_t>(p0 * NV + r) * sh.width + (k - r * M));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(to + 8 * k),
+                         "l"(from + static_cast<int64_t>(r) * sh.width + m)
+                         : "memory");
+            r += dr;
+            m += dm;
+            if (m >= M) m -= M, ++r;
         }
     };
-    stage_rows(0, fit);
+    auto rows_staged = [] { asm volatile("cp.async.wait_all;" ::: "memory"); };
+    if (M > 0) stage_rows(0, fit);
     // factor w (atom, excluded, hydration) of class c at grid point qq
     auto factor = [&](int c, int w, int qq) {
         double v = 0.0;
@@ -2185,6 +2201,7 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
             }
         }
     }
+    rows_staged();
     __syncthreads();
     double AA = 0, CC = 0, BB = 0, AC = 0, AB = 0, CB = 0;
     if (add_diag) {  // i = j terms
@@ -2205,6 +2222,7 @@ __global__ void __launch_bounds__(PD_PROF_THREADS)
         if (p0 > 0) {
             __syncthreads();  // the previous pairs' rows are read
             stage_rows(p0, n);
+            rows_staged();
             __syncthreads();
         }
         // groups per class pair (they share its moments)
@@ -3340,19 +3358,22 @@ cudaError_t launch_profiles(const double *red, const double *lat_sums, const PdC
     const int64_t blocks =
         static_cast<int64_t>(n_frames) * ((sh.nq + PD_PROF_Q - 1) / PD_PROF_Q);
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-    size_t smem = profile_smem(sh, n_cls);
-    const bool staged = smem <= PD_PROF_SMEM;
-    if (!staged) smem = profile_smem(sh, 0);
+    const bool staged = profile_smem(sh, PD_PROF_ROWS, n_cls) <= PD_PROF_SMEM;
+    const int64_t all = static_cast<int64_t>(sh.n_pairs) * nv * sh.max_moments;
+    const int rows = all <= 4 * PD_PROF_ROWS || blocks > 3 * 148 ? PD_PROF_ROWS
+                     : blocks > 148                              ? PD_PROF_ROWS_MANY
+                                                                 : PD_PROF_ROWS_MOST;
+    const size_t smem = profile_smem(sh, rows, staged ? n_cls : 0);
     auto kern = nv == 4 ? (staged ? pd_profiles<4, true> : pd_profiles<4, false>)
                         : (staged ? pd_profiles<1, true> : pd_profiles<1, false>);
     if (smem > 44 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(
-            kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(PD_PROF_SMEM));
+            kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (e != cudaSuccess) return e;
     }
     return chain_launch(after, kern, static_cast<unsigned>(blocks), PD_PROF_THREADS, smem, st, red,
                         lat_sums, cls, pairs, n_cls, sh, qv, frames, node_tab, ffA, ffC, ffW,
-                        add_diag, qmax, err, terms);
+                        add_diag, qmax, rows, err, terms);
 }
 
 cudaError_t launch_lattice(const double *xyz, const int32_t *perm, const PdLatDev *lat_dev,

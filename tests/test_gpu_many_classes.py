@@ -44,6 +44,36 @@ def test_species_without_a_bound(gpu_ctx, precision, mode, n, n_species, nq):
     assert np.all(err < TOL[precision]), err
 
 
+@pytest.mark.parametrize("mode,n_species,nq,n_frames", [
+    ("vacuum", 30, 1184, 1), ("vacuum", 30, 1185, 1), ("vacuum", 30, 400, 9),
+    ("vacuum", 5, 60, 1), ("weighted", 30, 1184, 1), ("weighted", 30, 1185, 1),
+    ("weighted", 30, 60, 60), ("weighted", 100, 30, 1), ("vacuum", 250, 30, 1)])
+def test_steps_of_staged_pair_rows(gpu_ctx, mode, n_species, nq, n_frames):
+    """Moments of the pairs of an elongated set: both sides of the block counts where the
+    steps change their length, one step and many, whole and with a last short one; every
+    profile against the compensated oracle, frames as the weighted mean."""
+    rng = np.random.default_rng(n_species * nq)
+    req = _request(140 if n_species < 100 else 300, n_species, nq, "fp32", mode, nq)
+    req.xyz = req.xyz * np.array([6.0, 0.5, 0.5])
+    qi = np.unique([0, 1, nq // 2, nq - 1])
+    if n_frames == 1:
+        got = solve(req, gpu_ctx)
+        err = term_errors(got[:, qi], O.terms_for_request(req, q_index=qi, precise=True))
+        assert np.all(err < TOL["fp32"]), err
+        return
+    base, frames = req.xyz, []
+    weights = rng.uniform(0.1, 2, n_frames)
+    want = 0.0
+    for k in range(n_frames):
+        req.xyz = base * rng.uniform(0.6, 1.0) + rng.normal(0, 0.3, base.shape)
+        frames.append(req.xyz)
+        want = want + weights[k] * O.terms_for_request(req, q_index=qi, precise=True)
+    req.xyz, req.frame_weights = np.stack(frames), weights
+    got = solve(req, gpu_ctx)
+    err = term_errors(got[:, qi], want / weights.sum())
+    assert np.all(err < TOL["fp32"]), err
+
+
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_many_species_in_a_stream(gpu_ctx, precision):
     """The same through a streamed trajectory: the mean of the frames' own solves."""

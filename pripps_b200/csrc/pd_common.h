@@ -111,8 +111,12 @@ constexpr int PD_MAX_MOMENTS = 512;
 // and the shared memory of the kernel that sums the class pairs.
 constexpr int PD_MAX_DIR_MOMENTS = 256;
 constexpr int PD_DIR_SMEM = 200 * 1024;
-// Lane operations that the pair form is charged beyond its pairs (frame_constants).
+// Lane operations that the moments of the pairs are charged for their longer chain of
+// short kernels (frame_constants).
 constexpr double PD_PAIRS_LATENCY = 1e7;
+// Nodes of directions that the class pairs' products are charged at least: with fewer the
+// kernel that forms them has SMs to spare.
+constexpr double PD_DIR_LEAST = 16000.0;
 constexpr int PD_DIR_DIRS = 8;  // directions of a work unit
 // Moments of its first block (FP32, FP64) and of each later one.
 constexpr int PD_DIR_MBLOCK = 128, PD_DIR_MBLOCK64 = 64;
@@ -127,10 +131,9 @@ struct PdMomentRule {
     // Cost of a pair: all grid points, the moment form per moment and per block (the
     // cheaper one sums the pairs), and the grid points in the directions' unit.
     double grid_cost, mom_cost, mom_block_cost, grid_dir_cost;
-    // What the grid points are charged beyond that, as PD_PAIRS_LATENCY: a thread's pass
-    // over its j atoms is a chain (FP32, 800 atoms, 1 to 16 points: 111 us, directions
-    // 75; FP64, 100 atoms: 2 us for each, 230 us, directions 62).
-    double grid_latency;
+    // What is charged beyond the pairs: their tiles, and at the grid points a thread's
+    // chain of atoms; and for each node of a direction the products of the class pairs.
+    double tile_cost, grid_latency, dir_pair_cost;
     // direction form (dir_cap = 0: never)
     int32_t dir_block;    // moments per unit
     int32_t dir_cap;      // directions the frame's table holds (a multiple of 32)

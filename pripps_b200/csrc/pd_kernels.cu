@@ -1371,11 +1371,10 @@ __global__ void __launch_bounds__(PD_CENT_THREADS)
 // The rule counts FP32 lane operations: a pair costs about 44 for its sequences and 12
 // for its share of the flushes (in each moment block) and 1.5 per moment, an atom in
 // one direction 14 (44 more for each later block) and 1.25 per moment, a direction
-// also n_cls·M terms per node in FP64;
-// PD_PAIRS_LATENCY stands for the pair form's longer chain of short kernels, the rule's
-// grid_latency for the chain of a thread's atoms at the grid points. The costs of the
-// pairs at the grid points and as moments, which decide between those two, are the
-// plan's (set_reduction). Whole solves on both sides (vacuum, µs): FP32, moments of the
+// also n_cls·M terms per node in FP64, and the class pairs' products there;
+// PD_PAIRS_LATENCY stands for the pair form's longer chain of short kernels. The costs of
+// the tiles, of the pairs at the grid points and as moments, which decide between those
+// two, and of the class pairs' products are the plan's (set_reduction). Whole solves on both sides (vacuum, µs): FP32, moments of the
 // pairs / directions, q_max 0.5, 200 / 300 / 600 / 1,200 atoms 68/65, 80/66, 83/70, 90/84,
 // q_max 1.0 71/75, 84/72, 89/82, 97/89, elongated 2.5 : 1, q_max 1.0, 300 / 500 / 800 atoms
 // 73/79, 82/92, 101/122; FP64, grid points / directions, 100 points, 100 / 300 / 600 atoms
@@ -1449,7 +1448,7 @@ __device__ __forceinline__ void frame_constants(double radius, const PdMomentRul
         }
     }
     pair_cost *= rule.n_tile_pairs;
-    pair_cost += fr.n_mom > 0 ? PD_PAIRS_LATENCY : rule.grid_latency;
+    pair_cost += rule.tile_cost + (fr.n_mom > 0 ? PD_PAIRS_LATENCY : rule.grid_latency);
     // ---- directions: 2h Gauss rings (upper half: h), enough points on each
     if (rule.dir_cap == 0) {
         if (part == 0 && threadIdx.x == 0) frames[f] = fr;
@@ -1483,7 +1482,8 @@ __device__ __forceinline__ void frame_constants(double radius, const PdMomentRul
     const double dir_cost =
         static_cast<double>(S) * (static_cast<double>(rule.n_atoms) * rule.nv2 *
                                       (44.0 * ablk - 30.0 + 1.25 * m8) +
-                                  4.0 * rule.n_cls * m8 * nodes);
+                                  4.0 * rule.n_cls * m8 * nodes) +
+        rule.dir_pair_cost * fmax(static_cast<double>(S) * nodes, PD_DIR_LEAST);
     const bool use = S > 0 && groups * 32 <= rule.dir_cap && mine > 0 &&
                      (groups + rule.world - 1) / rule.world <= rule.grp_cap &&
                      m8 <= rule.amp_cap && nodes <= rule.node_cap &&

@@ -746,8 +746,7 @@ static bool direction_only(Plan &P) {
     P.lptr.assign(static_cast<size_t>(P.n_pairs) * P.nqb + 1, 0);
     P.dir_only = true;
     set_reduction(P);
-    double pair_cost = P.mom.grid_dir_cost;
-    bool moments = false;
+    double pair_cost = P.mom.grid_dir_cost, latency = P.mom.grid_latency;
     if (P.mom.block > 0) {
         const double d = std::max(2.0 * 1.03 * P.radius_hint, 1e-6);
         const double z = P.qmax * d;  // the moments of pd_pack's pair form
@@ -757,12 +756,12 @@ static bool direction_only(Plan &P) {
         const double blocks = std::ceil(m8 / P.mom.block);
         if (m8 <= P.mom.max_moments && blocks <= P.nqb &&
             P.mom.mom_cost * m8 + P.mom.mom_block_cost * blocks < P.mom.grid_cost) {
-            moments = true;
             pair_cost = 56.0 * blocks + 1.5 * m8;
+            latency = PD_PAIRS_LATENCY;
         }
     }
     pair_cost *= P.mom.n_tile_pairs;
-    pair_cost += moments ? PD_PAIRS_LATENCY : P.mom.grid_latency;
+    pair_cost += P.mom.tile_cost + latency;
     const bool use = P.amp.dir_cap > 0 && P.dir_cost < pair_cost;
     if (!use) {
         P.dir_only = false;
@@ -777,7 +776,7 @@ static bool direction_only(Plan &P) {
     const int64_t per = std::min<int64_t>(
         P.dir_units, std::max<int64_t>(1, (1024 + P.n_frames - 1) / P.n_frames));
     P.jobs_per_frame = per;
-    P.job_cost = P.dir_cost / (3.0 * static_cast<double>(per));
+    P.job_cost = P.dir_work / (3.0 * static_cast<double>(per));
     if (P.precision == PD_FP64) P.job_cost *= 2.0;
     P.jobs.resize(static_cast<size_t>(per) * P.n_frames);
     for (int64_t o = 0; o < per; ++o)
@@ -854,9 +853,12 @@ static void set_directions(Plan &P) {
     P.amp.node_tile = static_cast<int32_t>(tile);
     P.amp.slot_cap = slots;
     const double ablk = static_cast<double>((m8 + P.amp.dir_block - 1) / P.amp.dir_block);
-    P.dir_cost = static_cast<double>(S) *
+    P.dir_work = static_cast<double>(S) *
                  (static_cast<double>(P.n_atoms) * P.amp.nv2 * (44.0 * ablk - 30.0 + 1.25 * m8) +
                   4.0 * P.n_cls * static_cast<double>(m8) * static_cast<double>(nodes));
+    P.dir_cost = P.dir_work + P.mom.dir_pair_cost *
+                                  std::max(static_cast<double>(S) * static_cast<double>(nodes),
+                                           PD_DIR_LEAST);
     P.dir_units = static_cast<int64_t>(P.amp.n_chunk) * P.amp.nv2 *
                   static_cast<int64_t>(ablk) * mine * (32 / PD_DIR_DIRS);
 }
@@ -895,15 +897,31 @@ void set_reduction(Plan &P) {
     const double points = static_cast<double>((P.nq + 15) & ~15);
     if (m.fp64) {
         m.grid_dir_cost = 0.29 * 110.0 * P.nqb * P.tun.K;
-        m.grid_latency = 8e6 * static_cast<double>(std::min<int64_t>(P.n_atoms, 256));
     } else {
         const bool weighted = P.mode == PD_MODE_WEIGHTED;
         m.grid_cost = (weighted ? 4.0 : 3.0) * points + 55.0 * P.nqb;
         m.mom_cost = weighted ? 2.1 : 1.25;
         m.mom_block_cost = weighted ? 72.0 + 2.0 * m.block : 60.0 + 0.625 * m.block;
         m.grid_dir_cost = 0.7 * m.grid_cost;
-        m.grid_latency = 4e7;
     }
+    // Beyond the pairs, each tile's jobs and a thread's pass over a class's atoms, which
+    // is a chain (FP32 4e7: 800 atoms, 1 to 16 points, 111 us, directions 75; FP64 4 us
+    // per atom of the largest class: 100 atoms of one class 490 us, directions 67, of
+    // eight classes 140 and 77); on the other side the class pairs' products at each node
+    // of each direction, an FP64 contraction of 2 to 7 ps for each. The constants are a
+    // fit to whole solves of 40 to 10,000 atoms, 1 to 100 species, 12 to 300 points: the
+    // form chosen is slower than the other by more than 10 % in 12 of 448 cases, by 31 %
+    // at most (63 and 5.8 times without these terms). Pairs / directions, us: FP64,
+    // weighted, 300 atoms of 16 species, 300 points 300 / 1,720, 1,000 atoms of 30, 60
+    // points 430 / 940; FP32, 10,000 atoms of 60, 60 points 950 / 1,980, 2,000 atoms of
+    // 84, 1,000 points 4,170 / 770.
+    const double tiles = 0.5 * static_cast<double>(P.n_pad / PD_IBLOCK) *
+                             (P.n_cls + static_cast<double>(P.n_pad) / P.tun.TJ) + 1.0;
+    double largest = 0.0;
+    for (const PdClassDev &c : P.cls) largest = std::max(largest, c.n);
+    m.tile_cost = 1.2e6 * tiles * P.nqb;
+    m.grid_latency = m.fp64 ? 2e7 * std::min(largest, 256.0) : 4e7;
+    m.dir_pair_cost = (m.fp64 ? 40.0 : 60.0) * P.n_pairs * P.nv;
     set_directions(P);
     m.dir_block = P.amp.dir_block;
     m.dir_cap = P.amp.dir_cap;

@@ -72,7 +72,8 @@ struct Plan {
     bool dir_only = false;
     bool no_directions = false;  // given up (drop_directions); a shard's share inherits it
     bool compact = false;        // the least memory (make_compact)
-    double dir_cost = 0.0;   // FP32 lane operations of a frame in the direction form
+    double dir_work = 0.0;   // FP32 lane operations of a frame's directions
+    double dir_cost = 0.0;   // and of its class pairs' products: the form's
     int64_t dir_units = 0;   // its work units
     double job_cost = 0.0;   // relative cost of a job (dir_only)
     double pair_bytes = 0.0; // at least what the tiles' plan would take (dir_only)

@@ -9,7 +9,7 @@ import pytest
 from conftest import term_errors
 from oracle import oracle as O
 from pripps_b200 import _lib, synth
-from pripps_b200.debye import DebyeRequest
+from pripps_b200.debye import DebyeRequest, solve
 
 pytestmark = pytest.mark.gpu
 GRID, MOMENTS, DIRECTIONS = 0, 1, 2
@@ -144,10 +144,37 @@ def test_cheaper_form_for_few_grid_points(gpu_ctx):
     assert form == [GRID], (form, mom)
 
 
+@pytest.mark.parametrize("precision,mode,n,n_species,qmax,nq,want", [
+    ("fp64", "weighted", 217, 30, 1.0, 59, GRID), ("fp64", "weighted", 217, 2, 1.0, 59, DIRECTIONS),
+    ("fp64", "vacuum", 1000, 60, 1.0, 60, GRID), ("fp64", "vacuum", 1000, 4, 1.0, 60, DIRECTIONS),
+    ("fp64", "weighted", 300, 16, 2.0, 300, GRID), ("fp64", "vacuum", 300, 1, 2.0, 300, DIRECTIONS),
+    ("fp32", "weighted", 500, 30, 0.5, 12, GRID), ("fp32", "weighted", 500, 2, 0.5, 12, DIRECTIONS),
+    ("fp32", "vacuum", 10000, 60, 1.0, 60, MOMENTS), ("fp32", "vacuum", 10000, 2, 1.0, 60, DIRECTIONS),
+    ("fp32", "vacuum", 2000, 84, 1.0, 1000, DIRECTIONS)])
+def test_many_classes_and_the_form(gpu_ctx, precision, mode, n, n_species, qmax, nq, want):
+    """The directions form every class pair's products at every node, the tiles of small
+    classes are short: the form follows the class count, and a solve, which decides on the
+    host, agrees with a plan's execution."""
+    rng = np.random.default_rng(n + n_species)
+    sp = rng.integers(0, n_species, n)
+    ff = rng.uniform(1, 8, (n_species, nq))
+    xyz = _ball(n, 1.6 * n ** (1 / 3))
+    extra = ((None,) * 3 if mode == "vacuum" else
+             (rng.uniform(0.2, 3, (n_species, nq)), rng.uniform(0, 2, n), rng.uniform(5, 10, nq)))
+    req = DebyeRequest(xyz, sp, ff, *extra, 0.0, qmax, nq, None, precision)
+    got, form, _ = _run(gpu_ctx, req)
+    assert form == [want] or (want != DIRECTIONS and form != [DIRECTIONS]), form
+    qi = np.array([0, nq // 2, nq - 1])
+    err = term_errors(got[:, qi], O.terms_for_request(req, q_index=qi, precise=True))
+    assert np.all(err < TOL[precision]), err
+    both = term_errors(solve(req, gpu_ctx), got)
+    assert np.all(both < (1e-13 if precision == "fp64" else 1e-6)), both
+
+
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_frames_of_a_batch_take_their_own_form(gpu_ctx, precision):
     xyz = _globule(800)
-    far = 8.0 if precision == "fp32" else 12.0  # (a grid point costs a double sin)
+    far = 8.0 if precision == "fp32" else 15.0  # (a grid point costs a double sin)
     frames = np.stack([xyz, far * xyz, xyz + 1.0])
     _, form, _ = _run(gpu_ctx, _request(frames, 0.6, 45, precision))
     assert form[0] == form[2] == DIRECTIONS and form[1] != DIRECTIONS, form

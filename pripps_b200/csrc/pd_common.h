@@ -117,6 +117,10 @@ constexpr double PD_PAIRS_LATENCY = 1e7;
 // Nodes of directions that the class pairs' products are charged at least: with fewer the
 // kernel that forms them has SMs to spare.
 constexpr double PD_DIR_LEAST = 16000.0;
+// Atoms that a chunk of the FP64 form is charged for: a block's 128 threads take an atom
+// each and add up their moments, whatever the chunk holds (per direction, 19 to 3,345
+// atoms in 1 to 60 chunks: as long as n_atoms + 80 to 116 per chunk).
+constexpr double PD_DIR_CHUNK64 = 130.0;
 constexpr int PD_DIR_DIRS = 8;  // directions of a work unit
 // Moments of its first block (FP32, FP64) and of each later one.
 constexpr int PD_DIR_MBLOCK = 128, PD_DIR_MBLOCK64 = 64;

@@ -1480,7 +1480,8 @@ __device__ __forceinline__ void frame_constants(double radius, const PdMomentRul
     const int ablk = (m8 + rule.dir_block - 1) / rule.dir_block;
     const int nodes = fp64 ? rule.nq : moments_needed(2.0 * fr.r1 * rule.qmax, true);
     const double dir_cost =
-        static_cast<double>(S) * (static_cast<double>(rule.n_atoms) * rule.nv2 *
+        static_cast<double>(S) * ((static_cast<double>(rule.n_atoms) +
+                                   (fp64 ? PD_DIR_CHUNK64 * rule.n_chunk : 0.0)) * rule.nv2 *
                                       (44.0 * ablk - 30.0 + 1.25 * m8) +
                                   4.0 * rule.n_cls * m8 * nodes) +
         rule.dir_pair_cost * fmax(static_cast<double>(S) * nodes, PD_DIR_LEAST);

@@ -854,7 +854,8 @@ static void set_directions(Plan &P) {
     P.amp.slot_cap = slots;
     const double ablk = static_cast<double>((m8 + P.amp.dir_block - 1) / P.amp.dir_block);
     P.dir_work = static_cast<double>(S) *
-                 (static_cast<double>(P.n_atoms) * P.amp.nv2 * (44.0 * ablk - 30.0 + 1.25 * m8) +
+                 ((static_cast<double>(P.n_atoms) + (fp64 ? PD_DIR_CHUNK64 * P.amp.n_chunk : 0.0)) *
+                      P.amp.nv2 * (44.0 * ablk - 30.0 + 1.25 * m8) +
                   4.0 * P.n_cls * static_cast<double>(m8) * static_cast<double>(nodes));
     P.dir_cost = P.dir_work + P.mom.dir_pair_cost *
                                   std::max(static_cast<double>(S) * static_cast<double>(nodes),
@@ -891,12 +892,12 @@ void set_reduction(Plan &P) {
     // Grid points / moments: a rod of 5,000 atoms, 160 moments, 150 points 511 / 414 us,
     // 300 points 819 / 414, weighted 708 / 757 and 1,040 / 757; 20,000 atoms, 208 moments,
     // 150 points 5.5 / 4.4 ms, weighted 7.8 / 10.0 and, 300 points, 12.3 / 10.0. The
-    // directions' own operations run at 57 % of the peak (FP64: 29 %), hence the
+    // directions' own operations run at 57 % of the peak (FP64: 23 %), hence the
     // factor 0.7. FP64: a grid point costs a double sin, 110 operations, for whole
     // q-blocks.
     const double points = static_cast<double>((P.nq + 15) & ~15);
     if (m.fp64) {
-        m.grid_dir_cost = 0.29 * 110.0 * P.nqb * P.tun.K;
+        m.grid_dir_cost = 0.23 * 110.0 * P.nqb * P.tun.K;
     } else {
         const bool weighted = P.mode == PD_MODE_WEIGHTED;
         m.grid_cost = (weighted ? 4.0 : 3.0) * points + 55.0 * P.nqb;
@@ -921,7 +922,7 @@ void set_reduction(Plan &P) {
     for (const PdClassDev &c : P.cls) largest = std::max(largest, c.n);
     m.tile_cost = 1.2e6 * tiles * P.nqb;
     m.grid_latency = m.fp64 ? 2e7 * std::min(largest, 256.0) : 4e7;
-    m.dir_pair_cost = (m.fp64 ? 40.0 : 60.0) * P.n_pairs * P.nv;
+    m.dir_pair_cost = (m.fp64 ? 30.0 : 60.0) * P.n_pairs * P.nv;
     set_directions(P);
     m.dir_block = P.amp.dir_block;
     m.dir_cap = P.amp.dir_cap;

@@ -748,11 +748,16 @@ int run_devplan(pd_ctx *ctx, DevPlan &dp, double *out_dev, cudaStream_t st,
     }
     if (!P.jobs.empty() && !P.dir_only) {
         NvtxRange nvtx("pd pair kernel");
+        const int grid = persistent_grid(ctx, P, static_cast<int64_t>(P.jobs.size()));
+        // Blocks that come while the packing runs go to the SMs it left free, two on
+        // each before the others have one, and in FP64 the first, longest jobs would share
+        // their SMs' pipe: with more blocks than SMs the pairs wait for the packing to end
+        // (4 frames of 2,043 atoms 1.39 -> 1.29 ms; where every block has its SM, 70
+        // against 71 us).
+        if (P.precision == PD_FP64 && P.amp.dir_cap == 0 && grid > ctx->sm_count) after = false;
         PD_CUDA(ctx, pd::launch_pairs(P.precision, P.tun.K, P.tun.NP, P.mode, dp.dptr<PdJob>(L.jobs),
                                       dp.dptr<int>(L.njobs), dp.dptr<PdReqDev>(L.req),
-                                      dp.dptr<int>(L.counter), P.n_frames,
-                                      persistent_grid(ctx, P, static_cast<int64_t>(P.jobs.size())),
-                                      st, after));
+                                      dp.dptr<int>(L.counter), P.n_frames, grid, st, after));
         ctx->launches += 1;
         after = true;
     }

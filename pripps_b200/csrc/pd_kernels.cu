@@ -937,14 +937,16 @@ __device__ __forceinline__ bool plan_sums_pairs(const PdReqDev &rq, int n_frames
 // The next job of a frame that sums pairs (one thread asks; n_jobs or more: none). The
 // jobs of frames in the direction form are passed over here, where a branch around a
 // whole tile cost the FP64 kernel's steps 13 % (5,000 atoms, 300 points: 13.3 ms
-// against 11.7 ms).
+// against 11.7 ms). A block's first job is its own number: the longest come first, and
+// blocks that wait for the frames' constants side by side would draw them in any order,
+// two long ones for one SM (4 frames of 2,043 atoms, FP64, one grid block: 1.29 or
+// 1.40 ms from one call to the next).
 __device__ __forceinline__ int next_pair_job(const PdJob *__restrict__ jobs, int n_jobs,
                                              const PdReqDev *__restrict__ reqs,
-                                             int *__restrict__ counter) {
-    int jid;
-    do
-        jid = atomicAdd(counter, 1);
-    while (jid < n_jobs && reqs[jobs[jid].req].frames[jobs[jid].frame].n_grp > 0);
+                                             int *__restrict__ counter, bool first) {
+    int jid = first ? blockIdx.x : gridDim.x + atomicAdd(counter, 1);
+    while (jid < n_jobs && reqs[jobs[jid].req].frames[jobs[jid].frame].n_grp > 0)
+        jid = gridDim.x + atomicAdd(counter, 1);
     return jid;
 }
 
@@ -988,8 +990,8 @@ __global__ void __launch_bounds__(PD_THREADS, fp32_min_blocks(K, MODE, NP))
     uint32_t phase = 0;  // bit b: parity of buffer b's next completion
     double *part = s_part + warp * NV * K;
     if (plan_frames > 0 && !plan_sums_pairs(reqs[0], plan_frames)) return;
-    for (;;) {
-        if (threadIdx.x == 0) s_job = next_pair_job(jobs, n_jobs, reqs, counter);
+    for (bool first = true;; first = false) {
+        if (threadIdx.x == 0) s_job = next_pair_job(jobs, n_jobs, reqs, counter, first);
         __syncthreads();
         const int jid = s_job;
         if (jid >= n_jobs) break;
@@ -1244,8 +1246,8 @@ __global__ void __launch_bounds__(PD_THREADS) pd_pairs_fp64(const PdJob *__restr
     const int n_jobs = *n_jobs_ptr;
     double *part = s_part + warp * NV * K;
     if (plan_frames > 0 && !plan_sums_pairs(reqs[0], plan_frames)) return;
-    for (;;) {
-        if (threadIdx.x == 0) s_job = next_pair_job(jobs, n_jobs, reqs, counter);
+    for (bool first = true;; first = false) {
+        if (threadIdx.x == 0) s_job = next_pair_job(jobs, n_jobs, reqs, counter, first);
         __syncthreads();
         const int jid = s_job;
         if (jid >= n_jobs) break;

@@ -178,3 +178,23 @@ def test_frames_of_a_batch_take_their_own_form(gpu_ctx, precision):
     frames = np.stack([xyz, far * xyz, xyz + 1.0])
     _, form, _ = _run(gpu_ctx, _request(frames, 0.6, 45, precision))
     assert form[0] == form[2] == DIRECTIONS and form[1] != DIRECTIONS, form
+
+
+@pytest.mark.parametrize("precision,n,n_frames", [
+    ("fp64", 9, 1), ("fp64", 9, 148), ("fp64", 9, 149), ("fp64", 9, 296), ("fp64", 9, 297),
+    ("fp64", 9, 700), ("fp64", 150, 3), ("fp32", 40, 148), ("fp32", 40, 445), ("fp32", 40, 900)])
+def test_every_job_is_taken_once(gpu_ctx, precision, n, n_frames):
+    """Fewer jobs than blocks, as many, and more: a block's first job is its own number and
+    the others are drawn. Each frame has its own weight, so a job left out or taken twice
+    shows; the frames' mean against the compensated oracle."""
+    rng = np.random.default_rng(n_frames)
+    frames = rng.uniform(-9, 9, (n_frames, n, 3))
+    req = _request(frames, 0.6, 20, precision)
+    req.frame_weights = rng.uniform(0.1, 2.0, n_frames)
+    want = 0.0
+    for x, w in zip(frames, req.frame_weights):
+        one = DebyeRequest(x, req.species, req.ff_atoms, None, None, None, 0.0, 0.6, 20, None,
+                           precision)
+        want = want + w * O.terms_for_request(one, q_index=np.array([0, 7, 19]), precise=True)
+    err = term_errors(solve(req, gpu_ctx)[:, [0, 7, 19]], want / req.frame_weights.sum())
+    assert np.all(err < TOL[precision]), err

@@ -111,12 +111,9 @@ constexpr int PD_MAX_MOMENTS = 512;
 // and the shared memory of the kernel that sums the class pairs.
 constexpr int PD_MAX_DIR_MOMENTS = 256;
 constexpr int PD_DIR_SMEM = 200 * 1024;
-// Lane operations that the moments of the pairs are charged for their longer chain of
-// short kernels (frame_constants).
-constexpr double PD_PAIRS_LATENCY = 1e7;
 // Nodes of directions that the class pairs' products are charged at least: with fewer the
 // kernel that forms them has SMs to spare.
-constexpr double PD_DIR_LEAST = 16000.0;
+constexpr double PD_DIR_LEAST = 12000.0;
 // Atoms that a chunk of the FP64 form is charged for: a block's 128 threads take an atom
 // each and add up their moments, whatever the chunk holds (per direction, 19 to 3,345
 // atoms in 1 to 60 chunks: as long as n_atoms + 80 to 116 per chunk).
@@ -135,9 +132,9 @@ struct PdMomentRule {
     // Cost of a pair: all grid points, the moment form per moment and per block (the
     // cheaper one sums the pairs), and the grid points in the directions' unit.
     double grid_cost, mom_cost, mom_block_cost, grid_dir_cost;
-    // What is charged beyond the pairs: their tiles, and at the grid points a thread's
-    // chain of atoms; and for each node of a direction the products of the class pairs.
-    double tile_cost, grid_latency, dir_pair_cost;
+    // What is charged beyond the pairs: their tiles, at the grid points a thread's chain of
+    // atoms, with moments the longer chain of short kernels; and for each node of a direction the products of the class pairs.
+    double tile_cost, grid_latency, mom_latency, dir_pair_cost;
     // direction form (dir_cap = 0: never)
     int32_t dir_block;    // moments per unit
     int32_t dir_cap;      // directions the frame's table holds (a multiple of 32)

@@ -1373,13 +1373,12 @@ __global__ void __launch_bounds__(PD_CENT_THREADS)
 // The rule counts FP32 lane operations: a pair costs about 44 for its sequences and 12
 // for its share of the flushes (in each moment block) and 1.5 per moment, an atom in
 // one direction 14 (44 more for each later block) and 1.25 per moment, a direction
-// also n_cls·M terms per node in FP64, and the class pairs' products there;
-// PD_PAIRS_LATENCY stands for the pair form's longer chain of short kernels. The costs of
+// also n_cls·M terms per node in FP64, and the class pairs' products there. The costs of
 // the tiles, of the pairs at the grid points and as moments, which decide between those
-// two, and of the class pairs' products are the plan's (set_reduction). Whole solves on both sides (vacuum, µs): FP32, moments of the
-// pairs / directions, q_max 0.5, 200 / 300 / 600 / 1,200 atoms 68/65, 80/66, 83/70, 90/84,
-// q_max 1.0 71/75, 84/72, 89/82, 97/89, elongated 2.5 : 1, q_max 1.0, 300 / 500 / 800 atoms
-// 73/79, 82/92, 101/122; FP64, grid points / directions, 100 points, 100 / 300 / 600 atoms
+// two, of the class pairs' products and of the chains are the plan's (set_reduction).
+// Whole solves on both sides (vacuum, µs): FP32, moments of the pairs / directions,
+// q_max 0.5, 200 / 300 / 600 / 1,200 atoms 68/65, 80/66, 83/70, 90/84, q_max 1.0 71/75,
+// 84/72, 89/82, 97/89, elongated 2.5 : 1, q_max 1.0, 300 / 500 / 800 atoms 73/79, 82/92, 101/122; FP64, grid points / directions, 100 points, 100 / 300 / 600 atoms
 // 233/59, 559/74, 983/75.
 constexpr int PD_PACK_THREADS = 256;
 
@@ -1450,7 +1449,7 @@ __device__ __forceinline__ void frame_constants(double radius, const PdMomentRul
         }
     }
     pair_cost *= rule.n_tile_pairs;
-    pair_cost += rule.tile_cost + (fr.n_mom > 0 ? PD_PAIRS_LATENCY : rule.grid_latency);
+    pair_cost += rule.tile_cost + (fr.n_mom > 0 ? rule.mom_latency : rule.grid_latency);
     // ---- directions: 2h Gauss rings (upper half: h), enough points on each
     if (rule.dir_cap == 0) {
         if (part == 0 && threadIdx.x == 0) frames[f] = fr;

@@ -757,7 +757,7 @@ static bool direction_only(Plan &P) {
         if (m8 <= P.mom.max_moments && blocks <= P.nqb &&
             P.mom.mom_cost * m8 + P.mom.mom_block_cost * blocks < P.mom.grid_cost) {
             pair_cost = 56.0 * blocks + 1.5 * m8;
-            latency = PD_PAIRS_LATENCY;
+            latency = P.mom.mom_latency;
         }
     }
     pair_cost *= P.mom.n_tile_pairs;
@@ -905,24 +905,33 @@ void set_reduction(Plan &P) {
         m.mom_block_cost = weighted ? 72.0 + 2.0 * m.block : 60.0 + 0.625 * m.block;
         m.grid_dir_cost = 0.7 * m.grid_cost;
     }
-    // Beyond the pairs, each tile's jobs and a thread's pass over a class's atoms, which
-    // is a chain (FP32 4e7: 800 atoms, 1 to 16 points, 111 us, directions 75; FP64 4 us
-    // per atom of the largest class: 100 atoms of one class 490 us, directions 67, of
-    // eight classes 140 and 77); on the other side the class pairs' products at each node
-    // of each direction, an FP64 contraction of 2 to 7 ps for each. The constants are a
-    // fit to whole solves of 40 to 10,000 atoms, 1 to 100 species, 12 to 300 points: the
-    // form chosen is slower than the other by more than 10 % in 12 of 448 cases, by 31 %
-    // at most (63 and 5.8 times without these terms). Pairs / directions, us: FP64,
-    // weighted, 300 atoms of 16 species, 300 points 300 / 1,720, 1,000 atoms of 30, 60
-    // points 430 / 940; FP32, 10,000 atoms of 60, 60 points 950 / 1,980, 2,000 atoms of
-    // 84, 1,000 points 4,170 / 770.
+    // Beyond the pairs: each tile's jobs, with moments a longer chain of short kernels
+    // (1e7), and at the grid points a thread's pass over a class's atoms, which is a chain
+    // (FP32 8e7: 800 atoms, 1 to 16 points, 111 us, directions 75; FP64 4 us per atom of
+    // the largest class: 100 atoms of one class 490 us, directions 67, of eight classes
+    // 140 and 77) and which a batch's frames run side by side. On the other side the
+    // class pairs' products at each node of each direction, an FP64 contraction of 2 to
+    // 7 ps for each. The constants are a fit to whole solves of both forms, 20 to 15,000
+    // atoms, 1 to 100 species, 2 to 600 points, 1 to 40 frames: the form chosen is slower
+    // than the other by more than 10 % in about 130 of 2,840 cases. Pairs / directions, us: FP64, weighted, 300
+    // atoms of 16 species, 300 points 300 / 1,720, 1,000 atoms of 30, 60 points 430 / 940,
+    // 40 frames of 100 atoms of 9, 30 points 251 / 1,108; FP32, 10,000 atoms of 60, 60
+    // points 950 / 1,980, 10 frames of 2,000 atoms of 30, 150 points 590 / 1,420, 2,000
+    // atoms of 84, 1,000 points 4,170 / 770.
+    const double all_pairs = 0.5 * static_cast<double>(P.n_atoms) * P.n_atoms;
+    m.n_tile_pairs = all_pairs;
+    for (const PdLatDev &d : P.lat)
+        m.n_tile_pairs -= 0.5 * static_cast<double>(d.n) * d.n;
     const double tiles = 0.5 * static_cast<double>(P.n_pad / PD_IBLOCK) *
-                             (P.n_cls + static_cast<double>(P.n_pad) / P.tun.TJ) + 1.0;
+                             (P.n_cls + static_cast<double>(P.n_pad) / P.tun.TJ) *
+                             (m.n_tile_pairs / all_pairs) + 1.0;
     double largest = 0.0;
     for (const PdClassDev &c : P.cls) largest = std::max(largest, c.n);
     m.tile_cost = 1.2e6 * tiles * P.nqb;
-    m.grid_latency = m.fp64 ? 2e7 * std::min(largest, 256.0) : 4e7;
-    m.dir_pair_cost = (m.fp64 ? 30.0 : 60.0) * P.n_pairs * P.nv;
+    // (In FP32 a frame's form, whose rounding shows, does not follow its batch's size.)
+    m.grid_latency = m.fp64 ? 2e7 * std::min(largest, 256.0) / P.n_frames : 8e7;
+    m.mom_latency = 1e7;
+    m.dir_pair_cost = (m.fp64 ? 30.0 : 100.0) * P.n_pairs * P.nv;
     set_directions(P);
     m.dir_block = P.amp.dir_block;
     m.dir_cap = P.amp.dir_cap;
@@ -936,9 +945,6 @@ void set_reduction(Plan &P) {
     m.world = P.amp.world;
     m.slot_cap = P.amp.slot_cap;
     m.n_atoms = P.n_atoms;
-    m.n_tile_pairs = 0.5 * static_cast<double>(P.n_atoms) * P.n_atoms;
-    for (const PdLatDev &d : P.lat)
-        m.n_tile_pairs -= 0.5 * static_cast<double>(d.n) * d.n;
     m.nq = P.nq;
     m.dir_only = P.dir_only ? 1 : 0;
     PdReduceShape &r = P.red;
